@@ -189,7 +189,6 @@ struct FwdLayout {
   size_t prog, cval, xrow, rows, bytes;
 };
 
-enum SetMode : int { kSingle = 0, kFlat = 1, kStrided = 2 };
 
 constexpr int kMaxVarRows = 16;  // variables held in rows; tapes over others take the general path
 
@@ -416,6 +415,13 @@ int max_dyn_smem() {
   return v;
 }
 
+int max_sm_smem() {
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 48 * 1024;
+  if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) return 48 * 1024;
+  return v;
+}
+
 int check_tape_args(int64_t B, int64_t M) {
   if (B < 0 || M < 0) { set_error("negative size"); return SR_ERR_INVALID_ARGUMENT; }
   if (M > kMaxNodes) {
@@ -485,10 +491,7 @@ static int launch_compile(const int64_t* ops, const int64_t* ch, int64_t B, int6
 
 bool pick_shape(const void* kern, size_t per_warp, int64_t work_items, Shape& sh, size_t reserve) {
   const int limit = max_dyn_smem();
-  int dev = 0, sm_bytes = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
-    return false;
+  const int sm_bytes = max_sm_smem();
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) return false;
   if (reserve && cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       cudaSharedmemCarveoutMaxShared) != cudaSuccess)

@@ -41,6 +41,10 @@ __device__ __forceinline__ void stream16(void* p, const double (&r)[2]) {
   __stcs(reinterpret_cast<double2*>(p), make_double2(r[0], r[1]));
 }
 
+// How a unit takes the K constant sets of its tape: one set (K = 1), all of them as N K
+// consecutive values per node, or one set whose values lie K elements apart.
+enum SetMode : int { kSingle = 0, kFlat = 1, kStrided = 2 };
+
 // NO_OP nodes count as operators: their value (NaN) and their adjoint check matter.
 __device__ __forceinline__ bool is_op_code(int code) { return code == NO_OP || arity_of(code) >= 1; }
 
@@ -105,6 +109,7 @@ __host__ __device__ __forceinline__ int table_rows(int Lmax) {
 
 int device_sm_count();
 int max_dyn_smem();
+int max_sm_smem();  // shared memory of an SM
 int check_tape_args(int64_t B, int64_t M);
 
 // Side stream and fork/join events per device, created on first use and kept for the

@@ -108,7 +108,8 @@ int sr_eval_forward_f64(const double *X_dev, int64_t N, int64_t n_x, const uint3
  * grad_C (B, M) (zero at non-constant nodes) and, when grad_X_dev is not NULL,
  * accumulates into grad_X (N, n_x), which the caller zeroes first.  status_dev
  * is zeroed and then receives 201 (nonzero gradient on a NO_OP node) or 204
- * (a/b with b = 0 and a nonzero gradient; 201 is kept over 204).  Replaces
+ * (a/b with b = 0 and a nonzero gradient; 201 is kept over 204; SR_MLP_TIMEOUT if a wait
+ * of the padding-row check ran out).  Replaces
  * SymbolicEvaluation::backward and evaluation_backward_step_k (reference
  * src/symbolic_evaluation.cpp:94-168, src/evaluation_kernels_cuda.cu:218-632, 654-673).
  * order_dev, max_len and the side stream (here the padding-row check) as for the

@@ -63,6 +63,7 @@ MLP_EPI_RELU, MLP_EPI_LINEAR, MLP_EPI_F32, MLP_EPI_RELU_GRAD, MLP_EPI_SPLIT_F32 
 MLP_VOCAB, MLP_EMB, MLP_FEATS, MLP_PROJ, MLP_IN = 64, 64, 32, 28, 128
 MLP_TIMEOUT = 601
 TAPE_EXCEEDS_LAUNCH = 602
+LIVE_ROWS_COUNTED = 1 << 30
 
 _SIGS = {
     "sr_last_error": ([], ctypes.c_char_p),

@@ -63,8 +63,9 @@ struct FitArgs {
   int max_iter, hist, ls_kind, ls_max, objective;
   double tol, eps;
   int Lmax, Kmax;
-  int Imax;         // rows of the per-warp node tables: largest count of operator nodes
-  int Amax;         // rows of the per-warp adjoint tables: most operator-node adjoints live at once
+  int Imax;         // program entries: largest count of operator nodes
+  int Amax;         // most operator-node adjoints live at once
+  int Rmax;         // rows of the per-warp table for operator values and adjoints (see stage_problem)
   int VR;           // rows of the per-warp table for variables (distinct variables of a tape)
   unsigned char* ws_hist;  // per CTA: the L-BFGS history block (hist_block_bytes), when not in shared memory
   int ring_off;            // > 0: the history block sits in shared memory at this byte offset
@@ -72,9 +73,9 @@ struct FitArgs {
   int32_t* status;
 };
 
-// Shared memory.  The CTA works on one problem at a time: the tape, the constants
-// published for the current trial point, the slot maps and the cross-warp
-// reduction buffers are shared; each warp owns the node table of its own points.
+// Shared memory.  The CTA works on one problem at a time: the tape, its program, the
+// constants published for the current trial point, the slot maps and the cross-warp
+// reduction buffers are shared; each warp owns the value and adjoint rows of its own points.
 // Float pair of a cascaded sum (Ogita, Rump and Oishi's Sum2): hi is the plain float
 // sum of the terms, lo the float sum of the exact rounding errors of those additions
 // (Knuth's TwoSum).  hi + lo is as accurate as a sum in twice the precision, rounded
@@ -86,109 +87,110 @@ struct F2 {
   float hi, lo;
 };
 
+// Values a lane works on at once: V points of a chunk of 32 V (the caller's points_per_lane),
+// in U chunks of its warp.  A row holds 32 lanes x P = U V floats, a lane's part in one place,
+// so that it is one shared-memory access.
+struct Layout {
+  int Lmax, Imax, Rmax, Kmax, VR, V, P, W;
+  // byte offsets from the start of shared memory: CTA tables
+  uint32_t red_g, red_l, pvec, red_e, task, info, rowvar, tape, node_slot, slot_node, row_of, adj_of, last, flags, frees,
+      fwd, rev, dst, bc, warps;
+  uint32_t vars, gl, warp_bytes;  // per warp: operator rows at 0, variable rows, gradient sums
+  size_t bytes;
+};
+
+__host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rmax, int Kmax, int V, int U, int W, int VR) {
+  Layout l;
+  l.Lmax = Lmax;
+  l.Imax = Imax > 0 ? Imax : 1;
+  l.Rmax = Rmax > 0 ? Rmax : 1;
+  l.Kmax = Kmax > 0 ? Kmax : 1;
+  l.VR = VR;
+  l.V = V;
+  l.P = V * U;
+  l.W = W;
+  size_t p = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = p;
+    p += fit_align16(bytes);
+    return (uint32_t)at;
+  };
+  const size_t n = (size_t)Lmax, I = (size_t)l.Imax, K = (size_t)l.Kmax;
+  l.red_g = take((size_t)W * K * 8);  // [W][K] per-warp gradient sums (F2)
+  l.red_l = take((size_t)W * 8);      // [W] per-warp loss sums (F2)
+  l.pvec = take(512);                 // [128] search direction computed by warp 0
+  l.red_e = take((size_t)W * 4);      // [W] per-warp error codes
+  l.task = take(8);                   // the CTA's current problem
+  l.info = take(48);                  // see stage_problem
+  l.rowvar = take((size_t)VR * 4);    // [VR] variable held in each variable row
+  l.tape = take(n * 4);
+  l.node_slot = take(n * 4);          // slot of a LEARNABLE node / program entry of an operator / row of a variable
+  l.slot_node = take(K * 4);
+  l.row_of = take(n * 4);             // value row of an operator node
+  l.fwd = take(I * 16);               // forward program: opcode, two operand words, destination row
+  l.rev = take(I * 16);               // reverse program: opcode | no parent << 8, two operand words, adjoint row
+  l.dst = take(I * 8);                // reverse program: where the operands' adjoints go
+  l.bc = take((1 + K + n) * 4 * (size_t)l.P);  // broadcast values, P copies each: 0, constants, fixed constants
+  p = (p + 127) & ~size_t(127);
+  l.warps = (uint32_t)p;
+  const uint32_t row = 128u * (uint32_t)l.P;
+  l.vars = (uint32_t)l.Rmax * row;
+  l.gl = l.vars + (uint32_t)VR * row;  // [K][32 V] per-lane, per-point gradient sums
+  l.warp_bytes = l.gl + (uint32_t)K * 128u * (uint32_t)V;
+  // scratch of stage_problem in the first warp's rows (adjoint rows, last uses, marks, free rows)
+  l.adj_of = l.warps;
+  l.last = l.adj_of + 4u * (uint32_t)n;
+  l.flags = l.last + 4u * (uint32_t)n;
+  l.frees = l.flags + 4u * (uint32_t)n;
+  const size_t scratch = 4 * n * 4 + 4 * (size_t)(l.Rmax > Lmax ? l.Rmax : Lmax);
+  size_t total = (size_t)W * l.warp_bytes;
+  if (total < scratch) total = scratch;
+  l.bytes = p + fit_align16(total);
+  return l;
+}
+
 struct WarpSmem {
-  uint32_t* tape;    // [Lmax]                      (CTA)
-  uint32_t* pcode;   // [Lmax] opcode of each operator node of the program       (CTA)
-  uint32_t* psa;     // [Lmax] operand 0 source word (see the program notes)     (CTA)
-  uint32_t* psb;     // [Lmax] operand 1 source word                             (CTA)
-  uint32_t* pda;     // [Lmax] operand 0 adjoint destination (byte offset)        (CTA)
-  uint32_t* pdb;     // [Lmax] operand 1 adjoint destination                      (CTA)
-  int* arow;         // [Lmax] adjoint row of each operator node (by liveness)    (CTA)
-  int* frees;        // [Lmax] free adjoint rows while they are assigned          (CTA)
-  int* rowvar;       // [VR] variable held in each variable row                  (CTA)
-  int* info;         // [8] operator nodes, root row, variable rows, root source, root destination (CTA)
-  int* node_slot;    // [Lmax] slot of a LEARNABLE node / row of an operator node / row of a variable (CTA)
-  int* slot_node;    // [Kmax]                      (CTA)
-  F2* red_g;         // [W][Kmax] per-warp gradient sums (CTA)
-  F2* red_l;         // [W] per-warp loss sums      (CTA)
-  float* pvec;       // [128] search direction computed by warp 0 (CTA)
-  int* red_e;        // [W] per-warp error codes    (CTA)
-  long long* task;   // the CTA's current problem   (CTA)
-  unsigned char* wb; // this warp's table base (warp):
-  float* bc;         //   [1 + Kmax + Lmax] broadcast values: 0, constants, fixed constants
-  float* vals;       //   [Imax + VR][32V] operator-node values, then variable values
-  float* adj;        //   [Amax + 1][32V] live operator-node adjoints, then a sink row
-  float* gl;         //   [Kmax][32V] per-lane, per-point gradient partial sums
+  unsigned char* base;  // start of shared memory; program words are byte offsets from it
+  uint32_t rows;        // this warp's operator rows
+  uint32_t* tape;
+  uint4* fwd;
+  uint4* rev;
+  uint2* dst;
+  int* rowvar;
+  int* info;
+  int* node_slot;
+  int* slot_node;
+  F2* red_g;
+  F2* red_l;
+  float* pvec;
+  int* red_e;
+  long long* task;
+  float* gl;  // this warp's gradient sums
 };
 
-// Per-warp table layout (byte offsets from the warp's base), V points per lane,
-// rows of RW = 32 V floats.
-struct WarpLayout {
-  uint32_t vals, adj, sink, gl, bytes;
-};
+// Problem facts in info: operator nodes, variable rows in use, the root's operand word, where
+// its adjoint goes, whether a constant has several parents, whether the rows suffice, and
+// whether the variable rows hold for every closure (see fill_variables).
+enum Info : int { kOps = 0, kVars = 1, kRootSrc = 2, kRootDst = 3, kSharedConst = 4, kTooFew = 5 };
 
-__host__ __device__ __forceinline__ WarpLayout warp_layout(int Lmax, int Imax, int Amax, int Kmax, int V, int VR) {
-  const uint32_t K = (uint32_t)(Kmax > 0 ? Kmax : 1), I = (uint32_t)(Imax > 0 ? Imax : 1);
-  const uint32_t Ar = (uint32_t)(Amax > 0 ? Amax : 1);
-  const uint32_t RW = 32u * (uint32_t)V * 4u;  // bytes per row
-  WarpLayout w;
-  w.vals = (uint32_t)((4u * (1u + K + (uint32_t)Lmax) + 127u) & ~127u);
-  w.adj = w.vals + (I + (uint32_t)VR) * RW;
-  w.sink = w.adj + Ar * RW;
-  w.gl = w.sink + RW;
-  w.bytes = w.gl + K * RW;
-  return w;
-}
-
-__host__ __device__ __forceinline__ size_t fit_shared_bytes(int Lmax, int Kmax, int W, int VR) {
-  const size_t K = (size_t)(Kmax > 0 ? Kmax : 1);
-  return fit_align16((size_t)Lmax * 4) * 9 + fit_align16(K * 4) + fit_align16((size_t)W * K * 8) +
-         fit_align16((size_t)W * 8) + fit_align16((size_t)W * 4) + fit_align16((size_t)VR * 4) + 32 + 16 + 512 +
-         128;  // + alignment of the warp tables
-}
-
-__host__ __device__ __forceinline__ size_t fit_cta_bytes(int Lmax, int Imax, int Amax, int Kmax, int V, int W,
-                                                         int VR) {
-  return fit_shared_bytes(Lmax, Kmax, W, VR) + (size_t)W * warp_layout(Lmax, Imax, Amax, Kmax, V, VR).bytes;
-}
-
-__device__ __forceinline__ WarpSmem carve(unsigned char* base, int Lmax, int Imax, int Amax, int Kmax, int V, int W,
-                                          int VR, int warp) {
+__device__ __forceinline__ WarpSmem carve(unsigned char* base, const Layout& l, int warp) {
   WarpSmem s;
-  const size_t K = (size_t)(Kmax > 0 ? Kmax : 1);
-  unsigned char* p = base;
-  s.red_g = reinterpret_cast<F2*>(p);
-  p += fit_align16((size_t)W * K * 8);
-  s.red_l = reinterpret_cast<F2*>(p);
-  p += fit_align16((size_t)W * 8);
-  s.pvec = reinterpret_cast<float*>(p);
-  p += 512;
-  s.tape = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.node_slot = reinterpret_cast<int*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.slot_node = reinterpret_cast<int*>(p);
-  p += fit_align16(K * 4);
-  s.red_e = reinterpret_cast<int*>(p);
-  p += fit_align16((size_t)W * 4);
-  s.task = reinterpret_cast<long long*>(p);
-  p += 16;
-  s.pcode = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.psa = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.psb = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.pda = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.pdb = reinterpret_cast<uint32_t*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.arow = reinterpret_cast<int*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.frees = reinterpret_cast<int*>(p);
-  p += fit_align16((size_t)Lmax * 4);
-  s.rowvar = reinterpret_cast<int*>(p);
-  p += fit_align16((size_t)VR * 4);
-  s.info = reinterpret_cast<int*>(p);
-  p += 32;
-  const WarpLayout L = warp_layout(Lmax, Imax, Amax, Kmax, V, VR);
-  unsigned char* t = base + fit_shared_bytes(Lmax, Kmax, W, VR) - 128;
-  t = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(t) + 127) & ~uintptr_t(127));
-  s.wb = t + (size_t)warp * L.bytes;
-  s.bc = reinterpret_cast<float*>(s.wb);
-  s.vals = reinterpret_cast<float*>(s.wb + L.vals);
-  s.adj = reinterpret_cast<float*>(s.wb + L.adj);
-  s.gl = reinterpret_cast<float*>(s.wb + L.gl);
+  s.base = base;
+  s.rows = l.warps + (uint32_t)warp * l.warp_bytes;
+  s.tape = reinterpret_cast<uint32_t*>(base + l.tape);
+  s.fwd = reinterpret_cast<uint4*>(base + l.fwd);
+  s.rev = reinterpret_cast<uint4*>(base + l.rev);
+  s.dst = reinterpret_cast<uint2*>(base + l.dst);
+  s.rowvar = reinterpret_cast<int*>(base + l.rowvar);
+  s.info = reinterpret_cast<int*>(base + l.info);
+  s.node_slot = reinterpret_cast<int*>(base + l.node_slot);
+  s.slot_node = reinterpret_cast<int*>(base + l.slot_node);
+  s.red_g = reinterpret_cast<F2*>(base + l.red_g);
+  s.red_l = reinterpret_cast<F2*>(base + l.red_l);
+  s.pvec = reinterpret_cast<float*>(base + l.pvec);
+  s.red_e = reinterpret_cast<int*>(base + l.red_e);
+  s.task = reinterpret_cast<long long*>(base + l.task);
+  s.gl = reinterpret_cast<float*>(base + s.rows + l.gl);
   return s;
 }
 
@@ -628,34 +630,17 @@ __device__ __forceinline__ void compact_update_direction(const History& H, int h
   for (int s = 0; s < SPL; ++s) q.v[s] = __fsub_rn(qs.v[s], qy.v[s]);
 }
 
-constexpr int kMaxRegVars = 4;  // X rows of up to this many variables are held in registers
-
-// Value of variable `var` at the lane's point: from registers when n_x is small.
-template <int V>
-__device__ __forceinline__ float var_value(const float (&xr)[V][kMaxRegVars], int v, int var, bool in_regs,
-                                           const float* __restrict__ X, int64_t nn, int64_t n_x) {
-  if (in_regs) {
-    float r = xr[v][0];
-    r = var == 1 ? xr[v][1] : r;
-    r = var == 2 ? xr[v][2] : r;
-    r = var == 3 ? xr[v][3] : r;
-    return r;
-  }
-  return __ldg(X + nn * n_x + var);
-}
-
 // ---------------------------------------------------------------------------------
 // Operator-node program.  Before the first closure of a problem its tape (nodes up
 // to the root) is rewritten as a list of operator nodes (arity >= 1, plus NO_OP
 // nodes, whose value NaN and adjoint check matter).  Leaves are not executed: every
-// operand is a precomputed address in the warp's table,
-//   source word  = byte offset (bits 0..23) | lane stride in bytes (bits 24..31):
-//                  an operator node's row or a variable's row (stride 4: one value
-//                  per lane and point) or a broadcast entry (stride 0: 0, a
-//                  constant slot, a fixed constant),
-//   destination  = byte offset of the row that receives the operand's adjoint: the
-//                  operator node's adjoint row, the constant slot's partial-sum
-//                  row, or a sink row for variables and fixed constants.
+// operand is a precomputed place,
+//   operand word      a row of the warp (bit 31 and its byte offset from the warp's rows: an
+//                     operator's value or a variable) or a broadcast entry of the CTA (its byte
+//                     offset: 0, a constant slot, a fixed constant);
+//   destination word  where the operand's adjoint goes: nowhere (0: variables and fixed
+//                     constants), into an operator's adjoint row as its first (1 << 30) or a
+//                     further contribution (2 << 30), or into a constant slot's sums (3 << 30).
 // So the interpreter fetches and stores operands without branching on their kind;
 // only the opcode dispatch remains (warp-uniform).
 // ---------------------------------------------------------------------------------
@@ -663,184 +648,243 @@ __device__ __forceinline__ bool is_operator_node(int code) { return code == NO_O
 
 __device__ __forceinline__ bool is_fixed_leaf(int code) { return code >= C1 && code <= E_; }
 
-// Source word and destination of operand node c (operator row / slot / variable row
-// numbers in node_slot).
-__device__ __forceinline__ void operand_words(const uint32_t* tape, const int* node_slot, const int* arow, int c,
-                                              int Kmax, int Imax, const WarpLayout& L, uint32_t RW, uint32_t& src,
-                                              uint32_t& dst) {
+// Whether the adjoint rule of an operator reads its operands' values (EXP reads its own).
+__device__ __forceinline__ bool adjoint_reads_operands(int code) {
+  return !(code == NO_OP || code == ADD || code == SUB || code == NEG || code == FLOOR || code == CEIL || code == EXP);
+}
+
+constexpr uint32_t kRowOperand = 0x80000000u;
+enum DstKind : uint32_t { kDstNone = 0, kDstFirst = 1, kDstAdd = 2, kDstSum = 3 };
+
+// Operand word of node c (value rows in row_of, slots and variable rows in node_slot).
+__device__ __forceinline__ uint32_t operand_word(const uint32_t* tape, const int* node_slot, const int* row_of, int c,
+                                                 const Layout& l) {
   const int code = code_of(tape[c]);
-  if (is_operator_node(code)) {
-    src = (L.vals + (uint32_t)node_slot[c] * RW) | (4u << 24);
-    dst = L.adj + (uint32_t)arow[node_slot[c]] * RW;
-  } else if (code == VAR) {
-    src = (L.vals + (uint32_t)(Imax + node_slot[c]) * RW) | (4u << 24);
-    dst = L.sink;
-  } else if (code == LEARNABLE) {
-    src = 4u * (1u + (uint32_t)node_slot[c]);
-    dst = L.gl + (uint32_t)node_slot[c] * RW;
-  } else if (is_fixed_leaf(code)) {
-    src = 4u * (1u + (uint32_t)Kmax + (uint32_t)c);
-    dst = L.sink;
+  const uint32_t row = 128u * (uint32_t)l.P, entry = 4u * (uint32_t)l.P;
+  if (is_operator_node(code)) return kRowOperand | ((uint32_t)row_of[c] * row);
+  if (code == VAR) return kRowOperand | (l.vars + (uint32_t)node_slot[c] * row);
+  if (code == LEARNABLE) return l.bc + entry * (1u + (uint32_t)node_slot[c]);
+  if (is_fixed_leaf(code)) return l.bc + entry * (1u + (uint32_t)l.Kmax + (uint32_t)c);
+  return l.bc;  // the zero entry
+}
+
+template <int P>
+__device__ __forceinline__ void lds_pack(const unsigned char* p, float (&r)[P]) {
+  if constexpr (P == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    r[0] = t.x; r[1] = t.y; r[2] = t.z; r[3] = t.w;
+  } else if constexpr (P == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    r[0] = t.x; r[1] = t.y;
   } else {
-    src = 0u;  // the zero entry
-    dst = L.sink;
+    r[0] = *reinterpret_cast<const float*>(p);
+  }
+}
+template <int P>
+__device__ __forceinline__ void sts_pack(unsigned char* p, const float (&r)[P]) {
+  if constexpr (P == 4) *reinterpret_cast<float4*>(p) = make_float4(r[0], r[1], r[2], r[3]);
+  else if constexpr (P == 2) *reinterpret_cast<float2*>(p) = make_float2(r[0], r[1]);
+  else *reinterpret_cast<float*>(p) = r[0];
+}
+
+// The operand of a word for this lane; lane_rows = the lane's place in row 0 of its warp.
+template <int P>
+__device__ __forceinline__ void fetch_operand(const unsigned char* base, uint32_t w, uint32_t lane_rows, float (&r)[P]) {
+  if ((int)w < 0) w += lane_rows - kRowOperand;
+  lds_pack<P>(base + w, r);
+}
+
+// Chunk indexes of a warp: pass t of a warp works on its chunks warp + (t U + u) W, u < U.  A
+// problem with a constant of several parents takes its chunks one at a time (u = 0 only),
+// because a lane's sum of that constant adds all of a chunk's terms before the next chunk's.
+template <int V, int U>
+struct PassPoints {
+  int64_t nn[V * U];
+  bool valid[V * U];
+};
+template <int V, int U>
+__device__ __forceinline__ PassPoints<V, U> pass_points(int64_t N, int64_t t, int lane, int warp, int W, int step) {
+  PassPoints<V, U> r;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t base = ((int64_t)warp + (t * step + u) * W) * (32 * V);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int64_t n = base + v * 32 + lane;
+      r.valid[u * V + v] = u < step && n < N;
+      r.nn[u * V + v] = r.valid[u * V + v] ? n : N - 1;
+    }
+  }
+  return r;
+}
+
+template <int V, int U>
+__device__ __forceinline__ void fill_variables(const FitArgs& A, const WarpSmem& S, const Layout& l,
+                                               const PassPoints<V, U>& q, int lane) {
+  constexpr int P = V * U;
+  const int nvr = S.info[kVars];
+  for (int r = 0; r < nvr; ++r) {
+    const int var = S.rowvar[r];
+    float x[P];
+#pragma unroll
+    for (int i = 0; i < P; ++i) x[i] = __ldg(A.X + q.nn[i] * A.n_x + var);
+    sts_pack<P>(S.base + S.rows + l.vars + (uint32_t)r * 128u * P + lane * 4u * P, x);
   }
 }
 
-template <int V>
-__device__ __forceinline__ float lds_src(const unsigned char* wb, uint32_t w, int li) {
-  return *reinterpret_cast<const float*>(wb + (w & 0xffffffu) + (uint32_t)li * (w >> 24));
-}
-
-__device__ __forceinline__ float* row_ptr(unsigned char* wb, uint32_t off, int li) {
-  return reinterpret_cast<float*>(wb + off) + li;
-}
-
 // ---------------------------------------------------------------------------------
-// One pass over the problem's points at the constants in the warp's broadcast
+// One pass over the problem's points at the constants in the broadcast
 // entries.  kPassGrad: loss + gradient (forward, residual, reverse sweep);
 // kPassYFinal: forward only, writing the root values to Y_final; kPassLoss: forward
 // and residuals only (the loss of a candidate start).  Adjoint contributions are
 // added in the reference's order (parents from the last to the first, child 0
-// before child 1).
+// before child 1).  What bounds it: the latency of a node's chain (operands, dispatch,
+// arithmetic, store) and the instructions around its arithmetic.  Two chunks at a time (U = 2)
+// run one decode and dispatch and two chains for both.  Measured with the row assignment of
+// stage_problem (fit kernel): 16384 ragged problems, N = 512, 91.9 to 63.2 ms; 2999 at N = 257
+// with backtracking 22.6 to 15.5 ms; 8192 README problems, N = 100, 12.9 to 9.8 ms.
 // ---------------------------------------------------------------------------------
 enum PassMode : int { kPassGrad = 0, kPassYFinal = 1, kPassLoss = 2 };
 
-template <int V, int kMode>
-__device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, int64_t b, int lane, int warp, int W,
-                                            int& err) {
+template <int V, int U, int kMode>
+__device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, const Layout& l, int64_t b, int lane,
+                                            int warp, int W, bool vars_hold, int& err) {
+  constexpr int P = V * U;
   const int64_t N = A.N;
   const float invN = 1.0f / (float)N;
   const float* __restrict__ Yrow = A.Y ? A.Y + b * N : nullptr;
-  const bool xin = A.n_x <= kMaxRegVars;
-  const int nI = S.info[0];              // operator nodes
-  const int root_row = S.info[1];        // the root's adjoint row, or -1 for a leaf root
-  const int nvr = S.info[2];             // variable rows in use
-  const uint32_t root_src = (uint32_t)S.info[3], root_dst = (uint32_t)S.info[4];
-  const uint32_t sink = (uint32_t)S.info[5];  // adjoints of variables and fixed constants go nowhere
-  const uint32_t RW = 32u * V;           // floats per row
-  unsigned char* wb = S.wb;
+  const int nI = S.info[kOps];
+  const uint32_t root_src = (uint32_t)S.info[kRootSrc], root_dst = (uint32_t)S.info[kRootDst];
+  const int step = U > 1 && S.info[kSharedConst] ? 1 : U;
+  unsigned char* const base = S.base;
+  const uint32_t lane_rows = S.rows + (uint32_t)lane * 4u * P;
+  unsigned char* const my_rows = base + lane_rows;
+  float* const gl = S.gl + lane;
   // per-lane partial sums in float (a lane sees N / (32 V W) points)
   float loss_part = 0.f;
-  for (int64_t base = (int64_t)warp * 32 * V; base < N; base += (int64_t)W * 32 * V) {
-    int64_t nn[V];
-    bool valid[V];
-    float xr[V][kMaxRegVars];
+  for (int64_t t = 0; ((int64_t)warp + t * step * W) * (32 * V) < N; ++t) {
+    const PassPoints<V, U> q = pass_points<V, U>(N, t, lane, warp, W, step);
+    float y[P];
+    if constexpr (kMode != kPassYFinal) {
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      const int64_t n = base + v * 32 + lane;
-      valid[v] = n < N;
-      nn[v] = valid[v] ? n : N - 1;
-#pragma unroll
-      for (int j = 0; j < kMaxRegVars; ++j) xr[v][j] = (xin && j < A.n_x) ? __ldg(A.X + nn[v] * A.n_x + j) : 0.f;
+      for (int i = 0; i < P; ++i) y[i] = A.objective == 0 ? __ldg(Yrow + q.nn[i]) : 0.f;
     }
-    // variable rows of this chunk
-    for (int r = 0; r < nvr; ++r) {
-      const int var = S.rowvar[r];
-#pragma unroll
-      for (int v = 0; v < V; ++v)
-        S.vals[(A.Imax + r) * RW + v * 32 + lane] = var_value<V>(xr, v, var, xin, A.X, nn[v], A.n_x);
-    }
-    __syncwarp();
+    if (!vars_hold) fill_variables<V, U>(A, S, l, q, lane);
     // ---- forward over the operator nodes ----
-    uint32_t cn = nI > 0 ? S.pcode[0] : 0u, san = nI > 0 ? S.psa[0] : 0u, sbn = nI > 0 ? S.psb[0] : 0u;
+    uint4 wn = nI > 0 ? S.fwd[0] : make_uint4(0u, 0u, 0u, 0u);
     for (int i = 0; i < nI; ++i) {
-      const int code = (int)(cn & 0xffu);
-      const uint32_t sa = san, sb = sbn;
-      if (i + 1 < nI) {
-        cn = S.pcode[i + 1];
-        san = S.psa[i + 1];
-        sbn = S.psb[i + 1];
-      }
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const int li = v * 32 + lane;
-        const float r = op_value<float>(code, lds_src<V>(wb, sa, li), lds_src<V>(wb, sb, li));
-        S.vals[i * RW + li] = r;
-      }
+      const uint4 w = wn;
+      if (i + 1 < nI) wn = S.fwd[i + 1];
+      float a[P], c[P], r[P];
+      fetch_operand<P>(base, w.y, lane_rows, a);
+      fetch_operand<P>(base, w.z, lane_rows, c);
+      op_value_v<float, P>((int)w.x, a, c, r);
+      sts_pack<P>(my_rows + w.w, r);
     }
-    float fval[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) fval[v] = lds_src<V>(wb, root_src, v * 32 + lane);
+    float f[P];
+    fetch_operand<P>(base, root_src, lane_rows, f);
     if constexpr (kMode == kPassYFinal) {
 #pragma unroll
-      for (int v = 0; v < V; ++v)
-        if (valid[v]) A.Y_final[b * N + nn[v]] = fval[v];
-      __syncwarp();
-      continue;
-    } else if constexpr (kMode == kPassLoss) {
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        if (valid[v]) {
-          if (A.objective == 0) {
-            const float rr = fval[v] - __ldg(Yrow + nn[v]);
-            loss_part = __fadd_rn(loss_part, __fmul_rn(rr, rr));
-          } else {
-            loss_part = __fadd_rn(loss_part, fval[v]);
-          }
-        }
-      }
-      __syncwarp();
-      continue;
+      for (int i = 0; i < P; ++i)
+        if (q.valid[i]) A.Y_final[b * N + q.nn[i]] = f[i];
     } else {
-    // ---- residuals: root adjoint (2 (f - y)) * (1/N), as autograd forms it ----
+      // ---- residuals: root adjoint (2 (f - y)) * (1/N), as autograd forms it ----
+      float groot[P];
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      float groot = 0.f;
-      if (valid[v]) {
-        if (A.objective == 0) {
-          const float rr = fval[v] - __ldg(Yrow + nn[v]);
-          loss_part = __fadd_rn(loss_part, __fmul_rn(rr, rr));
-          groot = __fmul_rn(rr * 2.0f, invN);
-        } else {
-          loss_part = __fadd_rn(loss_part, fval[v]);
-          groot = invN;
-        }
-      }
-      const int li = v * 32 + lane;
-      if (root_row >= 0) {
-        S.adj[root_row * RW + li] = groot;  // the seed of the root (its row holds 0)
-      } else if (groot != 0.f) {
-        float* d = row_ptr(wb, root_dst, li);  // a leaf root: its slot's row, or the sink
-        *d = __fadd_rn(*d, groot);
-      }
-    }
-    // ---- reverse sweep over the operator nodes ----
-    uint32_t cp = 0u, sap = 0u, sbp = 0u, dap = 0u, dbp = 0u;
-    if (nI > 0) {
-      cp = S.pcode[nI - 1]; sap = S.psa[nI - 1]; sbp = S.psb[nI - 1]; dap = S.pda[nI - 1]; dbp = S.pdb[nI - 1];
-    }
-    for (int i = nI - 1; i >= 0; --i) {
-      const int code = (int)(cp & 0xffu);
-      const uint32_t arow = (cp >> 8) * RW;  // the node's adjoint row (float offset)
-      const uint32_t sa = sap, sb = sbp, da = dap, db = dbp;
-      if (i > 0) {
-        cp = S.pcode[i - 1]; sap = S.psa[i - 1]; sbp = S.psb[i - 1]; dap = S.pda[i - 1]; dbp = S.pdb[i - 1];
-      }
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const int li = v * 32 + lane;
-        const float g = S.adj[arow + li];
-        S.adj[arow + li] = 0.f;  // read once: the row is free for the nodes swept next
-        bool a0, a1;
-        float r0, r1;
-        const int e = op_adjoint<float>(code, g, lds_src<V>(wb, sa, li), lds_src<V>(wb, sb, li), S.vals[i * RW + li],
-                                          a0, r0, a1, r1);
-        if (valid[v]) {
-          if (e && !err) err = e;
-          if (a0 && da != sink) {
-            float* d = row_ptr(wb, da, li);
-            *d = __fadd_rn(*d, r0);
-          }
-          if (a1 && db != sink) {
-            float* d = row_ptr(wb, db, li);
-            *d = __fadd_rn(*d, r1);
+      for (int i = 0; i < P; ++i) {
+        groot[i] = 0.f;
+        if (q.valid[i]) {
+          if (A.objective == 0) {
+            const float rr = f[i] - y[i];
+            loss_part = __fadd_rn(loss_part, __fmul_rn(rr, rr));
+            groot[i] = __fmul_rn(rr * 2.0f, invN);
+          } else {
+            loss_part = __fadd_rn(loss_part, f[i]);
+            groot[i] = invN;
           }
         }
       }
+      if constexpr (kMode == kPassLoss) continue;
+      const uint32_t rk = root_dst >> 30, ro = root_dst & 0x3fffffffu;
+      if (rk == kDstFirst) {
+        sts_pack<P>(my_rows + ro, groot);
+      } else if (rk == kDstSum) {  // a constant as the root
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+          if (groot[i] != 0.f) {
+            float* d = gl + ro + (i % V) * 32;
+            *d = __fadd_rn(*d, groot[i]);
+          }
+      }
+      // ---- reverse sweep over the operator nodes ----
+      int e2[P];
+#pragma unroll
+      for (int i = 0; i < P; ++i) e2[i] = 0;
+      uint4 rn = nI > 0 ? S.rev[nI - 1] : make_uint4(0u, 0u, 0u, 0u);
+      uint2 dn = nI > 0 ? S.dst[nI - 1] : make_uint2(0u, 0u);
+      for (int k = nI - 1; k >= 0; --k) {
+        const uint4 w = rn;
+        const uint2 d2 = dn;
+        if (k > 0) {
+          rn = S.rev[k - 1];
+          dn = S.dst[k - 1];
+        }
+        float g[P], a[P], c[P], o0[P], o1[P];
+        bool a0[P], a1[P];
+        int e[P];
+        lds_pack<P>(my_rows + w.w, g);
+        fetch_operand<P>(base, w.y, lane_rows, a);
+        fetch_operand<P>(base, w.z, lane_rows, c);
+        if (w.x & 0x100u) {  // a node without a parent: a zero adjoint
+#pragma unroll
+          for (int i = 0; i < P; ++i) g[i] = 0.f;
+        }
+        op_adjoint_v<float, P>((int)(w.x & 0xffu), g, a, c, a, a0, o0, a1, o1, e);
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          a0[i] = a0[i] && q.valid[i];
+          a1[i] = a1[i] && q.valid[i];
+          if (U == 1) {
+            if (e[i] && q.valid[i] && !err) err = e[i];
+          } else if (e[i] && q.valid[i] && !e2[i]) {
+            e2[i] = e[i];
+          }
+        }
+        auto give = [&](uint32_t d, const bool (&add)[P], const float (&o)[P]) {
+          const uint32_t kind = d >> 30, off = d & 0x3fffffffu;
+          if (kind == kDstNone) return;
+          if (kind == kDstSum) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              float x = gl[off + v * 32];
+#pragma unroll
+              for (int u = 0; u < U; ++u)
+                if (add[u * V + v]) x = __fadd_rn(x, o[u * V + v]);
+              gl[off + v * 32] = x;
+            }
+            return;
+          }
+          float x[P];
+          if (kind == kDstFirst) {
+#pragma unroll
+            for (int i = 0; i < P; ++i) x[i] = add[i] ? o[i] : 0.f;
+          } else {
+            lds_pack<P>(my_rows + off, x);
+#pragma unroll
+            for (int i = 0; i < P; ++i)
+              if (add[i]) x[i] = __fadd_rn(x[i], o[i]);
+          }
+          sts_pack<P>(my_rows + off, x);
+        };
+        give(d2.x, a0, o0);
+        give(d2.y, a1, o1);
+      }
+      if (U > 1) {  // the first error of a lane is that of its first chunk
+#pragma unroll
+        for (int i = 0; i < P; ++i)
+          if (!err) err = e2[i];
+      }
     }
-    __syncwarp();
-    }  // kPassGrad
   }
   return loss_part;
 }
@@ -897,25 +941,34 @@ __device__ __forceinline__ void reduce_slots(const float* __restrict__ gl, int V
   }
 }
 
+// The constants of a trial point into the broadcast entries (by one warp; a barrier follows).
+template <int SPL>
+__device__ __forceinline__ void publish_constants(const WarpSmem& S, const Layout& l, const Problem<SPL>& P,
+                                                  const Slots<SPL>& x) {
+  float* bc = reinterpret_cast<float*>(S.base + l.bc);
+#pragma unroll
+  for (int s = 0; s < SPL; ++s)
+    if (P.real(s))
+      for (int i = 0; i < l.P; ++i) bc[(1 + s * 32 + P.lane) * l.P + i] = x.v[s];
+}
+
 // Closure: publish the trial constants, run the pass over this warp's points,
 // reduce loss and gradient over the lanes (recursive halving) and then over the CTA's
 // warps in a fixed order, in float pairs on the FP32 pipe (GB300's FP64 rate is a
 // small fraction of its FP32 rate); every warp ends with the same bits.  Two CTA
 // barriers.
-template <int V, int SPL>
-__device__ __forceinline__ float closure(const FitArgs& A, const WarpSmem& S, const Problem<SPL>& P, int warp, int W,
-                                         const Slots<SPL>& xt, Slots<SPL>& grad, int& err) {
+template <int V, int U, int SPL>
+__device__ __forceinline__ float closure(const FitArgs& A, const WarpSmem& S, const Layout& l, const Problem<SPL>& P,
+                                         int warp, int W, bool vars_hold, const Slots<SPL>& xt, Slots<SPL>& grad,
+                                         int& err) {
   const int lane = P.lane;
-  // every warp holds the same trial point: each publishes it into its own broadcast entries
-#pragma unroll
-  for (int s = 0; s < SPL; ++s)
-    if (P.real(s)) S.bc[1 + s * 32 + lane] = xt.v[s];
+  if (warp == 0) publish_constants<SPL>(S, l, P, xt);  // every warp holds the same trial point
   for (int j = 0; j < P.K; ++j) {
 #pragma unroll
     for (int v = 0; v < V; ++v) S.gl[j * 32 * V + v * 32 + lane] = 0.f;
   }
   __syncthreads();  // also: every warp has read the previous closure's reduction buffers
-  const float lpart = tape_pass<V, kPassGrad>(A, S, P.b, lane, warp, W, err);
+  const float lpart = tape_pass<V, U, kPassGrad>(A, S, l, P.b, lane, warp, W, vars_hold, err);
   F2* out_g = S.red_g + warp * P.K;
   if (P.K < 32) {
     if (P.K < 1) reduce_slots<1>(S.gl, V, P.K, lpart, lane, out_g, S.red_l + warp);
@@ -976,22 +1029,37 @@ __device__ __forceinline__ bool problem_fits(const FitArgs& A, int64_t b, int L,
 }
 
 // Stages problem b (a tape of L = root + 1 nodes) for the CTA: the tape, the numbering
-// of its constant slots, operator nodes and variables, the adjoint rows by liveness,
-// the operator-node program (warp 0), then every warp's broadcast entries (0 and the
-// fixed constants) and zeroed adjoint rows.  Ends with the tables visible to the CTA;
-// false when the tape needs more live adjoint rows than the launch's max_live.
-template <int V>
-__device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& S, int64_t b, int L, int lane,
-                                              int warp) {
-  // stage the tape; number the constant slots, the operator nodes and the
-  // variables; write the operator-node program (warp 0), visible to the CTA
+// of its constant slots, operator nodes and variables, the rows, the operator-node program
+// and the broadcast entries of 0 and the fixed constants (warp 0).  Ends with the tables
+// visible to the CTA; false when the tape needs more rows than the launch's tables hold.
+//
+// Rows.  A value that the reverse sweep reads (an operand of a rule that uses its operands, EXP's
+// own) keeps its row for the whole pass; the others give it up after their last parent's
+// forward step.  An operator's adjoint holds a row from the sweep of its first parent to its
+// own.  The rows that come and go in the forward pass and those of the reverse sweep are the
+// same ones.  Rows are taken from a stack, so the assignment is the same in every run.  This
+// takes 38 rows for the ragged workload's tapes instead of the 43 + 12 of a value row per operator
+// beside the adjoint rows, which is what lets two CTAs with two chunks per warp onto an SM.
+template <int V, int U>
+__device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& S, const Layout& l, int64_t b, int L,
+                                              int lane, int warp) {
   if (warp == 0) {
-    for (int k = lane; k < L; k += 32) S.tape[k] = A.desc[b * A.M + k];
+    int* row_of = reinterpret_cast<int*>(S.base + l.row_of);
+    int* adj_of = reinterpret_cast<int*>(S.base + l.adj_of);
+    int* last = reinterpret_cast<int*>(S.base + l.last);      // last parent of a node, -1
+    int* flags = reinterpret_cast<int*>(S.base + l.flags);    // bit 0: read by the reverse sweep; then 2 x parents
+    int* frees = reinterpret_cast<int*>(S.base + l.frees);
+    for (int k = lane; k < L; k += 32) {
+      S.tape[k] = A.desc[b * A.M + k];
+      last[k] = -1;
+      flags[k] = 0;
+    }
     __syncwarp();
     int nslot = 0, nop = 0;
     for (int k0 = 0; k0 < L; k0 += 32) {
       const int k = k0 + lane;
-      const int code = k < L ? code_of(S.tape[k]) : -1;
+      const uint32_t d = k < L ? S.tape[k] : 0u;
+      const int code = k < L ? code_of(d) : -1;
       const bool lc = code == LEARNABLE;
       const bool opn = k < L && is_operator_node(code);
       const unsigned mc = __ballot_sync(0xffffffffu, lc);
@@ -1002,10 +1070,38 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
         S.node_slot[k] = slot;
         S.slot_node[slot] = k;
       }
-      if (opn) S.node_slot[k] = nop + __popc(mo & below);
+      if (opn) {
+        S.node_slot[k] = nop + __popc(mo & below);
+        const int ar = arity_of(code);
+        const bool reads = adjoint_reads_operands(code);
+        for (int j = 0; j < ar; ++j) {
+          const int c = j == 0 ? child0(d) : child1(d);
+          atomicMax(&last[c], k);
+          atomicAdd(&flags[c], 2);
+          if (reads) atomicOr(&flags[c], 1);
+        }
+        if (code == EXP) atomicOr(&flags[k], 1);
+      }
       nslot += __popc(mc);
       nop += __popc(mo);
     }
+    __syncwarp();
+    // rows kept for the pass, in node order
+    int kept = 0;
+    bool shared_const = false;
+    for (int k0 = 0; k0 < L; k0 += 32) {
+      const int k = k0 + lane;
+      const int code = k < L ? code_of(S.tape[k]) : -1;
+      const bool keep = k < L && is_operator_node(code) && (flags[k] & 1);
+      const unsigned mk = __ballot_sync(0xffffffffu, keep);
+      if (k < L) {
+        row_of[k] = keep ? kept + __popc(mk & ((1u << lane) - 1u)) : -1;
+        adj_of[k] = -1;
+      }
+      shared_const = __any_sync(0xffffffffu, code == LEARNABLE && flags[k < L ? k : 0] >= 4) || shared_const;
+      kept += __popc(mk);
+    }
+    __syncwarp();
     if (lane == 0) {  // one row per distinct variable, in order of first use
       int nvr = 0;
       for (int k = 0; k < L; ++k) {
@@ -1017,82 +1113,120 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
         if (r == nvr) S.rowvar[nvr++] = var;
         S.node_slot[k] = r;
       }
-      S.info[2] = nvr;
-      // adjoint rows by liveness: an operator node holds a row from the sweep of its
-      // first parent (the root from the start) to its own sweep, then frees it; rows
-      // are taken from a stack, so the assignment is the same in every run
+      S.info[kVars] = nvr;
+      bool over = kept > l.Rmax;
+      const int room = l.Rmax - kept;
+      // values that the reverse sweep does not read
       int top = 0;
-      for (int r = A.Amax - 1; r >= 0; --r) S.frees[top++] = r;
-      for (int i = 0; i < nop; ++i) S.arow[i] = -1;
-      bool over = false;
+      for (int r = room - 1; r >= 0; --r) frees[top++] = kept + r;
+      for (int k = 0; k < L && !over; ++k) {
+        const uint32_t d = S.tape[k];
+        const int code = code_of(d);
+        if (!is_operator_node(code)) continue;
+        const int ar = arity_of(code);
+        for (int j = 0; j < ar; ++j) {
+          const int c = j == 0 ? child0(d) : child1(d);
+          if (j == 1 && c == child0(d)) continue;
+          if (is_operator_node(code_of(S.tape[c])) && row_of[c] >= kept && last[c] == k) frees[top++] = row_of[c];
+        }
+        if (row_of[k] < 0) {
+          if (top == 0) { over = true; break; }
+          row_of[k] = frees[--top];
+          if (last[k] < 0 && k != L - 1) frees[top++] = row_of[k];  // a value that nothing uses
+        }
+      }
+      // adjoints; Amax bounds them as before
+      top = 0;
+      const int arooms = room < A.Amax ? room : A.Amax;
+      for (int r = arooms - 1; r >= 0; --r) frees[top++] = kept + r;
       const int R = L - 1;
-      if (is_operator_node(code_of(S.tape[R]))) {
-        if (top > 0) S.arow[S.node_slot[R]] = S.frees[--top];
+      if (!over && is_operator_node(code_of(S.tape[R]))) {
+        if (top > 0) adj_of[R] = frees[--top];
         else over = true;
       }
+      const uint32_t row = 128u * (uint32_t)l.P, sums = 32u * (uint32_t)l.V;
       for (int k = R; k >= 0 && !over; --k) {
         const uint32_t d = S.tape[k];
         const int code = code_of(d);
         if (!is_operator_node(code)) continue;
-        const int i = S.node_slot[k];
-        if (S.arow[i] < 0) {  // no parent: a zero row for the length of its own sweep
+        uint32_t x = (uint32_t)dense_op(code);
+        if (adj_of[k] < 0) {  // no parent: a zero adjoint for its own sweep
           if (top == 0) { over = true; break; }
-          S.arow[i] = S.frees[--top];
+          adj_of[k] = frees[--top];
+          x |= 0x100u;
         }
-        S.frees[top++] = S.arow[i];
+        frees[top++] = adj_of[k];
         const int ar = arity_of(code);
+        uint32_t to[2] = {0u, 0u};
         for (int j = 0; j < ar && !over; ++j) {
           const int c = j == 0 ? child0(d) : child1(d);
-          if (!is_operator_node(code_of(S.tape[c])) || S.arow[S.node_slot[c]] >= 0) continue;
-          if (top == 0) { over = true; break; }
-          S.arow[S.node_slot[c]] = S.frees[--top];
+          const int cc = code_of(S.tape[c]);
+          if (cc == LEARNABLE) {
+            to[j] = (kDstSum << 30) | ((uint32_t)S.node_slot[c] * sums);
+          } else if (is_operator_node(cc)) {
+            const bool first = adj_of[c] < 0;
+            if (first) {
+              if (top == 0) { over = true; break; }
+              adj_of[c] = frees[--top];
+            }
+            to[j] = ((first ? kDstFirst : kDstAdd) << 30) | ((uint32_t)adj_of[c] * row);
+          }
         }
+        const int i = S.node_slot[k];
+        S.rev[i].x = x;
+        S.rev[i].w = (uint32_t)adj_of[k] * row;
+        S.dst[i] = make_uint2(to[0], to[1]);
       }
-      S.info[6] = over ? 1 : 0;
+      const int rc = code_of(S.tape[R]);
+      S.info[kOps] = nop;
+      S.info[kRootDst] = is_operator_node(rc) ? (int)((kDstFirst << 30) | ((uint32_t)(over ? 0 : adj_of[R]) * row))
+                         : rc == LEARNABLE    ? (int)((kDstSum << 30) | ((uint32_t)S.node_slot[R] * sums))
+                                              : 0;
+      S.info[kSharedConst] = shared_const ? 1 : 0;
+      S.info[kTooFew] = over ? 1 : 0;
     }
     __syncwarp();
-    const WarpLayout WL = warp_layout(A.Lmax, A.Imax, A.Amax, A.Kmax, V, A.VR);
-    const uint32_t RWB = 32u * V * 4u;
-    for (int k = lane; k < L; k += 32) {
-      const uint32_t d = S.tape[k];
-      const int code = code_of(d);
-      if (!is_operator_node(code)) continue;
-      const int ar = arity_of(code);
-      uint32_t sa = 0u, sb = 0u, da = WL.sink, db = WL.sink;
-      if (ar >= 1) operand_words(S.tape, S.node_slot, S.arow, child0(d), A.Kmax, A.Imax, WL, RWB, sa, da);
-      if (ar == 2) operand_words(S.tape, S.node_slot, S.arow, child1(d), A.Kmax, A.Imax, WL, RWB, sb, db);
-      const int row = S.node_slot[k];
-      S.pcode[row] = (uint32_t)dense_op(code) | ((uint32_t)S.arow[row] << 8);  // opcode | adjoint row
-      S.psa[row] = sa;
-      S.psb[row] = sb;
-      S.pda[row] = da;
-      S.pdb[row] = db;
+    const uint32_t row = 128u * (uint32_t)l.P;
+    if (S.info[kTooFew] == 0) {
+      for (int k = lane; k < L; k += 32) {
+        const uint32_t d = S.tape[k];
+        const int code = code_of(d);
+        if (!is_operator_node(code)) continue;
+        const int ar = arity_of(code), i = S.node_slot[k];
+        uint32_t sa = l.bc, sb = l.bc;  // an operand that is not there reads the zero entry
+        if (ar >= 1) sa = operand_word(S.tape, S.node_slot, row_of, child0(d), l);
+        if (ar == 2) sb = operand_word(S.tape, S.node_slot, row_of, child1(d), l);
+        S.fwd[i] = make_uint4((uint32_t)dense_op(code), sa, sb, (uint32_t)row_of[k] * row);
+        const bool reads = adjoint_reads_operands(code);
+        S.rev[i].y = code == EXP ? (kRowOperand | ((uint32_t)row_of[k] * row)) : (reads ? sa : l.bc);
+        S.rev[i].z = reads ? sb : l.bc;
+      }
+      if (lane == 0) S.info[kRootSrc] = (int)operand_word(S.tape, S.node_slot, row_of, L - 1, l);
     }
-    if (lane == 0) {
-      const int R = (L - 1);
-      uint32_t rs, rdst;
-      operand_words(S.tape, S.node_slot, S.arow, R, A.Kmax, A.Imax, WL, RWB, rs, rdst);
-      S.info[0] = nop;
-      S.info[1] = is_operator_node(code_of(S.tape[R])) ? S.arow[S.node_slot[R]] : -1;  // the root's adjoint row
-      S.info[3] = (int)rs;
-      S.info[4] = (int)rdst;
-      S.info[5] = (int)WL.sink;
+    // broadcast entries: 0 and the fixed constants of the tape
+    float* bc = reinterpret_cast<float*>(S.base + l.bc);
+    if (lane < l.P) bc[lane] = 0.f;
+    for (int k = lane; k < L; k += 32) {
+      const int code = code_of(S.tape[k]);
+      if (is_fixed_leaf(code)) {
+        const float x = node_value<float>(code, 0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < l.P; ++i) bc[(1 + l.Kmax + k) * l.P + i] = x;
+      }
     }
   }
   __syncthreads();
-  const bool rows_suffice = S.info[6] == 0;  // written by warp 0 before the barrier
-  // this warp's broadcast entries: 0 and the fixed constants of the tape
-  if (lane == 0) S.bc[0] = 0.f;
-  for (int k = lane; k < L; k += 32) {
-    const int code = code_of(S.tape[k]);
-    if (is_fixed_leaf(code)) S.bc[1 + A.Kmax + k] = node_value<float>(code, 0.f, 0.f, 0.f, 0.f);
-  }
-  // this warp's adjoint rows start at zero; every sweep leaves them so (a node's row is
-  // reset when the node reads it)
-  for (int r = 0; r < A.Amax; ++r)
-    for (int v = 0; v < V; ++v) S.adj[r * 32 * V + v * 32 + lane] = 0.f;
-  __syncwarp();
-  return rows_suffice;
+  return S.info[kTooFew] == 0;
+}
+
+// Whether a warp's chunks fit one pass, so that its variable rows can be filled once per
+// problem and hold for every closure.
+template <int V, int U>
+__device__ __forceinline__ bool variables_once(const FitArgs& A, const WarpSmem& S, const Layout& l, int lane, int warp,
+                                               int W) {
+  const int step = U > 1 && S.info[kSharedConst] ? 1 : U;
+  if (((int64_t)warp + (int64_t)step * W) * (32 * V) < A.N) return false;
+  fill_variables<V, U>(A, S, l, pass_points<V, U>(A.N, 0, lane, warp, W, step), lane);
+  return true;
 }
 
 // Line-search phases of the per-problem state machine.  Every loop turn of the
@@ -1101,7 +1235,7 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
 // _alpha_zoom_corrected / _backtracking_line_search for one column.
 enum Phase : int { PH_INIT = 0, PH_BRACKET, PH_ZOOM_LO, PH_ZOOM, PH_BACKTRACK, PH_UPDATE, PH_DONE };
 
-template <int V, int SPL>
+template <int V, int U, int SPL>
 __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
   // L-BFGS constants in the iteration's arithmetic: eps as a float pair, the gradient
   // tolerance in float32 (the reference compares a float32 norm with it)
@@ -1109,7 +1243,8 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
   const float tolf = __double2float_rn(A.tol);
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const WarpSmem S = carve(smem, A.Lmax, A.Imax, A.Amax, A.Kmax, V, W, A.VR, warp);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR);
+  const WarpSmem S = carve(smem, l, warp);
   // the L-BFGS history of this CTA (used by warp 0)
   const History H = history_at<SPL>(
       A.ring_off ? smem + A.ring_off : A.ws_hist + (int64_t)blockIdx.x * (int64_t)hist_block_bytes(A.hist, SPL), A.hist);
@@ -1131,7 +1266,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
     P.nslots = P.K + (P.has_virtual ? 1 : 0);
     const int L = P.root + 1;
     // a caller's max_len / max_consts / max_operators / max_live too small: not fitted
-    if (!problem_fits(A, P.b, L, P.K, lane) || !stage_problem<V>(A, S, P.b, L, lane, warp)) {
+    if (!problem_fits(A, P.b, L, P.K, lane) || !stage_problem<V, U>(A, S, l, P.b, L, lane, warp)) {
       if (warp == 0) {
         const float qnan = __int_as_float(0x7fffffff);
         for (int64_t k = lane; k < A.M; k += 32) A.C_out[P.b * A.c_sb + k * A.c_sm] = A.C_init[P.b * A.c_sb + k * A.c_sm];
@@ -1147,6 +1282,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
       continue;
     }
 
+    const bool vars_hold = variables_once<V, U>(A, S, l, lane, warp, W);
     const float* Cin = A.C_init + P.b * A.c_sb;
     Slots<SPL> x, g, p, xn;
 #pragma unroll
@@ -1186,7 +1322,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
         default: xt = xn; break;  // PH_UPDATE
       }
       Point<SPL> cur;
-      cur.phi = closure<V, SPL>(A, S, P, warp, W, xt, cur.g, err);
+      cur.phi = closure<V, U, SPL>(A, S, l, P, warp, W, vars_hold, xt, cur.g, err);
       ++evals;
 
       // ---- advance the state machine ----
@@ -1476,14 +1612,12 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
         if (A.evals_out) A.evals_out[P.b] = evals;
       }
     }
-    // the final constants into every warp's broadcast entries for the Y_final pass
-#pragma unroll
-    for (int s = 0; s < SPL; ++s)
-      if (P.real(s)) S.bc[1 + s * 32 + lane] = x.v[s];
+    // the final constants into the broadcast entries for the Y_final pass
+    if (warp == 0) publish_constants<SPL>(S, l, P, x);
     __syncthreads();
     if (A.Y_final) {
       int dummy = 0;
-      tape_pass<V, kPassYFinal>(A, S, P.b, lane, warp, W, dummy);
+      tape_pass<V, U, kPassYFinal>(A, S, l, P.b, lane, warp, W, vars_hold, dummy);
     }
     __syncthreads();
   }
@@ -1496,17 +1630,18 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
 // loss_out[b, k] is the mean squared error from candidate k, as the fit's first
 // closure measures it (to the last bit but for the order of the lane sum).
 // Candidate k of problem b: C_sets + k c_sk + b c_sb, slot m at + m c_sm.
-template <int V>
+template <int V, int U>
 __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const float* __restrict__ C_sets, int64_t c_sk,
                                                             int64_t K, float* __restrict__ loss_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const WarpSmem S = carve(smem, A.Lmax, A.Imax, A.Amax, A.Kmax, V, W, A.VR, warp);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR);
+  const WarpSmem S = carve(smem, l, warp);
   for (int64_t b = blockIdx.x; b < A.B; b += gridDim.x) {
     const int L = A.meta[b * 4 + 1] + 1;
     const int Kc = A.meta[b * 4 + 2];
     // a caller's max_len / max_consts / max_operators / max_live too small
-    if (!problem_fits(A, b, L, Kc, lane) || !stage_problem<V>(A, S, b, L, lane, warp)) {
+    if (!problem_fits(A, b, L, Kc, lane) || !stage_problem<V, U>(A, S, l, b, L, lane, warp)) {
       if (threadIdx.x == 0) {
         report(A.status, kStatusTapeExceedsLaunch);
         for (int64_t k = 0; k < K; ++k) loss_out[b * K + k] = __int_as_float(0x7fffffff);
@@ -1514,12 +1649,17 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
       __syncthreads();  // the next problem's staging overwrites the tables
       continue;
     }
+    const bool vars_hold = variables_once<V, U>(A, S, l, lane, warp, W);
+    float* bc = reinterpret_cast<float*>(S.base + l.bc);
     for (int64_t k = 0; k < K; ++k) {
       const float* Cin = C_sets + k * c_sk + b * A.c_sb;
-      for (int j = lane; j < Kc; j += 32) S.bc[1 + j] = Cin[(int64_t)S.slot_node[j] * A.c_sm];
+      for (int j = threadIdx.x; j < Kc; j += blockDim.x) {
+        const float x = Cin[(int64_t)S.slot_node[j] * A.c_sm];
+        for (int i = 0; i < l.P; ++i) bc[(1 + j) * l.P + i] = x;
+      }
       __syncthreads();  // also: thread 0 has read the previous candidate's warp sums
       int dummy = 0;
-      const F2 lsum = warp_sum_f2(tape_pass<V, kPassLoss>(A, S, b, lane, warp, W, dummy));
+      const F2 lsum = warp_sum_f2(tape_pass<V, U, kPassLoss>(A, S, l, b, lane, warp, W, vars_hold, dummy));
       if (lane == 0) S.red_l[warp] = lsum;
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -1532,47 +1672,86 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
   }
 }
 
-// Rows the fit's liveness assignment needs per tape (the same events as in
-// stage_problem: a row is taken at the first parent's sweep, or at the node's own
-// sweep when it has no parent, and freed after the node's sweep), the batch's largest
-// into stats[5].  One warp per tape, lane 0 walks the tape; tapes longer than 128
-// nodes to the root count all their operator nodes (a bound).
-__global__ void __launch_bounds__(256) tape_live_kernel(const uint32_t* __restrict__ desc,
-                                                        const int32_t* __restrict__ meta, int64_t B, int64_t M,
-                                                        int32_t* __restrict__ stats) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  int best = 0;
-  for (int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < B; b += warps) {
-    if (lane != 0) continue;
+// What stage_problem's row assignment needs per tape, the batch's largest into stats[5]
+// (operator adjoints live at once) and stats[6] (rows in all: the values that the reverse
+// sweep reads, plus the larger of the adjoints and of the other values live at once).  One
+// thread per tape; tapes longer than 128 nodes to the root count all their operator nodes
+// (a bound).
+__global__ void __launch_bounds__(64) tape_live_kernel(const uint32_t* __restrict__ desc,
+                                                       const int32_t* __restrict__ meta, int64_t B, int64_t M,
+                                                       int32_t* __restrict__ stats) {
+  int best = 0, best_rows = 0;
+  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < B) {
     const int L = meta[b * 4 + 1] + 1;
     const uint32_t* d = desc + b * M;
-    int live = 0;
     if (L > 128) {
-      for (int k = 0; k < L; ++k) live += is_operator_node(code_of(d[k])) ? 1 : 0;
+      for (int k = 0; k < L; ++k) best += is_operator_node(code_of(d[k])) ? 1 : 0;
+      best_rows = 2 * best;
     } else {
-      uint64_t held[2] = {0ull, 0ull};
-      auto has = [&](int k) { return (held[k >> 6] >> (k & 63)) & 1ull; };
-      auto take = [&](int k, int& cur) { held[k >> 6] |= 1ull << (k & 63); ++cur; live = cur > live ? cur : live; };
+      uint64_t held[2] = {0ull, 0ull}, kept[2] = {0ull, 0ull}, used[2] = {0ull, 0ull};
+      auto has = [](const uint64_t(&m)[2], int k) { return (m[k >> 6] >> (k & 63)) & 1ull; };
+      auto set = [](uint64_t(&m)[2], int k) { m[k >> 6] |= 1ull << (k & 63); };
       int cur = 0;
+      auto take = [&](int k) {
+        set(held, k);
+        ++cur;
+        best = cur > best ? cur : best;
+      };
       const int R = L - 1;
-      if (is_operator_node(code_of(d[R]))) take(R, cur);
+      if (is_operator_node(code_of(d[R]))) take(R);
+      // the reverse sweep: adjoints, and which values it reads; going backwards, a value whose
+      // last parent is met comes alive and dies at its own node
+      int temps = 0, most = 0;
       for (int k = R; k >= 0; --k) {
         const uint32_t w = d[k];
         const int code = code_of(w);
         if (!is_operator_node(code)) continue;
-        if (!has(k)) take(k, cur);
+        if (!has(held, k)) take(k);
         --cur;
+        if (code == EXP) set(kept, k);
+        const int ar = arity_of(code);
+        const bool reads = adjoint_reads_operands(code);
+        for (int j = 0; j < ar; ++j) {
+          const int c = j == 0 ? child0(w) : child1(w);
+          if (!is_operator_node(code_of(d[c]))) continue;
+          if (!has(held, c)) take(c);
+          if (reads) set(kept, c);
+        }
+      }
+      // the other values: alive from their node to their last parent (a node's own comes after
+      // its operands' go)
+      for (int k = R; k >= 0; --k) {
+        const uint32_t w = d[k];
+        const int code = code_of(w);
+        if (!is_operator_node(code)) continue;
+        if (!has(kept, k)) {
+          // at k its value is alive: counted since its last parent, or for this step alone
+          const bool waits = has(used, k) || k == R;
+          if (k == R) ++temps;
+          const int now = temps + (waits ? 0 : 1);
+          most = now > most ? now : most;
+          if (waits) --temps;
+        }
         const int ar = arity_of(code);
         for (int j = 0; j < ar; ++j) {
           const int c = j == 0 ? child0(w) : child1(w);
-          if (is_operator_node(code_of(d[c])) && !has(c)) take(c, cur);
+          if (!is_operator_node(code_of(d[c])) || has(kept, c) || has(used, c)) continue;
+          set(used, c);
+          ++temps;
         }
+        most = temps > most ? temps : most;
       }
+      const int keep = __popcll(kept[0]) + __popcll(kept[1]);
+      best_rows = keep + (best > most ? best : most);
     }
-    best = live > best ? live : best;
   }
-  if (lane == 0 && best > 0) atomicMax(stats + 5, best);
+  best = __reduce_max_sync(0xffffffffu, best);
+  best_rows = __reduce_max_sync(0xffffffffu, best_rows);
+  if ((threadIdx.x & 31) == 0 && best_rows > 0) {
+    atomicMax(stats + 5, best);
+    atomicMax(stats + 6, best_rows);
+  }
 }
 
 static int fit_defaults(const sr_fit_options* o, sr_fit_options& r) {
@@ -1609,28 +1788,31 @@ static int spl_for(int Kmax) {
 }
 
 struct FitShape {
-  int V, SPL, warps, blocks, Imax, Amax, VR;
+  int V, U, SPL, warps, blocks, Imax, Amax, Rmax, VR;
   size_t smem;
   size_t ring_off;  // > 0: the L-BFGS history sits in shared memory from this byte offset
 };
 
 
-template <int V, int SPL>
+template <int V, int U, int SPL>
 static void* fit_kernel_ptr() {
-  return reinterpret_cast<void*>(fit_lbfgs_kernel<V, SPL>);
+  return reinterpret_cast<void*>(fit_lbfgs_kernel<V, U, SPL>);
 }
 
-static void* pick_kernel(int V, int SPL) {
-  switch (V * 10 + SPL) {
-    case 11: return fit_kernel_ptr<1, 1>();
-    case 12: return fit_kernel_ptr<1, 2>();
-    case 14: return fit_kernel_ptr<1, 4>();
-    case 21: return fit_kernel_ptr<2, 1>();
-    case 22: return fit_kernel_ptr<2, 2>();
-    case 24: return fit_kernel_ptr<2, 4>();
-    case 41: return fit_kernel_ptr<4, 1>();
-    case 42: return fit_kernel_ptr<4, 2>();
-    case 44: return fit_kernel_ptr<4, 4>();
+static void* pick_kernel(int V, int U, int SPL) {
+  switch (V * 100 + U * 10 + SPL) {
+    case 111: return fit_kernel_ptr<1, 1, 1>();
+    case 112: return fit_kernel_ptr<1, 1, 2>();
+    case 114: return fit_kernel_ptr<1, 1, 4>();
+    case 121: return fit_kernel_ptr<1, 2, 1>();
+    case 122: return fit_kernel_ptr<1, 2, 2>();
+    case 124: return fit_kernel_ptr<1, 2, 4>();
+    case 211: return fit_kernel_ptr<2, 1, 1>();
+    case 212: return fit_kernel_ptr<2, 1, 2>();
+    case 214: return fit_kernel_ptr<2, 1, 4>();
+    case 411: return fit_kernel_ptr<4, 1, 1>();
+    case 412: return fit_kernel_ptr<4, 1, 2>();
+    case 414: return fit_kernel_ptr<4, 1, 4>();
     default: return nullptr;
   }
 }
@@ -1644,13 +1826,19 @@ static void* pick_kernel(int V, int SPL) {
 // batch alone would leave the GPU short of 16 warps per SM and a warp still gets more
 // than 32 points (1024 README problems: 6.2 ms at W = 4 against 15.7 ms at W = 1).
 // The warp tables hold a row per distinct variable of a tape: VR = min(n_x, Lmax) rows.
+// U, the chunks a warp works on at once, changes no bit: 2 where some warp has a second chunk
+// (N > 32 W) and the rows for two, twice as large, leave at least half the CTAs on an SM.
 static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, const sr_fit_options& o, FitShape& sh) {
   const int Imax = (o.max_operators > 0 && o.max_operators < Lmax) ? o.max_operators : Lmax;
   sh.Imax = Imax;
   // adjoint rows: the most operator-node adjoints live at once (rows are assigned by
   // liveness), at most one per operator node
-  const int Amax = (o.max_live > 0 && o.max_live < Imax) ? o.max_live : Imax;
+  const bool counted = (o.max_live & SR_LIVE_ROWS_COUNTED) != 0;
+  const int live = counted ? (o.max_live & 0x7fff) : o.max_live, rows = counted ? (o.max_live >> 15 & 0x7fff) : 0;
+  const int Amax = (live > 0 && live < Imax) ? live : Imax;
   sh.Amax = Amax;
+  // rows for operator values and adjoints: what the batch's tapes take, or a bound
+  sh.Rmax = (rows > 0 && rows < Imax + Amax) ? rows : Imax + Amax;
   sh.VR = (int)(n_x < 1 ? 1 : (n_x < Lmax ? n_x : Lmax));
   sh.SPL = spl_for(Kmax);
   if (!sh.SPL) {
@@ -1670,29 +1858,39 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
     while (W < 8 && (int64_t)W * 32 < N && B * W < want_warps) W *= 2;
   }
   if (W > 8) W = 8;  // __launch_bounds__(256)
-  const int vc[3] = {1, 2, 4};
+  const int V = o.points_per_lane ? o.points_per_lane : 1;
   double best = -1.0;
-  int bestV = 0, bestPerSm = 0;
+  int bestPerSm = 0;
+  auto resident = [&](int u, int w, size_t& bytes) -> int {  // CTAs per SM, 0 if they do not fit, < 0 for an error
+    void* k = pick_kernel(V, u, sh.SPL);
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return -1;
+    bytes = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, u, w, sh.VR).bytes;
+    int per_sm = 0;
+    if (bytes > (size_t)optin ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, w * 32, bytes) != cudaSuccess)
+      return 0;
+    return per_sm;
+  };
   for (int w = W; w >= 1 && best < 0; w >>= 1) {
-    for (int vi = 0; vi < 3; ++vi) {
-      const int V = vc[vi];
-      if (o.points_per_lane ? V != o.points_per_lane : V != 1) continue;
-      void* k = pick_kernel(V, sh.SPL);
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) {
-        set_error("fit kernel shared memory attribute failed");
-        return SR_ERR_CUDA;
-      }
-      const size_t cb = fit_cta_bytes(Lmax, Imax, Amax, Kmax, V, w, sh.VR);
-      if (cb > (size_t)optin) continue;
-      int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, w * 32, cb) != cudaSuccess || per_sm < 1)
-        continue;
-      const double score = (double)per_sm * w;
-      if (score > best) {
-        best = score;
-        bestV = V;
-        bestPerSm = per_sm;
-        W = w;
+    size_t bytes = 0;
+    const int one = resident(1, w, bytes);
+    if (one < 0) {
+      set_error("fit kernel shared memory attribute failed");
+      return SR_ERR_CUDA;
+    }
+    if (one > 0) {
+      best = 1.0;
+      W = w;
+      sh.U = 1;
+      bestPerSm = one;
+      sh.smem = bytes;
+      if (V == 1 && N > (int64_t)32 * w) {
+        const int two = resident(2, w, bytes);
+        if (two > 0 && 2 * two >= one) {
+          sh.U = 2;
+          bestPerSm = two;
+          sh.smem = bytes;
+        }
       }
     }
     if (best < 0 && o.warps_per_block > 0) break;
@@ -1701,9 +1899,8 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
     set_error("tape of %d nodes does not fit in shared memory for the fit kernel", Lmax);
     return SR_ERR_UNSUPPORTED;
   }
-  sh.V = bestV;
+  sh.V = V;
   sh.warps = W;
-  sh.smem = fit_cta_bytes(Lmax, Imax, Amax, Kmax, bestV, W, sh.VR);
   // Warp 0 reads the L-BFGS history for every direction: keep it in shared memory
   // when that costs no resident CTA, else in the workspace.
   sh.ring_off = 0;
@@ -1711,7 +1908,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
     const size_t off = fit_align16(sh.smem), with = off + hist_block_bytes(o.history_size, sh.SPL);
     int per_sm = 0;
     if (with <= (size_t)optin &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(bestV, sh.SPL), W * 32, with) ==
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(V, sh.U, sh.SPL), W * 32, with) ==
             cudaSuccess &&
         per_sm >= bestPerSm) {
       sh.ring_off = off;
@@ -1758,9 +1955,8 @@ int sr_tape_live_rows(const uint32_t* desc, const int32_t* meta, int64_t B, int6
   if (M > sr::kMaxNodes) { sr::set_error("tapes longer than %d nodes are not supported", sr::kMaxNodes); return SR_ERR_UNSUPPORTED; }
   if (B == 0 || M == 0) return SR_OK;
   if (!desc || !meta || !stats) { sr::set_error("null pointer argument"); return SR_ERR_INVALID_ARGUMENT; }
-  int64_t blocks = (B + 7) / 8;
-  if (blocks > 65535) blocks = 65535;
-  sr::tape_live_kernel<<<(unsigned)blocks, 256, 0, sr::as_stream(stream)>>>(desc, meta, B, M, stats);
+  const int64_t blocks = (B + 63) / 64;
+  sr::tape_live_kernel<<<(unsigned)blocks, 64, 0, sr::as_stream(stream)>>>(desc, meta, B, M, stats);
   return sr::launch_check("tape_live_kernel");
 }
 
@@ -1815,10 +2011,12 @@ int sr_fit_screen(const float* X, int64_t N, int64_t n_x, const float* Y, const 
   A.desc = desc; A.meta = meta; A.B = B; A.M = M;
   A.c_sb = c_sb; A.c_sm = c_sm;
   A.objective = o.objective;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.VR = sh.VR;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
   A.status = status;
-  void* k = sh.V == 1 ? reinterpret_cast<void*>(fit_screen_kernel<1>)
-                      : (sh.V == 2 ? reinterpret_cast<void*>(fit_screen_kernel<2>) : reinterpret_cast<void*>(fit_screen_kernel<4>));
+  void* k = sh.V == 1 ? (sh.U == 2 ? reinterpret_cast<void*>(fit_screen_kernel<1, 2>)
+                                   : reinterpret_cast<void*>(fit_screen_kernel<1, 1>))
+                      : (sh.V == 2 ? reinterpret_cast<void*>(fit_screen_kernel<2, 1>)
+                                   : reinterpret_cast<void*>(fit_screen_kernel<4, 1>));
   int dev = 0, optin = 0;
   if (cuda_check(cudaGetDevice(&dev), "cudaGetDevice") ||
       cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory limit") ||
@@ -1876,14 +2074,14 @@ int sr_fit_lbfgs(const float* X, int64_t N, int64_t n_x, const float* Y, const u
   A.order = order;
   A.max_iter = o.max_iter; A.hist = o.history_size; A.ls_kind = o.line_search; A.ls_max = o.line_search_max_iter;
   A.objective = o.objective; A.tol = o.tolerance_grad; A.eps = o.eps;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.VR = sh.VR;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
   A.counter = reinterpret_cast<int*>(ws);
   A.ws_hist = sh.ring_off ? nullptr : ws + 256;
   A.ring_off = (int)sh.ring_off;
   A.status = status;
   rc = cuda_check(cudaMemsetAsync(ws, 0, 256, st), "work counter reset");
   if (rc) return rc;
-  void* k = pick_kernel(sh.V, sh.SPL);
+  void* k = pick_kernel(sh.V, sh.U, sh.SPL);
   void* args[] = {&A};
   rc = cuda_check(cudaLaunchKernel(k, dim3(sh.blocks), dim3(sh.warps * 32), args, sh.smem, st), "fit_lbfgs_kernel");
   return rc;

@@ -127,7 +127,7 @@ def _fit(X, Y, Ops, Ch, C_init, max_iter, history_size, tolerance_grad, line_sea
                            objective=int(objective), warps_per_block=int(warps_per_block),
                            points_per_lane=int(points_per_lane), grid_blocks=int(grid_blocks),
                            max_operators=int(max(tapes.max_operators, 1)),
-                           max_live=int(tapes.max_live))
+                           max_live=tapes.live_option)
     L = _lib.lib()
     C_out = torch.empty((B, M), dtype=torch.float32, device=dev)
     Y_out = torch.empty((B, N), dtype=torch.float32, device=dev) if want_y else None
@@ -197,7 +197,7 @@ def screen_starts(X, Y, Ops, Ch, C_sets, *, objective: int = 0, tapes=None) -> t
         tapes = compile_tapes(Ops, Ch, nx, live=True)
     opts = _lib.FitOptions(max_iter=0, history_size=1, tolerance_grad=0.0, line_search=0, line_search_max_iter=0,
                            eps=0.0, objective=int(objective), max_operators=int(max(tapes.max_operators, 1)),
-                           max_live=int(tapes.max_live))
+                           max_live=tapes.live_option)
     Cs = C_sets.to(torch.float32).contiguous()
     out = torch.empty((B, K), dtype=torch.float32, device=dev)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
@@ -230,7 +230,7 @@ def batch_launch_shape(X: torch.Tensor, Ops: torch.Tensor, Ch: torch.Tensor) -> 
     tapes = compile_tapes(Ops, Ch, nx, live=True)
     opts = _lib.FitOptions(max_iter=1, history_size=1, tolerance_grad=0.0, line_search=0, line_search_max_iter=0,
                            eps=0.0, objective=0, max_operators=int(max(tapes.max_operators, 1)),
-                           max_live=int(tapes.max_live))
+                           max_live=tapes.live_option)
     V, W = _launch_shape(_lib.lib(), B, N, nx, M, min(max(tapes.max_root, 1), M), tapes.max_consts, opts)
     return {"points_per_lane": V, "warps_per_block": W, "consts_floor": int(tapes.max_consts)}
 
@@ -332,7 +332,7 @@ class FitPlan:
                                     objective=int(objective), warps_per_block=int(warps_per_block),
                                     points_per_lane=int(points_per_lane), grid_blocks=int(grid_blocks),
                                     max_operators=int(max(self.tapes.max_operators, 1)),
-                                    max_live=int(self.tapes.max_live))
+                                    max_live=self.tapes.live_option)
         L = _lib.lib()
         self.max_len = min(max(self.tapes.max_root, 1), M)
         wsb = L.sr_fit_workspace_bytes(B, N, M, self.max_len, self.tapes.max_consts, self.opts)

@@ -27,7 +27,15 @@ class CompiledTapes:
     max_consts: int     # largest number of constants up to the root
     max_operators: int  # largest number of operator nodes (arity >= 1 or NO_OP) up to the root
     max_live: int = 0   # most operator-node adjoints live at once in a reverse sweep (0: not measured)
+    max_rows: int = 0   # most rows the fit's tables take for a tape, values and adjoints (0: not measured)
     _order: torch.Tensor | None = None
+
+    @property
+    def live_option(self) -> int:
+        """sr_fit_options.max_live: both measured counts where they fit its fields."""
+        if 0 < self.max_live <= 0x7fff and 0 < self.max_rows <= 0x7fff:
+            return _lib.LIVE_ROWS_COUNTED | self.max_rows << 15 | self.max_live
+        return self.max_live
 
     @property
     def order(self) -> torch.Tensor:
@@ -70,4 +78,4 @@ def compile_tapes(ops_bm: torch.Tensor, ch_bm: torch.Tensor, n_vars: int, valida
     if s[0]:
         raise RuntimeError(error_message(s[0], "input validation"))
     return CompiledTapes(desc=desc, meta=meta, B=B, M=M, max_len=s[1], max_root=s[2], max_consts=s[3],
-                         max_operators=s[4], max_live=s[5] if live else 0)
+                         max_operators=s[4], max_live=s[5] if live else 0, max_rows=s[6] if live else 0)

@@ -145,14 +145,20 @@ typedef struct sr_fit_options {
                                    (0 = max_len) */
   int32_t max_live;             /* largest number of operator-node adjoints live at once in a
                                    reverse sweep, stats[5] after sr_tape_live_rows; sizes the
-                                   adjoint tables (0 = max_operators) */
+                                   adjoint tables (0 = max_operators).  With SR_LIVE_ROWS_COUNTED:
+                                   stats[5] (at most 0x7fff) | stats[6] << 15 | the flag; sizes
+                                   the tables for what the tapes take (smaller) */
 } sr_fit_options;
+
+#define SR_LIVE_ROWS_COUNTED (1 << 30)
 
 /* The fit kernel keeps the adjoint of an operator node in a table row only from the
  * moment its first parent is swept until the node itself is: rows are assigned by
  * liveness.  This writes into stats_dev[5] (atomic max) the largest number of rows a
  * tape of the batch needs (exact for tapes of up to 128 nodes to the root, else its
- * operator-node count, a bound), to be passed as sr_fit_options.max_live.  desc_dev
+ * operator-node count, a bound), to be passed as sr_fit_options.max_live, and into
+ * stats_dev[6] the most rows a tape takes in all, values that the reverse sweep reads
+ * included (twice the operator-node count beyond 128 nodes).  desc_dev
  * and meta_dev as written by sr_tape_compile.  No counterpart in the reference.
  * Returns 0 or an error code. */
 int sr_tape_live_rows(const uint32_t *desc_dev, const int32_t *meta_dev, int64_t B, int64_t M, int32_t *stats_dev,

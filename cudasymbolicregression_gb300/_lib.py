@@ -70,6 +70,8 @@ _SIGS = {
     "sr_version": ([], ctypes.c_char_p),
     "sr_validate": ([vp, vp, i64, i64, i64, i64, i64, i64, i64, vp, vp], ctypes.c_int),
     "sr_tape_compile": ([vp, vp, i64, i64, i64, i64, i64, i64, i64, i32, vp, vp, vp, vp], ctypes.c_int),
+    "sr_tape_order": ([vp, i64, i64, i32, vp, vp], ctypes.c_int),
+    "sr_any_nonzero": ([vp, i64, vp, vp], ctypes.c_int),
     "sr_eval_forward_f32": ([vp, i64, i64, vp, vp, vp, i64, i64, i32, vp, i64, i64, vp, vp], ctypes.c_int),
     "sr_eval_forward_f64": ([vp, i64, i64, vp, vp, vp, i64, i64, i32, vp, i64, i64, vp, vp], ctypes.c_int),
     "sr_eval_backward_f32": ([vp, i64, i64, vp, vp, vp, i64, i64, i32, vp, i64, i64, vp, vp, vp, vp, vp, vp],
@@ -158,6 +160,14 @@ def ptr(t: torch.Tensor | None):
 
 def stream_ptr(device: torch.device):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def any_nonzero(words: torch.Tensor) -> bool:
+    """Whether any of the int64 words is not zero, found on the device: one flag is read
+    back instead of the words (one host synchronisation)."""
+    flag = torch.empty(1, dtype=torch.int32, device=words.device)
+    check(lib().sr_any_nonzero(ptr(words), words.numel(), ptr(flag), stream_ptr(words.device)), "sr_any_nonzero")
+    return bool(flag.item())
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:

@@ -718,10 +718,9 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
   int64_t most_warps = 0;
   for (int w = 1; w <= 8; w *= 2) {
     const size_t bytes = adjoint_layout<T>(Lhi, flat, w, !cache).bytes;
-    int blocks = 0;
-    if (bytes > (size_t)limit ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, w * 32, bytes) != cudaSuccess || blocks < 1)
-      break;
+    if (bytes > (size_t)limit) break;
+    int blocks = resident_ctas(kp, w * 32, bytes);
+    if (blocks < 1) break;
     if (w == 1 && units > (int64_t)sms * blocks) {
       // several waves: leave room for the padding check's CTA on every SM, its shared memory
       // (every CTA takes 1 KB besides its own) and the registers of its warps, as those of two
@@ -780,11 +779,9 @@ static int launch_backward(const T* X, int64_t N, int64_t n_x, const uint32_t* d
   const int Lmax = (max_len > 0 && max_len < M) ? max_len : (int)M;
   // the padding check runs on a side stream, forked from and joined back into the
   // caller's stream (a CUDA graph capture records the same fork and join)
-  Aux* aux = aux_for_current_device();
-  if (!aux) return SR_ERR_CUDA;
-  std::lock_guard<std::mutex> hold(aux->mu);
-  rc = cuda_check(cudaEventRecord(aux->fork, st), "fork event");
-  if (!rc) rc = cuda_check(cudaStreamWaitEvent(aux->stream, aux->fork, 0), "fork wait");
+  // (on the caller's stream when there is little to check, as in launch_forward)
+  SideStream side((double)B * M * N * K * sizeof(T) > (double)(8 << 20), st);
+  rc = side.begin();
   if (rc) return rc;
   // one persistent grid per class of tape lengths (Llo, Lhi], each with the tables its class
   // needs; a batch too small to fill the GPU class by class runs as one grid
@@ -811,7 +808,7 @@ static int launch_backward(const T* X, int64_t N, int64_t n_x, const uint32_t* d
     rc = cuda_check(cudaFuncSetAttribute(padding_check_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared), "check carveout");
     if (!rc) {
-      padding_check_kernel<T><<<(unsigned)pblocks, (kCheckWarps + 1) * 32, 0, aux->stream>>>(gout, meta, B, M, N * K,
+      padding_check_kernel<T><<<(unsigned)pblocks, (kCheckWarps + 1) * 32, 0, side.stream()>>>(gout, meta, B, M, N * K,
                                                                                             Lmax, status);
       rc = launch_check("padding_check_kernel");
     }
@@ -820,10 +817,8 @@ static int launch_backward(const T* X, int64_t N, int64_t n_x, const uint32_t* d
     rc = launch_backward_class<T>(X, N, n_x, desc, meta, order, B, M, cls[ci][0], cls[ci][1], C, c_sb, c_sm, c_sk, K,
                                   cache, gout, gC, gX, status, st);
   }
-  // join (also after a failed launch: the side stream must not outlive the call)
-  const int rj = cuda_check(cudaEventRecord(aux->join, aux->stream), "join event");
-  const int rw = rj ? rj : cuda_check(cudaStreamWaitEvent(st, aux->join, 0), "join wait");
-  return rc ? rc : rw;
+  const int rj = side.end();
+  return rc ? rc : rj;
 }
 
 }  // namespace sr

@@ -20,6 +20,12 @@ inline int cuda_check(cudaError_t e, const char* what) {
 
 inline int launch_check(const char* what) { return cuda_check(cudaGetLastError(), what); }
 
+// CTAs of a kernel that fit on an SM with this many threads and this much dynamic shared
+// memory (cudaOccupancyMaxActiveBlocksPerMultiprocessor; 0 for an error).  The answers, facts
+// of the kernel and the device, are kept in a table of fixed size: asking for the handful of
+// shapes that a launch chooses from took longer than a small launch.
+int resident_ctas(const void* kern, int threads, size_t smem);
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 __device__ __forceinline__ void report(int* status, int code) {

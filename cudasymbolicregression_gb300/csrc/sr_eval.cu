@@ -156,6 +156,71 @@ __global__ void __launch_bounds__(32) pad_fill_kernel(const int32_t* __restrict_
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// Work order: the tapes by falling meta[column], by one CTA (a histogram of the values, its
+// running sums, then a place for each tape).  The order decides only which warp takes which
+// tape, so tapes of one length come in any order.  What bounds it: two passes over meta by one
+// SM (65536 tapes: about 20 us); a library sort's five launches took the host longer than the
+// forward of a small batch.
+__global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restrict__ meta, int64_t B, int column,
+                                                          int add, int bins, int32_t* __restrict__ order) {
+  extern __shared__ int at[];  // per value: count, then the next place
+  __shared__ int warp_sum_[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < bins; i += blockDim.x) at[i] = 0;
+  __syncthreads();
+  const int64_t rounds = (B + blockDim.x - 1) / blockDim.x;
+  auto key = [&](int64_t b) {  // 0 for the largest value
+    const int v = meta[b * 4 + column] + add;
+    return bins - 1 - min(max(v, 0), bins - 1);
+  };
+  for (int64_t r = 0; r < rounds; ++r) {
+    const int64_t b = r * blockDim.x + tid;
+    const int k = b < B ? key(b) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, k);
+    if (k >= 0 && lane == __ffs((int)same) - 1) atomicAdd(&at[k], __popc(same));
+  }
+  __syncthreads();
+  // exclusive running sums over the bins, a run of consecutive bins per thread
+  const int per = (bins + (int)blockDim.x - 1) / (int)blockDim.x, lo = min(bins, tid * per), hi = min(bins, lo + per);
+  int sum = 0;
+  for (int i = lo; i < hi; ++i) sum += at[i];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_sum_[warp] = incl;
+  __syncthreads();
+  int before = incl - sum;
+  for (int w = 0; w < warp; ++w) before += warp_sum_[w];
+  for (int i = lo; i < hi; ++i) {
+    const int c = at[i];
+    at[i] = before;
+    before += c;
+  }
+  __syncthreads();
+  for (int64_t r = 0; r < rounds; ++r) {
+    const int64_t b = r * blockDim.x + tid;
+    const int k = b < B ? key(b) : -1;
+    const unsigned same = __match_any_sync(0xffffffffu, k);
+    const int leader = __ffs((int)same) - 1;
+    int base = 0;
+    if (k >= 0 && lane == leader) base = atomicAdd(&at[k], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (k >= 0) order[base + __popc(same & ((1u << lane) - 1u))] = (int32_t)b;
+  }
+}
+
+// Whether any of n words is not zero.
+__global__ void __launch_bounds__(256) any_nonzero_kernel(const int64_t* __restrict__ words, int64_t n,
+                                                          int32_t* __restrict__ out) {
+  bool nz = false;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    nz |= words[i] != 0;
+  if (__any_sync(0xffffffffu, nz) && (threadIdx.x & 31) == 0) atomicOr(out, 1);
+}
+
 // ------------------------------------------------------------------------------------
 // Forward.  Work unit = (tape, slice of its points); units are taken in grid-stride order
 // over the tapes sorted longest first, so every warp of the persistent grid gets a similar
@@ -422,6 +487,30 @@ int max_sm_smem() {
   return v;
 }
 
+int resident_ctas(const void* kern, int threads, size_t smem) {
+  struct Entry {
+    const void* kern;
+    int dev, threads, ctas;
+    size_t smem;
+  };
+  constexpr size_t kEntries = 256;  // direct-mapped: a shape that collides is asked for again
+  static Entry table[kEntries] = {};
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const size_t h = ((reinterpret_cast<uintptr_t>(kern) >> 4) * 31 + (size_t)dev * 17 + (size_t)threads + smem / 16 * 7) % kEntries;
+  {
+    std::lock_guard<std::mutex> hold(mu);
+    const Entry& e = table[h];
+    if (e.kern == kern && e.dev == dev && e.threads == threads && e.smem == smem) return e.ctas;
+  }
+  int ctas = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kern, threads, smem) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> hold(mu);
+  table[h] = Entry{kern, dev, threads, ctas, smem};
+  return ctas;
+}
+
 int check_tape_args(int64_t B, int64_t M) {
   if (B < 0 || M < 0) { set_error("negative size"); return SR_ERR_INVALID_ARGUMENT; }
   if (M > kMaxNodes) {
@@ -500,9 +589,7 @@ bool pick_shape(const void* kern, size_t per_warp, int64_t work_items, Shape& sh
   int w = 0, per_sm = 0, best = 0;
   for (int cand = 8; cand >= 1; cand >>= 1) {
     if (per_warp * cand > (size_t)limit) continue;
-    int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, cand * 32, per_warp * cand) != cudaSuccess)
-      continue;
+    int blocks = resident_ctas(kern, cand * 32, per_warp * cand);
     // every CTA takes 1 KB of its SM's shared memory besides its own
     const int room = (int)(((size_t)sm_bytes - reserve) / (per_warp * cand + 1024));
     if (reserve && blocks > room && room > 0) blocks = room;
@@ -547,11 +634,11 @@ static int launch_forward(const T* X, int64_t N, int64_t n_x, const uint32_t* de
   const int Lmax = (max_len > 0 && max_len < M) ? max_len : (int)M;
   const bool aligned = reinterpret_cast<uintptr_t>(cache) % 16 == 0;
   cudaStream_t st = as_stream(stream);
-  Aux* aux = aux_for_current_device();
-  if (!aux) return SR_ERR_CUDA;
-  std::lock_guard<std::mutex> hold(aux->mu);
-  rc = cuda_check(cudaEventRecord(aux->fork, st), "fork event");
-  if (!rc) rc = cuda_check(cudaStreamWaitEvent(aux->stream, aux->fork, 0), "fork wait");
+  // a small output is filled on the caller's stream: the fork and join take longer (8 MB are
+  // written in a few microseconds)
+  const bool fork = (double)B * M * N * K * sizeof(T) > (double)(8 << 20);
+  SideStream side(fork, st);
+  rc = side.begin();
   if (rc) return rc;
   {
     // one warp per SM, placed before the forward grids, which leave its shared memory free
@@ -561,7 +648,7 @@ static int launch_forward(const T* X, int64_t N, int64_t n_x, const uint32_t* de
     // ask for the largest shared memory, or whichever comes first locks the other out
     rc = cuda_check(cudaFuncSetAttribute(pad_fill_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared), "fill carveout");
-    pad_fill_kernel<T><<<(unsigned)fblocks, 32, 0, aux->stream>>>(meta, B, M, N * K, Lmax, cache);
+    pad_fill_kernel<T><<<(unsigned)fblocks, 32, 0, side.stream()>>>(meta, B, M, N * K, Lmax, cache);
     if (!rc) rc = launch_check("pad_fill_kernel");
   }
   // one persistent grid per class of tape lengths, as in launch_backward
@@ -593,9 +680,8 @@ static int launch_forward(const T* X, int64_t N, int64_t n_x, const uint32_t* de
                                                              nx_rows, C, c_sb, c_sm, c_sk, K, slice, nslices, cache);
     rc = launch_check("eval_forward_kernel");
   }
-  const int rj = cuda_check(cudaEventRecord(aux->join, aux->stream), "join event");
-  const int rw = rj ? rj : cuda_check(cudaStreamWaitEvent(st, aux->join, 0), "join wait");
-  return rc ? rc : rw;
+  const int rj = side.end();
+  return rc ? rc : rj;
 }
 
 }  // namespace sr
@@ -620,6 +706,30 @@ int sr_tape_compile(const int64_t* ops, const int64_t* ch, int64_t B, int64_t M,
                     int32_t* stats, void* stream) {
   return sr::launch_compile<true>(ops, ch, B, M, ops_sb, ops_sm, ch_sb, ch_sm, ch_si, n_vars, desc, meta, stats,
                                   stream);
+}
+
+int sr_tape_order(const int32_t* meta, int64_t B, int64_t M, int32_t column, int32_t* order, void* stream) {
+  using namespace sr;
+  int rc = check_tape_args(B, M);
+  if (rc) return rc;
+  if (column < 0 || column > 1 || B > INT32_MAX) { set_error("invalid column or too many tapes"); return SR_ERR_INVALID_ARGUMENT; }
+  if (B == 0) return SR_OK;
+  if (!meta || !order) { set_error("null pointer argument"); return SR_ERR_INVALID_ARGUMENT; }
+  const int bins = (int)M + 1;
+  tape_order_kernel<<<1, 1024, bins * sizeof(int), as_stream(stream)>>>(meta, B, column, column, bins, order);
+  return launch_check("tape_order_kernel");
+}
+
+int sr_any_nonzero(const int64_t* words, int64_t n, int32_t* out, void* stream) {
+  using namespace sr;
+  if (n < 0 || !out || (n > 0 && !words)) { set_error("invalid arguments"); return SR_ERR_INVALID_ARGUMENT; }
+  const int rc = cuda_check(cudaMemsetAsync(out, 0, sizeof(int32_t), as_stream(stream)), "flag reset");
+  if (rc || n == 0) return rc;
+  int64_t blocks = (n + 2047) / 2048;
+  const int64_t cap = (int64_t)device_sm_count() * 8;
+  if (blocks > cap) blocks = cap;
+  any_nonzero_kernel<<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(words, n, out);
+  return launch_check("any_nonzero_kernel");
 }
 
 int sr_eval_forward_f32(const float* X, int64_t N, int64_t n_x, const uint32_t* desc, const int32_t* meta,

@@ -121,6 +121,34 @@ struct Aux {
 };
 Aux* aux_for_current_device();
 
+// The side stream of one call, forked from the caller's stream and joined back into it (a CUDA
+// graph capture of the caller's stream records both); without a fork, the caller's stream.
+class SideStream {
+ public:
+  SideStream(bool fork, cudaStream_t st) : fork_(fork), st_(st) {}
+  int begin() {
+    if (!fork_) return SR_OK;
+    aux_ = aux_for_current_device();
+    if (!aux_) return SR_ERR_CUDA;
+    hold_ = std::unique_lock<std::mutex>(aux_->mu);
+    const int rc = cuda_check(cudaEventRecord(aux_->fork, st_), "fork event");
+    return rc ? rc : cuda_check(cudaStreamWaitEvent(aux_->stream, aux_->fork, 0), "fork wait");
+  }
+  cudaStream_t stream() const { return fork_ ? aux_->stream : st_; }
+  // also after a failed launch: the side stream must not outlive the call
+  int end() {
+    if (!fork_) return SR_OK;
+    const int rc = cuda_check(cudaEventRecord(aux_->join, aux_->stream), "join event");
+    return rc ? rc : cuda_check(cudaStreamWaitEvent(st_, aux_->join, 0), "join wait");
+  }
+
+ private:
+  bool fork_;
+  cudaStream_t st_;
+  Aux* aux_ = nullptr;
+  std::unique_lock<std::mutex> hold_;
+};
+
 // Persistent grid for an interpreter kernel: warps per CTA and CTAs from the
 // per-warp shared memory and the occupancy the kernel reaches.
 struct Shape {

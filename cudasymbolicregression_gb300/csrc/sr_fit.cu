@@ -1865,11 +1865,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
     void* k = pick_kernel(V, u, sh.SPL);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return -1;
     bytes = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, u, w, sh.VR).bytes;
-    int per_sm = 0;
-    if (bytes > (size_t)optin ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, w * 32, bytes) != cudaSuccess)
-      return 0;
-    return per_sm;
+    return bytes > (size_t)optin ? 0 : resident_ctas(k, w * 32, bytes);
   };
   for (int w = W; w >= 1 && best < 0; w >>= 1) {
     size_t bytes = 0;
@@ -1906,11 +1902,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
   sh.ring_off = 0;
   {
     const size_t off = fit_align16(sh.smem), with = off + hist_block_bytes(o.history_size, sh.SPL);
-    int per_sm = 0;
-    if (with <= (size_t)optin &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(V, sh.U, sh.SPL), W * 32, with) ==
-            cudaSuccess &&
-        per_sm >= bestPerSm) {
+    if (with <= (size_t)optin && resident_ctas(pick_kernel(V, sh.U, sh.SPL), W * 32, with) >= bestPerSm) {
       sh.ring_off = off;
       sh.smem = with;
     }

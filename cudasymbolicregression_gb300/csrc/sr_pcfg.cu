@@ -403,10 +403,8 @@ int sr_pcfg_sample_infix(const int32_t* nt_rule_ptr, const float* nt_rule_cum_pr
   int dev = 0, sms = 0, per_sm = 0;
   rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
   if (!rc) rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  if (!rc)
-    rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sample_infix_kernel, kThreads, smem),
-                    "occupancy");
   if (rc) return rc;
+  per_sm = resident_ctas(reinterpret_cast<const void*>(sample_infix_kernel), kThreads, smem);
   int64_t blocks = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
   const int64_t need = (B + kThreads - 1) / kThreads;
   if (blocks > need) blocks = need;

@@ -72,7 +72,8 @@ def get_postfix_children(postfix_ops: torch.Tensor, n_variables: int) -> torch.T
     rc = _lib.lib().sr_postfix_children(_lib.ptr(ops), B, M, int(n_variables), _lib.ptr(ch), _lib.ptr(err),
                                         _lib.stream_ptr(dev))
     _lib.check(rc, "sr_postfix_children")
-    _raise_for(err, "get postfix children", "postfix_ops")
+    if _lib.any_nonzero(err):  # the words only to report them
+        _raise_for(err, "get postfix children", "postfix_ops")
     return ch
 
 
@@ -86,7 +87,8 @@ def postfix_to_infix(postfix_ops: torch.Tensor, max_infix_len: int, n_variables:
     rc = _lib.lib().sr_postfix_to_infix(_lib.ptr(ops), B, M, int(n_variables), _lib.ptr(out), int(max_infix_len),
                                         _lib.ptr(err), _lib.stream_ptr(dev))
     _lib.check(rc, "sr_postfix_to_infix")
-    _raise_for(err, "postfix to infix conversion", "prefix_ops")
+    if _lib.any_nonzero(err):  # the words only to report them
+        _raise_for(err, "postfix to infix conversion", "prefix_ops")
     return out
 
 

@@ -135,11 +135,11 @@ def _fit(X, Y, Ops, Ch, C_init, max_iter, history_size, tolerance_grad, line_sea
     loss = torch.empty(B, dtype=torch.float32, device=dev)
     evals = torch.empty(B, dtype=torch.int32, device=dev)
     Cin = C_init.to(torch.float32).contiguous()
-    lens = tapes.meta[:, 1] + 1
     if order is None:
         # longest tapes first: the persistent warps then finish at about the same time
-        order = torch.argsort(lens, descending=True, stable=True).to(torch.int32)
-        classes = _length_classes(lens, order, class_width) if class_width > 0 else [(0, B, max(tapes.max_root, 1))]
+        order = tapes.order_by(1)
+        classes = (_length_classes(tapes.meta[:, 1] + 1, order, class_width) if class_width > 0
+                   else [(0, B, max(tapes.max_root, 1))])
     else:
         order = order.to(device=dev, dtype=torch.int32).contiguous()
         classes = [(0, B, max(tapes.max_root, 1))]
@@ -324,7 +324,7 @@ class FitPlan:
         self.X = X.contiguous()
         self.Y = None if Y is None else _targets(Y, B, N, dev)
         self.tapes = compile_tapes(Ops, Ch, nx, live=True)
-        self.order = torch.argsort(self.tapes.meta[:, 1] + 1, descending=True, stable=True).to(torch.int32)
+        self.order = self.tapes.order_by(1)
         self.opts = _lib.FitOptions(max_iter=int(max_iter), history_size=int(history_size),
                                     tolerance_grad=float(tolerance_grad),
                                     line_search=0 if line_search_fn == "strong_wolfe" else 1,

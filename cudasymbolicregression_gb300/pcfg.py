@@ -12,7 +12,7 @@ draws expressions on the device, each lane deriving one expression at a time
 (``sr_infix_to_postfix`` / ``sr_infix_to_prefix``); ``get_postfix_children`` and
 ``postfix_to_infix`` are the kernels of :mod:`.notation`.  ``sample(B)`` chains
 sampling, parsing and the child table on the device with one host
-synchronisation at the end (a two-number summary of the error words per kernel; the
+synchronisation at the end (one flag that says whether any error word is set; the
 words themselves are copied only to report an error), which is what a search loop
 feeds to the fit.
 
@@ -285,13 +285,6 @@ class ProbabilisticContextFreeGrammar:
                 msg += f"  {error_message(code)}: {counts[code]} occurrences.\n"
             raise RuntimeError(msg)
 
-    @staticmethod
-    def _any_error(errs: torch.Tensor) -> bool:
-        """Whether any per-row error word is nonzero, from the smallest and largest word of
-        each row of errs (one small device-to-host copy instead of all B words)."""
-        lo, hi = torch.aminmax(errs, dim=-1)
-        return bool(torch.stack((lo, hi)).ne(0).any().cpu())
-
     def sample_infix(self, B: int) -> torch.Tensor:
         """(B, padded_maximum_length) int64 infix token rows, NO_OP padded."""
         B = int(B)
@@ -299,7 +292,7 @@ class ProbabilisticContextFreeGrammar:
         err = torch.empty(B, dtype=torch.int64, device=self._device)
         if B:
             self._launch_sample(B, out, err)
-            if self._any_error(err):  # the full words only to report them
+            if _lib.any_nonzero(err):  # the full words only to report them
                 self._generation_error(err.cpu())
         return out
 
@@ -322,7 +315,7 @@ class ProbabilisticContextFreeGrammar:
                                            _lib.ptr(errs[1]), st), "sr_infix_to_postfix")
         _lib.check(lib.sr_postfix_children(_lib.ptr(post), B, L, self._n_variables, _lib.ptr(ch), _lib.ptr(errs[2]),
                                            st), "sr_postfix_children")
-        if self._any_error(errs):  # the full words only to report them
+        if _lib.any_nonzero(errs):  # the full words only to report them
             e = errs.cpu()
             self._generation_error(e[0])
             self._parsing_error(e[1], infix, "postfix parsing", 0, "infix_ops")
@@ -373,7 +366,8 @@ class ProbabilisticContextFreeGrammar:
         fn = _lib.lib().sr_infix_to_prefix if prefix else _lib.lib().sr_infix_to_postfix
         _lib.check(fn(_lib.ptr(x), B, M, self._n_variables, _lib.ptr(out), _lib.ptr(err), _lib.stream_ptr(dev)),
                    "sr_infix_to_prefix" if prefix else "sr_infix_to_postfix")
-        self._parsing_error(err.cpu(), x, "prefix parsing" if prefix else "postfix parsing", verbosity, "infix_ops")
+        if _lib.any_nonzero(err):  # the words only to report them
+            self._parsing_error(err.cpu(), x, "prefix parsing" if prefix else "postfix parsing", verbosity, "infix_ops")
         return out
 
     def infix_to_postfix(self, expressions: torch.Tensor, verbosity: int = 0) -> torch.Tensor:
@@ -401,7 +395,8 @@ class ProbabilisticContextFreeGrammar:
         if width is not None:
             args.append(int(width))
         _lib.check(getattr(_lib.lib(), fn)(*args, _lib.ptr(err), _lib.stream_ptr(dev)), fn)
-        self._parsing_error(err.cpu(), x, context, verbosity, check_kind)
+        if _lib.any_nonzero(err):  # the words only to report them
+            self._parsing_error(err.cpu(), x, context, verbosity, check_kind)
         return out
 
     def prefix_to_infix(self, expressions: torch.Tensor, max_infix_len: int, verbosity: int = 0) -> torch.Tensor:

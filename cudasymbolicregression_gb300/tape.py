@@ -41,8 +41,15 @@ class CompiledTapes:
     def order(self) -> torch.Tensor:
         """Tape indices, longest first (work order for the persistent kernels)."""
         if self._order is None:
-            self._order = torch.argsort(self.meta[:, 0], descending=True, stable=True).to(torch.int32)
+            self._order = self.order_by(0)
         return self._order
+
+    def order_by(self, column: int) -> torch.Tensor:
+        """Tape indices by falling meta[column] (``sr_tape_order``)."""
+        order = torch.empty(self.B, dtype=torch.int32, device=self.meta.device)
+        _lib.check(_lib.lib().sr_tape_order(_lib.ptr(self.meta), self.B, self.M, column, _lib.ptr(order),
+                                            _lib.stream_ptr(self.meta.device)), "sr_tape_order")
+        return order
 
 
 def compile_tapes(ops_bm: torch.Tensor, ch_bm: torch.Tensor, n_vars: int, validate_only: bool = False,
@@ -57,7 +64,7 @@ def compile_tapes(ops_bm: torch.Tensor, ch_bm: torch.Tensor, n_vars: int, valida
     B, M = ops_bm.shape
     L = _lib.lib()
     st = _lib.stream_ptr(dev)
-    stats = torch.zeros(8, dtype=torch.int32, device=dev)
+    stats = torch.empty(8, dtype=torch.int32, device=dev)  # zeroed by the call
     sb, sm = ops_bm.stride()
     cb, cm, ci = ch_bm.stride()
     if validate_only:

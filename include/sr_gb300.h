@@ -76,6 +76,16 @@ int sr_tape_compile(const int64_t *ops_dev, const int64_t *ch_dev, int64_t B, in
                     void *stream);
 
 /*
+ * Work order for the kernels below: order_dev (B) int32 lists the tapes by falling
+ * meta[column] (0: L_eff, 1: the root), tapes of one length in any order.  One launch.
+ */
+int sr_tape_order(const int32_t *meta_dev, int64_t B, int64_t M, int32_t column, int32_t *order_dev, void *stream);
+
+/* out_dev receives 1 if any of the n words is not zero, else 0 (the error words of the
+ * grammar and notation entry points, without copying them to the host). */
+int sr_any_nonzero(const int64_t *words_dev, int64_t n, int32_t *out_dev, void *stream);
+
+/*
  * Forward evaluation: cache (B, M, N) of every node at every point; NO_OP nodes
  * and the padding after the last real node are NaN.  Replaces the reference's
  * host loop of M launches of evaluation_forward_step_k

@@ -170,6 +170,10 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
 // residue p mod 32 K, that is to lane p mod 32 of the chunks s with s mod K = class: a warp
 // takes whole classes, so their sums are its own, and the set of a lane is fixed in a class.
 //
+// grad_X is an atomic sum over the tapes, constant sets and leaves.  A lane first adds up
+// the leaves of a variable at its value, so that there is one atomic for all of them (and the
+// sum over a tape's leaves has one order); more than 16 variables go straight to the atomics.
+//
 // Tapes whose child table is not that of a stack, or that need more rows than the table has,
 // take one adjoint row per node, set to its output gradient before the sweep, and one value
 // per lane.  So do calls without a cache, which recompute the node values into rows first.
@@ -180,14 +184,15 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
 // index; the nodes of the learnable constants; the constants' values (learnable j at j, fixed
 // f at L - 1 - f, one entry per set); the sums of ncap constants (32 K lanes each); the first
 // error of each point residue; then per warp the adjoint rows, without a cache a value row
-// per node and, with several warps, the terms of one pass.
+// per node, with several warps the terms of one pass, and with grad_X the sums of one pass
+// for each variable.
 struct AdjLayout {
-  size_t prog, cidx, lcon, cval, acc, errs, warps, warp_bytes, vals, crow, bytes;
+  size_t prog, cidx, lcon, cval, acc, errs, warps, warp_bytes, vals, crow, xacc, bytes;
   int ncap;
 };
 
 template <typename T>
-__host__ __device__ __forceinline__ AdjLayout adjoint_layout(int Lmax, int64_t K, int nwarp, bool recompute) {
+__host__ __device__ __forceinline__ AdjLayout adjoint_layout(int Lmax, int64_t K, int nwarp, bool recompute, int xrows) {
   AdjLayout l;
   // constants summed in one sweep: half the nodes of a tree are leaves, few of them
   // constants; a tape with more is swept again for the rest
@@ -206,10 +211,14 @@ __host__ __device__ __forceinline__ AdjLayout adjoint_layout(int Lmax, int64_t K
   l.warps = l.errs + 32 * 8 + 32;
   l.vals = (size_t)table_rows<T>(Lmax) * kRowBytes;
   l.crow = l.vals + (recompute ? (size_t)Lmax * 32 * sizeof(T) : 0);
-  l.warp_bytes = l.crow + (nwarp > 1 ? (size_t)cap * kRowBytes : 0);
+  l.xacc = l.crow + (nwarp > 1 ? (size_t)cap * kRowBytes : 0);
+  l.warp_bytes = l.xacc + (size_t)xrows * kRowBytes;
   l.bytes = l.warps + (size_t)nwarp * l.warp_bytes;
   return l;
 }
+
+// Variables whose sums over the leaves are kept in rows.
+__host__ __device__ __forceinline__ int x_sum_rows(int64_t n_x) { return n_x <= 16 ? (int)n_x : 0; }
 
 // Program words of operator node k:
 //   x: dense code (bits 0..4) | no parent (bit 5) | k << 8 | adjoint row << 20
@@ -264,6 +273,8 @@ struct GeneralSweep {
   const int *cidx, *lcon;
   const T* cv;           // the lane's constant entries
   T *accl, *adj, *vals;  // the lane's sums, adjoint rows and value rows
+  T* xs;                 // the lane's sums per variable, kRowBytes apart
+  unsigned xused;
   T* crow;
   const unsigned char* crows;
   size_t warp_bytes;
@@ -318,7 +329,14 @@ __device__ __noinline__ void general_sweep(const GeneralSweep<T>& q) {
         if (code_of(q.tape[k]) != VAR) return;
         const T g = q.adj[k * 32];
         q.adj[k * 32] = T(0);
-        if (g != T(0)) atomicAdd(q.gX + n * q.n_x + child0(q.tape[k]), g);
+        if (g == T(0)) return;
+        const int var = child0(q.tape[k]);
+        if (!q.xused) {
+          atomicAdd(q.gX + n * q.n_x + var, g);
+        } else {
+          T* t = q.xs + var * (int)(kRowBytes / sizeof(T));
+          *t = M_<T>::add(*t, g);
+        }
       };
       for (int i = q.nop - 1; i >= 0; --i) {
         const uint4 w = q.prog[i];
@@ -326,6 +344,12 @@ __device__ __noinline__ void general_sweep(const GeneralSweep<T>& q) {
         if (w.z >> 16 & 3u) leaf((int)(w.w >> 12));
       }
       for (int j = 0; j < q.norph; ++j) leaf((int)(q.orphan[-j] & 0xfffu));
+      for (unsigned m = q.xused; m; m &= m - 1) {
+        const int var = __ffs((int)m) - 1;
+        T* t = q.xs + var * (int)(kRowBytes / sizeof(T));
+        if (*t != T(0)) atomicAdd(q.gX + n * q.n_x + var, *t);
+        *t = T(0);
+      }
     }
     if (err && valid) {
       const int64_t kk = kMode == kFlat ? p - n * q.K : q.set, pchunks = (q.N + 31) / 32;
@@ -361,7 +385,8 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
   const int64_t total = N * K, rs = total * es;      // values per node, elements per node
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const unsigned below = (1u << lane) - 1u;
-  const AdjLayout ly = adjoint_layout<T>(Lhi, K, nwarp, !cache);
+  const int xrows = gX ? x_sum_rows(n_x) : 0;
+  const AdjLayout ly = adjoint_layout<T>(Lhi, K, nwarp, !cache, xrows);
   const int ncap = ly.ncap;
   uint32_t* tape = reinterpret_cast<uint32_t*>(smem);
   uint4* prog = reinterpret_cast<uint4*>(smem + ly.prog);
@@ -409,6 +434,7 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
       }
       __syncwarp();
       int ncon = 0, nfix = 0, norph = 0;
+      unsigned used = 0;  // variables of the tape
       for (int k0 = 0; k0 < L; k0 += 32) {
         const int k = k0 + lane;
         const int code = k < L ? code_of(tape[k]) : NO_OP;
@@ -416,6 +442,7 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
         const unsigned mc = __ballot_sync(0xffffffffu, con), mf = __ballot_sync(0xffffffffu, fix);
         const bool orph = (con || (var && gX)) && !parent[k];
         const unsigned mo = __ballot_sync(0xffffffffu, orph);
+        used |= __reduce_or_sync(0xffffffffu, var ? 1u << (child0(tape[k]) & 31) : 0u);
         const int j = ncon + __popc(mc & below);
         if (con) {
           cidx[k] = j;
@@ -483,11 +510,13 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
         info[1] = ncon;
         info[2] = norph;
         info[3] = stack ? 1 : 0;
+        info[4] = (int)used;
       }
     }
     __syncthreads();
     const int nop = info[0], ncon = info[1], norph = info[2];
     const bool stack = info[3] != 0;
+    const unsigned xused = xrows ? (unsigned)info[4] : 0u;
     for (int64_t i = threadIdx.x; i < (int64_t)ncon * K; i += blockDim.x) {
       const int64_t j = i / K, kk = i - j * K;
       cval[i] = __ldg(C + b * c_sb + (int64_t)lcon[j] * c_sm + (set + kk) * c_sk);
@@ -534,8 +563,7 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
               if (v < Vp) crow[(j * V + v) * 32 + lane] = (vm >> v & 1u) ? val[v] : T(0);
           }
         };
-        auto add_variable = [&](uint32_t var, const T (&val)[V]) {
-          if (!gXg) return;
+        auto to_grad_x = [&](uint32_t var, const T (&val)[V]) {
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             if ((vm >> v & 1u) && val[v] != T(0)) {
@@ -544,6 +572,24 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
             }
           }
         };
+        unsigned char* const xs = wb + ly.xacc + lane * 16;  // the lane's sums per variable
+        auto add_variable = [&](uint32_t var, const T (&val)[V]) {
+          if (!gXg) return;
+          if (!xrows) return to_grad_x(var, val);
+          T t[V];
+          load16(xs + var * kRowBytes, t);
+#pragma unroll
+          for (int v = 0; v < V; ++v)
+            if (val[v] != T(0)) t[v] = M_<T>::add(t[v], val[v]);
+          store16(xs + var * kRowBytes, t);
+        };
+        auto clear_variables = [&]() {
+          T zero[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) zero[v] = T(0);
+          for (unsigned m = xused; m; m &= m - 1) store16(xs + (__ffs((int)m) - 1) * kRowBytes, zero);
+        };
+        if (gXg) clear_variables();
         auto place = [&](int64_t round, int64_t& p, unsigned& m) {
           const int64_t q0 = (round * ranks + rank) * Vp;
           p = 32 * (cl + K * q0) + lane;
@@ -613,6 +659,14 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
                   if (w & (1u << 12)) add_variable(w >> 13, val);
                   else add_constant(w >> 13, val);
                 }
+                if (gXg && xused) {
+                  for (unsigned m = xused; m; m &= m - 1) {
+                    T t[V];
+                    load16(xs + (__ffs((int)m) - 1) * kRowBytes, t);
+                    to_grad_x((uint32_t)(__ffs((int)m) - 1), t);
+                  }
+                  clear_variables();
+                }
                 if (__any_sync(0xffffffffu, ep != 0)) {
 #pragma unroll
                   for (int v = 0; v < V; ++v) {
@@ -666,6 +720,7 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
           q.nq = nq; q.rounds = rounds;
           q.tape = tape; q.prog = prog; q.orphan = orphan; q.cidx = cidx; q.lcon = lcon; q.cv = cv; q.accl = accl;
           q.adj = reinterpret_cast<T*>(wb) + lane; q.vals = reinterpret_cast<T*>(wb + ly.vals) + lane;
+          q.xs = reinterpret_cast<T*>(xs); q.xused = xused;
           q.crow = crow; q.crows = smem + ly.warps + ly.crow; q.warp_bytes = ly.warp_bytes; q.errs = errs;
           q.L = L; q.nop = nop; q.norph = norph; q.g0 = g0; q.ng = ng; q.lane = lane; q.rank = rank; q.ranks = ranks;
           general_sweep<T, kMode>(q);
@@ -705,6 +760,7 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
                                cudaStream_t st) {
   auto kern = eval_adjoint_kernel<T, kMode>;
   const void* kp = reinterpret_cast<const void*>(kern);
+  const int xrows = gX ? x_sum_rows(n_x) : 0;
   const int64_t flat = kMode == kFlat ? K : 1, units = kMode == kStrided ? B * K : B;
   const int64_t chunks = (N * flat + 31) / 32;
   const int limit = max_dyn_smem(), sms = device_sm_count(), sm_bytes = max_sm_smem();
@@ -717,7 +773,7 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
   int best_w = 0, per_sm = 0;
   int64_t most_warps = 0;
   for (int w = 1; w <= 8; w *= 2) {
-    const size_t bytes = adjoint_layout<T>(Lhi, flat, w, !cache).bytes;
+    const size_t bytes = adjoint_layout<T>(Lhi, flat, w, !cache, xrows).bytes;
     if (bytes > (size_t)limit) break;
     int blocks = resident_ctas(kp, w * 32, bytes);
     if (blocks < 1) break;
@@ -744,7 +800,7 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
   }
   int64_t blocks = (int64_t)sms * per_sm;
   if (blocks > units) blocks = units;
-  kern<<<(unsigned)blocks, best_w * 32, adjoint_layout<T>(Lhi, flat, best_w, !cache).bytes, st>>>(
+  kern<<<(unsigned)blocks, best_w * 32, adjoint_layout<T>(Lhi, flat, best_w, !cache, xrows).bytes, st>>>(
       X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status);
   return launch_check("eval_adjoint_kernel");
 }
@@ -755,8 +811,9 @@ static int launch_backward_class(const T* X, int64_t N, int64_t n_x, const uint3
                                  int64_t c_sb, int64_t c_sm, int64_t c_sk, int64_t K, const T* cache, const T* gout,
                                  T* gC, T* gX, int32_t* status, cudaStream_t st) {
 #define SR_ADJ_ARGS X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status, st
+  const int xrows = gX ? x_sum_rows(n_x) : 0;
   if (K == 1) return launch_adjoint_mode<T, kSingle>(SR_ADJ_ARGS);
-  if (K <= 64 && adjoint_layout<T>(Lhi, K, 1, !cache).bytes <= (56u << 10)) return launch_adjoint_mode<T, kFlat>(SR_ADJ_ARGS);
+  if (K <= 64 && adjoint_layout<T>(Lhi, K, 1, !cache, xrows).bytes <= (56u << 10)) return launch_adjoint_mode<T, kFlat>(SR_ADJ_ARGS);
   return launch_adjoint_mode<T, kStrided>(SR_ADJ_ARGS);
 #undef SR_ADJ_ARGS
 }

@@ -58,7 +58,8 @@ __device__ __forceinline__ bool is_op_code(int code) { return code == NO_OP || a
 // that of a stack (a shared or a skipped subtree): such tapes take one row per node.
 // The check: the (right) child of k is k - 1, and a left child is the last node before k
 // whose result sits at the depth of k's own result.  last (L + 1 entries) is scratch.
-__device__ __forceinline__ int stack_rows(const uint32_t* tape, int L, int lane, int* last, int* row) {
+__device__ __forceinline__ int stack_rows(const uint32_t* tape, int L, int lane, int* last, int* row,
+                                          int* depth = nullptr) {
   const unsigned below = (1u << lane) - 1u, upto = below | (1u << lane);
   for (int d = lane; d <= L; d += 32) last[d] = -1;
   __syncwarp();
@@ -92,6 +93,7 @@ __device__ __forceinline__ int stack_rows(const uint32_t* tape, int L, int lane,
     S = __shfl_sync(0xffffffffu, s, end);
     D = __shfl_sync(0xffffffffu, r, end);
   }
+  if (depth) *depth = S;  // entries that are left (1: a single tree)
   return ok ? most : -1;
 }
 

@@ -38,8 +38,7 @@
 // NaN when the virtual slot was poisoned.
 #include <cstdint>
 
-#include "sr_common.cuh"
-#include "sr_ops.cuh"
+#include "sr_eval.cuh"
 
 namespace sr {
 
@@ -142,7 +141,7 @@ __host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rm
   l.last = l.adj_of + 4u * (uint32_t)n;
   l.flags = l.last + 4u * (uint32_t)n;
   l.frees = l.flags + 4u * (uint32_t)n;
-  const size_t scratch = 4 * n * 4 + 4 * (size_t)(l.Rmax > Lmax ? l.Rmax : Lmax);
+  const size_t scratch = 4 * n * 4 + 4 * (size_t)((l.Rmax > Lmax ? l.Rmax : Lmax) + 1);
   size_t total = (size_t)W * l.warp_bytes;
   if (total < scratch) total = scratch;
   l.bytes = p + fit_align16(total);
@@ -1037,10 +1036,13 @@ __device__ __forceinline__ bool problem_fits(const FitArgs& A, int64_t b, int L,
 // own) keeps its row for the whole pass; the others give it up after their last parent's
 // forward step.  An operator's adjoint holds a row from the sweep of its first parent to its
 // own.  The rows that come and go in the forward pass and those of the reverse sweep are the
-// same ones.  Rows are taken from a stack, so the assignment is the same in every run.  This
-// takes 38 rows for the ragged workload's tapes instead of the 43 + 12 of a value row per operator
+// same ones.  One lane walks the tape and takes rows from a stack; with kCount the rows of a
+// single tree in stack order are counted by all lanes instead (stack_rows).  The screening
+// kernel, which runs a pass or two per problem, counts (2048 problems of two starts: 237 us
+// with the walk, 147 us); the fit kernel, which runs tens of closures, walks, because the
+// larger code costs its closures 3%.  The assignment takes 38 rows for the ragged workload's tapes instead of the 43 + 12 of a value row per operator
 // beside the adjoint rows, which is what lets two CTAs with two chunks per warp onto an SM.
-template <int V, int U>
+template <int V, int U, bool kCount>
 __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& S, const Layout& l, int64_t b, int L,
                                               int lane, int warp) {
   if (warp == 0) {
@@ -1102,7 +1104,19 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
       kept += __popc(mk);
     }
     __syncwarp();
-    if (lane == 0) {  // one row per distinct variable, in order of first use
+    // one row per distinct variable
+    if (kCount && A.n_x <= 32) {
+      unsigned used = 0;
+      for (int k0 = 0; k0 < L; k0 += 32) {
+        const int k = k0 + lane;
+        const bool var = k < L && code_of(S.tape[k]) == VAR;
+        used |= __reduce_or_sync(0xffffffffu, var ? 1u << child0(S.tape[k]) : 0u);
+      }
+      for (int k = lane; k < L; k += 32)
+        if (code_of(S.tape[k]) == VAR) S.node_slot[k] = __popc(used & ((1u << child0(S.tape[k])) - 1u));
+      if (used >> lane & 1u) S.rowvar[__popc(used & ((1u << lane) - 1u))] = lane;
+      if (lane == 0) S.info[kVars] = __popc(used);
+    } else if (lane == 0) {
       int nvr = 0;
       for (int k = 0; k < L; ++k) {
         const uint32_t d = S.tape[k];
@@ -1114,6 +1128,59 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
         S.node_slot[k] = r;
       }
       S.info[kVars] = nvr;
+    }
+    __syncwarp();
+    const int R = L - 1;
+    const uint32_t row = 128u * (uint32_t)l.P, sums = 32u * (uint32_t)l.V;
+    int depth = 0, waiting = -1;
+    if (kCount) waiting = stack_rows(S.tape, L, lane, frees, adj_of, &depth);
+    __syncwarp();
+    if (kCount && waiting >= 0 && depth == 1) {
+      // a single tree in stack order: what waits is what the evaluation stack holds, so a
+      // row is a count of the entries below (a node's own row is also its left operand's: each
+      // lane has read what it holds before it writes there)
+      int T = 0, most = 0;
+      for (int k0 = 0; k0 < L; k0 += 32) {
+        const int k = k0 + lane;
+        const uint32_t d = k < L ? S.tape[k] : 0u;
+        const int ar = k < L ? arity_of(code_of(d)) : 0;
+        auto temp = [&](int c) { return is_operator_node(code_of(S.tape[c])) && !(flags[c] & 1); };
+        int delta = k < L && temp(k) ? 1 : 0;
+        if (ar >= 1 && temp(child0(d))) --delta;
+        if (ar == 2 && temp(child1(d))) --delta;
+        const unsigned up = __ballot_sync(0xffffffffu, delta > 0), down = __ballot_sync(0xffffffffu, delta < 0),
+                       two = __ballot_sync(0xffffffffu, delta < -1), upto = (2u << lane) - 1u;
+        const int t = T + __popc(up & upto) - __popc(down & upto) - __popc(two & upto);
+        most = max(most, __reduce_max_sync(0xffffffffu, k < L ? t : 0));
+        if (k < L && row_of[k] < 0) row_of[k] = kept + t - 1;  // (of no use to a leaf)
+        T = __shfl_sync(0xffffffffu, t, 31);
+      }
+      __syncwarp();
+      for (int k = lane; k < L; k += 32) {
+        const uint32_t d = S.tape[k];
+        const int code = code_of(d);
+        if (!is_operator_node(code)) continue;
+        const int ar = arity_of(code);
+        auto goes_to = [&](int c) -> uint32_t {
+          const int cc = code_of(S.tape[c]);
+          if (cc == LEARNABLE) return (kDstSum << 30) | ((uint32_t)S.node_slot[c] * sums);
+          return is_operator_node(cc) ? (kDstFirst << 30) | ((uint32_t)(kept + adj_of[c]) * row) : 0u;
+        };
+        const int i = S.node_slot[k];
+        S.rev[i].x = (uint32_t)dense_op(code);
+        S.rev[i].w = (uint32_t)(kept + adj_of[k]) * row;
+        S.dst[i] = make_uint2(ar >= 1 ? goes_to(child0(d)) : 0u, ar == 2 ? goes_to(child1(d)) : 0u);
+      }
+      if (lane == 0) {
+        const int rc = code_of(S.tape[R]);
+        S.info[kRootDst] = is_operator_node(rc) ? (int)((kDstFirst << 30) | ((uint32_t)(kept + adj_of[R]) * row))
+                           : rc == LEARNABLE    ? (int)((kDstSum << 30) | ((uint32_t)S.node_slot[R] * sums))
+                                                : 0;
+        S.info[kTooFew] = kept + max(waiting, most) > l.Rmax || waiting > A.Amax ? 1 : 0;
+      }
+    } else if (lane == 0) {
+      if (kCount)
+        for (int k = 0; k < L; ++k) adj_of[k] = -1;  // stack_rows has written there
       bool over = kept > l.Rmax;
       const int room = l.Rmax - kept;
       // values that the reverse sweep does not read
@@ -1139,12 +1206,10 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
       top = 0;
       const int arooms = room < A.Amax ? room : A.Amax;
       for (int r = arooms - 1; r >= 0; --r) frees[top++] = kept + r;
-      const int R = L - 1;
       if (!over && is_operator_node(code_of(S.tape[R]))) {
         if (top > 0) adj_of[R] = frees[--top];
         else over = true;
       }
-      const uint32_t row = 128u * (uint32_t)l.P, sums = 32u * (uint32_t)l.V;
       for (int k = R; k >= 0 && !over; --k) {
         const uint32_t d = S.tape[k];
         const int code = code_of(d);
@@ -1178,15 +1243,16 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
         S.dst[i] = make_uint2(to[0], to[1]);
       }
       const int rc = code_of(S.tape[R]);
-      S.info[kOps] = nop;
       S.info[kRootDst] = is_operator_node(rc) ? (int)((kDstFirst << 30) | ((uint32_t)(over ? 0 : adj_of[R]) * row))
                          : rc == LEARNABLE    ? (int)((kDstSum << 30) | ((uint32_t)S.node_slot[R] * sums))
                                               : 0;
-      S.info[kSharedConst] = shared_const ? 1 : 0;
       S.info[kTooFew] = over ? 1 : 0;
     }
+    if (lane == 0) {
+      S.info[kOps] = nop;
+      S.info[kSharedConst] = shared_const ? 1 : 0;
+    }
     __syncwarp();
-    const uint32_t row = 128u * (uint32_t)l.P;
     if (S.info[kTooFew] == 0) {
       for (int k = lane; k < L; k += 32) {
         const uint32_t d = S.tape[k];
@@ -1266,7 +1332,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
     P.nslots = P.K + (P.has_virtual ? 1 : 0);
     const int L = P.root + 1;
     // a caller's max_len / max_consts / max_operators / max_live too small: not fitted
-    if (!problem_fits(A, P.b, L, P.K, lane) || !stage_problem<V, U>(A, S, l, P.b, L, lane, warp)) {
+    if (!problem_fits(A, P.b, L, P.K, lane) || !stage_problem<V, U, false>(A, S, l, P.b, L, lane, warp)) {
       if (warp == 0) {
         const float qnan = __int_as_float(0x7fffffff);
         for (int64_t k = lane; k < A.M; k += 32) A.C_out[P.b * A.c_sb + k * A.c_sm] = A.C_init[P.b * A.c_sb + k * A.c_sm];
@@ -1641,7 +1707,7 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
     const int L = A.meta[b * 4 + 1] + 1;
     const int Kc = A.meta[b * 4 + 2];
     // a caller's max_len / max_consts / max_operators / max_live too small
-    if (!problem_fits(A, b, L, Kc, lane) || !stage_problem<V, U>(A, S, l, b, L, lane, warp)) {
+    if (!problem_fits(A, b, L, Kc, lane) || !stage_problem<V, U, true>(A, S, l, b, L, lane, warp)) {
       if (threadIdx.x == 0) {
         report(A.status, kStatusTapeExceedsLaunch);
         for (int64_t k = 0; k < K; ++k) loss_out[b * K + k] = __int_as_float(0x7fffffff);
@@ -1675,80 +1741,138 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
 // What stage_problem's row assignment needs per tape, the batch's largest into stats[5]
 // (operator adjoints live at once) and stats[6] (rows in all: the values that the reverse
 // sweep reads, plus the larger of the adjoints and of the other values live at once).  One
-// thread per tape; tapes longer than 128 nodes to the root count all their operator nodes
-// (a bound).
-__global__ void __launch_bounds__(64) tape_live_kernel(const uint32_t* __restrict__ desc,
-                                                       const int32_t* __restrict__ meta, int64_t B, int64_t M,
-                                                       int32_t* __restrict__ stats) {
-  int best = 0, best_rows = 0;
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < B) {
-    const int L = meta[b * 4 + 1] + 1;
-    const uint32_t* d = desc + b * M;
-    if (L > 128) {
-      for (int k = 0; k < L; ++k) best += is_operator_node(code_of(d[k])) ? 1 : 0;
-      best_rows = 2 * best;
-    } else {
-      uint64_t held[2] = {0ull, 0ull}, kept[2] = {0ull, 0ull}, used[2] = {0ull, 0ull};
-      auto has = [](const uint64_t(&m)[2], int k) { return (m[k >> 6] >> (k & 63)) & 1ull; };
-      auto set = [](uint64_t(&m)[2], int k) { m[k >> 6] |= 1ull << (k & 63); };
-      int cur = 0;
-      auto take = [&](int k) {
-        set(held, k);
-        ++cur;
-        best = cur > best ? cur : best;
-      };
-      const int R = L - 1;
-      if (is_operator_node(code_of(d[R]))) take(R);
-      // the reverse sweep: adjoints, and which values it reads; going backwards, a value whose
-      // last parent is met comes alive and dies at its own node
-      int temps = 0, most = 0;
-      for (int k = R; k >= 0; --k) {
-        const uint32_t w = d[k];
-        const int code = code_of(w);
-        if (!is_operator_node(code)) continue;
-        if (!has(held, k)) take(k);
-        --cur;
-        if (code == EXP) set(kept, k);
-        const int ar = arity_of(code);
-        const bool reads = adjoint_reads_operands(code);
-        for (int j = 0; j < ar; ++j) {
-          const int c = j == 0 ? child0(w) : child1(w);
-          if (!is_operator_node(code_of(d[c]))) continue;
-          if (!has(held, c)) take(c);
-          if (reads) set(kept, c);
-        }
+// warp per tape.  For a single tree in stack order the values and adjoints that wait are those
+// on the evaluation stack, so both counts are prefix sums (stack_rows); other tapes are walked
+// by one lane (2048 tapes of up to 64 nodes: 6 us this way, 56 us with a thread walking
+// each).  Tapes longer than 128 nodes to the root count all their operator nodes (a bound).
+constexpr int kLiveNodes = 128, kLiveWarps = 4;
+
+// The walk (see above): both counts of a tape whose words are d.
+__device__ __noinline__ void live_walk(const uint32_t* d, int L, int& best, int& rows) {
+    uint64_t held[2] = {0ull, 0ull}, kept[2] = {0ull, 0ull}, used[2] = {0ull, 0ull};
+    auto has = [](const uint64_t(&m)[2], int k) { return (m[k >> 6] >> (k & 63)) & 1ull; };
+    auto set = [](uint64_t(&m)[2], int k) { m[k >> 6] |= 1ull << (k & 63); };
+    int cur = 0;
+    auto take = [&](int k) {
+      set(held, k);
+      ++cur;
+      best = cur > best ? cur : best;
+    };
+    const int R = L - 1;
+    if (is_operator_node(code_of(d[R]))) take(R);
+    // the reverse sweep: adjoints, and which values it reads; going backwards, a value whose
+    // last parent is met comes alive and dies at its own node
+    int temps = 0, most = 0;
+    for (int k = R; k >= 0; --k) {
+      const uint32_t w = d[k];
+      const int code = code_of(w);
+      if (!is_operator_node(code)) continue;
+      if (!has(held, k)) take(k);
+      --cur;
+      if (code == EXP) set(kept, k);
+      const int ar = arity_of(code);
+      const bool reads = adjoint_reads_operands(code);
+      for (int j = 0; j < ar; ++j) {
+        const int c = j == 0 ? child0(w) : child1(w);
+        if (!is_operator_node(code_of(d[c]))) continue;
+        if (!has(held, c)) take(c);
+        if (reads) set(kept, c);
       }
-      // the other values: alive from their node to their last parent (a node's own comes after
-      // its operands' go)
-      for (int k = R; k >= 0; --k) {
-        const uint32_t w = d[k];
-        const int code = code_of(w);
-        if (!is_operator_node(code)) continue;
-        if (!has(kept, k)) {
-          // at k its value is alive: counted since its last parent, or for this step alone
-          const bool waits = has(used, k) || k == R;
-          if (k == R) ++temps;
-          const int now = temps + (waits ? 0 : 1);
-          most = now > most ? now : most;
-          if (waits) --temps;
-        }
-        const int ar = arity_of(code);
-        for (int j = 0; j < ar; ++j) {
-          const int c = j == 0 ? child0(w) : child1(w);
-          if (!is_operator_node(code_of(d[c])) || has(kept, c) || has(used, c)) continue;
-          set(used, c);
-          ++temps;
-        }
-        most = temps > most ? temps : most;
-      }
-      const int keep = __popcll(kept[0]) + __popcll(kept[1]);
-      best_rows = keep + (best > most ? best : most);
     }
+    // the other values: alive from their node to their last parent (a node's own comes after
+    // its operands' go)
+    for (int k = R; k >= 0; --k) {
+      const uint32_t w = d[k];
+      const int code = code_of(w);
+      if (!is_operator_node(code)) continue;
+      if (!has(kept, k)) {
+        // at k its value is alive: counted since its last parent, or for this step alone
+        const bool waits = has(used, k) || k == R;
+        if (k == R) ++temps;
+        const int now = temps + (waits ? 0 : 1);
+        most = now > most ? now : most;
+        if (waits) --temps;
+      }
+      const int ar = arity_of(code);
+      for (int j = 0; j < ar; ++j) {
+        const int c = j == 0 ? child0(w) : child1(w);
+        if (!is_operator_node(code_of(d[c])) || has(kept, c) || has(used, c)) continue;
+        set(used, c);
+        ++temps;
+      }
+      most = temps > most ? temps : most;
+    }
+  const int keep = __popcll(kept[0]) + __popcll(kept[1]);
+  rows = keep + (best > most ? best : most);
+}
+
+__global__ void __launch_bounds__(kLiveWarps * 32) tape_live_kernel(const uint32_t* __restrict__ desc,
+                                                                   const int32_t* __restrict__ meta, int64_t B,
+                                                                   int64_t M, int32_t* __restrict__ stats) {
+  __shared__ uint32_t words[kLiveWarps][kLiveNodes];
+  __shared__ int last_[kLiveWarps][kLiveNodes + 1], kept_[kLiveWarps][kLiveNodes];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t* d = words[warp];
+  int *last = last_[warp], *kept = kept_[warp];
+  int best = 0, best_rows = 0;
+  for (int64_t b = (int64_t)blockIdx.x * kLiveWarps + warp; b < B; b += (int64_t)gridDim.x * kLiveWarps) {
+    const int L = meta[b * 4 + 1] + 1;
+    int live = 0, rows = 0;
+    if (L > kLiveNodes) {
+      for (int k0 = 0; k0 < L; k0 += 32) {
+        const int k = k0 + lane;
+        live += __popc(__ballot_sync(0xffffffffu, k < L && is_operator_node(code_of(desc[b * M + k]))));
+      }
+      rows = 2 * live;
+    } else {
+      __syncwarp();
+      for (int k = lane; k < L; k += 32) d[k] = desc[b * M + k];
+      __syncwarp();
+      int depth = 0;
+      live = stack_rows(d, L, lane, last, kept, &depth);
+      if (live >= 0 && depth == 1) {
+        __syncwarp();
+        for (int k = lane; k < L; k += 32) kept[k] = code_of(d[k]) == EXP;
+        __syncwarp();
+        for (int k = lane; k < L; k += 32) {
+          const int code = code_of(d[k]), ar = arity_of(code);
+          if (!adjoint_reads_operands(code)) continue;
+          if (ar >= 1) kept[child0(d[k])] = 1;
+          if (ar == 2) kept[child1(d[k])] = 1;
+        }
+        __syncwarp();
+        int T = 0, most = 0, keep = 0;
+        for (int k0 = 0; k0 < L; k0 += 32) {
+          const int k = k0 + lane;
+          const uint32_t w = k < L ? d[k] : 0u;
+          const int ar = k < L ? arity_of(code_of(w)) : 0;
+          auto temp = [&](int c) { return is_operator_node(code_of(d[c])) && !kept[c]; };
+          const bool op = k < L && is_operator_node(code_of(w));
+          int delta = op && !kept[k] ? 1 : 0;
+          if (ar >= 1 && temp(child0(w))) --delta;
+          if (ar == 2 && temp(child1(w))) --delta;
+          const unsigned up = __ballot_sync(0xffffffffu, delta > 0), down = __ballot_sync(0xffffffffu, delta < 0),
+                         two = __ballot_sync(0xffffffffu, delta < -1), upto = (2u << lane) - 1u;
+          const int t = T + __popc(up & upto) - __popc(down & upto) - __popc(two & upto);
+          most = max(most, __reduce_max_sync(0xffffffffu, k < L ? t : 0));
+          keep += __popc(__ballot_sync(0xffffffffu, op && kept[k < L ? k : 0]));
+          T = __shfl_sync(0xffffffffu, t, 31);
+        }
+        rows = keep + max(live, most);
+      } else {
+        __syncwarp();
+        if (lane == 0) {
+          live = 0;
+          live_walk(d, L, live, rows);
+        }
+        live = __shfl_sync(0xffffffffu, live, 0);
+        rows = __shfl_sync(0xffffffffu, rows, 0);
+      }
+    }
+    best = max(best, live);
+    best_rows = max(best_rows, rows);
   }
-  best = __reduce_max_sync(0xffffffffu, best);
-  best_rows = __reduce_max_sync(0xffffffffu, best_rows);
-  if ((threadIdx.x & 31) == 0 && best_rows > 0) {
+  if (lane == 0 && best_rows > 0) {
     atomicMax(stats + 5, best);
     atomicMax(stats + 6, best_rows);
   }
@@ -1947,8 +2071,10 @@ int sr_tape_live_rows(const uint32_t* desc, const int32_t* meta, int64_t B, int6
   if (M > sr::kMaxNodes) { sr::set_error("tapes longer than %d nodes are not supported", sr::kMaxNodes); return SR_ERR_UNSUPPORTED; }
   if (B == 0 || M == 0) return SR_OK;
   if (!desc || !meta || !stats) { sr::set_error("null pointer argument"); return SR_ERR_INVALID_ARGUMENT; }
-  const int64_t blocks = (B + 63) / 64;
-  sr::tape_live_kernel<<<(unsigned)blocks, 64, 0, sr::as_stream(stream)>>>(desc, meta, B, M, stats);
+  int64_t blocks = (B + sr::kLiveWarps - 1) / sr::kLiveWarps;
+  const int64_t cap = (int64_t)sr::device_sm_count() * 16;
+  if (blocks > cap) blocks = cap;
+  sr::tape_live_kernel<<<(unsigned)blocks, sr::kLiveWarps * 32, 0, sr::as_stream(stream)>>>(desc, meta, B, M, stats);
   return sr::launch_check("tape_live_kernel");
 }
 
@@ -2005,20 +2131,26 @@ int sr_fit_screen(const float* X, int64_t N, int64_t n_x, const float* Y, const 
   A.objective = o.objective;
   A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
   A.status = status;
-  void* k = sh.V == 1 ? (sh.U == 2 ? reinterpret_cast<void*>(fit_screen_kernel<1, 2>)
-                                   : reinterpret_cast<void*>(fit_screen_kernel<1, 1>))
+  // a forward pass alone gains less from two chunks at once than it loses with the CTAs that
+  // the doubled rows displace (2048 problems of two starts, N = 512: 280 us against 237)
+  void* k = sh.V == 1 ? reinterpret_cast<void*>(fit_screen_kernel<1, 1>)
                       : (sh.V == 2 ? reinterpret_cast<void*>(fit_screen_kernel<2, 1>)
                                    : reinterpret_cast<void*>(fit_screen_kernel<4, 1>));
+  const size_t smem = fit_layout(Lmax, sh.Imax, sh.Rmax, max_consts, sh.V, 1, sh.warps, sh.VR).bytes;
   int dev = 0, optin = 0;
   if (cuda_check(cudaGetDevice(&dev), "cudaGetDevice") ||
       cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory limit") ||
       cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin), "screen smem attribute"))
     return SR_ERR_CUDA;
+  const int per_sm = resident_ctas(k, sh.warps * 32, smem);
+  int64_t blocks = (int64_t)device_sm_count() * (per_sm > 0 ? per_sm : 1);
+  if (o.grid_blocks > 0) blocks = o.grid_blocks;
+  if (blocks > B) blocks = B;
   const float* Cs = C_sets;
   int64_t csk = c_sk, kk = K;
   float* lo = loss_out;
   void* args[] = {&A, &Cs, &csk, &kk, &lo};
-  return cuda_check(cudaLaunchKernel(k, dim3(sh.blocks), dim3(sh.warps * 32), args, sh.smem, as_stream(stream)),
+  return cuda_check(cudaLaunchKernel(k, dim3((unsigned)blocks), dim3(sh.warps * 32), args, smem, as_stream(stream)),
                     "fit_screen_kernel");
 }
 

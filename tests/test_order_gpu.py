@@ -1,0 +1,32 @@
+"""The work order and the error-word summary against numpy."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("column", [0, 1])
+@pytest.mark.parametrize("B,M", [(1, 1), (31, 3), (1023, 64), (1024, 64), (1025, 64), (5000, 4095), (70001, 48)])
+def test_tape_order_lists_every_tape_by_falling_length(B, M, column):
+    from cudasymbolicregression_gb300 import _lib
+    rng = np.random.default_rng([B, M, column])
+    meta = np.zeros((B, 4), np.int32)
+    meta[:, column] = rng.integers(0, M + 1 - column, size=B)
+    m = torch.as_tensor(meta).cuda()
+    order = torch.full((B,), -1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().sr_tape_order(_lib.ptr(m), B, M, column, _lib.ptr(order), _lib.stream_ptr(m.device)), "order")
+    o = order.cpu().numpy()
+    assert np.array_equal(np.sort(o), np.arange(B))
+    assert (np.diff(meta[o, column]) <= 0).all()
+
+
+@pytest.mark.parametrize("n", [0, 1, 255, 2048, 2049, 300001])
+def test_any_nonzero(n):
+    from cudasymbolicregression_gb300 import _lib
+    w = torch.zeros(n, dtype=torch.int64, device="cuda")
+    assert not _lib.any_nonzero(w)
+    for i in {0, n // 2, n - 1} if n else ():
+        w[i] = 1 << 40
+        assert _lib.any_nonzero(w)
+        w[i] = 0

@@ -59,6 +59,22 @@ class MlpEpilogue(ctypes.Structure):
     ]
 
 
+class MlpNet(ctypes.Structure):
+    """Mirror of ``sr_mlp_net``."""
+    _fields_ = [
+        ("w", vp * 5), ("w_t", vp * 5), ("b", vp * 5),
+        ("hist", vp), ("hist_t", vp), ("x0", vp), ("x0_t", vp), ("h", vp * 3), ("h_t", vp * 3), ("out", vp),
+        ("d_out", vp), ("d_out_t", vp), ("dz", vp * 3), ("dz_t", vp * 3), ("dx0_t", vp),
+        ("part", vp), ("gw", vp * 5), ("gb", vp * 5), ("ld", i64), ("splits", i32), ("status", vp),
+    ]
+
+
+class MlpAdamTensor(ctypes.Structure):
+    """Mirror of ``sr_mlp_adam_tensor``."""
+    _fields_ = [("w", vp), ("g", vp), ("m", vp), ("v", vp), ("rows", i64), ("cols", i64), ("w_bf16", vp),
+                ("w_t_bf16", vp), ("weight_decay", ctypes.c_float)]
+
+
 MLP_EPI_RELU, MLP_EPI_LINEAR, MLP_EPI_F32, MLP_EPI_RELU_GRAD, MLP_EPI_SPLIT_F32 = 0, 1, 2, 3, 4
 MLP_VOCAB, MLP_EMB, MLP_FEATS, MLP_PROJ, MLP_IN = 64, 64, 32, 28, 128
 MLP_TIMEOUT = 601
@@ -108,6 +124,13 @@ _SIGS = {
     "sr_const_scatter": ([vp, i64, i64, i64, i64, vp, vp, vp, vp], ctypes.c_int),
     "sr_mlp_gemm": ([vp, i64, i64, i64, vp, i64, i64, ctypes.POINTER(MlpEpilogue), vp, vp], ctypes.c_int),
     "sr_mlp_gemm_splits_used": ([i64, i32], ctypes.c_int),
+    "sr_mlp_net_forward": ([ctypes.POINTER(MlpNet), i64, vp], ctypes.c_int),
+    "sr_mlp_net_backward": ([ctypes.POINTER(MlpNet), i64, vp], ctypes.c_int),
+    "sr_mlp_adam_all": ([ctypes.POINTER(MlpAdamTensor), i32, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                         ctypes.c_float, i32, vp], ctypes.c_int),
+    "sr_mlp_place_constants": ([vp, i64, i64, i64, i64, vp, i64, i32, ctypes.c_float, vp, vp, i64, i64, vp],
+                               ctypes.c_int),
+    "sr_mlp_pick_start": ([vp, vp, i64, i64, i64, vp, vp], ctypes.c_int),
     "sr_mlp_random_features": ([vp, i64, i64, vp, vp, vp, vp], ctypes.c_int),
     "sr_mlp_features": ([vp, i64, i64, i64, i64, vp, i64, vp, vp, vp, i64, vp, vp, vp, vp], ctypes.c_int),
     "sr_mlp_loss": ([vp, i64, i64, vp, vp, i32, ctypes.c_float, vp, vp, i64, vp, i64, vp], ctypes.c_int),

@@ -76,7 +76,8 @@ class _Workspace:
         self.dz = {i: (z(R, HIDDEN), z(HIDDEN, R)) for i in (1, 2, 3)}
         self.dx0_t = z(IN, R)
         self.splits = splits
-        self.part = f(splits, HIDDEN, HIDDEN)
+        # partial sums of every weight gradient (row counts padded to whole tiles)
+        self.part = f(splits * (2 * HIDDEN * HIDDEN + HIDDEN * IN + TILE * HIDDEN + TILE * VOCAB))
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
 
 
@@ -128,25 +129,19 @@ class WarmStartMLP:
     def _stream(self):
         return _lib.stream_ptr(self.device)
 
-    def _gemm(self, A, rows, k, lda, W, n, ldw, ws, **epi):
-        e = _lib.MlpEpilogue()
-        e.epilogue = epi.get("mode", _lib.MLP_EPI_LINEAR)
-        e.splits = epi.get("splits", 1)
-        e.bias = _p(epi.get("bias"))
-        e.gate = _p(epi.get("gate"))
-        e.ld_gate = epi.get("ld_gate", 0)
-        e.out = _p(epi.get("out"))
-        e.ld_out = epi.get("ld_out", 0)
-        e.out_col0 = epi.get("out_col0", 0)
-        e.out_t = _p(epi.get("out_t"))
-        e.ld_out_t = epi.get("ld_out_t", 0)
-        e.out_t_row0 = epi.get("out_t_row0", 0)
-        e.out_f32 = _p(epi.get("out_f32"))
-        e.ld_out_f32 = epi.get("ld_out_f32", 0)
-        e.split_stride = epi.get("split_stride", 0)
-        rc = self._lib().sr_mlp_gemm(_p(A), rows, k, lda, _p(W), n, ldw, ctypes.byref(e), _p(ws.status),
-                                     self._stream())
-        _lib.check(rc, "sr_mlp_gemm")
+    def _net(self, ws) -> "_lib.MlpNet":
+        """The buffers of a forward or backward pass, as the library takes them."""
+        n = _lib.MlpNet()
+        for i, name in enumerate(LAYERS):
+            n.w[i], n.w_t[i], n.gw[i] = (t[name].data_ptr() for t in (self.w_bf, self.w_bf_t, self.gw))
+            if name in self.b:
+                n.b[i], n.gb[i] = self.b[name].data_ptr(), self.gb[name].data_ptr()
+        for i in range(3):
+            (n.h[i], n.h_t[i]), (n.dz[i], n.dz_t[i]) = (tuple(t.data_ptr() for t in d[i + 1]) for d in (ws.h, ws.dz))
+        for name in ("hist", "hist_t", "x0", "x0_t", "out", "d_out", "d_out_t", "dx0_t", "part", "status"):
+            setattr(n, name, getattr(ws, name).data_ptr())
+        n.ld, n.splits = ws.R, ws.splits
+        return n
 
     def _pack(self):
         L = self._lib()
@@ -178,40 +173,11 @@ class WarmStartMLP:
                                      _p(ws.x0), _p(ws.x0_t), _p(ws.feats), self._stream()), "sr_mlp_features")
 
     def forward_ws(self, ws: _Workspace, rows: int):
-        R, ld = _pad_rows(rows), ws.R  # rows processed; leading dimension of the transposed buffers
-        # embedding of the bag of tokens -> x0[:, :64] and x0_t[:64]
-        self._gemm(ws.hist, R, VOCAB, VOCAB, self.w_bf["E"], EMB, VOCAB, ws, mode=_lib.MLP_EPI_LINEAR,
-                   out=ws.x0, ld_out=IN, out_col0=0, out_t=ws.x0_t, ld_out_t=ld, out_t_row0=0)
-        prev, k = ws.x0, IN
-        for i, name in ((1, "W1"), (2, "W2"), (3, "W3")):
-            h, h_t = ws.h[i]
-            self._gemm(prev, R, k, k, self.w_bf[name], HIDDEN, k, ws, mode=_lib.MLP_EPI_RELU, bias=self.b[name],
-                       out=h, ld_out=HIDDEN, out_t=h_t, ld_out_t=ld)
-            prev, k = h, HIDDEN
-        self._gemm(prev, R, HIDDEN, HIDDEN, self.w_bf["W4"], OUT_PAD, HIDDEN, ws, mode=_lib.MLP_EPI_F32,
-                   bias=self.b["W4"], out_f32=ws.out, ld_out_f32=OUT_PAD)
+        _lib.check(self._lib().sr_mlp_net_forward(ctypes.byref(self._net(ws)), _pad_rows(rows), self._stream()),
+                   "sr_mlp_net_forward")
         return ws.out[:rows, :N_OUT]
 
     # ---- backward ------------------------------------------------------------------
-    def _weight_grad(self, A_t, a_rows, B_t, n, R, ws, dst):
-        """dst (a_rows_real x n) = A_t (a_rows x R) . B_t (n x R)^T with a split reduction
-        (A_t and B_t have leading dimension ws.R)."""
-        L = self._lib()
-        splits = L.sr_mlp_gemm_splits_used(R, ws.splits)
-        stride = TILE * ((a_rows + TILE - 1) // TILE) * n
-        part = ws.part.view(-1)[: splits * stride].view(splits, -1)
-        e = _lib.MlpEpilogue()
-        e.epilogue = _lib.MLP_EPI_SPLIT_F32
-        e.splits = ws.splits
-        e.out_f32 = _p(part)
-        e.ld_out_f32 = n
-        e.split_stride = stride
-        _lib.check(L.sr_mlp_gemm(_p(A_t), a_rows, R, ws.R, _p(B_t), n, ws.R, ctypes.byref(e), _p(ws.status),
-                                 self._stream()), "sr_mlp_gemm")
-        count = dst.numel()
-        _lib.check(L.sr_mlp_reduce_splits(_p(part), splits, count, stride, _p(dst), self._stream()),
-                   "sr_mlp_reduce_splits")
-
     def backward_ws(self, ws: _Workspace, rows: int, out_grad: torch.Tensor | None = None):
         """Gradients into self.gw / self.gb of the mean over rows of sum_j mask (out - target)^2,
         or, with out_grad (rows, N_OUT) fp32 given, of a loss whose gradient with
@@ -227,42 +193,22 @@ class WarmStartMLP:
             g[:rows] = out_grad
             _lib.check(L.sr_mlp_output_grad(_p(g), R, N_OUT, N_OUT, 1.0 / max(rows, 1), _p(ws.d_out), OUT_PAD,
                                             _p(ws.d_out_t), ld, st), "sr_mlp_output_grad")
-        # output layer
-        self._weight_grad(ws.d_out_t, TILE, ws.h[3][1], HIDDEN, R, ws, self.gw["W4"])
-        _lib.check(L.sr_mlp_colsum(_p(ws.d_out_t), OUT_PAD, R, ld, _p(self.gb["W4"]), st), "sr_mlp_colsum")
-        dz_prev, k_prev = ws.d_out, OUT_PAD
-        for i, name, below in ((3, "W3", 2), (2, "W2", 1), (1, "W1", 0)):
-            up = {3: "W4", 2: "W3", 1: "W2"}[i]
-            dz, dz_t = ws.dz[i]
-            h = ws.h[i][0]
-            # dh_i = dz_{i+1} . W_{i+1}, gated by ReLU'(h_i)
-            self._gemm(dz_prev, R, k_prev, k_prev, self.w_bf_t[up], HIDDEN, k_prev, ws,
-                       mode=_lib.MLP_EPI_RELU_GRAD, gate=h, ld_gate=HIDDEN, out=dz, ld_out=HIDDEN, out_t=dz_t,
-                       ld_out_t=ld)
-            a_t, n_in = (ws.h[below][1], HIDDEN) if below else (ws.x0_t, IN)
-            self._weight_grad(dz_t, HIDDEN, a_t, n_in, R, ws, self.gw[name])
-            _lib.check(L.sr_mlp_colsum(_p(dz_t), HIDDEN, R, ld, _p(self.gb[name]), st), "sr_mlp_colsum")
-            dz_prev, k_prev = dz, HIDDEN
-        # d x0 = dz_1 . W1 (transposed copy only); its first 64 rows are d(embedding)
-        self._gemm(ws.dz[1][0], R, HIDDEN, HIDDEN, self.w_bf_t["W1"], IN, HIDDEN, ws, mode=_lib.MLP_EPI_LINEAR,
-                   out_t=ws.dx0_t, ld_out_t=ld)
-        gE = torch.empty(TILE, VOCAB, device=self.device)
-        self._weight_grad(ws.dx0_t, TILE, ws.hist_t, VOCAB, R, ws, gE)
-        self.gw["E"].copy_(gE[:EMB])
+        _lib.check(L.sr_mlp_net_backward(ctypes.byref(self._net(ws)), R, st), "sr_mlp_net_backward")
         return ws.row_loss[:rows]
 
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
-        L = self._lib()
         self.step_count += 1
-        st = self._stream()
-        for n in LAYERS:
-            o, i, has_b = LAYERS[n]
-            _lib.check(L.sr_mlp_adam(_p(self.w[n]), _p(self.gw[n]), _p(self.m[n]), _p(self.v[n]), o, i, lr, beta1,
-                                     beta2, eps, weight_decay, self.step_count, _p(self.w_bf[n]),
-                                     _p(self.w_bf_t[n]), st), "sr_mlp_adam")
-            if has_b:
-                _lib.check(L.sr_mlp_adam(_p(self.b[n]), _p(self.gb[n]), _p(self.mb[n]), _p(self.vb[n]), 1, o, lr,
-                                         beta1, beta2, eps, 0.0, self.step_count, None, None, st), "sr_mlp_adam")
+        items = (_lib.MlpAdamTensor * (len(self.w) + len(self.b)))()
+        for k, n in enumerate(list(self.w) + list(self.b)):
+            weight = k < len(self.w)
+            w, g, m, v = (d[n] for d in ((self.w, self.gw, self.m, self.v) if weight else
+                                         (self.b, self.gb, self.mb, self.vb)))
+            rows, cols = w.shape if weight else (1, w.shape[0])
+            items[k] = (w.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), rows, cols,
+                        self.w_bf[n].data_ptr() if weight else None, self.w_bf_t[n].data_ptr() if weight else None,
+                        weight_decay if weight else 0.0)
+        _lib.check(self._lib().sr_mlp_adam_all(items, len(items), lr, beta1, beta2, eps, self.step_count,
+                                               self._stream()), "sr_mlp_adam_all")
 
     def check_status(self):
         if self._ws is not None and int(self._ws.status.item()) != 0:
@@ -285,10 +231,10 @@ class WarmStartMLP:
         """One Adam step on a batch; returns the per-row losses (device tensor)."""
         rows = ops.shape[0]
         ws = self.workspace(rows)
-        ws.target.zero_()
-        ws.mask.zero_()
-        ws.target[:rows] = target
-        ws.mask[:rows] = mask
+        for buf, x in ((ws.target, target), (ws.mask, mask)):
+            buf[:rows] = x
+            if rows < _pad_rows(rows):
+                buf[rows:_pad_rows(rows)] = 0  # the rows that fill the last tile
         self.features(ops, X, Y, ws)
         self.forward_ws(ws, rows)
         loss = self.backward_ws(ws, rows)
@@ -381,9 +327,15 @@ def screened_start(X, Y, ops, ch, C_sets: torch.Tensor) -> torch.Tensor:
     counts as +inf and ties keep the earlier candidate (the plain start first)."""
     from .optimization import screen_starts
     loss = screen_starts(X, Y, ops, ch, C_sets)
-    loss = torch.where(torch.isfinite(loss), loss, torch.full_like(loss, float("inf")))
-    best = torch.argmin(loss, dim=1)
-    return C_sets[best, torch.arange(ops.shape[0], device=ops.device)]
+    K, B, M = C_sets.shape
+    if C_sets.requires_grad and torch.is_grad_enabled():  # a start that autograd can follow
+        loss = torch.where(torch.isfinite(loss), loss, torch.full_like(loss, float("inf")))
+        return C_sets[torch.argmin(loss, dim=1), torch.arange(B, device=ops.device)]
+    Cs = C_sets.contiguous()
+    out = torch.empty((B, M), dtype=Cs.dtype, device=Cs.device)
+    _lib.check(_lib.lib().sr_mlp_pick_start(_p(loss), _p(Cs), K, B, M, _p(out), _lib.stream_ptr(Cs.device)),
+               "sr_mlp_pick_start")
+    return out
 
 
 def gated_warm_start(net: WarmStartMLP, X, Y, ops, ch, C_plain, clip: float = 10.0) -> torch.Tensor:
@@ -396,13 +348,25 @@ def gated_warm_start(net: WarmStartMLP, X, Y, ops, ch, C_plain, clip: float = 10
 def warm_start_constants(net: WarmStartMLP, X, Y, ops, C_plain, clip: float = 10.0) -> torch.Tensor:
     """C_init with the first N_OUT learnable slots of every row set to the network's
     prediction (clipped to [-clip, clip]); every other slot keeps C_plain."""
-    pred = net.predict(ops, X, Y).clamp(-clip, clip)
-    is_c = ops == 1
-    rank = torch.cumsum(is_c.to(torch.int32), dim=1) - 1
-    sel = is_c & (rank < N_OUT)
-    C = C_plain.clone()
-    rows = torch.arange(ops.shape[0], device=ops.device).unsqueeze(1).expand_as(ops)
-    C[sel] = pred[rows[sel], rank[sel].long()]
+    _lib.require_cuda(ops, C_plain)
+    if C_plain.dtype != torch.float32 or C_plain.shape != ops.shape:
+        raise RuntimeError(f"C_plain must be float32 and shaped like ops {tuple(ops.shape)}, got {C_plain.dtype} "
+                           f"{tuple(C_plain.shape)}")
+    pred = net.predict(ops, X, Y)
+    if C_plain.requires_grad and torch.is_grad_enabled():  # a start that autograd can follow
+        sel, r, k = _first_slots(ops)
+        C = C_plain.clone()
+        C[sel] = pred.clamp(-clip, clip)[r, k]
+        return C
+    B, M = ops.shape
+    C = torch.empty_like(C_plain)
+    src = C_plain if C_plain.stride() == C.stride() else C_plain.contiguous()
+    if src.stride() != C.stride():
+        C = torch.empty_like(src)
+    sb, sm = ops.stride()
+    cb, cm = src.stride()
+    _lib.check(_lib.lib().sr_mlp_place_constants(_p(ops), B, M, sb, sm, _p(pred), pred.stride(0), N_OUT, clip, _p(src),
+                                                 _p(C), cb, cm, _lib.stream_ptr(ops.device)), "sr_mlp_place_constants")
     return C
 
 

@@ -418,6 +418,32 @@ int sr_mlp_gemm(const uint16_t *A_dev, int64_t rows, int64_t k, int64_t lda, con
 /* Number of K pieces sr_mlp_gemm uses for SR_MLP_EPI_SPLIT_F32 with this k and request. */
 int sr_mlp_gemm_splits_used(int64_t k, int32_t splits);
 
+/*
+ * The network's buffers, for sr_mlp_net_forward and sr_mlp_net_backward.  Weights (index 0..4:
+ * E (64, 64), W1 (256, 128), W2, W3 (256, 256), W4 (64, 256)) as bf16 copies w and their
+ * transposes w_t with fp32 biases b (index 1..4); activations for R rows (a multiple of 128,
+ * at most ld) with transposes of leading dimension ld; fp32 gradients gw, gb; part: partial
+ * sums of the weight gradients, splits x (2 x 64 Ki + 32 Ki + 32 Ki + 8 Ki) floats.
+ */
+typedef struct {
+  const uint16_t *w[5], *w_t[5];
+  const float *b[5];
+  uint16_t *hist, *hist_t, *x0, *x0_t, *h[3], *h_t[3];
+  float *out;
+  uint16_t *d_out, *d_out_t, *dz[3], *dz_t[3], *dx0_t;
+  float *part, *gw[5], *gb[5];
+  int64_t ld;
+  int32_t splits;
+  int32_t *status;
+} sr_mlp_net;
+
+/* All layers from hist and the feature columns of x0: five sr_mlp_gemm launches. */
+int sr_mlp_net_forward(const sr_mlp_net *net, int64_t R, void *stream);
+
+/* Every gradient from d_out: the nine sr_mlp_gemm launches of the layers, then the split
+ * reductions and bias sums (as sr_mlp_reduce_splits and sr_mlp_colsum) in one launch. */
+int sr_mlp_net_backward(const sr_mlp_net *net, int64_t R, void *stream);
+
 /* phi (N, SR_MLP_PROJ) = sqrt(2) cos(omega_j . x_n + beta_j); omega (SR_MLP_PROJ, n_x), beta (SR_MLP_PROJ). */
 int sr_mlp_random_features(const float *X_dev, int64_t N, int64_t n_x, const float *omega_dev,
                            const float *beta_dev, float *phi_dev, void *stream);
@@ -459,6 +485,36 @@ int sr_mlp_colsum(const uint16_t *xt_dev, int64_t n, int64_t rows, int64_t ld, f
 /* out (count) = sum over s < splits of part[s * split_stride + i], in order. */
 int sr_mlp_reduce_splits(const float *part_dev, int32_t splits, int64_t count, int64_t split_stride,
                          float *out_dev, void *stream);
+
+/* One tensor of sr_mlp_adam_all: the pointers and sizes of sr_mlp_adam. */
+typedef struct {
+  float *w;
+  const float *g;
+  float *m, *v;
+  int64_t rows, cols;
+  uint16_t *w_bf16, *w_t_bf16;
+  float weight_decay;
+} sr_mlp_adam_tensor;
+
+/* sr_mlp_adam of up to 16 tensors in one launch. */
+int sr_mlp_adam_all(const sr_mlp_adam_tensor *tensors, int32_t count, float lr, float beta1, float beta2, float eps,
+                    int32_t step, void *stream);
+
+/*
+ * Starting constants from predictions: out (B, M) = C with the first n_out
+ * LEARNABLE_CONSTANT slots of every row set to pred (B, ld_pred) clamped to [-clip, clip]
+ * (NaN stays NaN).  C and out: element (b, m) at b * c_sb + m * c_sm.
+ */
+int sr_mlp_place_constants(const int64_t *ops_dev, int64_t B, int64_t M, int64_t ops_sb, int64_t ops_sm,
+                           const float *pred_dev, int64_t ld_pred, int32_t n_out, float clip, const float *C_dev,
+                           float *out_dev, int64_t c_sb, int64_t c_sm, void *stream);
+
+/*
+ * Per problem, the candidate of C_sets (K, B, M) with the lowest loss (B, K) into out (B, M): a
+ * loss that is not finite counts as +inf, the first of equal ones wins.
+ */
+int sr_mlp_pick_start(const float *loss_dev, const float *C_sets_dev, int64_t K, int64_t B, int64_t M, float *out_dev,
+                      void *stream);
 
 /*
  * One Adam step (decoupled weight decay, bias correction for `step` >= 1) on fp32

@@ -4,7 +4,7 @@
 // the reference's CSR tables (src/pcfg.cpp:364-451): rules sorted by left-hand
 // side, nt_rule_ptr[s] .. nt_rule_ptr[s + 1] the rules of symbol s, their cumulative
 // probabilities, and the concatenated right-hand sides.  A lane derives one expression
-// at a time (the derivation is sequential; persistent warps hand a finished lane the
+// at a time (the derivation is sequential; persistent CTAs hand a finished lane the
 // next expression), leftmost first with an explicit stack,
 // exactly as the reference's sample_infix_kernel (src/pcfg_cuda.cu:10-118) does: a
 // try restarts when the stack would exceed 128 symbols or the output would exceed
@@ -21,7 +21,7 @@
 // that every operator has its operands and exactly one tree remains; to prefix it
 // runs the mirrored algorithm from the right end.  One thread per expression; the
 // stacks and the CTA's rows sit in shared memory, and rows are read and written by
-// the whole CTA in coalesced order.
+// the whole CTA in coalesced order; token ids below 254 take a byte there.
 #include <cstdint>
 
 #include "sr_common.cuh"
@@ -60,124 +60,268 @@ struct Stream {
   // uniform in (0, 1], 24 bits: the range the reference's curand_uniform draws from
   __device__ float uniform() {
     s += 0x9E3779B97F4A7C15ull;
-    return (float)((mix64(s) >> 40) + 1ull) * (1.0f / 16777216.0f);
+    return (float)((uint32_t)(mix64(s) >> 40) + 1u) * (1.0f / 16777216.0f);
   }
 };
 
-__global__ void __launch_bounds__(kThreads) sample_infix_kernel(
-    const int32_t* __restrict__ nt_ptr, const float* __restrict__ cum, const int32_t* __restrict__ rhs_ptr,
-    const int32_t* __restrict__ rhs, int32_t n_symbols, int32_t start, int64_t B, int32_t max_len,
-    int32_t max_tries, uint64_t seed, int64_t* __restrict__ out, int64_t* __restrict__ errors) {
-  // Persistent warps: warp w owns expressions [w per, (w + 1) per).  Every lane works on
-  // one expression and advances it by one symbol per loop turn (the same few branches in
-  // every lane); a lane whose expression is finished writes its row and takes the next
-  // expression of the warp's range.  So a warp pays for the sum of its lanes' work, not for
-  // 32 times its longest derivation (its tries included).  The draws of expression b come
-  // from its own stream, so the assignment of expressions to lanes changes no output.
-  extern __shared__ int16_t sm[];
-  const int t = threadIdx.x, lane = t & 31;
-  int16_t* stack = sm;                      // [kHardMax][kThreads]
-  int16_t* buf = sm + kHardMax * kThreads;  // [max_len][kThreads]
-  const int64_t nwarps = (int64_t)gridDim.x * (kThreads / 32);
-  const int64_t w = (int64_t)blockIdx.x * (kThreads / 32) + (t >> 5);
-  const int64_t per = (B + nwarps - 1) / nwarps;
-  const int64_t wbeg = w * per < B ? w * per : B, wend = wbeg + per < B ? wbeg + per : B;
-  const unsigned below = (1u << lane) - 1u;
-  int64_t b = wbeg + lane;
-  int64_t next = wbeg + 32;
-  bool active = b < wend;
-  Stream rng(seed, (uint64_t)(active ? b : 0));
-  int tries = 0, sp = 0, len = 0, err = 0;
-  bool fin = false;
-  // a new expression: its first try (or 303 at once when no try is allowed)
-  auto begin = [&]() {
-    rng = Stream(seed, (uint64_t)b);
-    tries = 0;
-    err = 0;
-    len = 0;
-    sp = 0;
-    fin = false;
-    if (max_tries <= 0) {
-      err = GEN_MAX_TRIES;
-      fin = true;
-    } else {
-      stack[t] = (int16_t)start;
-      sp = 1;
+__host__ __device__ __forceinline__ int odd_stride(int bytes) { return ((bytes + 3) / 4 | 1) * 4; }
+
+// The grammar as the caller gave it.  rules() gives a symbol's first rule and how many it has
+// (0: a terminal; an id outside [0, n_symbols) reads no table), choose() the first rule whose
+// cumulative probability reaches u (-1: none), length() a rule's symbols.
+struct WideGrammar {
+  const int32_t *nt_ptr, *rhs_ptr, *rhs;
+  const float* cum;
+  int n_symbols;
+  __device__ __forceinline__ int rules(int sym, int& r0) const {
+    if ((unsigned)sym >= (unsigned)n_symbols) return 0;
+    r0 = nt_ptr[sym];
+    return nt_ptr[sym + 1] - r0;
+  }
+  __device__ __forceinline__ int choose(int r0, int n, float u) const {
+    for (int r = r0; r < r0 + n; ++r)
+      if (u <= cum[r]) return r;
+    return -1;
+  }
+  __device__ __forceinline__ int length(int rule) const {
+    const int n = rhs_ptr[rule + 1] - rhs_ptr[rule];
+    return n > 0 ? n : 0;
+  }
+  // pushes all but the first symbol, last first; returns the first
+  template <typename Tok>
+  __device__ __forceinline__ int push(int rule, int n, Tok* stack, int& sp) const {
+    const int32_t* p = rhs + rhs_ptr[rule];
+    for (int i = n - 1; i >= 1; --i) stack[sp++] = (Tok)p[i];
+    return n > 0 ? (int)(Tok)p[0] : 0;
+  }
+};
+
+// A grammar with symbols below 256 whose tables take kTableBytes at most, in shared memory:
+// one word per symbol and two per rule (its first four symbols, and where all of them are),
+// so that a step waits for three reads, one after the other.
+constexpr int kTableBytes = 4096;
+struct SmallGrammar {
+  const uint32_t* nt;    // [256] first rule | rules << 16
+  const float* cum;      // [rules]
+  const uint2* rule;     // [rules] first four symbols, offset | symbols << 16
+  const uint8_t* rhs;
+  __device__ __forceinline__ int rules(int sym, int& r0) const {
+    const uint32_t e = nt[sym];
+    r0 = (int)(e & 0xffffu);
+    return (int)(e >> 16);
+  }
+  __device__ __forceinline__ int choose(int r0, int n, float u) const {
+    const int last = r0 + n - 1;
+    for (int r = r0; r <= last; r += 4) {  // four reads at once
+      const int r1 = min(r + 1, last), r2 = min(r + 2, last), r3 = min(r + 3, last);
+      const float c0 = cum[r], c1 = cum[r1], c2 = cum[r2], c3 = cum[r3];
+      int at = -1;  // the first of the four, without branches that the lanes would part at
+      if (u <= c3) at = r3;
+      if (u <= c2) at = r2;
+      if (u <= c1) at = r1;
+      if (u <= c0) at = r;
+      if (at >= 0) return at;
     }
+    return -1;
+  }
+  __device__ __forceinline__ int length(int r) const { return (int)(rule[r].y >> 16); }
+  template <typename Tok>
+  __device__ __forceinline__ int push(int r, int n, Tok* stack, int& sp) const {
+    const uint2 e = rule[r];
+    for (int i = n - 1; i >= 4; --i) stack[sp++] = (Tok)rhs[(e.y & 0xffffu) + i];
+    if (n > 3) stack[sp++] = (Tok)(e.x >> 24);
+    if (n > 2) stack[sp++] = (Tok)((e.x >> 16) & 0xffu);
+    if (n > 1) stack[sp++] = (Tok)((e.x >> 8) & 0xffu);
+    return (int)(e.x & 0xffu);
+  }
+};
+
+// The CTA's copy of a small grammar at `at`; false (in every thread) if it is not one.
+__device__ __forceinline__ bool stage_grammar(const WideGrammar& W, int start, unsigned char* at, SmallGrammar& G) {
+  const int t = threadIdx.x;
+  if (W.n_symbols > 256 || start > 255) return false;
+  const int rules = W.nt_ptr[W.n_symbols];
+  if (rules < 0 || rules > kTableBytes / 12) return false;
+  const int total = W.rhs_ptr[rules];
+  if (total < 0 || 1024 + 12 * rules + total > kTableBytes) return false;
+  uint32_t* nt = reinterpret_cast<uint32_t*>(at);
+  uint2* rule = reinterpret_cast<uint2*>(at + 1024);
+  float* cum = reinterpret_cast<float*>(at + 1024 + 8 * rules);
+  uint8_t* rhs = at + 1024 + 12 * rules;
+  bool ok = true;
+  for (int i = t; i < total; i += blockDim.x) {
+    const int v = W.rhs[i];
+    ok &= v >= 0 && v < 256;
+    rhs[i] = (uint8_t)v;
+  }
+  for (int i = t; i < 256; i += blockDim.x) {
+    int r0 = 0, n = 0;
+    if (i < W.n_symbols) {
+      r0 = W.nt_ptr[i];
+      n = W.nt_ptr[i + 1] - r0;
+      ok &= r0 >= 0 && n >= 0 && r0 + n <= rules;
+    }
+    nt[i] = (uint32_t)(n > 0 ? r0 : 0) | (uint32_t)n << 16;
+  }
+  for (int r = t; r < rules; r += blockDim.x) {
+    const int lo = W.rhs_ptr[r], n = W.rhs_ptr[r + 1] - lo;
+    const bool in = lo >= 0 && n >= 0 && lo + n <= total;
+    ok &= in;
+    uint32_t first = 0;
+    for (int i = 0; in && i < n && i < 4; ++i) first |= (uint32_t)(W.rhs[lo + i] & 0xff) << (8 * i);
+    rule[r] = make_uint2(first, (uint32_t)lo | (uint32_t)n << 16);
+    cum[r] = W.cum[r];
+  }
+  G = SmallGrammar{nt, cum, rule, rhs};
+  return __syncthreads_and(ok);
+}
+
+// The CTA's warps derive the expressions [beg, beg + count).  Every lane works on one
+// expression; a turn of the loop emits at most one terminal and expands at most one
+// non-terminal of it, with the next symbol in a register and the next random number drawn
+// ahead.  A lane whose expression is finished takes the CTA's next one (`queue`), so that a
+// warp does not wait for its longest derivation before it goes on.  The draws of expression b
+// come from its own stream, so the assignment of expressions to lanes changes no output.
+template <typename Tok, typename G>
+__device__ __forceinline__ void derive(const G& g, int start, int64_t beg, int64_t count, int* queue, int max_len,
+                                       int max_tries, uint64_t seed, unsigned char* stacks, unsigned char* bufs,
+                                       int64_t* __restrict__ out, int64_t* __restrict__ errors) {
+  const int t = threadIdx.x, lane = t & 31;
+  const int buf_bytes = odd_stride(max_len * (int)sizeof(Tok));
+  Tok* stack = reinterpret_cast<Tok*>(stacks + t * odd_stride(kHardMax * (int)sizeof(Tok)));
+  Tok* buf = reinterpret_cast<Tok*>(bufs + t * buf_bytes);
+  const unsigned below = (1u << lane) - 1u;
+  int64_t b = t;  // within the CTA's expressions
+  bool active = b < count;
+  Stream rng(seed, 0);
+  float u = 0.0f;
+  // cur: the symbol to work on; the stack holds the sp symbols after it
+  int cur = start, tries = 0, sp = 0, len = 0, err = 0;
+  // a new expression: its first try
+  auto begin = [&]() {
+    rng = Stream(seed, (uint64_t)(beg + b));
+    u = rng.uniform();
+    cur = start;
+    tries = sp = len = err = 0;
   };
   if (active) begin();
   while (__any_sync(0xffffffffu, active)) {
-    if (active && !fin) {
-      // one symbol of the derivation, leftmost first
-      bool restart = false;
-      const int sym = stack[(--sp) * kThreads + t];
-      // an id outside [0, n_symbols) has no rules (a terminal): no table read for it
-      const bool has_rules = (unsigned)sym < (unsigned)n_symbols;
-      const int r0 = has_rules ? nt_ptr[sym] : 0;
-      const int r1 = has_rules ? nt_ptr[sym + 1] : 0;
-      if (r0 != r1) {  // a non-terminal: choose a rule, push its right-hand side reversed
-        const float u = rng.uniform();
-        int chosen = -1;
-        for (int r = r0; r < r1; ++r) {
-          if (u <= cum[r]) {
-            chosen = r;
-            break;
+    bool done = false;
+    if (active) {
+      enum { kGoOn, kEnded, kRestart, kNoRule };
+      int state = kGoOn;
+      int r0 = 0, n = g.rules(cur, r0);
+      if (n == 0) {  // a terminal: emit it and take the next symbol
+        if (len >= max_len) {  // past the padded length
+          state = kRestart;
+        } else {
+          buf[len++] = (Tok)cur;
+          if (sp == 0) {
+            state = kEnded;
+          } else {
+            cur = stack[--sp];
+            n = g.rules(cur, r0);
           }
         }
+      }
+      if (n != 0) {  // a non-terminal: choose a rule, leftmost symbol next
+        const int chosen = g.choose(r0, n, u);
+        u = rng.uniform();
         if (chosen < 0) {
+          state = kNoRule;
+        } else {
+          const int k = g.length(chosen);
+          if (sp + k > kHardMax) {
+            state = kRestart;
+          } else {
+            cur = g.push(chosen, k, stack, sp);
+            if (k == 0) {  // an empty right-hand side
+              if (sp == 0) state = kEnded;
+              else cur = stack[--sp];
+            }
+          }
+        }
+      }
+      // a try ends: without a rule, restarted, or derived completely (an empty derivation
+      // fails too)
+      if (state != kGoOn) {
+        done = true;
+        if (state == kNoRule) {
           err = GEN_NO_RULE;
           len = 0;
-          fin = true;
-        } else {
-          for (int i = rhs_ptr[chosen + 1] - 1; i >= rhs_ptr[chosen]; --i) {
-            if (sp >= kHardMax) {
-              restart = true;
-              break;
-            }
-            stack[(sp++) * kThreads + t] = (int16_t)rhs[i];
+        } else if (state == kRestart || len == 0) {
+          len = 0;
+          if (++tries >= max_tries) {
+            err = GEN_MAX_TRIES;
+          } else {
+            cur = start;
+            sp = 0;
+            done = false;
           }
         }
-      } else if (len >= max_len) {  // a terminal past the padded length
-        restart = true;
-      } else {  // a terminal: emit it
-        buf[(len++) * kThreads + t] = (int16_t)sym;
-      }
-      // a try ends: restarted, or derived completely (an empty derivation fails too)
-      if (!fin && (restart || sp == 0)) {
-        if (!restart && len > 0) {
-          fin = true;
-        } else if (++tries >= max_tries) {
-          err = GEN_MAX_TRIES;
-          len = 0;
-          fin = true;
-        } else {
-          stack[t] = (int16_t)start;
-          sp = 1;
-          len = 0;
-        }
       }
     }
-    const bool done = active && fin;
     const unsigned m = __ballot_sync(0xffffffffu, done);
+    if (m == 0) continue;
     // the warp writes the rows finished in this turn together, one row at a time, its
     // lanes on consecutive tokens (coalesced), while no lane waits on another's row
-    if (m) __syncwarp();  // the finished rows' tokens, written by their lanes
+    int first = 0;
+    if (lane == 0) first = atomicAdd(queue, __popc(m));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    __syncwarp();  // the finished rows' tokens, written by their lanes
     for (unsigned mm = m; mm; mm &= mm - 1) {
       const int src = __ffs(mm) - 1;
-      const int64_t bs = __shfl_sync(0xffffffffu, b, src);
+      const int64_t bs = beg + __shfl_sync(0xffffffffu, b, src);
       const int ls = __shfl_sync(0xffffffffu, len, src);
       const int es = __shfl_sync(0xffffffffu, err, src);
-      const int ts = (t & ~31) + src;
-      for (int i = lane; i < max_len; i += 32) out[bs * max_len + i] = i < ls ? (int64_t)buf[i * kThreads + ts] : NO_OP;
+      const Tok* row = reinterpret_cast<const Tok*>(bufs + ((t & ~31) + src) * buf_bytes);
+      for (int i = lane; i < max_len; i += 32) out[bs * max_len + i] = i < ls ? (int64_t)row[i] : NO_OP;
       if (lane == 0) errors[bs] = es;
     }
-    if (m) __syncwarp();  // read before their lanes start the next expressions
+    __syncwarp();  // read before their lanes start the next expressions
     if (done) {
-      b = next + __popc(m & below);
-      active = b < wend;
+      b = (int64_t)first + __popc(m & below);
+      active = b < count;
       if (active) begin();
     }
-    next += __popc(m);
+  }
+}
+
+// Persistent CTAs, each with an equal share of the expressions.  What bounds it: the longest
+// derivations of a CTA's share (a few hundred steps where the mean is 33), so the latency of
+// a step: the symbol at hand in a register, the tables in shared memory and packed
+// (SmallGrammar), rows of an odd number of words per thread (no bank conflicts when a warp
+// writes a finished row), and symbols in a byte, which put 28 warps on an SM instead of 16.
+// 262144 expressions of up to 64 tokens take 320 us where one symbol per turn, the tables
+// read from L1 and 16-bit symbols took 513; 1000 take 144 us (before: 226), 1000000 take 590
+// (1051).  Fewer CTAs per SM, each with a longer queue, are slower: 425 us with two.
+// Other grammars keep 16-bit symbols and their tables in global memory; `wide_threads`
+// threads of the CTA then work (all of them, or the half that shared memory sized for bytes
+// holds).
+__global__ void __launch_bounds__(kThreads) sample_infix_kernel(
+    const int32_t* __restrict__ nt_ptr, const float* __restrict__ cum, const int32_t* __restrict__ rhs_ptr,
+    const int32_t* __restrict__ rhs, int32_t n_symbols, int32_t start, int64_t B, int32_t max_len,
+    int32_t max_tries, uint64_t seed, int wide_threads, int64_t* __restrict__ out, int64_t* __restrict__ errors) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int queue;
+  const int64_t per = (B + gridDim.x - 1) / gridDim.x, beg = per * blockIdx.x;
+  const int64_t count = B - beg < per ? (B - beg > 0 ? B - beg : 0) : per;
+  if (max_tries <= 0) {  // no try is allowed
+    for (int64_t j = threadIdx.x; j < count * max_len; j += kThreads) out[beg * max_len + j] = NO_OP;
+    for (int64_t j = threadIdx.x; j < count; j += kThreads) errors[beg + j] = GEN_MAX_TRIES;
+    return;
+  }
+  const WideGrammar W{nt_ptr, rhs_ptr, rhs, cum, n_symbols};
+  SmallGrammar S;
+  const bool small = stage_grammar(W, start, smem, S);
+  if (threadIdx.x == 0) queue = small ? kThreads : wide_threads;
+  __syncthreads();
+  if (small) {
+    derive<uint8_t>(S, start, beg, count, &queue, max_len, max_tries, seed, smem + kTableBytes,
+                    smem + kTableBytes + kThreads * odd_stride(kHardMax), out, errors);
+  } else if ((int)threadIdx.x < wide_threads) {
+    derive<int16_t>(W, start, beg, count, &queue, max_len, max_tries, seed, smem,
+                    smem + wide_threads * odd_stride(kHardMax * (int)sizeof(int16_t)), out, errors);
   }
 }
 
@@ -342,6 +486,174 @@ __global__ void __launch_bounds__(kThreads) infix_parse_kernel(const int64_t* __
   }
 }
 
+// The same parsers for rows of up to 128 tokens and token ids below 254, a token per byte.
+// What bounds them: the passes of one thread over its row, over the warps that shared memory
+// lets reside.  Each thread's row, stack and queue are rows of an odd number of words (no bank
+// conflicts between the threads of a warp), the checks of the whole row go word by word, a
+// table says what a token does, and only the tokens before the padding are parsed: 243 us for 262144 rows of 64 tokens with 16-bit tokens and six
+// token-by-token passes, 90 us this way.
+constexpr uint32_t kByteNegative = 0xff, kByteRange = 0xfe;  // tokens that fail the checks
+constexpr int kByteLimit = 0xfe;
+
+// Tokens of rows r < rows of the CTA's block into bytes, consecutive threads on consecutive tokens.
+__device__ __forceinline__ void stage_bytes(const int64_t* __restrict__ src, int rows, int M, int stride, int64_t limit,
+                                            unsigned char* dst) {
+  const int total = rows * M, dr = kThreads / M, di = kThreads % M;
+  int r = threadIdx.x / M, i = threadIdx.x - r * M;
+#pragma unroll 8
+  for (int j = threadIdx.x; j < total; j += kThreads) {
+    const int64_t tok = src[j];
+    dst[r * stride + i] = (unsigned char)(tok < 0 ? kByteNegative : (tok >= limit ? kByteRange : (uint32_t)tok));
+    r += dr;
+    i += di;
+    if (i >= M) {
+      i -= M;
+      ++r;
+    }
+  }
+}
+
+// Row checks, four tokens at a time: a token that failed (BAD_*), the tokens before the first
+// NO_OP (len), whether a token follows it.
+__device__ __forceinline__ void check_row(const uint32_t* words, int n_words, int& bad, int& len, bool& follows) {
+  bad = 0;
+  len = 0;
+  follows = false;
+  bool ended = false;
+  for (int w = 0; w < n_words; ++w) {
+    const uint32_t x = words[w];
+    if (__vcmpeq4(x, 0xffffffffu)) bad = BAD_NEGATIVE;
+    else if (__vcmpeq4(x, 0xfefefefeu) && bad == 0) bad = BAD_RANGE;
+    if (ended) {
+      follows |= x != 0;
+      continue;
+    }
+    const uint32_t zero = __vcmpeq4(x, 0u);
+    if (!zero) {
+      len += 4;
+    } else {
+      const int at = (__ffs((int)zero) - 1) & ~7;  // bit of the first NO_OP
+      len += at >> 3;
+      ended = true;
+      follows |= (x >> at) != 0;
+    }
+  }
+}
+
+template <bool kPrefix>
+__global__ void __launch_bounds__(kThreads) infix_parse_bytes_kernel(const int64_t* __restrict__ infix, int64_t B,
+                                                                     int M, int32_t n_vars, int64_t* __restrict__ outp,
+                                                                     int64_t* __restrict__ errors) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  // What the parser needs to know of a token: its precedence on the stack (an opening
+  // parenthesis 0), from which precedence on the stack's operators go to the queue before it
+  // is taken, and what is then done with it.
+  constexpr int kOperand = 0, kPush = 1, kClose = 2, kNever = 7;
+  __shared__ uint8_t table[256];  // precedence | threshold << 3 | kind << 6
+  __shared__ uint8_t counts[kThreads];  // tokens of each output row
+  const int t = threadIdx.x, stride = odd_stride(M), n_words = (M + 3) / 4;
+  unsigned char* row = smem + t * stride;
+  unsigned char* ops = smem + (kThreads + t) * stride;  // operator stack
+  // The output queue.  To postfix it lives in the row itself (see infix_parse_kernel); to
+  // prefix, which scans from the right end, it fills an array of its own from the right end.
+  unsigned char* queues = kPrefix ? smem + 2 * kThreads * stride : smem;
+  unsigned char* queue = queues + t * stride;
+  const int64_t b0 = (int64_t)blockIdx.x * kThreads;
+  const int rows = (int)(B - b0 < kThreads ? B - b0 : kThreads);
+  const int lp = VAR + n_vars, rp = lp + 1;
+  const int open = kPrefix ? rp : lp, close = kPrefix ? lp : rp;
+  for (int k = t; k < 256; k += kThreads) {
+    // to postfix: an operator takes off those that bind at least as tightly (left-assoc) or
+    // more tightly (right-assoc); to prefix the two conditions swap
+    const int p = precedence(k, lp, rp);
+    int e = p | (p + (right_assoc(k) != kPrefix ? 1 : 0)) << 3 | kPush << 6;
+    if (p == 0) e = kNever << 3 | kOperand << 6;
+    if (k == open) e = kNever << 3 | kPush << 6;
+    if (k == close) e = 1 << 3 | kClose << 6;
+    table[k] = (uint8_t)e;
+  }
+  reinterpret_cast<uint32_t*>(row)[n_words - 1] = 0u;  // bytes past the last token
+  __syncthreads();
+  stage_bytes(infix + b0 * M, rows, M, stride, rp + 1, smem);
+  __syncthreads();
+  if (t < rows) {
+    int bad, len, n_out = 0, err = 0;
+    bool follows;
+    check_row(reinterpret_cast<const uint32_t*>(row), n_words, bad, len, follows);
+    if (follows) err = PARSE_UNEXPECTED;
+    int sp = 0, depth = 0;
+    int missing = 0;  // first operator of the postfix row without its operands
+    auto enqueue = [&](int tok, int p) {
+      queue[kPrefix ? M - 1 - n_out : n_out] = (unsigned char)tok;
+      ++n_out;
+      if (!kPrefix) {
+        const int ar = p == 0 ? 0 : (p == 4 ? 1 : 2);
+        if (depth < ar && !missing) missing = ar == 1 ? PARSE_UNARY_MISSING : PARSE_BINARY_MISSING;
+        depth = depth - ar + 1;
+      }
+    };
+    // A turn either queues the top of the stack or takes the next token, so that the lanes of
+    // a warp go through their rows side by side, whatever each row needs.  The end of the row
+    // empties the stack as a closing parenthesis does.
+    const int end = 1 << 3 | kClose << 6;
+    int step = 0, top = 0, ptop = 0;
+    auto next = [&](int& tok) {
+      tok = step < len ? (int)row[kPrefix ? len - 1 - step : step] : -1;
+      return step < len ? (int)table[tok] : end;
+    };
+    auto look = [&]() {  // the stack's new top
+      top = sp > 0 ? (int)ops[sp - 1] : 0;
+      ptop = sp > 0 ? table[top] & 7 : 0;
+    };
+    int tok, e = next(tok);
+    while (!err && !bad) {
+      const int kind = e >> 6;
+      if (ptop >= ((e >> 3) & 7)) {
+        enqueue(top, ptop);
+        --sp;
+        look();
+        continue;
+      }
+      if (kind == kOperand) {
+        enqueue(tok, 0);
+      } else if (kind == kPush) {
+        ops[sp++] = (unsigned char)tok;
+        top = tok;
+        ptop = e & 7;
+      } else {
+        // the stack is empty or an opening parenthesis is on top
+        if (tok < 0 && sp == 0) break;
+        if (tok < 0 || sp == 0) {
+          err = PARSE_PAREN;
+          break;
+        }
+        --sp;
+        look();
+      }
+      ++step;
+      e = next(tok);
+    }
+    if (!kPrefix && !err && !bad && n_out > 0) err = missing ? missing : (depth != 1 ? PARSE_MALFORMED : 0);
+    if (err || bad) n_out = 0;
+    errors[b0 + t] = bad ? bad : err;
+    counts[t] = (uint8_t)n_out;
+  }
+  __syncthreads();
+  const int total = rows * M, dr = kThreads / M, di = kThreads % M;
+  int r = t / M, i = t - r * M;
+#pragma unroll 8
+  for (int j = t; j < total; j += kThreads) {
+    const int n = counts[r];
+    outp[b0 * M + j] = i < n ? (int64_t)queues[r * stride + (kPrefix ? M - n + i : i)] : (int64_t)NO_OP;
+    r += dr;
+    i += di;
+    if (i >= M) {
+      i -= M;
+      ++r;
+    }
+  }
+}
+
 static int max_smem_optin() {
   int dev = 0, v = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 48 * 1024;
@@ -361,6 +673,15 @@ static int launch_parse(const int64_t* infix, int64_t B, int64_t M, int32_t n_va
   if (B == 0) return SR_OK;
   if (!errors || (M > 0 && (!infix || !outp))) { set_error("null pointer argument"); return SR_ERR_INVALID_ARGUMENT; }
   const int64_t arrays = kPrefix ? 3 : 2;  // row, operator stack (, queue)
+  if (M >= 1 && VAR + n_vars + 2 <= kByteLimit) {
+    const size_t bytes = (size_t)arrays * kThreads * odd_stride((int)M);
+    auto kern = infix_parse_bytes_kernel<kPrefix>;
+    const int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem");
+    if (rc) return rc;
+    kern<<<(unsigned)((B + kThreads - 1) / kThreads), kThreads, bytes, as_stream(stream)>>>(infix, B, (int)M, n_vars, outp,
+                                                                                           errors);
+    return launch_check(kPrefix ? "infix_parse_bytes_kernel<prefix>" : "infix_parse_bytes_kernel<postfix>");
+  }
   const size_t smem = (size_t)(arrays * M > 0 ? arrays * M : 1) * kThreads * sizeof(int16_t);
   auto kern = infix_parse_kernel<kPrefix>;
   int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
@@ -394,7 +715,13 @@ int sr_pcfg_sample_infix(const int32_t* nt_rule_ptr, const float* nt_rule_cum_pr
     set_error("null pointer argument");
     return SR_ERR_INVALID_ARGUMENT;
   }
-  const size_t smem = (size_t)(kHardMax + max_length) * kThreads * sizeof(int16_t);
+  // Grammars that may have symbols below 256 get shared memory for those (and for half as
+  // many threads with 16-bit symbols, should an id or the tables turn out larger).
+  const bool bytes = n_symbols <= 256 && start_symbol < 256;
+  const int wide_threads = bytes ? kThreads / 2 : kThreads;
+  size_t smem = (size_t)wide_threads * (odd_stride(2 * kHardMax) + odd_stride(2 * max_length));
+  const size_t narrow = (size_t)kTableBytes + (size_t)kThreads * (odd_stride(kHardMax) + odd_stride(max_length));
+  if (bytes && narrow > smem) smem = narrow;
   if ((int)smem > max_smem_optin()) { set_error("sampling tables do not fit in shared memory"); return SR_ERR_UNSUPPORTED; }
   int rc = cuda_check(cudaFuncSetAttribute(sample_infix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                       "smem");
@@ -406,11 +733,11 @@ int sr_pcfg_sample_infix(const int32_t* nt_rule_ptr, const float* nt_rule_cum_pr
   if (rc) return rc;
   per_sm = resident_ctas(reinterpret_cast<const void*>(sample_infix_kernel), kThreads, smem);
   int64_t blocks = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
-  const int64_t need = (B + kThreads - 1) / kThreads;
+  const int64_t need = (B + wide_threads - 1) / wide_threads;
   if (blocks > need) blocks = need;
   sample_infix_kernel<<<(unsigned)blocks, kThreads, smem, as_stream(stream)>>>(
       nt_rule_ptr, nt_rule_cum_probs, rhs_ptr, rhs_concat, n_symbols, start_symbol, B, max_length, max_tries, seed,
-      out, errors);
+      wide_threads, out, errors);
   return launch_check("sample_infix_kernel");
 }
 

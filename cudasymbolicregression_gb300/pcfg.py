@@ -303,12 +303,13 @@ class ProbabilisticContextFreeGrammar:
         B, L = int(B), self._padded_maximum_length
         dev = self._device
         infix = torch.empty((B, L), dtype=torch.int64, device=dev)
+        errs = torch.empty((3, B), dtype=torch.int64, device=dev)  # every word is written
+        if B:
+            self._launch_sample(B, infix, errs[0])
         post = torch.empty((B, L), dtype=torch.int64, device=dev)
         ch = torch.empty((B, L, 2), dtype=torch.int64, device=dev)
-        errs = torch.zeros((3, B), dtype=torch.int64, device=dev)
         if B == 0:
             return post, ch
-        self._launch_sample(B, infix, errs[0])
         st = _lib.stream_ptr(dev)
         lib = _lib.lib()
         _lib.check(lib.sr_infix_to_postfix(_lib.ptr(infix), B, L, self._n_variables, _lib.ptr(post),
@@ -362,7 +363,7 @@ class ProbabilisticContextFreeGrammar:
         if M > HARD_MAX_LENGTH:
             raise ValueError(f"M must be less than or equal to HARD_MAX_LENGTH, but got {M} > {HARD_MAX_LENGTH}.")
         out = torch.empty((B, M), dtype=torch.int64, device=dev)
-        err = torch.zeros(B, dtype=torch.int64, device=dev)
+        err = torch.empty(B, dtype=torch.int64, device=dev)
         fn = _lib.lib().sr_infix_to_prefix if prefix else _lib.lib().sr_infix_to_postfix
         _lib.check(fn(_lib.ptr(x), B, M, self._n_variables, _lib.ptr(out), _lib.ptr(err), _lib.stream_ptr(dev)),
                    "sr_infix_to_prefix" if prefix else "sr_infix_to_postfix")
@@ -384,13 +385,14 @@ class ProbabilisticContextFreeGrammar:
         return notation.postfix_to_infix(expressions, max_infix_len, self._n_variables)
 
     def _convert(self, fn: str, expressions: torch.Tensor, context: str, check_kind: str, verbosity: int,
-                 width=None, fill=int(Operator.NO_OP)) -> torch.Tensor:
+                 width=None) -> torch.Tensor:
         _check_token_rows(expressions)
         dev = _lib.require_cuda(expressions)
         x = expressions.to(torch.int64).contiguous()
         B, M = x.shape
-        out = torch.full((B, M if width is None else int(width)), fill, dtype=torch.int64, device=dev)
-        err = torch.zeros(B, dtype=torch.int64, device=dev)
+        # the kernels write every word of both
+        out = torch.empty((B, M if width is None else int(width)), dtype=torch.int64, device=dev)
+        err = torch.empty(B, dtype=torch.int64, device=dev)
         args = [_lib.ptr(x), B, M, self._n_variables, _lib.ptr(out)]
         if width is not None:
             args.append(int(width))
@@ -416,7 +418,7 @@ class ProbabilisticContextFreeGrammar:
 
     def get_prefix_parent(self, prefix_ops: torch.Tensor, verbosity: int = 0) -> torch.Tensor:
         """(B, M) prefix -> (B, M) index of every node's parent (-1: root or padding)."""
-        return self._convert("sr_prefix_parent", prefix_ops, "get prefix parent", "prefix_ops", verbosity, fill=-1)
+        return self._convert("sr_prefix_parent", prefix_ops, "get prefix parent", "prefix_ops", verbosity)
 
     def get_postfix_children(self, postfix_ops: torch.Tensor, verbosity: int = 0) -> torch.Tensor:
         """(B, M) postfix -> (B, M, 2) child table (NULL_CHILD = -1)."""

@@ -33,6 +33,9 @@ void set_error(const char* fmt, ...) {
 // (101); the count must equal the arity (102).  Inputs the reference accepts but
 // then reads out of bounds (a counted child < 0, or a unary node whose only child
 // sits in the second slot) are reported as 101 here.
+// The batch summary is one maximum per CTA, by warps that each take several tapes: with an
+// atomic per tape the 65536 atomics on four words bound the kernel (16384 tapes of 64 nodes:
+// 46 us; 10 us so).
 // ------------------------------------------------------------------------------------
 template <bool kStage>
 __global__ void __launch_bounds__(256) tape_compile_kernel(const int64_t* __restrict__ ops,
@@ -44,6 +47,7 @@ __global__ void __launch_bounds__(256) tape_compile_kernel(const int64_t* __rest
                                                            int32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (blockDim.x >> 5);
+  int max_len = 0, max_root = 0, max_kroot = 0, max_ops = 0;  // of this warp's tapes
   for (int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < B; b += warps_total) {
     int count = 0, last = -1;
     int err = 0;
@@ -102,13 +106,25 @@ __global__ void __launch_bounds__(256) tape_compile_kernel(const int64_t* __rest
         meta[b * 4 + 1] = root;
         meta[b * 4 + 2] = kroot;
         meta[b * 4 + 3] = kall;
-        // batch summary: stats[1] = max L_eff, stats[2] = max root + 1, stats[3] = max constants to root
-        atomicMax(status + 1, last + 1);
-        atomicMax(status + 2, root + 1);
-        atomicMax(status + 3, kroot);
-        atomicMax(status + 4, nops);
       }
+      max_len = max(max_len, last + 1);
+      max_root = max(max_root, root + 1);
+      max_kroot = max(max_kroot, kroot);
+      max_ops = max(max_ops, nops);
     }
+  }
+  if (kStage) {
+    // batch summary: stats[1] = max L_eff, stats[2] = max root + 1, stats[3] = max constants
+    // to the root, stats[4] = max operator nodes
+    __shared__ int cta_max[4];
+    if (threadIdx.x < 4) cta_max[threadIdx.x] = 0;
+    __syncthreads();
+    if (lane < 4) {
+      const int mine = lane == 0 ? max_len : lane == 1 ? max_root : lane == 2 ? max_kroot : max_ops;
+      atomicMax(&cta_max[lane], mine);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) atomicMax(status + 1 + threadIdx.x, cta_max[threadIdx.x]);
   }
 }
 
@@ -159,8 +175,12 @@ __global__ void __launch_bounds__(32) pad_fill_kernel(const int32_t* __restrict_
 // Work order: the tapes by falling meta[column], by one CTA (a histogram of the values, its
 // running sums, then a place for each tape).  The order decides only which warp takes which
 // tape, so tapes of one length come in any order.  What bounds it: two passes over meta by one
-// SM (65536 tapes: about 20 us); a library sort's five launches took the host longer than the
+// SM, so a thread reads kOrderLoads tapes at once and counts with plain
+// shared-memory atomics (16384 tapes: 13.5 us, all of one length 18; with the lanes of a warp
+// grouped by value first, 31); a library sort's five launches took the host longer than the
 // forward of a small batch.
+constexpr int kOrderLoads = 8;
+
 __global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restrict__ meta, int64_t B, int column,
                                                           int add, int bins, int32_t* __restrict__ order) {
   extern __shared__ int at[];  // per value: count, then the next place
@@ -168,17 +188,24 @@ __global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restr
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < bins; i += blockDim.x) at[i] = 0;
   __syncthreads();
-  const int64_t rounds = (B + blockDim.x - 1) / blockDim.x;
-  auto key = [&](int64_t b) {  // 0 for the largest value
-    const int v = meta[b * 4 + column] + add;
-    return bins - 1 - min(max(v, 0), bins - 1);
+  // f(b, key) for every tape, the lanes of a warp together; key 0 for the largest value, -1
+  // past the last tape
+  auto each_tape = [&](auto f) {
+    for (int64_t b0 = 0; b0 < B; b0 += (int64_t)kOrderLoads * blockDim.x) {
+      int k[kOrderLoads];
+#pragma unroll
+      for (int j = 0; j < kOrderLoads; ++j) {
+        const int64_t b = b0 + j * (int)blockDim.x + tid;
+        k[j] = b < B ? bins - 1 - min(max(meta[b * 4 + column] + add, 0), bins - 1) : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < kOrderLoads; ++j)
+        if (b0 + j * (int)blockDim.x < B) f(b0 + j * (int)blockDim.x + tid, k[j]);
+    }
   };
-  for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t b = r * blockDim.x + tid;
-    const int k = b < B ? key(b) : -1;
-    const unsigned same = __match_any_sync(0xffffffffu, k);
-    if (k >= 0 && lane == __ffs((int)same) - 1) atomicAdd(&at[k], __popc(same));
-  }
+  each_tape([&](int64_t, int k) {
+    if (k >= 0) atomicAdd(&at[k], 1);
+  });
   __syncthreads();
   // exclusive running sums over the bins, a run of consecutive bins per thread
   const int per = (bins + (int)blockDim.x - 1) / (int)blockDim.x, lo = min(bins, tid * per), hi = min(bins, lo + per);
@@ -200,16 +227,9 @@ __global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restr
     before += c;
   }
   __syncthreads();
-  for (int64_t r = 0; r < rounds; ++r) {
-    const int64_t b = r * blockDim.x + tid;
-    const int k = b < B ? key(b) : -1;
-    const unsigned same = __match_any_sync(0xffffffffu, k);
-    const int leader = __ffs((int)same) - 1;
-    int base = 0;
-    if (k >= 0 && lane == leader) base = atomicAdd(&at[k], __popc(same));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (k >= 0) order[base + __popc(same & ((1u << lane) - 1u))] = (int32_t)b;
-  }
+  each_tape([&](int64_t b, int k) {
+    if (k >= 0) order[atomicAdd(&at[k], 1)] = (int32_t)b;
+  });
 }
 
 // Whether any of n words is not zero.
@@ -571,7 +591,7 @@ static int launch_compile(const int64_t* ops, const int64_t* ch, int64_t B, int6
   if (rc || B == 0) return rc;
   const int threads = 256;
   int64_t blocks = (B + 7) / 8;
-  const int64_t cap = (int64_t)device_sm_count() * 16;
+  const int64_t cap = (int64_t)device_sm_count() * 8;
   if (blocks > cap) blocks = cap;
   tape_compile_kernel<kStage><<<(unsigned)blocks, threads, 0, st>>>(ops, ch, B, M, ops_sb, ops_sm, ch_sb, ch_sm,
                                                                     ch_si, n_vars, desc, meta, status);

@@ -30,3 +30,21 @@ def test_any_nonzero(n):
         w[i] = 1 << 40
         assert _lib.any_nonzero(w)
         w[i] = 0
+
+
+@pytest.mark.parametrize("M", [1, 33, 64])
+@pytest.mark.parametrize("B", [1, 8, 9, 9728, 9729, 30001])
+def test_compile_summary_is_the_maximum_over_tapes(B, M):
+    """Batches below, at and above the tapes that the grid's warps take at once; the longest
+    tape first, last or in between."""
+    from cudasymbolicregression_gb300 import tape, tapes
+    tb = tapes.generate(B, M, seed=B + M, mean_length=min(5, M), n_vars=2, p_const_leaf=0.5)
+    ops = tb.ops.copy()
+    for at in {0, B // 2, B - 1}:
+        rows = ops.copy()
+        rows[at] = 1  # constants only: the root is the last of them
+        want = ((rows != 0) * np.arange(1, M + 1)).max(), (rows != 0).sum(1).max(), (rows == 1).sum(1).max()
+        ch = tb.ch.copy()
+        ch[at] = -1
+        c = tape.compile_tapes(torch.as_tensor(rows).cuda(), torch.as_tensor(ch).cuda(), 2)
+        assert (c.max_len, c.max_root, c.max_consts) == want

@@ -97,13 +97,15 @@ struct WideGrammar {
 };
 
 // A grammar with symbols below 256 whose tables take kTableBytes at most, in shared memory:
-// one word per symbol and two per rule (its first four symbols, and where all of them are),
-// so that a step waits for three reads, one after the other.
-constexpr int kTableBytes = 4096;
+// one word per symbol and three per rule (its cumulative probability, its first four symbols,
+// and where all of them are).  A symbol's rules start at a multiple of four and are filled up
+// with NaN, which no number reaches, so a step waits for three reads, one after the other:
+// the symbol's word, four probabilities at once, the rule.
+constexpr int kTableBytes = 5120, kTableRules = 208, kTableSymbols = kTableBytes - 1024 - 12 * kTableRules;
 struct SmallGrammar {
   const uint32_t* nt;    // [256] first rule | rules << 16
-  const float* cum;      // [rules]
-  const uint2* rule;     // [rules] first four symbols, offset | symbols << 16
+  const float* cum;      // [kTableRules]
+  const uint2* rule;     // [kTableRules] first four symbols, offset | symbols << 16
   const uint8_t* rhs;
   __device__ __forceinline__ int rules(int sym, int& r0) const {
     const uint32_t e = nt[sym];
@@ -111,15 +113,13 @@ struct SmallGrammar {
     return (int)(e >> 16);
   }
   __device__ __forceinline__ int choose(int r0, int n, float u) const {
-    const int last = r0 + n - 1;
-    for (int r = r0; r <= last; r += 4) {  // four reads at once
-      const int r1 = min(r + 1, last), r2 = min(r + 2, last), r3 = min(r + 3, last);
-      const float c0 = cum[r], c1 = cum[r1], c2 = cum[r2], c3 = cum[r3];
+    for (int r = r0; r < r0 + n; r += 4) {
+      const float4 c = *reinterpret_cast<const float4*>(cum + r);
       int at = -1;  // the first of the four, without branches that the lanes would part at
-      if (u <= c3) at = r3;
-      if (u <= c2) at = r2;
-      if (u <= c1) at = r1;
-      if (u <= c0) at = r;
+      if (u <= c.w) at = r + 3;
+      if (u <= c.z) at = r + 2;
+      if (u <= c.y) at = r + 1;
+      if (u <= c.x) at = r;
       if (at >= 0) return at;
     }
     return -1;
@@ -141,36 +141,54 @@ __device__ __forceinline__ bool stage_grammar(const WideGrammar& W, int start, u
   const int t = threadIdx.x;
   if (W.n_symbols > 256 || start > 255) return false;
   const int rules = W.nt_ptr[W.n_symbols];
-  if (rules < 0 || rules > kTableBytes / 12) return false;
+  if (rules < 0 || rules > kTableRules) return false;
   const int total = W.rhs_ptr[rules];
-  if (total < 0 || 1024 + 12 * rules + total > kTableBytes) return false;
+  if (total < 0 || total > kTableSymbols) return false;
   uint32_t* nt = reinterpret_cast<uint32_t*>(at);
-  uint2* rule = reinterpret_cast<uint2*>(at + 1024);
-  float* cum = reinterpret_cast<float*>(at + 1024 + 8 * rules);
-  uint8_t* rhs = at + 1024 + 12 * rules;
+  float* cum = reinterpret_cast<float*>(at + 1024);
+  uint2* rule = reinterpret_cast<uint2*>(at + 1024 + 4 * kTableRules);
+  uint8_t* rhs = at + 1024 + 12 * kTableRules;
   bool ok = true;
   for (int i = t; i < total; i += blockDim.x) {
     const int v = W.rhs[i];
     ok &= v >= 0 && v < 256;
     rhs[i] = (uint8_t)v;
   }
-  for (int i = t; i < 256; i += blockDim.x) {
-    int r0 = 0, n = 0;
-    if (i < W.n_symbols) {
-      r0 = W.nt_ptr[i];
-      n = W.nt_ptr[i + 1] - r0;
-      ok &= r0 >= 0 && n >= 0 && r0 + n <= rules;
+  if (t < 32) {  // a lane per symbol: its rules' place is a sum over the symbols before it
+    int placed = 0;
+    for (int s0 = 0; s0 < 256; s0 += 32) {
+      const int s = s0 + t;
+      int from = 0, n = 0;
+      if (s < W.n_symbols) {
+        from = W.nt_ptr[s];
+        n = W.nt_ptr[s + 1] - from;
+        const bool in = from >= 0 && n >= 0 && from <= rules - n;
+        ok &= in;
+        if (!in) n = 0;
+      }
+      const int room = (n + 3) & ~3;
+      int upto = room;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (t >= o) upto += x;
+      }
+      const int r0 = placed + upto - room;
+      placed += __shfl_sync(0xffffffffu, upto, 31);
+      const bool fits = placed <= kTableRules;
+      ok &= fits;
+      nt[s] = (uint32_t)(n > 0 ? r0 : 0) | (uint32_t)n << 16;
+      for (int j = 0; fits && j < room; ++j) {
+        const bool real = j < n;
+        const int lo = real ? W.rhs_ptr[from + j] : 0, k = real ? W.rhs_ptr[from + j + 1] - lo : 0;
+        const bool in = lo >= 0 && k >= 0 && lo <= total - k;
+        ok &= in;
+        uint32_t first = 0;
+        for (int i = 0; in && i < k && i < 4; ++i) first |= (uint32_t)(W.rhs[lo + i] & 0xff) << (8 * i);
+        rule[r0 + j] = make_uint2(first, (uint32_t)lo | (uint32_t)k << 16);
+        cum[r0 + j] = real ? W.cum[from + j] : __int_as_float(0x7fffffff);
+      }
     }
-    nt[i] = (uint32_t)(n > 0 ? r0 : 0) | (uint32_t)n << 16;
-  }
-  for (int r = t; r < rules; r += blockDim.x) {
-    const int lo = W.rhs_ptr[r], n = W.rhs_ptr[r + 1] - lo;
-    const bool in = lo >= 0 && n >= 0 && lo + n <= total;
-    ok &= in;
-    uint32_t first = 0;
-    for (int i = 0; in && i < n && i < 4; ++i) first |= (uint32_t)(W.rhs[lo + i] & 0xff) << (8 * i);
-    rule[r] = make_uint2(first, (uint32_t)lo | (uint32_t)n << 16);
-    cum[r] = W.cum[r];
   }
   G = SmallGrammar{nt, cum, rule, rhs};
   return __syncthreads_and(ok);
@@ -292,9 +310,11 @@ __device__ __forceinline__ void derive(const G& g, int start, int64_t beg, int64
 // a step: the symbol at hand in a register, the tables in shared memory and packed
 // (SmallGrammar), rows of an odd number of words per thread (no bank conflicts when a warp
 // writes a finished row), and symbols in a byte, which put 28 warps on an SM instead of 16.
-// 262144 expressions of up to 64 tokens take 320 us where one symbol per turn, the tables
-// read from L1 and 16-bit symbols took 513; 1000 take 144 us (before: 226), 1000000 take 590
-// (1051).  Fewer CTAs per SM, each with a longer queue, are slower: 425 us with two.
+// 262144 expressions of up to 64 tokens take 283 us where one symbol per turn, the tables
+// read from L1 and 16-bit symbols took 513; 1000 take 132 us (before: 226), 1000000 take 501
+// (1051).  With the probabilities read one by one (indexes clamped to the symbol's last) the
+// first took 320 us; with two CTAs per SM, each with a longer queue, 425; with the streams of
+// 32 expressions seeded ahead by all lanes, 343.
 // Other grammars keep 16-bit symbols and their tables in global memory; `wide_threads`
 // threads of the CTA then work (all of them, or the half that shared memory sized for bytes
 // holds).

@@ -97,19 +97,19 @@ GEMM_REPS = 512  # GEMMs per step of the gemm workload (a step long enough to sa
 # The fit kernel's traffic per problem is set by N, M and the history, not by the
 # operator set, so the warm-start line's held-out problems (same lengths, M and N)
 # scale the same B=4096 ragged capture.
-FIT_TRAFFIC_BYTES = {("ragged", 16384, 512): 4 * (10738176 + 2048),
-                     ("warmstart", 65536, 512): 16 * (10738176 + 2048)}
+FIT_TRAFFIC_BYTES = {("ragged", 16384, 512): 4 * (10265344 + 1536),
+                     ("warmstart", 65536, 512): 16 * (10265344 + 1536)}
 # Pipe and issue utilisation of the fit kernel (percent of peak, active cycles) from the
-# same capture, the kernel of commit a0a780f (profiles/fit_lbfgs_ragged_B16384_N512.txt):
+# same capture, the kernel of commit 66b7445 (profiles/fit_lbfgs_ragged_B16384_N512.txt):
 # an interpreter whose instructions are mostly integer and control work.
-FIT_PROFILE = {"commit": "a0a780f", "issue_active_pct": 53.9, "fp32_pipe_pct": 14.9, "xu_pipe_pct": 1.73,
-               "alu_pipe_pct": 48.7, "lsu_pipe_pct": 25.1, "fp64_pipe_pct": 1.68, "warps_active_pct": 23.1,
+FIT_PROFILE = {"commit": "66b7445", "issue_active_pct": 54.8, "fp32_pipe_pct": 15.8, "xu_pipe_pct": 2.5,
+               "alu_pipe_pct": 51.3, "lsu_pipe_pct": 13.9, "fp64_pipe_pct": 2.4, "warps_active_pct": 23.2,
                "capture": "ncu --set full, ragged B=4096, N=512"}
-# The adjoint call: its length-class grids (which stage the cached value rows of the real
-# nodes beside the grad_out rows) and the concurrent padding check, captured with three
-# classes; the split of the longest class at 48 nodes moves the same rows.
+# The adjoint call: its length-class grids (which read the cached value rows of the real
+# nodes beside the grad_out rows) and the concurrent padding check, captured with an earlier
+# kernel that staged the same rows in shared memory.
 EVAL_TRAFFIC_BYTES = {("eval_forward_kernel", 65536, 1024): 16 * (1611520 + 1012199000),
-                      ("eval_backward_kernel", 65536, 1024): 16 * (1364424192 + 13661696)}
+                      ("eval_adjoint_kernel", 65536, 1024): 16 * (1364424192 + 13661696)}
 
 
 def peaks():
@@ -577,9 +577,10 @@ def run_fit(args, rank, world, local):
                            f"history 10, max_iter={max_iter}, strong_wolfe, tol 1e-7, plain randn init",
                  "readme": f"README problem: B={B} expressions of the README grammar (infix <= 32 tokens), "
                            f"N={N}, Y = 2.5 cos(X0) - 1.5, max_iter={max_iter}, strong_wolfe, tol 1e-7"}
-        # per step: tape staging + fit; the warm arm adds the network (random features,
-        # features, 5 GEMMs), and tape staging + one screening launch
-        launches_per_step = 2 + (9 if warm else 0)
+        # per step: tape staging, live rows, work order, fit; the warm arm adds the network
+        # (random features, features, 5 GEMMs), the placed constants, staging and live rows,
+        # one screening launch and the chosen starts
+        launches_per_step = 4 + (12 if warm else 0)
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": head_t * 1000.0, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -732,7 +733,7 @@ def run_eval(args, rank, world, local):
                    "sr_eval_backward_f32")
 
     ktimes = {}
-    for name, fn in (("eval_forward_kernel", fwd_k), ("eval_backward_kernel", bwd_k)):
+    for name, fn in (("eval_forward_kernel", fwd_k), ("eval_adjoint_kernel", bwd_k)):
         for _ in range(3):
             fn()
         ts = []
@@ -787,7 +788,7 @@ def run_eval(args, rank, world, local):
         pk, pk_kind = peaks()
         hbm = float(pk["hbm_gbs"])
         dom = max(ktimes, key=ktimes.get)
-        dom_bytes = bwd_bytes if dom == "eval_backward_kernel" else fwd_bytes
+        dom_bytes = bwd_bytes if dom == "eval_adjoint_kernel" else fwd_bytes
         ach = dom_bytes / ktimes[dom] / 1e9
         line = {"metric": EVAL_METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": t_step * 1000.0, "higher_is_better": True, "scaling": "weak",
@@ -798,12 +799,12 @@ def run_eval(args, rank, world, local):
                 "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                              "traffic": EVAL_TRAFFIC_BYTES.get((dom, B, N)), "kernel": dom, "peak_kind": pk_kind},
                 "kernels": {k: {"ms": v * 1000.0,
-                                "GB/s": (bwd_bytes if k == "eval_backward_kernel" else fwd_bytes) / v / 1e9}
+                                "GB/s": (bwd_bytes if k == "eval_adjoint_kernel" else fwd_bytes) / v / 1e9}
                             for k, v in ktimes.items()},
                 "expressions_per_s": B * world / t_step,
-                # per step: tape compile, padding fill, padding check, and one forward and
-                # one adjoint grid per length class (<= 16, <= 32, longer) the batch reaches
-                "gpu_launches": (3 + 2 * (1 + (tapes.max_len > 16) + (tapes.max_len > 32))) * args.steps,
+                # per step: tape compile, work order, padding fill, padding check, and one forward
+                # and one adjoint grid per length class the batch reaches (three at these lengths)
+                "gpu_launches": (4 + 2 * (1 + (tapes.max_len > 16) + (tapes.max_len > 32))) * args.steps,
                 "clocks": clk.summary()}
         if e2e:
             line["e2e"] = e2e
@@ -978,7 +979,8 @@ def run_sample(args, rank, world, local):
     ok = int((ops != 0).any(dim=1).sum())
     mean_len = float((ops != 0).sum(dim=1).float().mean())
 
-    # the three kernels alone, through the C ABI, on the launching stream
+    # the three kernels alone, through the C ABI, on the launching stream (a sampled batch
+    # also launches the summary of its error words)
     lib, st = _lib.lib(), _lib.stream_ptr(dev)
     nt, cum, rp, rc = pcfg._tables
     infix = torch.empty((B, L), dtype=torch.int64, device=dev)
@@ -1051,7 +1053,7 @@ def run_sample(args, rank, world, local):
                 "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                              "traffic": None, "kernel": dom, "peak_kind": pk_kind},
                 "kernels": {k: {"ms": v * 1000.0, "GB/s": algo[k] / v / 1e9} for k, v in ktimes.items()},
-                "gpu_launches": 3 * args.steps, "clocks": clk.summary()}
+                "gpu_launches": 4 * args.steps, "clocks": clk.summary()}
         if e2e:
             line["e2e"] = e2e
         if cpu:

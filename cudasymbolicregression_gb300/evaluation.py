@@ -12,9 +12,9 @@ and the C++ entry src/symbolic_evaluation.cpp:306-355):
   per tape into a (B, M, N, K) cache (reference symbolic_torch/evaluation.py:36-65);
   ``evaluate_multiple_constant_backend`` is its M-first entry point.
 
-The cache is written directly in (B, M, N) order by one kernel launch (the
-reference launches one kernel per tape position); the adjoint recomputes node
-values and never reads the cache.  Shape, dtype and validation errors carry the
+The cache is written directly in (B, M, N) order by one persistent grid per class of
+tape lengths (the reference launches one kernel per tape position), with the NaN
+padding filled beside it; the adjoint reads the saved cache.  Shape, dtype and validation errors carry the
 reference's messages.
 """
 from __future__ import annotations

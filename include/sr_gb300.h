@@ -91,9 +91,10 @@ int sr_any_nonzero(const int64_t *words_dev, int64_t n, int32_t *out_dev, void *
  * host loop of M launches of evaluation_forward_step_k
  * (reference src/symbolic_evaluation.cpp:39-92, src/evaluation_kernels_cuda.cu:51-216,
  * 634-652).  One warp interprets one tape, lanes over data points, one grid per
- * class of tape lengths; the NaN padding rows are written by a kernel on a
- * library-owned side stream, forked from `stream` and joined back into it before the
- * call returns (a CUDA graph capture of `stream` records both).
+ * class of tape lengths; the NaN padding rows of an output above 8 MB are written by a
+ * kernel on a library-owned side stream, forked from `stream` and joined back into it
+ * before the call returns (a CUDA graph capture of `stream` records both), those of a
+ * smaller one on `stream` itself.
  * max_len: largest meta[0] of the batch (stats[1] of sr_tape_compile), or 0 for M;
  * it sizes the per-warp shared-memory node tables, and a tape whose meta[0] exceeds
  * it is not evaluated: its whole (M, N) block is NaN.  order_dev (B) int32, or NULL:

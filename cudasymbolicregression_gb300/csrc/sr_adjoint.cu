@@ -26,8 +26,11 @@ __device__ __forceinline__ void report_adjoint(int* status, int code) {
 // any bit but its sign is).  What bounds it: HBM reads, together with the adjoint's own.  The
 // copies keep 32 KB of every SM in flight from one warp; the vector loads before it held
 // 16 warps and a quarter of the registers that the adjoint beside it needs (65536 tapes: the
-// two together 5.48 ms with them, 4.12 ms with the copies; 16384 tapes with 3 stages 1160 us,
-// 4 stages 1046, 6 stages 1081).  Every wait gives up after about a second (status 601).
+// two together 5.48 ms with them, 4.5 to 4.9 ms with the copies; 16384 tapes with 3 stages
+// 1160 us, 4 stages 1046, 6 stages 1081).  Two adjoint CTAs leave an SM 4096 registers, too few
+// for this CTA, so where it comes first one of them waits for it.  Three readers of 32 registers
+// fit beside both: 4.08 ms, but 5.9 ms instead of 5.6 where every tape has a gradient, so they
+// are not used.  Every wait gives up after about a second (status 601).
 // A tape longer than the max_len the call was given is adjoined by no class grid: it
 // is reported (status 602) instead of being skipped silently.
 constexpr int kCheckWarps = 4;          // readers
@@ -157,10 +160,11 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
 // each).  The kernel before it staged every grad_out and value row of a chunk in shared
 // memory (256 bytes per node and warp: 12 warps per SM for 64 nodes) and swept one point per
 // lane.  Measured with the check above: 16384 tapes of mean length 20 at N = 1024, 1390 to
-// 1060 us; 65536 tapes 4.90 to 4.12 ms; 1003 tapes at N = 777, 834 to 96 us; 512 float64 tapes
-// at N = 1000, 1850 to 172 us; 1000 tapes at N = 256, K = 8, 1214 to 166 us.  (One warp per
-// tape left most of the GPU idle in the last three.)  A launch bound of three CTAs per SM
-// (80 registers instead of 118) undoes the loads ahead: 1450 us.
+// 1060 us; 1003 tapes at N = 777, 834 to 96 us; 512 float64 tapes at N = 1000, 1850 to 172 us;
+// 1000 tapes at N = 256, K = 8, 1214 to 166 us.  (One warp per tape left most of the GPU idle
+// in the last three.)  At 65536 tapes it is no faster: 4.3 ms became 4.5 to 4.9 with a gradient
+// on the tapes of moderate values only, 4.9 became 5.7 with one on every tape.  A launch bound
+// of three CTAs per SM (80 registers instead of 118) undoes the loads ahead: 1450 us.
 //
 // Sums keep one order whatever the split.  A child's adjoint is its output gradient plus its
 // parent's contribution.  A constant's gradient is summed per residue of the point index mod

@@ -110,7 +110,6 @@ __host__ __device__ __forceinline__ int table_rows(int Lmax) {
 }
 
 int device_sm_count();
-int max_dyn_smem();
 int max_sm_smem();  // shared memory of an SM
 int check_tape_args(int64_t B, int64_t M);
 

@@ -692,11 +692,6 @@ fail:
 
 static unsigned row_blocks(int64_t B) { return (unsigned)((B + sr::kRowThreads - 1) / sr::kRowThreads); }
 
-static int byte_smem(const void* kern, size_t smem) {
-  if (smem <= 48 * 1024) return SR_OK;
-  return sr::cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
-}
-
 // Rows whose tokens, the ids up to `last` included, fit the byte kernels.
 static bool byte_rows(int64_t M, int64_t last) { return M >= 1 && M <= sr::kStackLimit && last <= 255; }
 
@@ -715,7 +710,7 @@ int sr_postfix_children(const int64_t* ops, int64_t B, int64_t M, int32_t n_vars
     const size_t smem = (size_t)3 * kRowThreads * row_stride((int)M);
     auto kern = reinterpret_cast<uintptr_t>(ch) % 16 ? postfix_children_bytes_kernel<false>
                                                      : postfix_children_bytes_kernel<true>;
-    if (const int rc = byte_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
+    if (const int rc = sr::allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
     kern<<<row_blocks(B), kRowThreads, smem, as_stream(stream)>>>(ops, B, (int)M, n_operators, ch, err);
     return launch_check("postfix_children_bytes_kernel");
   }
@@ -737,7 +732,7 @@ int sr_postfix_to_infix(const int64_t* ops, int64_t B, int64_t M, int32_t n_vars
   if (byte_rows(M, n_operators + 1) && M_out <= INT32_MAX / kRowThreads) {
     const int cap = (int)(M_out < 3 * M ? M_out : 3 * M);
     const size_t smem = (size_t)kRowThreads * (2 * row_stride((int)M) + row_stride(cap));
-    if (const int rc = byte_smem(reinterpret_cast<const void*>(postfix_to_infix_bytes_kernel), smem)) return rc;
+    if (const int rc = sr::allow_dynamic_smem(reinterpret_cast<const void*>(postfix_to_infix_bytes_kernel), smem)) return rc;
     postfix_to_infix_bytes_kernel<<<row_blocks(B), kRowThreads, smem, as_stream(stream)>>>(ops, B, (int)M, n_operators,
                                                                                         infix, M_out, cap, err);
     return launch_check("postfix_to_infix_bytes_kernel");
@@ -757,7 +752,7 @@ static int launch_reorder(const int64_t* in, int64_t B, int64_t M, int32_t n_var
   using namespace sr;
   const size_t smem = (size_t)2 * kRowThreads * row_stride((int)M);
   auto kern = reorder_bytes_kernel<kFromPrefix>;
-  if (const int rc = byte_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
+  if (const int rc = sr::allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return rc;
   kern<<<row_blocks(B), kRowThreads, smem, as_stream(stream)>>>(in, B, (int)M, (int64_t)VAR + n_vars, out, err);
   return launch_check(kFromPrefix ? "reorder_bytes_kernel<prefix>" : "reorder_bytes_kernel<postfix>");
 }

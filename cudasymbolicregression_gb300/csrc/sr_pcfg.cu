@@ -674,13 +674,6 @@ __global__ void __launch_bounds__(kThreads) infix_parse_bytes_kernel(const int64
   }
 }
 
-static int max_smem_optin() {
-  int dev = 0, v = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 48 * 1024;
-  if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 48 * 1024;
-  return v;
-}
-
 template <bool kPrefix>
 static int launch_parse(const int64_t* infix, int64_t B, int64_t M, int32_t n_vars, int64_t* outp, int64_t* errors,
                         void* stream) {
@@ -696,7 +689,7 @@ static int launch_parse(const int64_t* infix, int64_t B, int64_t M, int32_t n_va
   if (M >= 1 && VAR + n_vars + 2 <= kByteLimit) {
     const size_t bytes = (size_t)arrays * kThreads * odd_stride((int)M);
     auto kern = infix_parse_bytes_kernel<kPrefix>;
-    const int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem");
+    const int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), bytes);
     if (rc) return rc;
     kern<<<(unsigned)((B + kThreads - 1) / kThreads), kThreads, bytes, as_stream(stream)>>>(infix, B, (int)M, n_vars, outp,
                                                                                            errors);
@@ -704,7 +697,7 @@ static int launch_parse(const int64_t* infix, int64_t B, int64_t M, int32_t n_va
   }
   const size_t smem = (size_t)(arrays * M > 0 ? arrays * M : 1) * kThreads * sizeof(int16_t);
   auto kern = infix_parse_kernel<kPrefix>;
-  int rc = cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem");
+  int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
   const int64_t blocks = (B + kThreads - 1) / kThreads;
   kern<<<(unsigned)blocks, kThreads, smem, as_stream(stream)>>>(infix, B, M, n_vars, outp, errors);
@@ -742,9 +735,8 @@ int sr_pcfg_sample_infix(const int32_t* nt_rule_ptr, const float* nt_rule_cum_pr
   size_t smem = (size_t)wide_threads * (odd_stride(2 * kHardMax) + odd_stride(2 * max_length));
   const size_t narrow = (size_t)kTableBytes + (size_t)kThreads * (odd_stride(kHardMax) + odd_stride(max_length));
   if (bytes && narrow > smem) smem = narrow;
-  if ((int)smem > max_smem_optin()) { set_error("sampling tables do not fit in shared memory"); return SR_ERR_UNSUPPORTED; }
-  int rc = cuda_check(cudaFuncSetAttribute(sample_infix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                      "smem");
+  if (smem > (size_t)max_dyn_smem()) { set_error("sampling tables do not fit in shared memory"); return SR_ERR_UNSUPPORTED; }
+  int rc = allow_dynamic_smem(reinterpret_cast<const void*>(sample_infix_kernel), smem);
   if (rc) return rc;
   // persistent grid: the CTAs that fit at once, or fewer when B is small
   int dev = 0, sms = 0, per_sm = 0;

@@ -145,3 +145,42 @@ def test_sampler_symbol_and_table_sizes(B, length, offset, n_symbols):
     want, want_err = oracle.pcfg_sample(tables, E, B, length, 5, 99)
     np.testing.assert_array_equal(err.cpu().numpy(), want_err)
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+def test_calls_of_several_threads_keep_their_shared_memory():
+    """Threads whose calls need different amounts of shared memory launch the same kernels at
+    the same time: no launch is refused, and every row is right."""
+    import threading
+
+    from cudasymbolicregression_gb300 import _lib
+    L = _lib.lib()
+    sizes = [(128, 384), (128, 200), (100, 300), (128, 300)]
+    rows = [_postfix(300, M, i) for i, (M, _) in enumerate(sizes)]
+    want = [_call("sr_postfix_to_infix", x, 2, width) + _call("sr_postfix_children", x, 2, last=(2,))
+            for x, (_, width) in zip(rows, sizes)]
+    failed = []
+
+    def work(x, width, want):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            xd = torch.tensor(x).cuda()
+            B, M = x.shape
+            out, ch = torch.empty((B, width), dtype=torch.int64).cuda(), torch.empty((B, M, 2), dtype=torch.int64).cuda()
+            err, err_ch = (torch.empty(B, dtype=torch.int64).cuda() for _ in range(2))
+            st = _lib.stream_ptr(xd.device)
+            for _ in range(3000):
+                if L.sr_postfix_to_infix(_lib.ptr(xd), B, M, 2, _lib.ptr(out), width, _lib.ptr(err), st) or \
+                        L.sr_postfix_children(_lib.ptr(xd), B, M, 2, _lib.ptr(ch), _lib.ptr(err_ch), st):
+                    failed.append(L.sr_last_error())
+                    return
+            stream.synchronize()
+            got = [t.cpu().numpy() for t in (out, err, ch, err_ch)]
+            if not all(np.array_equal(a, b) for a, b in zip(got, want)):
+                failed.append("rows differ")
+
+    threads = [threading.Thread(target=work, args=(x, w, e)) for x, (_, w), e in zip(rows, sizes, want)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed

@@ -64,6 +64,7 @@ struct FitArgs {
   int Lmax, Kmax;
   int Imax;         // program entries: largest count of operator nodes
   int Amax;         // most operator-node adjoints live at once
+  int tight;        // see fit_layout
   int Rmax;         // rows of the per-warp table for operator values and adjoints (see stage_problem)
   int VR;           // rows of the per-warp table for variables (distinct variables of a tape)
   unsigned char* ws_hist;  // per CTA: the L-BFGS history block (hist_block_bytes), when not in shared memory
@@ -90,15 +91,23 @@ struct F2 {
 // in U chunks of its warp.  A row holds 32 lanes x P = U V floats, a lane's part in one place,
 // so that it is one shared-memory access.
 struct Layout {
-  int Lmax, Imax, Rmax, Kmax, VR, V, P, W;
+  int Lmax, Imax, Rmax, Kmax, VR, V, U, P, W;
   // byte offsets from the start of shared memory: CTA tables
-  uint32_t red_g, red_l, pvec, red_e, task, info, rowvar, tape, node_slot, slot_node, row_of, adj_of, last, flags, frees,
-      fwd, rev, dst, bc, warps;
+  uint32_t red_g, red_l, pvec, red_e, task, info, rowvar, slot_node, fwd, rev, dst, bc, warps;
+  uint32_t tape, node_slot, row_of, adj_of, last, flags, frees;  // of stage_problem
   uint32_t vars, gl, warp_bytes;  // per warp: operator rows at 0, variable rows, gradient sums
   size_t bytes;
 };
 
-__host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rmax, int Kmax, int V, int U, int W, int VR) {
+constexpr int kFixedLeaves = E_ - C1 + 1;  // fixed constants
+
+// The tables that only stage_problem uses (the tape words; the slot of a LEARNABLE node, program
+// entry of an operator or row of a variable; the value row of an operator) have a place of their
+// own unless that makes the layout too large (tight): then they too sit in the first warps' rows,
+// which are free while it runs.  Always there, they cost the screening kernel 8 to 20% (4096 tapes
+// with shared subtrees, three starts: 590 us against 493).
+__host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rmax, int Kmax, int V, int U, int W, int VR,
+                                                      bool tight) {
   Layout l;
   l.Lmax = Lmax;
   l.Imax = Imax > 0 ? Imax : 1;
@@ -106,6 +115,7 @@ __host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rm
   l.Kmax = Kmax > 0 ? Kmax : 1;
   l.VR = VR;
   l.V = V;
+  l.U = U;
   l.P = V * U;
   l.W = W;
   size_t p = 0;
@@ -122,26 +132,34 @@ __host__ __device__ __forceinline__ Layout fit_layout(int Lmax, int Imax, int Rm
   l.task = take(8);                   // the CTA's current problem
   l.info = take(48);                  // see stage_problem
   l.rowvar = take((size_t)VR * 4);    // [VR] variable held in each variable row
-  l.tape = take(n * 4);
-  l.node_slot = take(n * 4);          // slot of a LEARNABLE node / program entry of an operator / row of a variable
+  if (!tight) {
+    l.tape = take(n * 4);
+    l.node_slot = take(n * 4);
+    l.row_of = take(n * 4);
+  }
   l.slot_node = take(K * 4);
-  l.row_of = take(n * 4);             // value row of an operator node
   l.fwd = take(I * 16);               // forward program: opcode, two operand words, destination row
   l.rev = take(I * 16);               // reverse program: opcode | no parent << 8, two operand words, adjoint row
   l.dst = take(I * 8);                // reverse program: where the operands' adjoints go
-  l.bc = take((1 + K + n) * 4 * (size_t)l.P);  // broadcast values, P copies each: 0, constants, fixed constants
+  l.bc = take((1 + K + kFixedLeaves) * 4 * (size_t)U);  // broadcast values, U copies each: 0, constants, fixed constants
   p = (p + 127) & ~size_t(127);
   l.warps = (uint32_t)p;
   const uint32_t row = 128u * (uint32_t)l.P;
   l.vars = (uint32_t)l.Rmax * row;
   l.gl = l.vars + (uint32_t)VR * row;  // [K][32 V] per-lane, per-point gradient sums
   l.warp_bytes = l.gl + (uint32_t)K * 128u * (uint32_t)V;
-  // scratch of stage_problem in the first warp's rows (adjoint rows, last uses, marks, free rows)
-  l.adj_of = l.warps;
+  uint32_t at = l.warps;
+  if (tight) {
+    l.tape = at;
+    l.node_slot = l.tape + 4u * (uint32_t)n;
+    l.row_of = l.node_slot + 4u * (uint32_t)n;
+    at = l.row_of + 4u * (uint32_t)n;
+  }
+  l.adj_of = at;
   l.last = l.adj_of + 4u * (uint32_t)n;
   l.flags = l.last + 4u * (uint32_t)n;
   l.frees = l.flags + 4u * (uint32_t)n;
-  const size_t scratch = 4 * n * 4 + 4 * (size_t)((l.Rmax > Lmax ? l.Rmax : Lmax) + 1);
+  const size_t scratch = (tight ? 7 : 4) * n * 4 + 4 * (size_t)((l.Rmax > Lmax ? l.Rmax : Lmax) + 1);
   size_t total = (size_t)W * l.warp_bytes;
   if (total < scratch) total = scratch;
   l.bytes = p + fit_align16(total);
@@ -168,8 +186,7 @@ struct WarpSmem {
 };
 
 // Problem facts in info: operator nodes, variable rows in use, the root's operand word, where
-// its adjoint goes, whether a constant has several parents, whether the rows suffice, and
-// whether the variable rows hold for every closure (see fill_variables).
+// its adjoint goes, whether a constant has several parents, whether the rows do not suffice.
 enum Info : int { kOps = 0, kVars = 1, kRootSrc = 2, kRootDst = 3, kSharedConst = 4, kTooFew = 5 };
 
 __device__ __forceinline__ WarpSmem carve(unsigned char* base, const Layout& l, int warp) {
@@ -661,11 +678,11 @@ enum DstKind : uint32_t { kDstNone = 0, kDstFirst = 1, kDstAdd = 2, kDstSum = 3 
 __device__ __forceinline__ uint32_t operand_word(const uint32_t* tape, const int* node_slot, const int* row_of, int c,
                                                  const Layout& l) {
   const int code = code_of(tape[c]);
-  const uint32_t row = 128u * (uint32_t)l.P, entry = 4u * (uint32_t)l.P;
+  const uint32_t row = 128u * (uint32_t)l.P, entry = 4u * (uint32_t)l.U;
   if (is_operator_node(code)) return kRowOperand | ((uint32_t)row_of[c] * row);
   if (code == VAR) return kRowOperand | (l.vars + (uint32_t)node_slot[c] * row);
   if (code == LEARNABLE) return l.bc + entry * (1u + (uint32_t)node_slot[c]);
-  if (is_fixed_leaf(code)) return l.bc + entry * (1u + (uint32_t)l.Kmax + (uint32_t)c);
+  if (is_fixed_leaf(code)) return l.bc + entry * (1u + (uint32_t)l.Kmax + (uint32_t)(code - C1));
   return l.bc;  // the zero entry
 }
 
@@ -689,8 +706,17 @@ __device__ __forceinline__ void sts_pack(unsigned char* p, const float (&r)[P]) 
 }
 
 // The operand of a word for this lane; lane_rows = the lane's place in row 0 of its warp.
-template <int P>
+// A broadcast entry holds U copies: with one chunk at a time a single value serves all points.
+template <int U, int P>
 __device__ __forceinline__ void fetch_operand(const unsigned char* base, uint32_t w, uint32_t lane_rows, float (&r)[P]) {
+  if constexpr (U != P) {
+    if ((int)w >= 0) {
+      const float x = *reinterpret_cast<const float*>(base + w);
+#pragma unroll
+      for (int i = 0; i < P; ++i) r[i] = x;
+      return;
+    }
+  }
   if ((int)w < 0) w += lane_rows - kRowOperand;
   lds_pack<P>(base + w, r);
 }
@@ -779,8 +805,8 @@ __device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, 
     if (nI > 0) {
       uint4 wn = S.fwd[0], wnn = nI > 1 ? S.fwd[1] : wn;
       float an[P], cn[P];
-      fetch_operand<P>(base, wn.y, lane_rows, an);
-      fetch_operand<P>(base, wn.z, lane_rows, cn);
+      fetch_operand<U, P>(base, wn.y, lane_rows, an);
+      fetch_operand<U, P>(base, wn.z, lane_rows, cn);
       for (int i = 0; i < nI; ++i) {
         const uint4 w = wn;
         wn = wnn;
@@ -791,8 +817,8 @@ __device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, 
           a[j] = an[j];
           c[j] = cn[j];
         }
-        fetch_operand<P>(base, wn.y, lane_rows, an);
-        fetch_operand<P>(base, wn.z, lane_rows, cn);
+        fetch_operand<U, P>(base, wn.y, lane_rows, an);
+        fetch_operand<U, P>(base, wn.z, lane_rows, cn);
         op_value_v<float, P>((int)(w.x & 0xffu), a, c, r);
         sts_pack<P>(my_rows + w.w, r);
 #pragma unroll
@@ -803,7 +829,7 @@ __device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, 
       }
     }
     float f[P];
-    fetch_operand<P>(base, root_src, lane_rows, f);
+    fetch_operand<U, P>(base, root_src, lane_rows, f);
     if constexpr (kMode == kPassYFinal) {
 #pragma unroll
       for (int i = 0; i < P; ++i)
@@ -854,8 +880,8 @@ __device__ __forceinline__ float tape_pass(const FitArgs& A, const WarpSmem& S, 
         bool a0[P], a1[P];
         int e[P];
         lds_pack<P>(my_rows + w.w, g);
-        fetch_operand<P>(base, w.y, lane_rows, a);
-        fetch_operand<P>(base, w.z, lane_rows, c);
+        fetch_operand<U, P>(base, w.y, lane_rows, a);
+        fetch_operand<U, P>(base, w.z, lane_rows, c);
         if (w.x & 0x100u) {  // a node without a parent: a zero adjoint
 #pragma unroll
           for (int i = 0; i < P; ++i) g[i] = 0.f;
@@ -970,7 +996,7 @@ __device__ __forceinline__ void publish_constants(const WarpSmem& S, const Layou
 #pragma unroll
   for (int s = 0; s < SPL; ++s)
     if (P.real(s))
-      for (int i = 0; i < l.P; ++i) bc[(1 + s * 32 + P.lane) * l.P + i] = x.v[s];
+      for (int i = 0; i < l.U; ++i) bc[(1 + s * 32 + P.lane) * l.U + i] = x.v[s];
 }
 
 // Closure: publish the trial constants, run the pass over this warp's points,
@@ -1296,13 +1322,12 @@ __device__ __forceinline__ bool stage_problem(const FitArgs& A, const WarpSmem& 
     }
     // broadcast entries: 0 and the fixed constants of the tape
     float* bc = reinterpret_cast<float*>(S.base + l.bc);
-    if (lane < l.P) bc[lane] = 0.f;
-    for (int k = lane; k < L; k += 32) {
-      const int code = code_of(S.tape[k]);
-      if (is_fixed_leaf(code)) {
-        const float x = node_value<float>(code, 0.f, 0.f, 0.f, 0.f);
-        for (int i = 0; i < l.P; ++i) bc[(1 + l.Kmax + k) * l.P + i] = x;
-      }
+    if (lane < l.U) bc[lane] = 0.f;
+    if (lane < kFixedLeaves) {
+      const float x = lane == PI_ - C1  ? node_value<float>(PI_, 0.f, 0.f, 0.f, 0.f)
+                      : lane == E_ - C1 ? node_value<float>(E_, 0.f, 0.f, 0.f, 0.f)
+                                        : (float)(lane + 1);
+      for (int i = 0; i < l.U; ++i) bc[(1 + l.Kmax + lane) * l.U + i] = x;
     }
   }
   __syncthreads();
@@ -1334,7 +1359,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
   const float tolf = __double2float_rn(A.tol);
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, A.tight != 0);
   const WarpSmem S = carve(smem, l, warp);
   // the L-BFGS history of this CTA (used by warp 0)
   const History H = history_at<SPL>(
@@ -1726,7 +1751,7 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
                                                             int64_t K, float* __restrict__ loss_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, A.tight != 0);
   const WarpSmem S = carve(smem, l, warp);
   for (int64_t b = blockIdx.x; b < A.B; b += gridDim.x) {
     const int L = A.meta[b * 4 + 1] + 1;
@@ -1746,7 +1771,7 @@ __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const flo
       const float* Cin = C_sets + k * c_sk + b * A.c_sb;
       for (int j = threadIdx.x; j < Kc; j += blockDim.x) {
         const float x = Cin[(int64_t)S.slot_node[j] * A.c_sm];
-        for (int i = 0; i < l.P; ++i) bc[(1 + j) * l.P + i] = x;
+        for (int i = 0; i < l.U; ++i) bc[(1 + j) * l.U + i] = x;
       }
       __syncthreads();  // also: thread 0 has read the previous candidate's warp sums
       int dummy = 0;
@@ -1938,6 +1963,7 @@ static int spl_for(int Kmax) {
 
 struct FitShape {
   int V, U, SPL, warps, blocks, Imax, Amax, Rmax, VR;
+  bool tight;
   size_t smem;
   size_t ring_off;  // > 0: the L-BFGS history sits in shared memory from this byte offset
 };
@@ -2010,14 +2036,16 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
   const int V = o.points_per_lane ? o.points_per_lane : 1;
   double best = -1.0;
   int bestPerSm = 0;
+  bool tight = false;
   auto resident = [&](int u, int w, size_t& bytes) -> int {  // CTAs per SM, 0 if they do not fit, < 0 for an error
     void* k = pick_kernel(V, u, sh.SPL);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return -1;
-    bytes = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, u, w, sh.VR).bytes;
+    bytes = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, u, w, sh.VR, tight).bytes;
     return bytes > (size_t)optin ? 0 : resident_ctas(k, w * 32, bytes);
   };
   for (int w = W; w >= 1 && best < 0; w >>= 1) {
     size_t bytes = 0;
+    tight = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, 1, w, sh.VR, false).bytes > (size_t)optin;
     const int one = resident(1, w, bytes);
     if (one < 0) {
       set_error("fit kernel shared memory attribute failed");
@@ -2027,6 +2055,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
       best = 1.0;
       W = w;
       sh.U = 1;
+      sh.tight = tight;
       bestPerSm = one;
       sh.smem = bytes;
       if (V == 1 && N > (int64_t)32 * w) {
@@ -2154,14 +2183,14 @@ int sr_fit_screen(const float* X, int64_t N, int64_t n_x, const float* Y, const 
   A.desc = desc; A.meta = meta; A.B = B; A.M = M;
   A.c_sb = c_sb; A.c_sm = c_sm;
   A.objective = o.objective;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR; A.tight = sh.tight;
   A.status = status;
   // a forward pass alone gains less from two chunks at once than it loses with the CTAs that
   // the doubled rows displace (2048 problems of two starts, N = 512: 280 us against 237)
   void* k = sh.V == 1 ? reinterpret_cast<void*>(fit_screen_kernel<1, 1>)
                       : (sh.V == 2 ? reinterpret_cast<void*>(fit_screen_kernel<2, 1>)
                                    : reinterpret_cast<void*>(fit_screen_kernel<4, 1>));
-  const size_t smem = fit_layout(Lmax, sh.Imax, sh.Rmax, max_consts, sh.V, 1, sh.warps, sh.VR).bytes;
+  const size_t smem = fit_layout(Lmax, sh.Imax, sh.Rmax, max_consts, sh.V, 1, sh.warps, sh.VR, sh.tight).bytes;
   int dev = 0, optin = 0;
   if (cuda_check(cudaGetDevice(&dev), "cudaGetDevice") ||
       cuda_check(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev), "shared memory limit") ||
@@ -2223,7 +2252,7 @@ int sr_fit_lbfgs(const float* X, int64_t N, int64_t n_x, const float* Y, const u
   A.order = order;
   A.max_iter = o.max_iter; A.hist = o.history_size; A.ls_kind = o.line_search; A.ls_max = o.line_search_max_iter;
   A.objective = o.objective; A.tol = o.tolerance_grad; A.eps = o.eps;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR; A.tight = sh.tight;
   A.counter = reinterpret_cast<int*>(ws);
   A.ws_hist = sh.ring_off ? nullptr : ws + 256;
   A.ring_off = (int)sh.ring_off;

@@ -67,3 +67,22 @@ def test_shared_subtrees_bit_identical(N, W, share_constants):
     first = oracle.optimize(X, Y, ops, ch, C, max_iter=0, dot_mode=2, warps=W, points_per_lane=1)["loss"]
     fine = np.isfinite(first)
     np.testing.assert_allclose(losses[fine], first[fine], rtol=1e-6)
+
+
+@pytest.mark.parametrize("L", [741, 743, 781])
+def test_longest_tapes_that_the_tables_hold(L):
+    """Chains of operators, whose tables take the most shared memory: up to 781 nodes fit."""
+    import cudasymbolicregression_gb300 as sr
+    from parity import fit_bits_differ, oracle_fit_like
+    rng = np.random.default_rng(L)
+    B, N = 3, 40
+    ops = np.zeros((B, L), np.int64)
+    ch = np.full((B, L, 2), -1, np.int64)
+    ops[:, :3], ch[:, 2] = (50, 1, 40), (0, 1)
+    ops[:, 3:] = rng.choice((10, 11, 27), size=(B, L - 3))
+    ch[:, 3:, 0] = np.arange(2, L - 1)
+    X = rng.uniform(-1, 1, (N, 1)).astype(np.float32)
+    Y = rng.uniform(-1, 1, (B, N)).astype(np.float32)
+    C = rng.uniform(-1, 1, (B, L)).astype(np.float32)
+    r = sr.optimize_ex(cuda(X), cuda(Y), cuda(ops), cuda(ch), cuda(C), max_iter=3, raise_errors=False)
+    assert not fit_bits_differ(r, oracle_fit_like(r, X, Y, ops, ch, C, max_iter=3)).any()

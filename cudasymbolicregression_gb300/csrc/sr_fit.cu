@@ -1963,6 +1963,7 @@ static int spl_for(int Kmax) {
 
 struct FitShape {
   int V, U, SPL, warps, blocks, Imax, Amax, Rmax, VR;
+  int blocks_one;  // the grid with one chunk at a time (U = 1), whose CTAs fit at least as often
   bool tight;
   size_t smem;
   size_t ring_off;  // > 0: the L-BFGS history sits in shared memory from this byte offset
@@ -2035,7 +2036,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
   if (W > 8) W = 8;  // __launch_bounds__(256)
   const int V = o.points_per_lane ? o.points_per_lane : 1;
   double best = -1.0;
-  int bestPerSm = 0;
+  int bestPerSm = 0, onePerSm = 0;
   bool tight = false;
   auto resident = [&](int u, int w, size_t& bytes) -> int {  // CTAs per SM, 0 if they do not fit, < 0 for an error
     void* k = pick_kernel(V, u, sh.SPL);
@@ -2056,7 +2057,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
       W = w;
       sh.U = 1;
       sh.tight = tight;
-      bestPerSm = one;
+      bestPerSm = onePerSm = one;
       sh.smem = bytes;
       if (V == 1 && N > (int64_t)32 * w) {
         const int two = resident(2, w, bytes);
@@ -2085,18 +2086,28 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
       sh.smem = with;
     }
   }
-  int64_t blocks = o.grid_blocks > 0 ? o.grid_blocks : (int64_t)sms * bestPerSm;
-  if (blocks > B) blocks = B;  // one problem per CTA at a time
-  if (blocks < 1) blocks = 1;
-  sh.blocks = (int)blocks;
+  auto grid = [&](int per_sm) {
+    int64_t blocks = o.grid_blocks > 0 ? o.grid_blocks : (int64_t)sms * per_sm;
+    if (blocks > B) blocks = B;  // one problem per CTA at a time
+    return (int)(blocks < 1 ? 1 : blocks);
+  };
+  sh.blocks = grid(bestPerSm);
+  sh.blocks_one = grid(onePerSm);
   return SR_OK;
 }
 
-// Workspace of a launch: the work counter, and the L-BFGS history unless it sits in
-// shared memory (rings_anyway: the size with the history, an upper bound for any n_x).
-static int64_t ws_bytes_for(const FitShape& sh, int hist, bool rings_anyway = false) {
-  if (sh.ring_off && !rings_anyway) return 256;
-  return 256 + (int64_t)sh.blocks * (int64_t)hist_block_bytes(hist, sh.SPL);
+// Workspace of a launch: the work counter, and the L-BFGS history of every CTA unless it sits in
+// shared memory.
+static int64_t ws_bytes_for(const FitShape& sh, int hist) {
+  return 256 + (sh.ring_off ? 0 : (int64_t)sh.blocks * (int64_t)hist_block_bytes(hist, sh.SPL));
+}
+
+// The grid that a workspace of this size holds: fewer persistent CTAs only lengthen each one's
+// share of the queue.
+static void fit_workspace(FitShape& sh, int hist, int64_t bytes) {
+  if (sh.ring_off || ws_bytes_for(sh, hist) <= bytes) return;
+  const int64_t blocks = (bytes - 256) / (int64_t)hist_block_bytes(hist, sh.SPL);
+  sh.blocks = blocks < 1 ? 1 : (int)blocks;
 }
 
 }  // namespace sr
@@ -2112,12 +2123,12 @@ int64_t sr_fit_workspace_bytes(int64_t B, int64_t N, int64_t M, int32_t max_len,
     return -1;
   }
   sr::FitShape sh;
-  // the same node-table size sr_fit_lbfgs uses; one variable row gives the smallest
-  // tables, hence the most resident CTAs: an upper bound for any n_x (sr_fit_lbfgs
-  // shrinks its grid to the workspace it is given)
+  // the same node-table size sr_fit_lbfgs uses; one variable row and one chunk at a time
+  // give the smallest tables, hence the most resident CTAs of these warps: an upper bound for
+  // any n_x (sr_fit_lbfgs takes the grid that the workspace it is given holds)
   const int Lmax = (max_len > 0 && max_len < M) ? max_len : (int)(M < 1 ? 1 : M);
   if (sr::fit_shape(B, N, 1, Lmax, max_consts, o, sh)) return -1;
-  return sr::ws_bytes_for(sh, o.history_size, true);
+  return 256 + (int64_t)sh.blocks_one * (int64_t)sr::hist_block_bytes(o.history_size, sh.SPL);
 }
 
 int sr_tape_live_rows(const uint32_t* desc, const int32_t* meta, int64_t B, int64_t M, int32_t* stats, void* stream) {
@@ -2235,9 +2246,7 @@ int sr_fit_lbfgs(const float* X, int64_t N, int64_t n_x, const float* Y, const u
   const int Lmax = (max_len > 0 && max_len < M) ? max_len : (int)M;
   rc = fit_shape(B, N, n_x, Lmax, max_consts, o, sh);
   if (rc) return rc;
-  // fewer persistent CTAs only lengthen each one's share of the queue
-  while (sh.blocks > 1 && ws_bytes_for(sh, o.history_size) > workspace_bytes)
-    sh.blocks = sh.blocks > 8 ? sh.blocks * 3 / 4 : sh.blocks - 1;
+  fit_workspace(sh, o.history_size, workspace_bytes);
   const int64_t need = ws_bytes_for(sh, o.history_size);
   if (workspace_bytes < need) {
     set_error("workspace too small: %lld < %lld bytes", (long long)workspace_bytes, (long long)need);
@@ -2310,32 +2319,23 @@ extern "C" int sr_fit_lbfgs_static_scratch(const float* X, int64_t N, int64_t n_
   if (B == 0 || M == 0) return sr_fit_lbfgs(X, N, n_x, Y, desc, meta, B, M, C_init, C_out, c_sb, c_sm, Y_final,
                                             iters_out, loss_out, evals_out, order, max_len, max_consts, &o, nullptr,
                                             0, status, stream);
-  // Persistent grid: fewer CTAs only lengthen the work queue per warp, so shrink the
-  // grid until its L-BFGS history fits in the static array.
+  // the grid whose L-BFGS history fits in the static array
   FitShape sh;
   const int Lmax = (max_len > 0 && max_len < M) ? max_len : (int)M;
   rc = fit_shape(B, N, n_x, Lmax, max_consts, o, sh);
   if (rc) return rc;
-  int64_t blocks = sh.blocks;
-  while (blocks >= 1) {
-    FitShape t = sh;
-    t.blocks = (int)blocks;
-    if (ws_bytes_for(t, o.history_size) <= kStaticFitScratchBytes) break;
-    blocks = blocks > 8 ? blocks * 3 / 4 : blocks - 1;
-  }
-  if (blocks < 1) {
-    FitShape t = sh;
-    t.blocks = 1;
+  fit_workspace(sh, o.history_size, kStaticFitScratchBytes);
+  if (ws_bytes_for(sh, o.history_size) > kStaticFitScratchBytes) {
     set_error("static fit scratch is %lld bytes; one CTA of %d warps needs %lld (history_size=%d, up to %d constants); "
               "use sr_fit_lbfgs with a caller workspace",
-              (long long)kStaticFitScratchBytes, sh.warps, (long long)ws_bytes_for(t, o.history_size), o.history_size,
+              (long long)kStaticFitScratchBytes, sh.warps, (long long)ws_bytes_for(sh, o.history_size), o.history_size,
               max_consts);
     return SR_ERR_WORKSPACE;
   }
   void* scratch = nullptr;
   rc = static_scratch_address(&scratch);
   if (rc) return rc;
-  o.grid_blocks = (int32_t)blocks;
+  o.grid_blocks = sh.blocks;
   o.warps_per_block = sh.warps;
   o.points_per_lane = sh.V;
   return sr_fit_lbfgs(X, N, n_x, Y, desc, meta, B, M, C_init, C_out, c_sb, c_sm, Y_final, iters_out, loss_out,

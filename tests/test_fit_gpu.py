@@ -609,3 +609,23 @@ def test_shards_fitted_with_the_batch_launch_shape_equal_the_whole_fit():
     assert alone[1].shapes[0][2] == 8 and whole.shapes[0][2] == 4
     C_alone = torch.cat([a.C for a in alone]).cpu().numpy()
     assert not np.array_equal(bits(C_alone), bits(whole.C.cpu().numpy()))
+
+
+@pytest.mark.parametrize("n_x", [1, 2, 8, 16, 40])
+@pytest.mark.parametrize("N,max_len,ops,live,rows,consts,W", [(256, 96, 60, 40, 88, 30, 4), (400, 200, 100, 60, 121, 8, 2),
+                                                              (512, 64, 43, 12, 38, 12, 8)])
+def test_workspace_holds_the_grid_of_any_number_of_variables(n_x, N, max_len, ops, live, rows, consts, W):
+    """sr_fit_workspace_bytes, which is not told n_x, covers the history of every CTA that a
+    launch takes: where more variable rows turn the passes over two chunks off, more CTAs fit."""
+    import ctypes
+
+    from cudasymbolicregression_gb300 import _lib
+    L = _lib.lib()
+    B = 100000
+    o = _lib.FitOptions(max_iter=10, history_size=10, tolerance_grad=1e-7, line_search=0, line_search_max_iter=10,
+                        eps=1e-10, warps_per_block=W, max_operators=ops,
+                        max_live=_lib.LIVE_ROWS_COUNTED | rows << 15 | live)
+    block = L.sr_fit_workspace_bytes(1, N, max_len, max_len, consts, o) - 256  # one CTA's history
+    shape = (ctypes.c_int32 * 3)()
+    assert L.sr_fit_launch_shape(B, N, n_x, max_len, max_len, consts, o, ctypes.cast(shape, ctypes.c_void_p)) == 0
+    assert L.sr_fit_workspace_bytes(B, N, max_len, max_len, consts, o) >= 256 + shape[2] * block

@@ -1,5 +1,7 @@
 // sr_adjoint.cu -- adjoint of the forward evaluation for a dense output gradient: the
 // padding-row check and the adjoint proper.
+#include <type_traits>
+
 #include "sr_eval.cuh"
 
 namespace sr {
@@ -25,12 +27,8 @@ __device__ __forceinline__ void report_adjoint(int* status, int code) {
 // with bulk copies, and the others look for a nonzero word (a float or double is nonzero when
 // any bit but its sign is).  What bounds it: HBM reads, together with the adjoint's own.  The
 // copies keep 32 KB of every SM in flight from one warp; the vector loads before it held
-// 16 warps and a quarter of the registers that the adjoint beside it needs (65536 tapes: the
-// two together 5.48 ms with them, 4.5 to 4.9 ms with the copies; 16384 tapes with 3 stages
-// 1160 us, 4 stages 1046, 6 stages 1081).  Two adjoint CTAs leave an SM 4096 registers, too few
-// for this CTA, so where it comes first one of them waits for it.  Three readers of 32 registers
-// fit beside both: 4.08 ms, but 5.9 ms instead of 5.6 where every tape has a gradient, so they
-// are not used.  Every wait gives up after about a second (status 601).
+// 16 warps and a quarter of the registers that the adjoint beside it needs (16384 tapes with 3 stages
+// 1160 us, 4 stages 1046, 6 stages 1081).  Every wait gives up after about a second (status 601).
 // A tape longer than the max_len the call was given is adjoined by no class grid: it
 // is reported (status 602) instead of being skipped silently.
 constexpr int kCheckWarps = 4;          // readers
@@ -91,14 +89,21 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
       ++turn;
       return true;
     };
-    for (int64_t b = blockIdx.x; b < B && !stuck; b += gridDim.x) {
-      const int64_t L = meta[b * 4];
+    // the lengths of its next 32 tapes at once, and as often a look at whether there is anything
+    // left to find
+    int lens = 0;
+    int64_t seen = 0;
+    for (int64_t b = blockIdx.x; b < B && !stuck; b += gridDim.x, ++seen) {
+      if ((seen & 31) == 0) {
+        const int64_t mine = b + (int64_t)lane * gridDim.x;
+        lens = mine < B ? meta[mine * 4] : 0;
+        if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int32_t*>(status), 0) == ERR_GRAD_ON_NO_OP) break;
+      }
+      const int64_t L = __shfl_sync(0xffffffffu, lens, (int)(seen & 31));
       if (L > Lmax) {
         if (lane == 0) report(status, SR_TAPE_EXCEEDS_LAUNCH);
         continue;
       }
-      // nothing more to find once a 201 is recorded
-      if (__shfl_sync(0xffffffffu, *reinterpret_cast<volatile int32_t*>(status), 0) == ERR_GRAD_ON_NO_OP) break;
       const T* p = gout + (size_t)b * M * N + (size_t)L * N;
       const size_t count = (size_t)(M - L) * N;
       size_t head = ((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(T);
@@ -144,6 +149,61 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
   if (__any_sync(0xffffffffu, stuck) && lane == 0) report(status, SR_MLP_TIMEOUT);
 }
 
+// The check beside the staged kernel, which takes the shared memory that the ring needs: one CTA
+// per tape (grid-stride), 16-byte streaming loads, four in flight per thread.
+template <typename T>
+__global__ void __launch_bounds__(256) padding_check_direct_kernel(const T* __restrict__ gout,
+                                                                   const int32_t* __restrict__ meta, int64_t B,
+                                                                   int64_t M, int64_t N, int Lmax,
+                                                                   int32_t* __restrict__ status) {
+  constexpr int kVec = 16 / sizeof(T);
+  for (int64_t b = blockIdx.x; b < B; b += gridDim.x) {
+    // the whole CTA stops once a 201 is recorded (uniform decision)
+    if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int32_t*>(status) == ERR_GRAD_ON_NO_OP))
+      return;
+    const int64_t L = meta[b * 4];
+    if (L > Lmax) {
+      if (threadIdx.x == 0) report(status, SR_TAPE_EXCEEDS_LAUNCH);
+      continue;
+    }
+    const T* p = gout + (size_t)b * M * N + (size_t)L * N;
+    const size_t count = (size_t)(M - L) * N;
+    size_t head = (size_t)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(T);
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(T)) head = count;  // unaligned elements: one by one
+    if (head > count) head = count;
+    bool nz = false;
+    for (size_t i = threadIdx.x; i < head; i += blockDim.x) nz |= __ldcs(p + i) != T(0);
+    const size_t nvec = (count - head) / kVec;
+    const float4* q = reinterpret_cast<const float4*>(p + head);
+    size_t i = threadIdx.x;
+    for (; i + 3 * blockDim.x < nvec; i += 4 * blockDim.x) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldcs(q + i + u * blockDim.x);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (sizeof(T) == 4) {
+          nz |= (v[u].x != 0.f) | (v[u].y != 0.f) | (v[u].z != 0.f) | (v[u].w != 0.f);
+        } else {
+          const double* d = reinterpret_cast<const double*>(&v[u]);
+          nz |= (d[0] != 0.0) | (d[1] != 0.0);
+        }
+      }
+    }
+    for (; i < nvec; i += blockDim.x) {
+      const float4 v = __ldcs(q + i);
+      if (sizeof(T) == 4) {
+        nz |= (v.x != 0.f) | (v.y != 0.f) | (v.z != 0.f) | (v.w != 0.f);
+      } else {
+        const double* d = reinterpret_cast<const double*>(&v);
+        nz |= (d[0] != 0.0) | (d[1] != 0.0);
+      }
+    }
+    for (size_t j = head + nvec * kVec + threadIdx.x; j < count; j += blockDim.x) nz |= __ldcs(p + j) != T(0);
+    if (__syncthreads_or(nz) && threadIdx.x == 0) report_adjoint(status, ERR_GRAD_ON_NO_OP);
+  }
+}
+
 // ------------------------------------------------------------------------------------
 // Adjoint.  Work unit = (tape, all or one of its constant sets), one warp or,
 // for small batches, several warps of a CTA.  The unit's values per node (points, or points x
@@ -162,9 +222,10 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
 // lane.  Measured with the check above: 16384 tapes of mean length 20 at N = 1024, 1390 to
 // 1060 us; 1003 tapes at N = 777, 834 to 96 us; 512 float64 tapes at N = 1000, 1850 to 172 us;
 // 1000 tapes at N = 256, K = 8, 1214 to 166 us.  (One warp per tape left most of the GPU idle
-// in the last three.)  At 65536 tapes it is no faster: 4.3 ms became 4.5 to 4.9 with a gradient
-// on the tapes of moderate values only, 4.9 became 5.7 with one on every tape.  A launch bound
-// of three CTAs per SM (80 registers instead of 118) undoes the loads ahead: 1450 us.
+// in the last three.)  It issues as many instructions per value as the kernel before it did, so
+// large batches, which fill the GPU either way, go to that one (see eval_adjoint_staged_kernel).  A
+// launch bound of three CTAs per SM (80 registers) undoes the loads ahead: 1450 us; prefetching
+// the next pass's rows into L2 adds instructions and gains nothing (5.9 to 7.4 ms at 65536).
 //
 // Sums keep one order whatever the split.  A child's adjoint is its output gradient plus its
 // parent's contribution.  A constant's gradient is summed per residue of the point index mod
@@ -178,61 +239,74 @@ __global__ void __launch_bounds__((kCheckWarps + 1) * 32) padding_check_kernel(c
 // the leaves of a variable at its value, so that there is one atomic for all of them (and the
 // sum over a tape's leaves has one order); more than 16 variables go straight to the atomics.
 //
-// Tapes whose child table is not that of a stack, or that need more rows than the table has,
-// take one adjoint row per node, set to its output gradient before the sweep, and one value
-// per lane.  So do calls without a cache, which recompute the node values into rows first.
+// Tapes whose child table is not that of a stack, or that need more rows than the table has, take
+// a general sweep: one adjoint row per operator, and per leaf with several parents, of one or two
+// values per lane, as many as the table then holds.  A node's first parent in the sweep starts
+// from its output gradient, the others add to the row, and a leaf's last one hands the sum on.
+// Calls without a cache take it with one value per lane and recompute the node values into rows.
 // ------------------------------------------------------------------------------------
 
 // Shared memory of a CTA: the tape words (offset 0); the program, from the front 16 bytes per
 // operator and from the back 4 bytes per leaf without a parent; per node its row or constant
-// index; the nodes of the learnable constants; the constants' values (learnable j at j, fixed
+// index; the nodes of the learnable constants (and from the back those of the variables); the
+// constants' values (learnable j at j, fixed
 // f at L - 1 - f, one entry per set); the sums of ncap constants (32 K lanes each); the first
 // error of each point residue; then per warp the adjoint rows, without a cache a value row
 // per node, with several warps the terms of one pass, and with grad_X the sums of one pass
 // for each variable.
 struct AdjLayout {
   size_t prog, cidx, lcon, cval, acc, errs, warps, warp_bytes, vals, crow, xacc, bytes;
-  int ncap;
 };
 
 template <typename T>
-__host__ __device__ __forceinline__ AdjLayout adjoint_layout(int Lmax, int64_t K, int nwarp, bool recompute, int xrows) {
+__host__ __device__ __forceinline__ AdjLayout adjoint_layout(int Lmax, int64_t K, int nwarp, bool recompute, int xrows,
+                                                             int ncap) {
   AdjLayout l;
-  // constants summed in one sweep: half the nodes of a tree are leaves, few of them
-  // constants; a tape with more is swept again for the rest
-  int cap = (Lmax + 1) / 2;
-  if (cap > 12) cap = 12;
-  const int64_t room = (int64_t)(24 << 10) / (K * 32 * (int64_t)sizeof(T));
-  if (cap > room) cap = room < 1 ? 1 : (int)room;
-  if (nwarp > 1 && cap > 8) cap = 8;
-  l.ncap = cap;
   l.prog = align16((size_t)Lmax * 4);
   l.cidx = l.prog + 16 * (size_t)Lmax;
   l.lcon = l.cidx + align16((size_t)Lmax * 4);
   l.cval = l.lcon + align16((size_t)Lmax * 4);
   l.acc = l.cval + align16((size_t)Lmax * (size_t)K * sizeof(T));
-  l.errs = l.acc + (size_t)cap * (size_t)K * 32 * sizeof(T);
+  l.errs = l.acc + (size_t)ncap * (size_t)K * 32 * sizeof(T);
   l.warps = l.errs + 32 * 8 + 32;
   l.vals = (size_t)table_rows<T>(Lmax) * kRowBytes;
   l.crow = l.vals + (recompute ? (size_t)Lmax * 32 * sizeof(T) : 0);
-  l.xacc = l.crow + (nwarp > 1 ? (size_t)cap * kRowBytes : 0);
+  l.xacc = l.crow + (nwarp > 1 ? (size_t)ncap * kRowBytes : 0);
   l.warp_bytes = l.xacc + (size_t)xrows * kRowBytes;
   l.bytes = l.warps + (size_t)nwarp * l.warp_bytes;
   return l;
+}
+
+// Constants summed in one sweep: half the nodes of a tree are leaves, few of them constants; a
+// tape with more is swept again for the rest.  Long tapes get more, beside rows that are larger
+// anyway (256 tapes of 200 to 400 nodes, N = 256: 979 us with 8, 343 with an eighth of the
+// nodes).
+template <typename T>
+static int sum_capacity(int Lmax, int64_t K, int nwarp) {
+  int cap = nwarp > 1 ? 8 : 12;
+  if (cap < Lmax / 8) cap = Lmax / 8;
+  if (cap > (Lmax + 1) / 2) cap = (Lmax + 1) / 2;
+  const int64_t room = (int64_t)(24 << 10) / (K * 32 * (int64_t)sizeof(T));
+  return cap > room ? (room < 1 ? 1 : (int)room) : cap;
 }
 
 // Variables whose sums over the leaves are kept in rows.
 __host__ __device__ __forceinline__ int x_sum_rows(int64_t n_x) { return n_x <= 16 ? (int)n_x : 0; }
 
 // Program words of operator node k:
-//   x: dense code (bits 0..4) | no parent (bit 5) | k << 8 | adjoint row << 20
+//   x: dense code (bits 0..4) | no parent (bit 5) | one child twice (bit 6) | k << 8 |
+//      adjoint row << 20
 //   y, z: for child 0 and 1: where its value comes from (bits 0..1: nowhere, its cache row,
 //      a constant entry, the node's own cache row), the constant index (bits 2..13), where
 //      its adjoint goes (bits 16..17: nowhere, a row, a constant's sum, grad_X), the row,
-//      constant or variable index (bits 18..29)
+//      constant or variable index (bits 18..29); for a node with several parents whether an
+//      earlier parent has left its adjoint in the row (bit 30), and for such a leaf at its last
+//      parent (bit 31) that bits 18..29 are the row and bits 2..13 the constant or variable
 //   w: child 0 | child 1 << 12
 enum ValueFrom : uint32_t { kNoValue = 0, kChildRow = 1, kConstant = 2, kOwnRow = 3 };
 enum AdjointTo : uint32_t { kNowhere = 0, kRow = 1, kSum = 2, kGradX = 3 };
+constexpr uint32_t kNoParent = 1u << 5, kSameChild = 1u << 6, kEdgeAdd = 1u << 30, kEdgeLeaf = 1u << 31;
+constexpr uint32_t kNothing = 31u;  // the code of the one entry of a tape without operators
 
 // Whether the adjoint rule of an operator reads its operands' values (node_adjoint).
 __device__ __forceinline__ bool reads_operands(int code) {
@@ -263,487 +337,843 @@ __device__ __forceinline__ void op_adjoint_onto(int d, const T (&g)[V], const T 
   }
 }
 
-// The general path over one class of a unit's chunks: one adjoint row per node and one value
-// per lane.  Kept out of line: its code and registers would otherwise weigh on the sweep that
-// nearly every tape takes (1050 us became 1486 for 16384 tapes, M = 64, N = 1024).
+// Whether a tape of the class takes the sweep over stack rows: its rows fit the table, and rows of
+// the cache have less than 4 GB (that sweep's offsets have 32 bits).
 template <typename T>
-struct GeneralSweep {
+__device__ __forceinline__ bool in_stack_order(int need, int Lhi, int64_t rs) {
+  return need >= 0 && need <= table_rows<T>(Lhi) && rs <= (int64_t)0xffffffff / (int64_t)sizeof(T);
+}
+
+// A lane's part of a row: VV values.
+template <typename T, int VV>
+__device__ __forceinline__ void load_part(const void* p, T (&r)[VV]) {
+  if constexpr (VV * sizeof(T) == 16) {
+    load16(p, r);
+  } else if constexpr (VV == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    r[0] = t.x; r[1] = t.y;
+  } else {
+    r[0] = *reinterpret_cast<const T*>(p);
+  }
+}
+template <typename T, int VV>
+__device__ __forceinline__ void store_part(void* p, const T (&r)[VV]) {
+  if constexpr (VV * sizeof(T) == 16) store16(p, r);
+  else if constexpr (VV == 2) *reinterpret_cast<float2*>(p) = make_float2(r[0], r[1]);
+  else *reinterpret_cast<T*>(p) = r[0];
+}
+
+// What a warp sweeps: one class of a unit's chunks.
+template <typename T>
+struct Sweep {
   const T *X, *Cc, *G;  // Cc: null without a cache
   T* gX;
-  int64_t N, n_x, rs, es, total, K, set, cl, nq, rounds;
+  int64_t N, n_x, rs, es, total, K, set, cl, nq;
   const uint32_t* tape;
   const uint4* prog;
-  const uint32_t* orphan;
-  const int *cidx, *lcon;
-  const T* cv;           // the lane's constant entries
-  T *accl, *adj, *vals;  // the lane's sums, adjoint rows and value rows
-  T* xs;                 // the lane's sums per variable, kRowBytes apart
-  unsigned xused;
-  T* crow;
-  const unsigned char* crows;
+  const uint32_t* orphan;  // leaf j without a parent at orphan[-j]
+  const int *vars, *cidx;  // variable leaf j at vars[-j]
+  const T* cv;             // the lane's constant entries
+  T* accl;                 // the lane's sums
+  unsigned char* wb;       // the warp's rows
+  const unsigned char* rows0;  // the first warp's rows
+  uint32_t vals, crow, xacc;   // in the warp's rows: values, terms of a pass, sums per variable
   size_t warp_bytes;
   unsigned long long* errs;
-  int L, nop, norph, g0, ng, lane, rank, ranks;
+  unsigned xused;
+  int xrows, L, nop, norph, nvar, g0, ng, lane, rank, ranks;
 };
 
-template <typename T, int kMode>
-__device__ __noinline__ void general_sweep(const GeneralSweep<T>& q) {
-  constexpr int V = Pack<T>::V;  // the stride of crow
-  for (int64_t round = 0; round < q.rounds; ++round) {
-    const int64_t p = 32 * (q.cl + q.K * (round * q.ranks + q.rank)) + q.lane;
-    const bool valid = p < q.total;
-    const int64_t pv = valid ? p : q.total - 1, n = kMode == kFlat ? pv / q.K : pv;
-    for (int k = 0; k < q.L; ++k) q.adj[k * 32] = valid ? __ldg(q.G + (int64_t)k * q.rs + p * q.es) : T(0);
-    // a node's value: a constant's entry, its cache row, or what is recomputed here
-    auto node = [&](int k) -> T {
+// The sweep, VV values per lane.  kShared: nodes may have several parents.  Not kCached: the node
+// values are recomputed into rows at the start of a pass (VV is 1).
+template <typename T, int kMode, int VV, bool kShared, bool kCached>
+__device__ __forceinline__ void sweep(const Sweep<T>& q) {
+  constexpr uint32_t RB = 32u * VV * (uint32_t)sizeof(T);  // bytes of an adjoint row
+  constexpr bool kFold = kMode != kFlat;
+  const int64_t K = kFold ? 1 : q.K, es = kMode == kStrided ? q.es : 1;
+  const int lane = q.lane, ranks = kFold ? q.ranks : 1, rank = kFold ? q.rank : 0;
+  const int64_t rounds = (q.nq + (int64_t)ranks * VV - 1) / ((int64_t)ranks * VV);
+  const int64_t vs = 32 * K * es;  // elements from one of a lane's values to the next
+  using RowBytes = std::conditional_t<kShared, uint64_t, uint32_t>;
+  const RowBytes row_bytes = (RowBytes)(q.rs * (int64_t)sizeof(T));
+  T* const gX = q.gX;
+  T* const accl = q.accl;
+  T* const crow = reinterpret_cast<T*>(q.wb + q.crow);
+  unsigned char* const rows = q.wb + lane * (VV * (int)sizeof(T));
+  unsigned char* const xs = q.wb + q.xacc + lane * 16;  // the lane's sums per variable
+  T* const vals = reinterpret_cast<T*>(q.wb + q.vals) + lane;
+  int64_t p0 = 0;   // value index of the lane's first value in this pass
+  unsigned vm = 0;  // which of its values exist
+  uint32_t ep = 0;  // first error of each value: two bits (1 = 201, 2 = 204)
+  auto point = [&](int64_t p) -> int64_t {  // the point of a value
+    if (kMode != kFlat) return p;
+    return q.total <= (int64_t)0xffffffff ? (int64_t)((uint32_t)p / (uint32_t)K) : p / K;
+  };
+  // a value's term of constant j
+  auto add_constant = [&](uint32_t idx, const T (&val)[VV]) {
+    const int j = (int)idx - q.g0;
+    if (j < 0 || j >= q.ng) return;
+    if (ranks == 1) {
+      T t = accl[j * 32];
+#pragma unroll
+      for (int v = 0; v < VV; ++v)
+        if ((vm >> v & 1u) && val[v] != T(0)) t = M_<T>::add(t, val[v]);
+      accl[j * 32] = t;
+    } else {
+#pragma unroll
+      for (int v = 0; v < VV; ++v) crow[(j * VV + v) * 32 + lane] = (vm >> v & 1u) ? val[v] : T(0);
+    }
+  };
+  auto to_grad_x = [&](uint32_t var, const T (&val)[VV]) {
+#pragma unroll
+    for (int v = 0; v < VV; ++v)
+      if ((vm >> v & 1u) && val[v] != T(0)) atomicAdd(gX + point(p0 + v * 32 * K) * q.n_x + var, val[v]);
+  };
+  auto add_variable = [&](uint32_t var, const T (&val)[VV]) {
+    if (!gX) return;
+    if (!q.xrows) return to_grad_x(var, val);
+    T t[VV];
+    load_part<T, VV>(xs + var * kRowBytes, t);
+#pragma unroll
+    for (int v = 0; v < VV; ++v)
+      if (val[v] != T(0)) t[v] = M_<T>::add(t[v], val[v]);
+    store_part<T, VV>(xs + var * kRowBytes, t);
+  };
+  auto clear_variables = [&]() {
+    T zero[VV];
+#pragma unroll
+    for (int v = 0; v < VV; ++v) zero[v] = T(0);
+    for (unsigned m = q.xused; m; m &= m - 1) store_part<T, VV>(xs + (__ffs((int)m) - 1) * kRowBytes, zero);
+  };
+  if (gX) clear_variables();
+  auto place = [&](int64_t round, int64_t& p, unsigned& m) {
+    const int64_t q0 = (round * ranks + rank) * VV;
+    p = 32 * (q.cl + K * q0) + lane;
+    m = 0;
+#pragma unroll
+    for (int v = 0; v < VV; ++v)
+      if (p + v * 32 * K < q.total) m |= 1u << v;
+  };
+  auto row = [&](const T* at, uint32_t k, unsigned m, T (&x)[VV]) {  // at: the lane's first value of node 0
+    const T* r = reinterpret_cast<const T*>(reinterpret_cast<const char*>(at) + (uint64_t)k * row_bytes);
+#pragma unroll
+    for (int v = 0; v < VV; ++v) x[v] = (m >> v & 1u) ? __ldg(r + v * vs) : T(0);
+  };
+  // next: the loads of the node to come (operand values, children's output gradients,
+  // and its own for a node without a parent); cur: the node at hand
+  struct Loads {
+    uint4 w;
+    T a[VV], b[VV], s0[VV], s1[VV], g[VV];
+  } next, cur;
+  next.w = make_uint4(0u, 0u, 0u, 0u);
+  auto value = [&](uint32_t w, uint32_t child, uint32_t own, const T* cp, unsigned m, T (&x)[VV]) {
+    const uint32_t from = w & 3u;
+    if (!kCached) {
+      if (from != kNoValue) x[0] = vals[(from == kOwnRow ? own : child) * 32];
+    } else if (from == kConstant) {
+      const T t = q.cv[(int64_t)(w >> 2 & 0xfffu) * K];
+#pragma unroll
+      for (int v = 0; v < VV; ++v) x[v] = t;
+    } else if (from != kNoValue) {
+      row(cp, from == kOwnRow ? own : child, m, x);
+    }
+  };
+  // a child's adjoint: its output gradient plus the contributions
+  auto give = [&](uint32_t w, const T (&val)[VV]) {
+    const uint32_t to = w >> 16 & 3u;
+    const uint32_t idx = kShared && (w & kEdgeLeaf) ? w >> 2 & 0xfffu : w >> 18 & 0xfffu;
+    if (to == kRow) store_part<T, VV>(rows + idx * RB, val);
+    else if (to == kSum) add_constant(idx, val);
+    else if (to == kGradX) add_variable(idx, val);
+  };
+  auto from_gout = [&](uint32_t w) { return (w >> 16 & 3u) && !(kShared && (w & kEdgeAdd)); };
+  if constexpr (!kCached) {
+    for (int k = 0; k < q.L; ++k) {
       const int code = code_of(q.tape[k]);
-      if (!is_op_code(code) && code != VAR) return q.cv[(int64_t)q.cidx[k] * q.K];
-      return q.Cc ? __ldg(q.Cc + (int64_t)k * q.rs + pv * q.es) : q.vals[k * 32];
-    };
-    if (!q.Cc) {
-      for (int k = 0; k < q.L; ++k) {
-        const uint32_t d = q.tape[k];
-        const int code = code_of(d), ar = arity_of(code);
-        if (code == VAR) q.vals[k * 32] = __ldg(q.X + n * q.n_x + child0(d));
-        else if (is_op_code(code))
-          q.vals[k * 32] =
-              op_value<T>(dense_op(code), ar >= 1 ? node(child0(d)) : T(0), ar == 2 ? node(child1(d)) : T(0));
-      }
+      if (!is_op_code(code) && code != VAR) vals[k * 32] = q.cv[(int64_t)q.cidx[k] * K];
     }
-    int err = 0;
-    for (int i = q.nop - 1; i >= 0; --i) {
+  }
+  auto recompute = [&]() {
+    const int64_t n = point(p0 < q.total ? p0 : q.total - 1);
+    for (int j = 0; j < q.nvar; ++j) {
+      const int k = q.vars[-j];
+      vals[k * 32] = __ldg(q.X + n * q.n_x + child0(q.tape[k]));
+    }
+    for (int i = 0; i < q.nop; ++i) {
       const uint4 w = q.prog[i];
-      const int own = (int)(w.x >> 8 & 0xfffu), c0 = (int)(w.w & 0xfffu), c1 = (int)(w.w >> 12);
-      const T a = (w.y & 3u) == kNoValue ? T(0) : node((w.y & 3u) == kOwnRow ? own : c0);
-      const T b = (w.z & 3u) == kNoValue ? T(0) : node(c1);
-      T o0, o1;
-      bool a0, a1;
-      const int e = op_adjoint<T>((int)(w.x & 31u), q.adj[own * 32], a, b, a, a0, o0, a1, o1);
-      if (e && !err) err = e;
-      if (a0 && (w.y >> 16 & 3u)) q.adj[c0 * 32] = M_<T>::add(q.adj[c0 * 32], o0);
-      if (a1 && (w.z >> 16 & 3u)) q.adj[c1 * 32] = M_<T>::add(q.adj[c1 * 32], o1);
+      vals[(w.x >> 8 & 0xfffu) * 32] = op_value<T>((int)(w.x & 31u), vals[(w.w & 0xfffu) * 32], vals[(w.w >> 12) * 32]);
     }
-    for (int j = 0; j < q.ng; ++j) {
-      const T g = valid ? q.adj[q.lcon[q.g0 + j] * 32] : T(0);
-      if (q.ranks > 1) q.crow[j * V * 32 + q.lane] = g;
-      else if (g != T(0)) q.accl[j * 32] = M_<T>::add(q.accl[j * 32], g);
+  };
+  int64_t pl = 0;  // first value, and which exist, of the pass that is being loaded
+  unsigned ml = 0;
+  int64_t round = 0, rcur = 0;         // the pass that is being loaded, the pass at hand
+  int in = q.nop - 1, icur = -1;       // the node to load next, the node at hand
+  if (rounds > 0) place(0, pl, ml);
+  while (true) {
+    const bool more = round < rounds;
+    cur = next;
+    if (more) {
+      next.w = q.prog[in];
+      const uint32_t own = next.w.x >> 8 & 0xfffu, c0 = next.w.w & 0xfffu, c1 = next.w.w >> 12;
+      const T* gp = q.G + pl * es;
+      if constexpr (kCached) {
+        const T* cp = q.Cc + pl * es;
+        value(next.w.y, c0, own, cp, ml, next.a);
+        value(next.w.z, c1, own, cp, ml, next.b);
+      }
+      if (from_gout(next.w.y)) row(gp, c0, ml, next.s0);
+      if (from_gout(next.w.z)) row(gp, c1, ml, next.s1);
+      if (next.w.x & kNoParent) row(gp, own, ml, next.g);
     }
-    if (q.gX && valid) {  // in the order of the sweep, each variable leaf once
-      auto leaf = [&](int k) {
-        if (code_of(q.tape[k]) != VAR) return;
-        const T g = q.adj[k * 32];
-        q.adj[k * 32] = T(0);
-        if (g == T(0)) return;
-        const int var = child0(q.tape[k]);
-        if (!q.xused) {
-          atomicAdd(q.gX + n * q.n_x + var, g);
-        } else {
-          T* t = q.xs + var * (int)(kRowBytes / sizeof(T));
-          *t = M_<T>::add(*t, g);
+    if (icur >= 0) {
+      if constexpr (!kCached) {
+        if (icur == q.nop - 1) recompute();
+        const uint32_t own = cur.w.x >> 8 & 0xfffu;
+        value(cur.w.y, cur.w.w & 0xfffu, own, nullptr, vm, cur.a);
+        value(cur.w.z, cur.w.w >> 12, own, nullptr, vm, cur.b);
+      }
+      if (!(cur.w.x & kNoParent)) load_part<T, VV>(rows + (cur.w.x >> 20) * RB, cur.g);
+      if constexpr (kShared) {
+        if (cur.w.y & kEdgeAdd) load_part<T, VV>(rows + (cur.w.y >> 18 & 0xfffu) * RB, cur.s0);
+        if (cur.w.z & kEdgeAdd) load_part<T, VV>(rows + (cur.w.z >> 18 & 0xfffu) * RB, cur.s1);
+        if (cur.w.x & kSameChild) {
+#pragma unroll
+          for (int v = 0; v < VV; ++v) cur.s1[v] = T(0);
         }
-      };
-      for (int i = q.nop - 1; i >= 0; --i) {
-        const uint4 w = q.prog[i];
-        if (w.y >> 16 & 3u) leaf((int)(w.w & 0xfffu));
-        if (w.z >> 16 & 3u) leaf((int)(w.w >> 12));
       }
-      for (int j = 0; j < q.norph; ++j) leaf((int)(q.orphan[-j] & 0xfffu));
-      for (unsigned m = q.xused; m; m &= m - 1) {
-        const int var = __ffs((int)m) - 1;
-        T* t = q.xs + var * (int)(kRowBytes / sizeof(T));
-        if (*t != T(0)) atomicAdd(q.gX + n * q.n_x + var, *t);
-        *t = T(0);
-      }
-    }
-    if (err && valid) {
-      const int64_t kk = kMode == kFlat ? p - n * q.K : q.set, pchunks = (q.N + 31) / 32;
-      atomicMin(&q.errs[n & 31],
-                ((unsigned long long)(kk * pchunks + n / 32) << 16) | (unsigned long long)err);
-    }
-    if (q.ranks > 1) {
-      __syncthreads();
-      for (int j = q.rank; j < q.ng; j += q.ranks) {
-        T t = q.accl[j * 32];
-        for (int r = 0; r < q.ranks && round * q.ranks + r < q.nq; ++r) {
-          const T x = reinterpret_cast<const T*>(q.crows + (size_t)r * q.warp_bytes)[j * V * 32 + q.lane];
-          if (x != T(0)) t = M_<T>::add(t, x);
+      op_adjoint_onto<T, VV>((int)(cur.w.x & 31u), cur.g, cur.a, cur.b, cur.s0, cur.s1, ep);
+      if constexpr (kShared) {
+        if (cur.w.x & kSameChild) {  // (its second edge goes nowhere)
+#pragma unroll
+          for (int v = 0; v < VV; ++v) cur.s0[v] = M_<T>::add(cur.s0[v], cur.s1[v]);
         }
-        q.accl[j * 32] = t;
       }
-      __syncthreads();
+      give(cur.w.y, cur.s0);
+      give(cur.w.z, cur.s1);
+      if (icur == 0) {  // the pass ends
+        for (int j = 0; j < q.norph; ++j) {  // leaves without a parent: their output gradient alone
+          const uint32_t w = q.orphan[-j];
+          T val[VV];
+          row(q.G + p0 * es, w & 0xfffu, vm, val);
+          if (w & (1u << 12)) add_variable(w >> 13, val);
+          else add_constant(w >> 13, val);
+        }
+        if (gX && q.xused) {
+          for (unsigned m = q.xused; m; m &= m - 1) {
+            T t[VV];
+            load_part<T, VV>(xs + (__ffs((int)m) - 1) * kRowBytes, t);
+            to_grad_x((uint32_t)(__ffs((int)m) - 1), t);
+          }
+          clear_variables();
+        }
+        if (__any_sync(0xffffffffu, ep != 0)) {
+          const int64_t pchunks = (q.N + 31) / 32;
+#pragma unroll
+          for (int v = 0; v < VV; ++v) {
+            const uint32_t e = ep >> (2 * v) & 3u;
+            if (e && (vm >> v & 1u)) {
+              const int64_t p = p0 + v * 32 * K, n = point(p);
+              const int64_t kk = kMode == kFlat ? p - n * K : q.set;
+              atomicMin(&q.errs[n & 31], ((unsigned long long)(kk * pchunks + n / 32) << 16) |
+                                             (unsigned long long)(e == 2 ? ERR_DIV_BY_ZERO : ERR_GRAD_ON_NO_OP));
+            }
+          }
+          ep = 0;
+        }
+        if (ranks > 1) {
+          __syncthreads();
+          for (int j = rank; j < q.ng; j += ranks) {
+            T t = accl[j * 32];
+            for (int r = 0; r < ranks; ++r) {
+              const T* cr = reinterpret_cast<const T*>(q.rows0 + (size_t)r * q.warp_bytes + q.crow);
+              const int64_t q0 = (rcur * ranks + r) * VV;
+#pragma unroll
+              for (int v = 0; v < VV; ++v) {
+                if (q0 + v < q.nq) {
+                  const T x = cr[(j * VV + v) * 32 + lane];
+                  if (x != T(0)) t = M_<T>::add(t, x);
+                }
+              }
+            }
+            accl[j * 32] = t;
+          }
+          __syncthreads();
+        }
+      }
+    }
+    if (!more) break;
+    if (in == q.nop - 1) {  // the first node of a pass is loaded: the pass begins
+      p0 = pl;
+      vm = ml;
+      rcur = round;
+    }
+    icur = in;
+    if (--in < 0) {
+      in = q.nop - 1;
+      if (++round < rounds) place(round, pl, ml);
     }
   }
 }
 
-template <typename T, int kMode>
-__global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
-    const T* __restrict__ X, const T* __restrict__ cache, int64_t N, int64_t n_x, const uint32_t* __restrict__ desc,
-    const int32_t* __restrict__ meta, const int32_t* __restrict__ order, int64_t B, int64_t M, int Llo, int Lhi,
-    const T* __restrict__ C, int64_t c_sb, int64_t c_sm, int64_t c_sk, int64_t Ktot, const T* __restrict__ gout,
-    T* __restrict__ gC, T* __restrict__ gX, int32_t* __restrict__ status) {
-  constexpr int V = Pack<T>::V;
+// The arguments of the kernel below.
+template <typename T>
+struct AdjArgs {
+  const T *X, *cache;
+  int64_t N, n_x;
+  const uint32_t* desc;
+  const int32_t *meta, *order;
+  int64_t B, M;
+  int Llo, Lhi, xrows, ncap;
+  const T* C;
+  int64_t c_sb, c_sm, c_sk, Ktot;
+  const T* gout;
+  T *gC, *gX;
+  int32_t* status;
+};
+
+// A CTA's view of its unit: sizes and the tables in shared memory.
+template <typename T, int kMode, bool kCached>
+struct UnitView {
+  int64_t K, es, total, rs, nchunks;  // sets; elements between values; values per node; elements per node
+  int lane, warp, nwarp, ranks, rank;
+  AdjLayout ly;
+  uint32_t* tape;
+  uint4* prog;
+  uint32_t* orphan;  // leaf j without a parent at orphan[-j]
+  int *cidx, *lcon, *vars;  // variable leaf j at vars[-j] (without a cache)
+  T *cval, *acc;
+  unsigned long long* errs;
+  int* info;  // operators, constants, orphans, variable leaves, variables, values per lane
+  unsigned char* wb;
+  __device__ __forceinline__ UnitView(const AdjArgs<T>& A, unsigned char* smem) {
+    K = kMode == kFlat ? A.Ktot : 1;
+    es = kMode == kStrided ? A.Ktot : 1;
+    total = A.N * K;
+    rs = total * es;
+    nchunks = (total + 31) / 32;
+    lane = threadIdx.x & 31;
+    warp = threadIdx.x >> 5;
+    nwarp = blockDim.x >> 5;
+    // with one set the warps of a unit take turns over its passes (ranks), else whole classes
+    ranks = kMode == kFlat ? 1 : nwarp;
+    rank = kMode == kFlat ? 0 : warp;
+    ly = adjoint_layout<T>(A.Lhi, K, nwarp, !kCached, A.xrows, A.ncap);
+    tape = reinterpret_cast<uint32_t*>(smem);
+    prog = reinterpret_cast<uint4*>(smem + ly.prog);
+    orphan = reinterpret_cast<uint32_t*>(smem + ly.cidx) - 1;
+    cidx = reinterpret_cast<int*>(smem + ly.cidx);
+    lcon = reinterpret_cast<int*>(smem + ly.lcon);
+    vars = lcon + A.Lhi - 1;
+    cval = reinterpret_cast<T*>(smem + ly.cval);
+    acc = reinterpret_cast<T*>(smem + ly.acc);
+    errs = reinterpret_cast<unsigned long long*>(smem + ly.errs);
+    info = reinterpret_cast<int*>(smem + ly.errs + 32 * 8);
+    wb = smem + ly.warps + (size_t)warp * ly.warp_bytes;
+  }
+};
+
+// The sweeps of one unit, once its program stands, and its gradients of the constants.
+template <typename T, int kMode, int VV, bool kShared, bool kCached>
+__device__ __forceinline__ void sweep_unit(const AdjArgs<T>& A, const UnitView<T, kMode, kCached>& u, unsigned char* smem,
+                                           int64_t b, int64_t set, int L) {
+  const int K = (int)u.K, ncap = A.ncap, ncon = u.info[1];
+  // sweeps of ncap constants each: one, but for tapes with more of them
+  for (int g0 = 0; g0 == 0 || g0 < ncon; g0 += ncap) {
+    const int ng = min(ncap, ncon - g0);
+    for (int i = threadIdx.x; i < ncap * K * 32; i += blockDim.x) u.acc[i] = T(0);
+    __syncthreads();
+    for (int cl = kMode == kFlat ? u.warp : 0; cl < K; cl += kMode == kFlat ? u.nwarp : 1) {
+      Sweep<T> q;
+      q.X = A.X;
+      q.Cc = kCached ? A.cache + (size_t)b * A.M * u.rs + set : nullptr;
+      q.G = A.gout + (size_t)b * A.M * u.rs + set;
+      q.gX = g0 == 0 ? A.gX : nullptr;
+      q.N = A.N; q.n_x = A.n_x; q.rs = u.rs; q.es = u.es; q.total = u.total; q.K = K; q.set = set;
+      q.cl = cl;
+      q.nq = cl < u.nchunks ? (u.nchunks - cl + K - 1) / K : 0;  // chunks of this class
+      q.tape = u.tape; q.prog = u.prog; q.orphan = u.orphan; q.vars = u.vars; q.cidx = u.cidx;
+      q.cv = u.cval + (kMode == kFlat ? (32 * cl + u.lane) % K : 0);
+      q.accl = u.acc + (int64_t)cl * ncap * 32 + u.lane;
+      q.wb = u.wb; q.rows0 = smem + u.ly.warps; q.vals = (uint32_t)u.ly.vals; q.crow = (uint32_t)u.ly.crow;
+      q.xacc = (uint32_t)u.ly.xacc; q.warp_bytes = u.ly.warp_bytes; q.errs = u.errs;
+      q.xused = A.xrows ? (unsigned)u.info[4] : 0u;
+      q.xrows = A.xrows;
+      q.L = L; q.nop = u.info[0]; q.norph = u.info[2]; q.nvar = u.info[3]; q.g0 = g0; q.ng = ng;
+      q.lane = u.lane; q.rank = u.rank; q.ranks = u.ranks;
+      sweep<T, kMode, VV, kShared, kCached>(q);
+    }
+    __syncthreads();  // every class's sums are complete
+    for (int i = u.warp; i < ng * K; i += u.nwarp) {
+      const int j = i / K, kk = i - j * K, pos = u.lane * K + kk;
+      const T s = warp_sum(u.acc[((pos >> 5) * ncap + j) * 32 + (pos & 31)]);
+      if (u.lane == 0) A.gC[(b * A.M + u.lcon[g0 + j]) * A.Ktot + set + kk] = s;
+    }
+    __syncthreads();
+  }
+}
+
+// The same for the tapes that the sweep over stack rows does not take, out of line: its code and
+// registers would otherwise weigh on that sweep (1050 us became 1486 for 16384 tapes, M = 64,
+// N = 1024), and so would values that the caller keeps across it.
+template <typename T, int kMode, int VV>
+__device__ __noinline__ void general_unit(const AdjArgs<T>& A, int64_t b, int64_t set, int L) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int64_t K = kMode == kFlat ? Ktot : 1;       // sets of a unit
-  const int64_t es = kMode == kStrided ? Ktot : 1;   // elements between its values
-  const int64_t sets = kMode == kStrided ? Ktot : 1;
-  const int64_t total = N * K, rs = total * es;      // values per node, elements per node
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const UnitView<T, kMode, true> u(A, smem);
+  sweep_unit<T, kMode, VV, true, true>(A, u, smem, b, set, L);
+}
+
+// Not kGeneral: the tapes that are not in stack order are left to the staged kernel below (118
+// registers, where the call of the general sweeps makes it 128 and 17 resident warps 16).
+template <typename T, int kMode, bool kCached, bool kGeneral>
+__global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(const __grid_constant__ AdjArgs<T> A) {
+  constexpr int V = Pack<T>::V;
+  constexpr int G = V / 2;  // values per lane of the wider of the two general sweeps
+  extern __shared__ __align__(16) unsigned char smem[];
+  const UnitView<T, kMode, kCached> v(A, smem);
+  const int64_t K = v.K, rs = v.rs, sets = kMode == kStrided ? A.Ktot : 1;
+  const int64_t N = A.N, M = A.M;
+  const int lane = v.lane, warp = v.warp, Lhi = A.Lhi;
   const unsigned below = (1u << lane) - 1u;
-  const int xrows = gX ? x_sum_rows(n_x) : 0;
-  const AdjLayout ly = adjoint_layout<T>(Lhi, K, nwarp, !cache, xrows);
-  const int ncap = ly.ncap;
-  uint32_t* tape = reinterpret_cast<uint32_t*>(smem);
-  uint4* prog = reinterpret_cast<uint4*>(smem + ly.prog);
-  uint32_t* orphan = reinterpret_cast<uint32_t*>(smem + ly.cidx) - 1;  // leaf j without a parent at orphan[-j]
-  int* cidx = reinterpret_cast<int*>(smem + ly.cidx);
-  int* lcon = reinterpret_cast<int*>(smem + ly.lcon);
-  T* cval = reinterpret_cast<T*>(smem + ly.cval);
-  T* acc = reinterpret_cast<T*>(smem + ly.acc);
-  unsigned long long* errs = reinterpret_cast<unsigned long long*>(smem + ly.errs);
-  int* info = reinterpret_cast<int*>(smem + ly.errs + 32 * 8);  // operators, constants, orphans, stack order
-  unsigned char* wb = smem + ly.warps + (size_t)warp * ly.warp_bytes;
-  T* crow = reinterpret_cast<T*>(wb + ly.crow);
-  // with one set the warps of a unit take turns over its passes (ranks), else whole classes
-  const int ranks = kMode == kFlat ? 1 : nwarp, rank = kMode == kFlat ? 0 : warp;
-  const int64_t nchunks = (total + 31) / 32, pchunks = (N + 31) / 32;
+  T* const gX = A.gX;
+  uint32_t *tape = v.tape, *orphan = v.orphan;
+  uint4* prog = v.prog;
+  int *cidx = v.cidx, *lcon = v.lcon, *vars = v.vars, *info = v.info;
+  T* cval = v.cval;
+  unsigned char* wb = v.wb;
 
   // The units come longest first: a CTA takes them there and back (i, 2 G - 1 - i, 2 G + i, ...),
   // so that the ones with the longest first unit get the shortest next.
-  const int64_t units = B * sets;
+  const int64_t units = A.B * sets;
   for (int64_t turn = 0; turn * gridDim.x < units; ++turn) {
     const int64_t u = turn * gridDim.x + (turn & 1 ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
     if (u >= units) continue;
     const int64_t ti = kMode == kStrided ? u / sets : u, set = u - ti * sets;
-    const int64_t b = order ? (int64_t)order[ti] : ti;
-    const int L = meta[b * 4];
-    if (L <= Llo || L > Lhi) continue;  // another class's grid takes it (the same in every thread)
+    const int64_t b = A.order ? (int64_t)A.order[ti] : ti;
+    const int L = A.meta[b * 4];
+    if (L <= A.Llo || L > Lhi) continue;  // another class's grid takes it (the same in every thread)
     __syncthreads();                    // every warp is done with the previous unit's tables
-    for (int k = threadIdx.x; k < L; k += blockDim.x) tape[k] = desc[b * M + k];
-    if (threadIdx.x < 32) errs[threadIdx.x] = ~0ull;
+    for (int k = threadIdx.x; k < L; k += blockDim.x) tape[k] = A.desc[b * M + k];
+    if (threadIdx.x < 32) v.errs[threadIdx.x] = ~0ull;
     __syncthreads();
     if (warp == 0) {
-      int* last = reinterpret_cast<int*>(wb);  // scratch in the rows' place
-      int* parent = last + L + 1;
-      const int need = stack_rows(tape, L, lane, last, cidx);
-      // the general path also takes a tape of leaves alone, a call without a cache, and rows
-      // of 4 GB or more (the sweep's row offsets have 32 bits)
-      const bool stack = need >= 1 && need <= table_rows<T>(Lhi) && cache && rs <= (int64_t)0xffffffff / (int64_t)sizeof(T);
-      for (int k = lane; k < L; k += 32) parent[k] = 0;
+      int* scratch = reinterpret_cast<int*>(wb);  // in the rows' place
+      int need = -1;
+      if (kCached) need = stack_rows(tape, L, lane, scratch, cidx);
+      const int R = table_rows<T>(Lhi);
+      const bool stack = in_stack_order<T>(need, Lhi, rs);
+      if (!kGeneral && !stack) {
+        if (lane == 0) info[5] = 0;
+      } else {
+        int *first = scratch, *final = scratch + L, *rowof = scratch + 2 * L;  // parents that the sweep meets first and last
+        for (int k = lane; k < L; k += 32) {
+          first[k] = -1;
+          final[k] = L;
+        }
+        __syncwarp();
+        for (int k = lane; k < L; k += 32) {
+          const uint32_t d = tape[k];
+          const int ar = arity_of(code_of(d));
+          if (stack) {
+            if (ar >= 1) first[child0(d)] = k;
+            if (ar == 2) first[child1(d)] = k;
+          } else {
+            for (int j = 0; j < ar; ++j) {
+              const int c = j == 0 ? child0(d) : child1(d);
+              atomicMax(&first[c], k);
+              atomicMin(&final[c], k);
+            }
+          }
+        }
+        __syncwarp();
+        // a leaf whose adjoint has to wait for further parents in a row
+        auto waits = [&](int c, bool leaf) { return leaf && first[c] >= 0 && first[c] != final[c]; };
+        int ncon = 0, nfix = 0, norph = 0, nvar = 0, nrow = 0;
+        unsigned used = 0;  // variables of the tape
+        for (int k0 = 0; k0 < L; k0 += 32) {
+          const int k = k0 + lane;
+          const bool in = k < L;
+          const int code = in ? code_of(tape[k]) : NO_OP;
+          const bool con = code == LEARNABLE, var = code == VAR, fix = !is_op_code(code) && !con && !var;
+          const unsigned mc = __ballot_sync(0xffffffffu, con), mf = __ballot_sync(0xffffffffu, fix);
+          const bool orph = (con || (var && gX)) && first[k] < 0;
+          const unsigned mo = __ballot_sync(0xffffffffu, orph);
+          used |= __reduce_or_sync(0xffffffffu, var ? 1u << (child0(tape[k]) & 31) : 0u);
+          const int j = ncon + __popc(mc & below);
+          if (!stack) {
+            const bool has = in && (is_op_code(code) || waits(k, con || (var && gX)));
+            const unsigned mr = __ballot_sync(0xffffffffu, has);
+            if (in) rowof[k] = need >= 0 ? cidx[k] : nrow + __popc(mr & below);
+            nrow += __popc(mr);
+          }
+          if (!kCached) {
+            const unsigned mv = __ballot_sync(0xffffffffu, var);
+            if (var) vars[-(nvar + __popc(mv & below))] = k;
+            nvar += __popc(mv);
+          }
+          if (con) {
+            cidx[k] = j;
+            lcon[j] = k;
+          }
+          if (fix) {
+            const int f = L - 1 - (nfix + __popc(mf & below));
+            cidx[k] = f;
+            const T x = node_value<T>(code, T(0), T(0), T(0), T(0));
+            for (int kk = 0; kk < (int)K; ++kk) cval[(int64_t)f * K + kk] = x;
+          }
+          if (orph)
+            orphan[-(norph + __popc(mo & below))] =
+                (uint32_t)k | (var ? 1u << 12 : 0u) | ((uint32_t)(var ? child0(tape[k]) : j) << 13);
+          ncon += __popc(mc);
+          nfix += __popc(mf);
+          norph += __popc(mo);
+        }
+        if (need >= 0) nrow = need;
+        __syncwarp();
+        auto operand = [&](int code, int k, int c, bool merged) -> uint32_t {
+          const int cc = code_of(tape[c]);
+          const bool op = is_op_code(cc), con = cc == LEARNABLE, var = cc == VAR;
+          uint32_t w = 0;
+          if (reads_operands(code)) {
+            if (code == EXP) w = kOwnRow;  // its rule uses the node's own value
+            else if (op || var) w = kChildRow;
+            else w = kConstant | ((uint32_t)cidx[c] << 2);
+          }
+          const bool leaf = con || (var && gX);
+          if (merged || !(op || leaf)) return w;
+          const uint32_t kind = con ? kSum : kGradX, at = con ? (uint32_t)cidx[c] : (uint32_t)child0(tape[c]);
+          if (stack) return w | (op ? (kRow << 16) | ((uint32_t)cidx[c] << 18) : (kind << 16) | (at << 18));
+          const bool wait = waits(c, leaf);
+          if (!op && !wait) return w | (kind << 16) | (at << 18);
+          w |= ((uint32_t)rowof[c] << 18) | (k == first[c] ? 0u : kEdgeAdd);
+          if (op || k != final[c]) return w | (kRow << 16);
+          return w | (kind << 16) | (at << 2) | kEdgeLeaf;
+        };
+        int nop = 0;
+        for (int k0 = 0; k0 < L; k0 += 32) {
+          const int k = k0 + lane;
+          const uint32_t d = k < L ? tape[k] : 0u;
+          const int code = code_of(d), ar = arity_of(code);
+          const bool op = k < L && is_op_code(code);
+          const unsigned mo = __ballot_sync(0xffffffffu, op);
+          if (op) {
+            uint4 w = make_uint4((uint32_t)dense_op(code) | ((uint32_t)k << 8) |
+                                     ((uint32_t)(stack ? cidx[k] : rowof[k]) << 20), 0u, 0u, 0u);
+            if (first[k] < 0) w.x |= kNoParent;
+            if (ar >= 1) {
+              w.y = operand(code, k, child0(d), false);
+              w.w = (uint32_t)child0(d);
+            }
+            if (ar == 2) {
+              const bool same = child0(d) == child1(d);
+              if (same) w.x |= kSameChild;
+              w.z = operand(code, k, child1(d), same);
+              w.w |= (uint32_t)child1(d) << 12;
+            }
+            prog[nop + __popc(mo & below)] = w;
+          }
+          nop += __popc(mo);
+        }
+        if (lane == 0) {
+          if (nop == 0) prog[nop++] = make_uint4(kNothing, 0u, 0u, 0u);
+          info[0] = nop;
+          info[1] = ncon;
+          info[2] = norph;
+          info[3] = nvar;
+          info[4] = (int)used;
+          // values per lane: G where the rows hold them and a warp has more than one chunk
+          info[5] = stack ? V : nrow * G <= R * V && N > 32 * v.ranks ? G : 1;
+        }
+      }
+    }
+    __syncthreads();
+    const int ncon = info[1], VV = info[5];
+    if (!kGeneral && VV != V) continue;
+    for (int i = threadIdx.x; i < ncon * (int)K; i += blockDim.x) {
+      const int j = i / (int)K, kk = i - j * (int)K;
+      cval[i] = __ldg(A.C + b * A.c_sb + (int64_t)lcon[j] * A.c_sm + (set + kk) * A.c_sk);
+    }
+    // every other node's gradient is zero
+    for (int i = threadIdx.x; i < (int)M * (int)K; i += blockDim.x) {
+      const int k = i / (int)K, kk = i - k * (int)K;
+      if (!(k < L && code_of(tape[k]) == LEARNABLE)) A.gC[(b * M + k) * A.Ktot + set + kk] = T(0);
+    }
+    if constexpr (!kCached) {
+      sweep_unit<T, kMode, 1, true, false>(A, v, smem, b, set, L);
+    } else {
+      if (VV == V) sweep_unit<T, kMode, V, false, true>(A, v, smem, b, set, L);
+      else if (kGeneral && G > 1 && VV == G) general_unit<T, kMode, G>(A, b, set, L);
+      else if (kGeneral) general_unit<T, kMode, 1>(A, b, set, L);
+    }
+    if (warp == 0) {
+      int err = v.errs[lane] == ~0ull ? 0 : (int)(v.errs[lane] & 0xffffu);
+      err = __reduce_max_sync(0xffffffffu, err);
+      if (err && lane == 0) report_adjoint(A.status, err);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------
+// Adjoint with staged rows.  One warp per tape, one value per lane.  A chunk's output gradients
+// and node values are copied into shared memory at once (16 bytes per lane where the rows are
+// aligned), then swept from there through precomputed byte offsets: half the
+// instructions per value of the sweep above with one value per lane, and level with its four values
+// per lane, but 256 bytes per node and warp, and nothing to split a tape over.  It takes
+//   - tapes that the sweep above would give one or two values per lane, where the batch alone
+//     fills the GPU, in grids of their own after those of the tapes in stack order (4096 tapes of
+//     50 nodes with shared subtrees, N = 1024: 735 us, 2020 in the general sweep);
+//   - calls of such batches without a cache (65536 tapes, N = 1024: 6.6 ms, 14 by the sweep);
+//   - batches of one set from 192 tapes per SM on (65536 tapes, N = 1024, a gradient on every root:
+//     4.6 ms, 5.1 by the sweep; with quotients, so with infinite and huge arguments, 5.0 and 6.5;
+//     at 24576 tapes the sweep is still ahead, 2.48 and 2.60 ms);
+//   - few points, where a pass of the sweep would be mostly empty (5000 tapes at N = 7: 64 us, 99;
+//     20000 at N = 64, K = 3: 317 and 530).
+// Sums and orders are the same, grad_X's within a tape included.
+// ------------------------------------------------------------------------------------
+template <int kBytes>
+__device__ __forceinline__ void cp_async(void* dst_smem, const void* src, int src_bytes) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst_smem));
+  if (kBytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(d), "l"(src), "r"(src_bytes), "n"(kBytes) : "memory");
+}
+
+// Copies 32 values from p on of rows node(0), ..., node(n - 1) of a block into rows of 32 of buf
+// (zero past the last value).  vec16: every row's start is 16-byte aligned.
+template <typename T, typename Node>
+__device__ __forceinline__ void stage_rows(T* buf, const T* block, int n, Node node, int64_t total, int64_t rs, int64_t es,
+                                           int64_t p, int lane, bool vec16) {
+  if (vec16) {
+    constexpr int E = 16 / sizeof(T), kLanes = 32 / E, kRows = 32 / kLanes;
+    const int e = (lane % kLanes) * E;
+    const int64_t left = total - (p + e);
+    const int bytes = left >= E ? 16 : (left > 0 ? (int)left * (int)sizeof(T) : 0);
+    for (int r = lane / kLanes; r < n; r += kRows) {
+      const int k = node(r);
+      cp_async<16>(buf + k * 32 + e, bytes ? block + (size_t)k * rs + p + e : block, bytes);
+    }
+  } else {
+    const int bytes = p + lane < total ? (int)sizeof(T) : 0;
+    for (int r = 0; r < n; ++r) {
+      const int k = node(r);
+      cp_async<(int)sizeof(T)>(buf + k * 32 + lane, bytes ? block + (size_t)k * rs + (p + lane) * es : block, bytes);
+    }
+  }
+}
+
+// Shared memory of a warp: the tape words (offset 0); per operator its code, the operands' source
+// words (byte offset, bits 0..23, lane stride, bits 24..31), its value row and the operands'
+// adjoint rows; the learnable and the variable leaves; the broadcast entries; a value and an adjoint row
+// per node.  A learnable constant's value row holds its lanes' sums.
+struct StagedLayout {
+  uint32_t code, sa, sb, own, da, db, lcon, lvar, bc, vals, adj, bytes;
+};
+template <typename T>
+__host__ __device__ __forceinline__ StagedLayout staged_layout(int Lmax) {
+  const uint32_t lb = (uint32_t)align16((size_t)Lmax * 4), rows = (uint32_t)Lmax * 32u * (uint32_t)sizeof(T);
+  StagedLayout l;
+  l.code = lb;
+  l.sa = 2 * lb;
+  l.sb = 3 * lb;
+  l.own = 4 * lb;
+  l.da = 5 * lb;
+  l.db = 6 * lb;
+  l.lcon = 7 * lb;
+  l.lvar = 8 * lb;
+  l.bc = 9 * lb;
+  l.vals = l.bc + (uint32_t)align16((size_t)(Lmax + 1) * sizeof(T));
+  l.adj = l.vals + rows;
+  l.bytes = l.adj + rows;
+  return l;
+}
+
+template <typename T, bool kMulti, bool kCached>
+__global__ void __launch_bounds__(256, 4) eval_adjoint_staged_kernel(
+    const T* __restrict__ X, const T* __restrict__ cache, int64_t N, int64_t n_x, const uint32_t* __restrict__ desc,
+    const int32_t* __restrict__ meta, const int32_t* __restrict__ order, int64_t B, int64_t M, int Llo, int Lhi,
+    bool general_only, const T* __restrict__ C, int64_t c_sb, int64_t c_sm, int64_t c_sk, int64_t K_,
+    const T* __restrict__ gout, T* __restrict__ gC, T* __restrict__ gX, int32_t* __restrict__ status, bool vec16) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int64_t K = kMulti ? K_ : 1, rs = N * K;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  constexpr uint32_t RB = 32u * (uint32_t)sizeof(T), kRowStride = (uint32_t)sizeof(T) << 24;
+  const StagedLayout ly = staged_layout<T>(Lhi);
+  unsigned char* wb = smem + (size_t)warp * ly.bytes;
+  uint32_t* tape = reinterpret_cast<uint32_t*>(wb);
+  auto table = [&](uint32_t at) { return reinterpret_cast<uint32_t*>(wb + at); };
+  uint32_t *code_ = table(ly.code), *psa = table(ly.sa), *psb = table(ly.sb), *pown = table(ly.own), *pda = table(ly.da),
+           *pdb = table(ly.db), *lcon = table(ly.lcon), *lvar = table(ly.lvar);
+  T* bc = reinterpret_cast<T*>(wb + ly.bc);
+  T* vals = reinterpret_cast<T*>(wb + ly.vals);
+  T* adj = reinterpret_cast<T*>(wb + ly.adj);
+  const uint32_t adj_delta = ly.adj - ly.vals;
+  const unsigned below = (1u << lane) - 1u;
+  auto at = [&](uint32_t off) -> T& { return reinterpret_cast<T*>(wb + off)[lane]; };
+  auto operand = [&](uint32_t w) { return *reinterpret_cast<const T*>(wb + (w & 0xffffffu) + (uint32_t)lane * (w >> 24)); };
+  for (int64_t ti = (int64_t)blockIdx.x * nwarp + warp; ti < B; ti += (int64_t)gridDim.x * nwarp) {
+    const int64_t b = order ? (int64_t)order[ti] : ti;
+    const int L = meta[b * 4];
+    if (L <= Llo || L > Lhi) continue;  // another class's grid takes it (warp-uniform)
+    for (int k = lane; k < L; k += 32) tape[k] = desc[b * M + k];
+    if (lane == 0) bc[0] = T(0);
+    __syncwarp();
+    if (general_only) {
+      int* scratch = reinterpret_cast<int*>(adj);
+      const int need = stack_rows(tape, L, lane, scratch, scratch + L + 1);
+      __syncwarp();
+      if (in_stack_order<T>(need, Lhi, rs)) continue;  // eval_adjoint_kernel takes it
+    }
+    // the operators, learnable and variable leaves; the broadcast entries of fixed leaves (and of
+    // codes that evaluate to 0) now
+    int nop = 0, ncon = 0, nvar = 0;
+    for (int k0 = 0; k0 < L; k0 += 32) {
+      const int k = k0 + lane;
+      const uint32_t d = k < L ? tape[k] : 0u;
+      const int code = k < L ? code_of(d) : -1;
+      const bool op = k < L && is_op_code(code), con = code == LEARNABLE, var = code == VAR;
+      const unsigned mo = __ballot_sync(0xffffffffu, op), mc = __ballot_sync(0xffffffffu, con),
+                     mv = __ballot_sync(0xffffffffu, var);
+      // source word of operand node c: its value row, or its broadcast entry
+      auto src = [&](int c) -> uint32_t {
+        const int cc = code_of(tape[c]);
+        if (is_op_code(cc) || cc == VAR) return (ly.vals + (uint32_t)c * RB) | kRowStride;
+        return ly.bc + (uint32_t)(1 + c) * (uint32_t)sizeof(T);
+      };
+      if (op) {
+        const int ar = arity_of(code), i = nop + __popc(mo & below);
+        const uint32_t none = ly.adj + (uint32_t)k * RB;  // never written through (arity < 2)
+        code_[i] = (uint32_t)dense_op(code);
+        pown[i] = ly.vals + (uint32_t)k * RB;
+        psa[i] = ar >= 1 ? src(child0(d)) : ly.bc;
+        pda[i] = ar >= 1 ? ly.adj + (uint32_t)child0(d) * RB : none;
+        psb[i] = ar == 2 ? src(child1(d)) : ly.bc;
+        pdb[i] = ar == 2 ? ly.adj + (uint32_t)child1(d) * RB : none;
+      } else if (k < L && !con && !var) {
+        bc[1 + k] = node_value<T>(code, T(0), T(0), T(0), T(0));
+      }
+      if (con) lcon[ncon + __popc(mc & below)] = (uint32_t)k;
+      if (var) lvar[nvar + __popc(mv & below)] = (uint32_t)k;
+      nop += __popc(mo);
+      ncon += __popc(mc);
+      nvar += __popc(mv);
+    }
+    __syncwarp();
+    if (gX && nvar > 0) {
+      // the variable leaves in the order in which the sweep meets their last parents (leaves without
+      // one at the end), each with the first of its variable in bits 12..23: that one's
+      // adjoint row takes the sum
+      int* key = reinterpret_cast<int*>(adj);
+      uint32_t* sorted = reinterpret_cast<uint32_t*>(adj) + L;
+      for (int k = lane; k < L; k += 32) key[k] = 0x7fffffff;
       __syncwarp();
       for (int k = lane; k < L; k += 32) {
         const uint32_t d = tape[k];
         const int ar = arity_of(code_of(d));
-        if (ar >= 1) parent[child0(d)] = 1;
-        if (ar == 2) parent[child1(d)] = 1;
+        if (ar >= 1) atomicMin(&key[child0(d)], 2 * k);
+        if (ar == 2) atomicMin(&key[child1(d)], 2 * k + 1);
       }
       __syncwarp();
-      int ncon = 0, nfix = 0, norph = 0;
-      unsigned used = 0;  // variables of the tape
-      for (int k0 = 0; k0 < L; k0 += 32) {
-        const int k = k0 + lane;
-        const int code = k < L ? code_of(tape[k]) : NO_OP;
-        const bool con = code == LEARNABLE, var = code == VAR, fix = !is_op_code(code) && !con && !var;
-        const unsigned mc = __ballot_sync(0xffffffffu, con), mf = __ballot_sync(0xffffffffu, fix);
-        const bool orph = (con || (var && gX)) && !parent[k];
-        const unsigned mo = __ballot_sync(0xffffffffu, orph);
-        used |= __reduce_or_sync(0xffffffffu, var ? 1u << (child0(tape[k]) & 31) : 0u);
-        const int j = ncon + __popc(mc & below);
-        if (con) {
-          cidx[k] = j;
-          lcon[j] = k;
-        }
-        if (fix) {
-          const int f = L - 1 - (nfix + __popc(mf & below));
-          cidx[k] = f;
-          const T x = node_value<T>(code, T(0), T(0), T(0), T(0));
-          for (int64_t kk = 0; kk < K; ++kk) cval[(int64_t)f * K + kk] = x;
-        }
-        if (orph)
-          orphan[-(norph + __popc(mo & below))] =
-              (uint32_t)k | (var ? 1u << 12 : 0u) | ((uint32_t)(var ? child0(tape[k]) : j) << 13);
-        ncon += __popc(mc);
-        nfix += __popc(mf);
-        norph += __popc(mo);
+      auto later = [&](int c) { return key[c] == 0x7fffffff ? -1 - c : (key[c] ^ 1) + 1; };  // falls along the sweep
+      for (int j = lane; j < nvar; j += 32) {
+        const int mine = later((int)lvar[j]);
+        int place = 0;
+        for (int i = 0; i < nvar; ++i) place += later((int)lvar[i]) > mine ? 1 : 0;
+        sorted[place] = lvar[j];
       }
       __syncwarp();
-      auto operand = [&](int code, int k, int c) -> uint32_t {
-        const int cc = code_of(tape[c]);
-        const bool op = is_op_code(cc), con = cc == LEARNABLE, var = cc == VAR;
-        uint32_t w = 0;
-        if (reads_operands(code)) {
-          if (code == EXP) w = kOwnRow;  // its rule uses the node's own value
-          else if (op || var) w = kChildRow;
-          else w = kConstant | ((uint32_t)cidx[c] << 2);
-        }
-        if (!stack) {
-          if (op || con || var) w |= (kRow << 16) | ((uint32_t)c << 18);
-        } else if (op) {
-          w |= (kRow << 16) | ((uint32_t)cidx[c] << 18);
-        } else if (con) {
-          w |= (kSum << 16) | ((uint32_t)cidx[c] << 18);
-        } else if (var && gX) {
-          w |= (kGradX << 16) | ((uint32_t)child0(tape[c]) << 18);
-        }
-        return w;
-      };
-      int nop = 0;
-      for (int k0 = 0; k0 < L; k0 += 32) {
-        const int k = k0 + lane;
-        const uint32_t d = k < L ? tape[k] : 0u;
-        const int code = code_of(d), ar = arity_of(code);
-        const bool op = k < L && is_op_code(code);
-        const unsigned mo = __ballot_sync(0xffffffffu, op);
-        if (op) {
-          uint4 w = make_uint4((uint32_t)dense_op(code) | ((uint32_t)k << 8) | ((uint32_t)(stack ? cidx[k] : k) << 20),
-                               0u, 0u, 0u);
-          if (!parent[k]) w.x |= 1u << 5;
-          if (ar >= 1) {
-            w.y = operand(code, k, child0(d));
-            w.w = (uint32_t)child0(d);
-          }
-          if (ar == 2) {
-            w.z = operand(code, k, child1(d));
-            w.w |= (uint32_t)child1(d) << 12;
-          }
-          prog[nop + __popc(mo & below)] = w;
-        }
-        nop += __popc(mo);
+      for (int j = lane; j < nvar; j += 32) {
+        const int var = child0(tape[sorted[j]]);
+        int i = 0;
+        while (child0(tape[sorted[i]]) != var) ++i;
+        lvar[j] = sorted[j] | sorted[i] << 12;
       }
-      if (lane == 0) {
-        info[0] = nop;
-        info[1] = ncon;
-        info[2] = norph;
-        info[3] = stack ? 1 : 0;
-        info[4] = (int)used;
-      }
+      __syncwarp();
     }
-    __syncthreads();
-    const int nop = info[0], ncon = info[1], norph = info[2];
-    const bool stack = info[3] != 0;
-    const unsigned xused = xrows ? (unsigned)info[4] : 0u;
-    for (int64_t i = threadIdx.x; i < (int64_t)ncon * K; i += blockDim.x) {
-      const int64_t j = i / K, kk = i - j * K;
-      cval[i] = __ldg(C + b * c_sb + (int64_t)lcon[j] * c_sm + (set + kk) * c_sk);
-    }
-    // every other node's gradient is zero
-    for (int64_t i = threadIdx.x; i < M * K; i += blockDim.x) {
-      const int64_t k = i / K, kk = i - k * K;
-      if (!(k < L && code_of(tape[k]) == LEARNABLE)) gC[(b * M + k) * Ktot + set + kk] = T(0);
-    }
-    const T* G = gout + (size_t)b * M * rs + set;
-    const T* Cc = cache ? cache + (size_t)b * M * rs + set : nullptr;
-    const int64_t vs = 32 * K * es;  // elements from one of a lane's values to the next
-    const uint32_t row_bytes = (uint32_t)(rs * (int64_t)sizeof(T));
-    const int Vp = stack ? V : 1;    // chunks in a pass
-
-    // sweeps of ncap constants each: one, but for tapes with more of them
-    for (int g0 = 0; g0 == 0 || g0 < ncon; g0 += ncap) {
-      const int ng = min(ncap, ncon - g0);
-      for (int i = threadIdx.x; i < ncap * (int)K * 32; i += blockDim.x) acc[i] = T(0);
-      __syncthreads();
-      T* const gXg = g0 == 0 ? gX : nullptr;
-      for (int64_t cl = kMode == kFlat ? warp : 0; cl < K; cl += kMode == kFlat ? nwarp : 1) {
-        const int64_t nq = cl < nchunks ? (nchunks - cl + K - 1) / K : 0;  // chunks of this class
-        const int64_t rounds = (nq + (int64_t)ranks * Vp - 1) / ((int64_t)ranks * Vp);
-        const int64_t kkl = kMode == kFlat ? (32 * cl + lane) % K : 0;
-        const T* const cv = cval + kkl;
-        T* const accl = acc + cl * ncap * 32 + lane;
-        int64_t p0 = 0;    // value index of the lane's first value in this pass
-        unsigned vm = 0;   // which of its values exist
-        uint32_t ep = 0;   // first error of each value: two bits (1 = 201, 2 = 204)
-        // a value's term of constant j
-        auto add_constant = [&](uint32_t idx, const T (&val)[V]) {
-          const int j = (int)idx - g0;
-          if (j < 0 || j >= ng) return;
-          if (ranks == 1) {
-            T t = accl[j * 32];
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-              if ((vm >> v & 1u) && val[v] != T(0)) t = M_<T>::add(t, val[v]);
-            accl[j * 32] = t;
-          } else {
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-              if (v < Vp) crow[(j * V + v) * 32 + lane] = (vm >> v & 1u) ? val[v] : T(0);
-          }
-        };
-        auto to_grad_x = [&](uint32_t var, const T (&val)[V]) {
-#pragma unroll
-          for (int v = 0; v < V; ++v) {
-            if ((vm >> v & 1u) && val[v] != T(0)) {
-              const int64_t p = p0 + v * 32 * K;
-              atomicAdd(gXg + (kMode == kFlat ? p / K : p) * n_x + var, val[v]);
-            }
-          }
-        };
-        unsigned char* const xs = wb + ly.xacc + lane * 16;  // the lane's sums per variable
-        auto add_variable = [&](uint32_t var, const T (&val)[V]) {
-          if (!gXg) return;
-          if (!xrows) return to_grad_x(var, val);
-          T t[V];
-          load16(xs + var * kRowBytes, t);
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-            if (val[v] != T(0)) t[v] = M_<T>::add(t[v], val[v]);
-          store16(xs + var * kRowBytes, t);
-        };
-        auto clear_variables = [&]() {
-          T zero[V];
-#pragma unroll
-          for (int v = 0; v < V; ++v) zero[v] = T(0);
-          for (unsigned m = xused; m; m &= m - 1) store16(xs + (__ffs((int)m) - 1) * kRowBytes, zero);
-        };
-        if (gXg) clear_variables();
-        auto place = [&](int64_t round, int64_t& p, unsigned& m) {
-          const int64_t q0 = (round * ranks + rank) * Vp;
-          p = 32 * (cl + K * q0) + lane;
-          m = 0;
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-            if (v < Vp && p + v * 32 * K < total) m |= 1u << v;
-        };
-        auto row = [&](const T* at, uint32_t k, unsigned m, T (&x)[V]) {  // at: the lane's first value of node 0
-          const T* r = reinterpret_cast<const T*>(reinterpret_cast<const char*>(at) + (uint64_t)k * row_bytes);
-#pragma unroll
-          for (int v = 0; v < V; ++v) x[v] = (m >> v & 1u) ? __ldg(r + v * vs) : T(0);
-        };
-        if (stack) {
-          // next: the loads of the node to come (operand values, children's output gradients,
-          // and its own for a node without a parent); cur: the node at hand
-          struct Loads {
-            uint4 w;
-            T a[V], b[V], s0[V], s1[V], g[V];
-          } next, cur;
-          next.w = make_uint4(0u, 0u, 0u, 0u);
-          auto value = [&](uint32_t w, uint32_t child, uint32_t own, const T* cp, unsigned m, T (&x)[V]) {
-            const uint32_t from = w & 3u;
-            if (from == kConstant) {
-              const T t = cv[(int64_t)(w >> 2 & 0xfffu) * K];
-#pragma unroll
-              for (int v = 0; v < V; ++v) x[v] = t;
-            } else if (from != kNoValue) {
-              row(cp, from == kOwnRow ? own : child, m, x);
-            }
-          };
-          // a child's adjoint: its output gradient plus the contribution
-          auto give = [&](uint32_t w, const T (&val)[V]) {
-            const uint32_t to = w >> 16 & 3u, idx = w >> 18 & 0xfffu;
-            if (to == kRow) store16(wb + idx * kRowBytes + lane * 16, val);
-            else if (to == kSum) add_constant(idx, val);
-            else if (to == kGradX) add_variable(idx, val);
-          };
-          int64_t pl = 0;      // first value, and which exist, of the pass that is being loaded
-          unsigned ml = 0;
-          int64_t round = 0, rcur = 0;  // the pass that is being loaded, the pass at hand
-          int in = nop - 1, icur = -1;  // the node to load next, the node at hand
-          if (rounds > 0) place(0, pl, ml);
-          while (true) {
-            const bool more = round < rounds;
-            cur = next;
-            if (more) {
-              next.w = prog[in];
-              const uint32_t own = next.w.x >> 8 & 0xfffu, c0 = next.w.w & 0xfffu, c1 = next.w.w >> 12;
-              const T *cp = Cc + pl * es, *gp = G + pl * es;
-              value(next.w.y, c0, own, cp, ml, next.a);
-              value(next.w.z, c1, own, cp, ml, next.b);
-              if (next.w.y >> 16 & 3u) row(gp, c0, ml, next.s0);
-              if (next.w.z >> 16 & 3u) row(gp, c1, ml, next.s1);
-              if (next.w.x & 32u) row(gp, own, ml, next.g);
-            }
-            if (icur >= 0) {
-              if (!(cur.w.x & 32u)) load16(wb + (cur.w.x >> 20) * kRowBytes + lane * 16, cur.g);
-              op_adjoint_onto<T, V>((int)(cur.w.x & 31u), cur.g, cur.a, cur.b, cur.s0, cur.s1, ep);
-              give(cur.w.y, cur.s0);
-              give(cur.w.z, cur.s1);
-              if (icur == 0) {  // the pass ends
-                for (int j = 0; j < norph; ++j) {  // leaves without a parent: their output gradient alone
-                  const uint32_t w = orphan[-j];
-                  T val[V];
-                  row(G + p0 * es, w & 0xfffu, vm, val);
-                  if (w & (1u << 12)) add_variable(w >> 13, val);
-                  else add_constant(w >> 13, val);
-                }
-                if (gXg && xused) {
-                  for (unsigned m = xused; m; m &= m - 1) {
-                    T t[V];
-                    load16(xs + (__ffs((int)m) - 1) * kRowBytes, t);
-                    to_grad_x((uint32_t)(__ffs((int)m) - 1), t);
-                  }
-                  clear_variables();
-                }
-                if (__any_sync(0xffffffffu, ep != 0)) {
-#pragma unroll
-                  for (int v = 0; v < V; ++v) {
-                    const uint32_t e = ep >> (2 * v) & 3u;
-                    if (e && (vm >> v & 1u)) {
-                      const int64_t p = p0 + v * 32 * K, n = kMode == kFlat ? p / K : p;
-                      const int64_t kk = kMode == kFlat ? p - n * K : set;
-                      atomicMin(&errs[n & 31], ((unsigned long long)(kk * pchunks + n / 32) << 16) |
-                                                   (unsigned long long)(e == 2 ? ERR_DIV_BY_ZERO : ERR_GRAD_ON_NO_OP));
-                    }
-                  }
-                  ep = 0;
-                }
-                if (ranks > 1) {
-                  __syncthreads();
-                  for (int j = rank; j < ng; j += ranks) {
-                    T t = accl[j * 32];
-                    for (int r = 0; r < ranks; ++r) {
-                      const T* cr = reinterpret_cast<const T*>(smem + ly.warps + (size_t)r * ly.warp_bytes + ly.crow);
-                      const int64_t q0 = (rcur * ranks + r) * V;
-#pragma unroll
-                      for (int v = 0; v < V; ++v) {
-                        if (q0 + v < nq) {
-                          const T x = cr[(j * V + v) * 32 + lane];
-                          if (x != T(0)) t = M_<T>::add(t, x);
-                        }
-                      }
-                    }
-                    accl[j * 32] = t;
-                  }
-                  __syncthreads();
-                }
-              }
-            }
-            if (!more) break;
-            if (in == nop - 1) {  // the first node of a pass is loaded: the pass begins
-              p0 = pl;
-              vm = ml;
-              rcur = round;
-            }
-            icur = in;
-            if (--in < 0) {
-              in = nop - 1;
-              if (++round < rounds) place(round, pl, ml);
-            }
-          }
-        } else {
-          GeneralSweep<T> q;
-          q.X = X; q.Cc = Cc; q.G = G; q.gX = gXg;
-          q.N = N; q.n_x = n_x; q.rs = rs; q.es = es; q.total = total; q.K = K; q.set = set; q.cl = cl;
-          q.nq = nq; q.rounds = rounds;
-          q.tape = tape; q.prog = prog; q.orphan = orphan; q.cidx = cidx; q.lcon = lcon; q.cv = cv; q.accl = accl;
-          q.adj = reinterpret_cast<T*>(wb) + lane; q.vals = reinterpret_cast<T*>(wb + ly.vals) + lane;
-          q.xs = reinterpret_cast<T*>(xs); q.xused = xused;
-          q.crow = crow; q.crows = smem + ly.warps + ly.crow; q.warp_bytes = ly.warp_bytes; q.errs = errs;
-          q.L = L; q.nop = nop; q.norph = norph; q.g0 = g0; q.ng = ng; q.lane = lane; q.rank = rank; q.ranks = ranks;
-          general_sweep<T, kMode>(q);
+    int err = 0;
+    const int64_t nchunks = (N + 31) / 32;
+    // the sets one after the other: set kk of node k, point n is at ((b M + k) N + n) K + kk
+    for (int64_t kk = 0; kk < K; ++kk) {
+      const T* Crow = C + b * c_sb + kk * c_sk;
+      for (int j = lane; j < ncon; j += 32) bc[1 + lcon[j]] = __ldg(Crow + (int64_t)lcon[j] * c_sm);
+      for (int j = 0; j < ncon; ++j) vals[lcon[j] * 32 + lane] = T(0);
+      const T* G = gout + (size_t)b * M * rs + kk;
+      const T* Cc = kCached ? cache + (size_t)b * M * rs + kk : nullptr;
+      __syncwarp();
+      for (int64_t c = 0; c < nchunks; ++c) {
+        const int64_t n = c * 32 + lane, nn = n < N ? n : N - 1;
+        const bool valid = n < N;
+        // the adjoints start as the output gradients
+        stage_rows(adj, G, L, [](int r) { return r; }, N, rs, K, c * 32, lane, vec16);
+        if constexpr (kCached) {
+          auto node = [&](int r) { return r < nop ? (int)((pown[r] - ly.vals) / RB) : (int)(lvar[r - nop] & 0xfffu); };
+          stage_rows(vals, Cc, nop + nvar, node, N, rs, K, c * 32, lane, vec16);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if constexpr (!kCached) {
+          for (int j = 0; j < nvar; ++j) {
+            const int k = (int)(lvar[j] & 0xfffu);
+            vals[k * 32 + lane] = __ldg(X + nn * n_x + child0(tape[k]));
+          }
+          for (int i = 0; i < nop; ++i) {
+            const int code = (int)code_[i];
+            const uint32_t sa = psa[i], sb = psb[i], own = pown[i];
+            at(own) = op_value<T>(code, operand(sa), operand(sb));
+          }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        for (int i = nop - 1; i >= 0; --i) {
+          const int code = (int)code_[i];
+          const uint32_t sa = psa[i], sb = psb[i], own = pown[i], da = pda[i], db = pdb[i];
+          T g[1], a[1], c1[1], v[1], o0[1], o1[1];
+          bool a0[1], a1[1];
+          int e[1];
+          g[0] = at(own + adj_delta);
+          a[0] = operand(sa);
+          c1[0] = operand(sb);
+          v[0] = at(own);
+          op_adjoint_v<T, 1>(code, g, a, c1, v, a0, o0, a1, o1, e);
+          if (valid) {
+            if (e[0] && !err) err = e[0];
+            if (a0[0]) { T& x = at(da); x = M_<T>::add(x, o0[0]); }
+            if (a1[0]) { T& x = at(db); x = M_<T>::add(x, o1[0]); }
+          }
+        }
+        // leaves: every contribution from the parents has arrived
+        for (int j = 0; j < ncon; ++j) {
+          const T g = adj[lcon[j] * 32 + lane];
+          T& x = vals[lcon[j] * 32 + lane];
+          if (valid && g != T(0)) x = M_<T>::add(x, g);
+        }
+        if (gX) {
+          for (int j = 1; j < nvar; ++j) {
+            const uint32_t k = lvar[j] & 0xfffu, first = lvar[j] >> 12;
+            const T g = adj[k * 32 + lane];
+            T& x = adj[first * 32 + lane];
+            if (k != first && g != T(0)) x = M_<T>::add(x, g);
+          }
+          for (int j = 0; j < nvar; ++j) {
+            const uint32_t k = lvar[j] & 0xfffu;
+            const T g = adj[k * 32 + lane];
+            if (k == lvar[j] >> 12 && valid && g != T(0)) atomicAdd(gX + nn * n_x + child0(tape[k]), g);
+          }
+        }
+        __syncwarp();  // every lane is done with the rows before the next chunk's land
       }
-      __syncthreads();  // every class's sums are complete
-      for (int i = warp; i < ng * (int)K; i += nwarp) {
-        const int j = i / (int)K, kk = i - j * (int)K;
-        const int pos = lane * (int)K + kk;
-        const T s = warp_sum(acc[((pos >> 5) * ncap + j) * 32 + (pos & 31)]);
-        if (lane == 0) gC[(b * M + lcon[g0 + j]) * Ktot + set + kk] = s;
+      // the constants' sums (lane partials in chunk order, then a butterfly) replace
+      // their values in the broadcast entries
+      for (int j = 0; j < ncon; ++j) {
+        const T part = warp_sum(vals[lcon[j] * 32 + lane]);
+        if (lane == 0) bc[1 + lcon[j]] = part;
       }
-      __syncthreads();
+      __syncwarp();
+      for (int64_t k = lane; k < M; k += 32)
+        gC[(b * M + k) * K + kk] = k < L && code_of(tape[k]) == LEARNABLE ? bc[1 + k] : T(0);
+      __syncwarp();
     }
-    if (warp == 0) {
-      int err = errs[lane] == ~0ull ? 0 : (int)(errs[lane] & 0xffffu);
-      err = __reduce_max_sync(0xffffffffu, err);
-      if (err && lane == 0) report_adjoint(status, err);
-    }
+    err = __reduce_max_sync(0xffffffffu, err);
+    if (err && lane == 0) report_adjoint(status, err);
+    __syncwarp();
   }
 }
 
@@ -757,14 +1187,14 @@ __global__ void __launch_bounds__(256, 2) eval_adjoint_kernel(
 //   warps: the power of two that puts the most warps on the GPU at once, as far as the points
 //          reach: one when the batch alone fills it (1003 tapes at N = 777: 97 us with 4 warps,
 //          167 us with 2).
-template <typename T, int kMode>
+template <typename T, int kMode, bool kCached, bool kGeneral>
 static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_x, const uint32_t* desc, const int32_t* meta,
                                const int32_t* order, int64_t B, int64_t M, int Llo, int Lhi, const T* C, int64_t c_sb,
                                int64_t c_sm, int64_t c_sk, int64_t K, const T* gout, T* gC, T* gX, int32_t* status,
                                cudaStream_t st) {
-  auto kern = eval_adjoint_kernel<T, kMode>;
+  auto kern = eval_adjoint_kernel<T, kMode, kCached, kGeneral>;
+  constexpr int V = kCached ? Pack<T>::V / 2 : 1;  // as few points per warp as a general sweep can use
   const void* kp = reinterpret_cast<const void*>(kern);
-  const int xrows = gX ? x_sum_rows(n_x) : 0;
   const int64_t flat = kMode == kFlat ? K : 1, units = kMode == kStrided ? B * K : B;
   const int64_t chunks = (N * flat + 31) / 32;
   const int limit = max_dyn_smem(), sms = device_sm_count(), sm_bytes = max_sm_smem();
@@ -773,11 +1203,17 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
     rc = cuda_check(cudaFuncSetAttribute(kp, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared), "adjoint carveout");
   if (rc) return rc;
-  const int64_t most = kMode == kFlat ? flat : (chunks + Pack<T>::V - 1) / Pack<T>::V;
+  // a tape that only just fits gets one constant at a time and no sums per variable
+  int xrows = gX ? x_sum_rows(n_x) : 0;
+  auto bytes_of = [&](int w, int cap) { return adjoint_layout<T>(Lhi, flat, w, !kCached, xrows, cap).bytes; };
+  const bool tight = bytes_of(1, sum_capacity<T>(Lhi, flat, 1)) > (size_t)limit;
+  if (tight) xrows = 0;
+  auto capacity = [&](int w) { return tight ? 1 : sum_capacity<T>(Lhi, flat, w); };
+  const int64_t most = kMode == kFlat ? flat : (chunks + V - 1) / V;
   int best_w = 0, per_sm = 0;
   int64_t most_warps = 0;
   for (int w = 1; w <= 8; w *= 2) {
-    const size_t bytes = adjoint_layout<T>(Lhi, flat, w, !cache, xrows).bytes;
+    const size_t bytes = bytes_of(w, capacity(w));
     if (bytes > (size_t)limit) break;
     int blocks = resident_ctas(kp, w * 32, bytes);
     if (blocks < 1) break;
@@ -804,22 +1240,48 @@ static int launch_adjoint_mode(const T* X, const T* cache, int64_t N, int64_t n_
   }
   int64_t blocks = (int64_t)sms * per_sm;
   if (blocks > units) blocks = units;
-  kern<<<(unsigned)blocks, best_w * 32, adjoint_layout<T>(Lhi, flat, best_w, !cache, xrows).bytes, st>>>(
-      X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status);
+  const AdjArgs<T> args{X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, xrows, capacity(best_w), C, c_sb, c_sm, c_sk, K, gout, gC, gX, status};
+  kern<<<(unsigned)blocks, best_w * 32, bytes_of(best_w, capacity(best_w)), st>>>(args);
   return launch_check("eval_adjoint_kernel");
 }
 
-template <typename T>
-static int launch_backward_class(const T* X, int64_t N, int64_t n_x, const uint32_t* desc, const int32_t* meta,
-                                 const int32_t* order, int64_t B, int64_t M, int Llo, int Lhi, const T* C,
-                                 int64_t c_sb, int64_t c_sm, int64_t c_sk, int64_t K, const T* cache, const T* gout,
-                                 T* gC, T* gX, int32_t* status, cudaStream_t st) {
-#define SR_ADJ_ARGS X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status, st
+template <typename T, bool kCached>
+static int launch_streaming(const T* X, const T* cache, int64_t N, int64_t n_x, const uint32_t* desc, const int32_t* meta,
+                            const int32_t* order, int64_t B, int64_t M, int Llo, int Lhi, const T* C, int64_t c_sb,
+                            int64_t c_sm, int64_t c_sk, int64_t K, const T* gout, T* gC, T* gX, int32_t* status,
+                            bool stack_only, cudaStream_t st) {
+#define SR_ADJ_ARGS \
+  X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status, st
   const int xrows = gX ? x_sum_rows(n_x) : 0;
-  if (K == 1) return launch_adjoint_mode<T, kSingle>(SR_ADJ_ARGS);
-  if (K <= 64 && adjoint_layout<T>(Lhi, K, 1, !cache, xrows).bytes <= (56u << 10)) return launch_adjoint_mode<T, kFlat>(SR_ADJ_ARGS);
-  return launch_adjoint_mode<T, kStrided>(SR_ADJ_ARGS);
+  if (K == 1)
+    return stack_only ? launch_adjoint_mode<T, kSingle, true, false>(SR_ADJ_ARGS)
+                      : launch_adjoint_mode<T, kSingle, kCached, true>(SR_ADJ_ARGS);
+  if (K <= 64 && adjoint_layout<T>(Lhi, K, 1, !kCached, xrows, sum_capacity<T>(Lhi, K, 1)).bytes <= (56u << 10))
+    return launch_adjoint_mode<T, kFlat, kCached, true>(SR_ADJ_ARGS);
+  return launch_adjoint_mode<T, kStrided, kCached, true>(SR_ADJ_ARGS);
 #undef SR_ADJ_ARGS
+}
+
+template <typename T, bool kCached>
+static int launch_staged(const T* X, const T* cache, int64_t N, int64_t n_x, const uint32_t* desc, const int32_t* meta,
+                         const int32_t* order, int64_t B, int64_t M, int Llo, int Lhi, const T* C, int64_t c_sb,
+                         int64_t c_sm, int64_t c_sk, int64_t K, const T* gout, T* gC, T* gX, int32_t* status,
+                         bool general_only, cudaStream_t st) {
+  auto kern = K == 1 ? eval_adjoint_staged_kernel<T, false, kCached> : eval_adjoint_staged_kernel<T, true, kCached>;
+  Shape sh;
+  // beside the padding check's ring, which a large batch keeps busy meanwhile (16384 tapes with
+  // shared subtrees 1.98 to 1.85 ms; 4096 of them 743 to 910 us)
+  const size_t reserve = general_only && B >= (int64_t)device_sm_count() * 32 ? kCheckReserve : 0;
+  if (!pick_shape(reinterpret_cast<const void*>(kern), staged_layout<T>(Lhi).bytes, B, sh, reserve)) {
+    set_error("tape of %d nodes does not fit in shared memory", Lhi);
+    return SR_ERR_UNSUPPORTED;
+  }
+  auto aligned = [&](const T* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  const bool vec16 = K == 1 && aligned(gout) && aligned(cache) && N % Pack<T>::V == 0;
+  kern<<<(unsigned)sh.blocks, sh.warps * 32, sh.smem, st>>>(X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi,
+                                                           general_only, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status,
+                                                           vec16);
+  return launch_check("eval_adjoint_staged_kernel");
 }
 
 template <typename T>
@@ -844,13 +1306,23 @@ static int launch_backward(const T* X, int64_t N, int64_t n_x, const uint32_t* d
   SideStream side((double)B * M * N * K * sizeof(T) > (double)(8 << 20), st);
   rc = side.begin();
   if (rc) return rc;
+  // which kernel takes what (see eval_adjoint_staged_kernel, whose tables hold fewer nodes).  A batch
+  // fills the GPU when at least half of that kernel's warps that fit get a tape.
+  const int64_t sms = device_sm_count();
+  const size_t staged_bytes = staged_layout<T>(Lmax).bytes;
+  const int64_t per_sm = (int64_t)(max_sm_smem() / staged_bytes) < 32 ? (int64_t)(max_sm_smem() / staged_bytes) : 32;
+  const bool holds = staged_bytes <= (size_t)max_dyn_smem(), fills = holds && K <= 4 && 2 * B >= sms * per_sm;
+  const bool few = holds && N <= 16 * Pack<T>::V && K <= 4;
+  const bool all_staged = few || (fills && (!cache || (K == 1 && B >= sms * 192)));
+  const bool general_staged = fills && K == 1 && !all_staged;
   // one persistent grid per class of tape lengths (Llo, Lhi], each with the tables its class
-  // needs; a batch too small to fill the GPU class by class runs as one grid
-  const int bound[3] = {64, 32, 16};
+  // needs; a batch too small to fill the GPU class by class runs as one grid.  The staged kernel's
+  // tables are the larger: its longest class is split at 48 rather than 64.
+  const int bound[3] = {all_staged ? 48 : 64, 32, 16};
   int cls[4][2], nc = 0, hi = Lmax;
-  const bool split = B * K >= (int64_t)device_sm_count() * 32;
+  const bool split = B * K >= sms * 32;
   for (int j = 0; j < 3; ++j) {
-    if (hi > bound[j] && (split || bound[j] == 64)) {
+    if (hi > bound[j] && (split || hi > 64)) {
       cls[nc][0] = bound[j];
       cls[nc][1] = hi;
       ++nc;
@@ -860,23 +1332,37 @@ static int launch_backward(const T* X, int64_t N, int64_t n_x, const uint32_t* d
   cls[nc][0] = -1;
   cls[nc][1] = hi;
   ++nc;
-  {
+  auto check = [&]() -> int {
+    if (all_staged) {
+      const int64_t pblocks = sms * 2 < B ? sms * 2 : B;
+      padding_check_direct_kernel<T><<<(unsigned)pblocks, 256, 0, side.stream()>>>(gout, meta, B, M, N * K, Lmax, status);
+      return launch_check("padding_check_direct_kernel");
+    }
     // one CTA per SM, placed before the adjoint's grids, which leave it its shared memory.  An
     // SM cannot change its split of L1 and shared memory while a CTA is on it, so both ask for
     // the largest shared memory, or whichever comes first locks the other out
-    int64_t pblocks = device_sm_count();
-    if (pblocks > B) pblocks = B;
-    rc = cuda_check(cudaFuncSetAttribute(padding_check_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                         cudaSharedmemCarveoutMaxShared), "check carveout");
-    if (!rc) {
-      padding_check_kernel<T><<<(unsigned)pblocks, (kCheckWarps + 1) * 32, 0, side.stream()>>>(gout, meta, B, M, N * K,
-                                                                                            Lmax, status);
-      rc = launch_check("padding_check_kernel");
-    }
-  }
+    const int64_t pblocks = sms < B ? sms : B;
+    const int e = cuda_check(cudaFuncSetAttribute(padding_check_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                  cudaSharedmemCarveoutMaxShared), "check carveout");
+    if (e) return e;
+    padding_check_kernel<T><<<(unsigned)pblocks, (kCheckWarps + 1) * 32, 0, side.stream()>>>(gout, meta, B, M, N * K,
+                                                                                          Lmax, status);
+    return launch_check("padding_check_kernel");
+  };
+  if (!all_staged) rc = check();
   for (int ci = 0; ci < nc && !rc; ++ci) {
-    rc = launch_backward_class<T>(X, N, n_x, desc, meta, order, B, M, cls[ci][0], cls[ci][1], C, c_sb, c_sm, c_sk, K,
-                                  cache, gout, gC, gX, status, st);
+    const int Llo = cls[ci][0], Lhi = cls[ci][1];
+    auto streaming = cache ? launch_streaming<T, true> : launch_streaming<T, false>;
+    auto staged = cache ? launch_staged<T, true> : launch_staged<T, false>;
+    if (!all_staged)
+      rc = streaming(X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status,
+                     general_staged, st);
+    if (!rc && (all_staged || general_staged))
+      rc = staged(X, cache, N, n_x, desc, meta, order, B, M, Llo, Lhi, C, c_sb, c_sm, c_sk, K, gout, gC, gX, status,
+                  general_staged, st);
+    // enqueued after the first grid, whose CTAs are placed first: the check's CTAs take the
+    // registers and warp slots they leave
+    if (!rc && all_staged && ci == 0) rc = check();
   }
   const int rj = side.end();
   return rc ? rc : rj;

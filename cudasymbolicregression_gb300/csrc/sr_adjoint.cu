@@ -344,25 +344,6 @@ __device__ __forceinline__ bool in_stack_order(int need, int Lhi, int64_t rs) {
   return need >= 0 && need <= table_rows<T>(Lhi) && rs <= (int64_t)0xffffffff / (int64_t)sizeof(T);
 }
 
-// A lane's part of a row: VV values.
-template <typename T, int VV>
-__device__ __forceinline__ void load_part(const void* p, T (&r)[VV]) {
-  if constexpr (VV * sizeof(T) == 16) {
-    load16(p, r);
-  } else if constexpr (VV == 2) {
-    const float2 t = *reinterpret_cast<const float2*>(p);
-    r[0] = t.x; r[1] = t.y;
-  } else {
-    r[0] = *reinterpret_cast<const T*>(p);
-  }
-}
-template <typename T, int VV>
-__device__ __forceinline__ void store_part(void* p, const T (&r)[VV]) {
-  if constexpr (VV * sizeof(T) == 16) store16(p, r);
-  else if constexpr (VV == 2) *reinterpret_cast<float2*>(p) = make_float2(r[0], r[1]);
-  else *reinterpret_cast<T*>(p) = r[0];
-}
-
 // What a warp sweeps: one class of a unit's chunks.
 template <typename T>
 struct Sweep {

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "sr_eval.cuh"
 
@@ -134,7 +135,8 @@ __global__ void __launch_bounds__(256) tape_compile_kernel(const int64_t* __rest
 // memory: the copy engine moves the bytes, so the fill takes next to none of the issue slots
 // and warp places that the forward needs (as a kernel of vector stores it held 64 warps of
 // every SM, and the forward grids waited for it: 16384 tapes of mean length 20, M = 64,
-// N = 1024: 925 us with it, 697 us with the copies, for 4.3 GB).
+// N = 1024: 925 us with it, 697 us with the copies, for 4.3 GB).  Short ranges go 32 at a time, a
+// lane each: one after the other they were what 5000 short tapes waited for.
 // A tape longer than the max_len the call was given is evaluated by no class grid: its
 // whole block is NaN, so no row keeps what the buffer held before.
 constexpr int kFillBytes = 4096;          // one bulk copy
@@ -150,24 +152,42 @@ __global__ void __launch_bounds__(32) pad_fill_kernel(const int32_t* __restrict_
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
   const uint32_t src = static_cast<uint32_t>(__cvta_generic_to_shared(block));
-  for (int64_t b = blockIdx.x; b < B; b += gridDim.x) {
-    int64_t L = meta[b * 4];
-    if (L > Lmax) L = 0;
-    T* p = cache + (size_t)b * M * NK + (size_t)L * NK;
-    const size_t count = (size_t)(M - L) * NK;
+  // 32 tapes at a time: a lane for each while their ranges take one copy (or none), else the warp
+  // for one after the other
+  auto range = [&](int64_t b, int64_t L, T*& p, size_t& count, size_t& head) -> size_t {
+    p = cache + (size_t)b * M * NK + (size_t)L * NK;
+    count = (size_t)(M - L) * NK;
     // bulk copies start and end on 16-byte boundaries
-    size_t head = ((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(T);
+    head = ((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / sizeof(T);
     if (head > count) head = count;
-    const size_t body = (count - head) * sizeof(T) & ~size_t(15), tail = head + body / sizeof(T);
-    if ((size_t)lane < head) __stcs(p + lane, qnan);
-    unsigned char* q = reinterpret_cast<unsigned char*>(p + head);
-    for (size_t off = (size_t)lane * kFillBytes; off < body; off += 32 * (size_t)kFillBytes) {
-      const uint32_t bytes = (uint32_t)(body - off < (size_t)kFillBytes ? body - off : (size_t)kFillBytes);
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(q + off), "r"(src), "r"(bytes)
-                   : "memory");
+    return (count - head) * sizeof(T) & ~size_t(15);
+  };
+  auto copy = [&](void* to, size_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(to), "r"(src), "r"((uint32_t)bytes)
+                 : "memory");
+  };
+  for (int64_t b0 = blockIdx.x; b0 < B; b0 += 32 * (int64_t)gridDim.x) {
+    const int64_t mine = b0 + (int64_t)lane * gridDim.x;
+    int L = mine < B ? meta[mine * 4] : 0;
+    if (L > Lmax) L = 0;
+    T* p;
+    size_t count = 0, head = 0, body = 0;
+    if (mine < B) body = range(mine, L, p, count, head);
+    if (!__any_sync(0xffffffffu, body > (size_t)kFillBytes)) {
+      for (size_t i = 0; i < head; ++i) __stcs(p + i, qnan);
+      if (body) copy(p + head, body);
+      for (size_t i = head + body / sizeof(T); i < count; ++i) __stcs(p + i, qnan);
+    } else {
+      for (int t = 0; t < 32 && b0 + (int64_t)t * gridDim.x < B; ++t) {
+        body = range(b0 + (int64_t)t * gridDim.x, __shfl_sync(0xffffffffu, L, t), p, count, head);
+        const size_t tail = head + body / sizeof(T);
+        if ((size_t)lane < head) __stcs(p + lane, qnan);
+        for (size_t off = (size_t)lane * kFillBytes; off < body; off += 32 * (size_t)kFillBytes)
+          copy(reinterpret_cast<unsigned char*>(p + head) + off, body - off < (size_t)kFillBytes ? body - off : (size_t)kFillBytes);
+        if (tail + lane < count) __stcs(p + tail + lane, qnan);
+      }
     }
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    if (tail + lane < count) __stcs(p + tail + lane, qnan);
   }
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
@@ -257,6 +277,14 @@ __global__ void __launch_bounds__(256) any_nonzero_kernel(const int64_t* __restr
 // 128.  Measured with the fill kernel above: 16384 tapes of mean length 20 at N = 1024, 914 to
 // 697 us (6.2 TB/s); 65536 tapes 3500 to 2770 us; 1003 tapes at N = 777, 135 to 72 us.
 //
+// Tapes out of stack order take a row per operator, and as many values per lane (V, V / 2 or 1)
+// as the table then holds: with one value and a row per node 4096 tapes with shared subtrees took
+// 302 us where this takes 239, deep tapes (20 results waiting) 568 and 355; where every tape
+// has 30 operators out of order (422 us) the kernel of one point per lane, with more warps, took
+// 382.  Variables beyond the rows are numbered by the tape's distinct ones (17 variables: 394 to
+// 270 us).  Few points skip the search for the stack's order, as a pass of V values per lane
+// would be half empty: 20000 tapes at N = 16, 72 to 43 us with the fill's change.
+//
 // With K constant sets the cache is (B, M, N, K): node k's values are the N K consecutive
 // elements p = n K + kk, and the lanes run over them as over points (coalesced stores for
 // any K; stores K elements apart took 537 us for 1000 tapes at N = 256, K = 8, where this takes
@@ -271,18 +299,19 @@ __global__ void __launch_bounds__(256) any_nonzero_kernel(const int64_t* __restr
 // constants' values (K entries for each learnable or fixed leaf), the rows of the variables,
 // and the rows of the operator results.
 struct FwdLayout {
-  size_t prog, cval, xrow, rows, bytes;
+  size_t prog, cval, xvar, xrow, rows, bytes;
 };
 
 
-constexpr int kMaxVarRows = 16;  // variables held in rows; tapes over others take the general path
+constexpr int kMaxVarRows = 16;  // variables held in rows
 
 template <typename T>
 __host__ __device__ __forceinline__ FwdLayout forward_layout(int Lmax, int nx_rows, int64_t K) {
   FwdLayout l;
   l.prog = align16((size_t)Lmax * 4);
   l.cval = l.prog + 16 * (size_t)Lmax;
-  l.xrow = l.cval + align16((size_t)Lmax * (size_t)K * sizeof(T));
+  l.xvar = l.cval + align16((size_t)Lmax * (size_t)K * sizeof(T));
+  l.xrow = l.xvar + (nx_rows > 0 ? kMaxVarRows * 4 : 0);
   l.rows = l.xrow + (size_t)nx_rows * kRowBytes;
   l.bytes = l.rows + (size_t)table_rows<T>(Lmax) * kRowBytes;
   return l;
@@ -302,14 +331,15 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
                                                            int64_t c_sk, int64_t K_, int64_t slice, int64_t nslices,
                                                            T* __restrict__ cache) {
   constexpr int V = Pack<T>::V;
+  constexpr int G = V / 2;  // values per lane where the rows do not hold V
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr bool kMulti = kMode == kFlat;
   const int64_t K = kMulti ? K_ : 1;            // sets in one pass (one: the index arithmetic folds)
   const int64_t es = kMode == kStrided ? K_ : 1;  // elements between the values of a unit
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const FwdLayout fl = forward_layout<T>(Lhi, nx_rows, K);
-  const struct { uint32_t prog, cval, xrow, rows; } ly{(uint32_t)fl.prog, (uint32_t)fl.cval, (uint32_t)fl.xrow,
-                                                       (uint32_t)fl.rows};
+  const struct { uint32_t prog, cval, xvar, xrow, rows; } ly{(uint32_t)fl.prog, (uint32_t)fl.cval, (uint32_t)fl.xvar,
+                                                             (uint32_t)fl.xrow, (uint32_t)fl.rows};
   const int R = table_rows<T>(Lhi);
   unsigned char* wb = smem + (size_t)warp * fl.bytes;
   uint32_t* tape = reinterpret_cast<uint32_t*>(wb);
@@ -330,17 +360,60 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
     __syncwarp();
     // the rows: while the program is built their place holds the scratch of stack_rows
     int* row = reinterpret_cast<int*>(wb + ly.rows);
-    const int need = stack_rows(tape, L, lane, row + L, row);
-    bool stack = need >= 0 && need <= R;
-    unsigned used = 0;  // variables of the tape
+    int* xvar = reinterpret_cast<int*>(wb + ly.xvar);  // variable of each row, where not the row's number
+    // few points: no pass of 32 V values, so rows are not short and stack order is not looked for
+    const bool few = total <= 16 * V;
+    int need = few ? -1 : stack_rows(tape, L, lane, row + L, row);
+    // variables of the tape in rows: row v for variable v, or the distinct ones in the order found
+    const bool by_number = n_x <= nx_rows;
+    unsigned used = 0;
+    int nvr = 0;  // rows taken
     for (int k0 = 0; k0 < L; k0 += 32) {
       const int k = k0 + lane;
       const bool isvar = k < L && code_of(tape[k]) == VAR;
       const int var = isvar ? child0(tape[k]) : 0;
-      if (__any_sync(0xffffffffu, isvar && var >= nx_rows)) stack = false;
-      used |= __reduce_or_sync(0xffffffffu, isvar ? 1u << (var & 31) : 0u);
+      if (by_number) {
+        used |= __reduce_or_sync(0xffffffffu, isvar ? 1u << (var & 31) : 0u);
+        nvr = max(nvr, __reduce_max_sync(0xffffffffu, isvar ? var + 1 : 0));
+      } else if (nvr <= nx_rows) {
+        int at = -1;  // its row
+        for (int r = 0; r < nvr; ++r) at = isvar && xvar[r] == var ? r : at;
+        const unsigned same = __match_any_sync(0xffffffffu, isvar ? var : -1 - lane);
+        const bool fresh = isvar && at < 0 && (same & below) == 0;
+        const unsigned mf = __ballot_sync(0xffffffffu, fresh);
+        if (fresh) {
+          at = nvr + __popc(mf & below);
+          if (at < nx_rows) xvar[at] = var;
+        }
+        at = __shfl_sync(0xffffffffu, at, __ffs((int)same) - 1);
+        if (isvar) row[k] = at;
+        nvr += __popc(mf);
+        __syncwarp();
+      }
     }
-    const uint32_t row_bytes = stack ? kRowBytes : 32u * (uint32_t)sizeof(T);
+    // more variables than rows: every variable leaf takes a row of its own among the operators'
+    const bool own_rows = nvr > nx_rows;
+    const uint32_t vrow = own_rows ? ly.rows : ly.xrow;
+    if (own_rows) {
+      need = -1;
+      used = 0;
+      nvr = 0;
+    }
+    if (need < 0) {  // a row for each operator (and such leaf)
+      need = 0;
+      for (int k0 = 0; k0 < L; k0 += 32) {
+        const int k = k0 + lane;
+        const int code = k < L ? code_of(tape[k]) : ZERO;
+        const bool has = is_op_code(code) || (own_rows && code == VAR);
+        const unsigned mh = __ballot_sync(0xffffffffu, has);
+        if (has) row[k] = need + __popc(mh & below);
+        need += __popc(mh);
+      }
+      __syncwarp();
+    }
+    // values per lane: as many as the rows hold
+    const int VV = need <= R && !few ? V : G > 1 && need * G <= R * V && total > 32 ? G : 1;
+    const uint32_t row_bytes = 32u * (uint32_t)VV * (uint32_t)sizeof(T);
     // a leaf's constant index is its position among the broadcast leaves (written first: the
     // program's operand words need it)
     int nleaf = 0, nbc = 0;
@@ -351,7 +424,12 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
       const unsigned ml = __ballot_sync(0xffffffffu, isleaf), mb = __ballot_sync(0xffffffffu, isleaf && !isvar);
       const int j = nbc + __popc(mb & below);
       if (isleaf) {
-        const uint32_t idx = isvar ? (uint32_t)child0(tape[k]) : (uint32_t)j;
+        int xr = 0;  // a variable's row
+        if (isvar) {
+          xr = by_number && !own_rows ? child0(tape[k]) : row[k];
+          row[k] = xr;
+        }
+        const uint32_t idx = isvar ? (uint32_t)xr : (uint32_t)j;
         leaf[-(nleaf + __popc(ml & below))] = (uint32_t)k | (isvar ? 1u << 12 : 0u) | (idx << 13);
         if (!isvar) {
           row[k] = j;  // a broadcast leaf has no row: its place holds the constant index
@@ -367,9 +445,8 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
     __syncwarp();
     auto operand = [&](int c) -> uint32_t {
       const int cc = code_of(tape[c]);
-      if (is_op_code(cc)) return ly.rows + (uint32_t)(stack ? row[c] : c) * row_bytes;
-      if (cc == VAR)
-        return stack ? ly.xrow + (uint32_t)child0(tape[c]) * kRowBytes : ly.rows + (uint32_t)c * row_bytes;
+      if (is_op_code(cc)) return ly.rows + (uint32_t)row[c] * row_bytes;
+      if (cc == VAR) return vrow + (uint32_t)row[c] * row_bytes;
       return kConstOperand | (ly.cval + (uint32_t)row[c] * (uint32_t)K * (uint32_t)sizeof(T));
     };
     int nop = 0;
@@ -381,7 +458,7 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
       const unsigned mo = __ballot_sync(0xffffffffu, isop);
       if (isop) {
         // an operand that is not there reads the node's own row (its value is not used)
-        const uint32_t own = ly.rows + (uint32_t)(stack ? row[k] : k) * row_bytes;
+        const uint32_t own = ly.rows + (uint32_t)row[k] * row_bytes;
         prog[nop + __popc(mo & below)] = make_uint4((uint32_t)dense_op(code) | ((uint32_t)k << 8), own,
                                                     ar >= 1 ? operand(child0(d)) : own, ar == 2 ? operand(child1(d)) : own);
       }
@@ -390,95 +467,89 @@ __global__ void __launch_bounds__(256) eval_forward_kernel(const T* __restrict__
     __syncwarp();
     T* out = cache + (size_t)b * M * rs + set;
     const int64_t e0 = sl * slice, e1 = min(total, e0 + slice);
-    if (stack) {
-      for (int64_t base = e0; base < e1; base += 32 * V) {
+    auto passes = [&](auto width) {
+      constexpr int W = decltype(width)::value;  // values per lane
+      for (int64_t base = e0; base < e1; base += 32 * W) {
         // element, point and constant-set index of each of the lane's values
-        int64_t p[V];
-        uint32_t kko[V];
-        bool valid[V];
-        int64_t n[V];
+        int64_t p[W];
+        uint32_t kko[W];
+        bool valid[W];
+        int64_t n[W];
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          p[v] = base + (kVec ? lane * V + v : 32 * v + lane);
+        for (int v = 0; v < W; ++v) {
+          p[v] = base + (kVec ? lane * W + v : 32 * v + lane);
           valid[v] = p[v] < e1;
           const int64_t q = valid[v] ? p[v] : e1 - 1;
-          n[v] = kMulti ? q / K : q;
+          n[v] = !kMulti ? q : total <= (int64_t)0xffffffff ? (int64_t)((uint32_t)q / (uint32_t)K) : q / K;
           kko[v] = kMulti ? (uint32_t)(q - n[v] * K) * (uint32_t)sizeof(T) : 0u;
         }
-        auto put = [&](int64_t k, const T (&x)[V]) {
+        unsigned char* const mine = wb + lane * (W * (int)sizeof(T));
+        auto put = [&](int64_t k, const T (&x)[W]) {
           T* o = out + k * rs;
           if (kVec) {  // the row's elements come in whole packs
-            if (valid[0]) stream16(o + p[0], x);
+            if (valid[0]) stream_part<T, W>(o + p[0], x);
           } else {
 #pragma unroll
-            for (int v = 0; v < V; ++v)
+            for (int v = 0; v < W; ++v)
               if (valid[v]) __stcs(o + p[v] * es, x[v]);
           }
         };
-        auto constant = [&](uint32_t off, T (&x)[V]) {
+        auto constant = [&](uint32_t off, T (&x)[W]) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) x[v] = *reinterpret_cast<const T*>(wb + off + kko[v]);
+          for (int v = 0; v < W; ++v) x[v] = *reinterpret_cast<const T*>(wb + off + kko[v]);
         };
-        auto fetch = [&](uint32_t w, T (&x)[V]) {
+        auto fetch = [&](uint32_t w, T (&x)[W]) {
           if (w & kConstOperand) constant(w & ~kConstOperand, x);
-          else load16(wb + w + lane * 16, x);
+          else load_part<T, W>(mine + w, x);
         };
-        for (unsigned m = used; m; m &= m - 1) {
-          const int var = __ffs((int)m) - 1;
-          T x[V];
+        auto variable = [&](int var, T (&x)[W]) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) x[v] = __ldg(X + n[v] * n_x + var);
-          store16(wb + ly.xrow + (uint32_t)var * kRowBytes + lane * 16, x);
+          for (int v = 0; v < W; ++v) x[v] = __ldg(X + n[v] * n_x + var);
+        };
+        if (by_number) {
+          for (unsigned m = used; m; m &= m - 1) {
+            const int var = __ffs((int)m) - 1;
+            T x[W];
+            variable(var, x);
+            store_part<T, W>(mine + vrow + (uint32_t)var * row_bytes, x);
+          }
+        } else {
+          for (int r = 0; r < nvr; ++r) {
+            T x[W];
+            variable(xvar[r], x);
+            store_part<T, W>(mine + vrow + (uint32_t)r * row_bytes, x);
+          }
+        }
+        if (own_rows) {
+          for (int j = 0; j < nleaf; ++j) {
+            const uint32_t w = leaf[-j];
+            T x[W];
+            if (!(w & (1u << 12))) continue;
+            variable(child0(tape[w & 0xfffu]), x);
+            store_part<T, W>(mine + vrow + (w >> 13) * row_bytes, x);
+          }
         }
         for (int j = 0; j < nleaf; ++j) {
           const uint32_t w = leaf[-j];
-          T x[V];
-          if (w & (1u << 12)) load16(wb + ly.xrow + (w >> 13) * kRowBytes + lane * 16, x);
+          T x[W];
+          if (w & (1u << 12)) load_part<T, W>(mine + vrow + (w >> 13) * row_bytes, x);
           else constant(ly.cval + (w >> 13) * (uint32_t)K * (uint32_t)sizeof(T), x);
           put(w & 0xfffu, x);
         }
         for (int i = 0; i < nop; ++i) {
           const uint4 w = prog[i];
-          T a[V], c[V], r[V];
+          T a[W], c[W], r[W];
           fetch(w.z, a);
           fetch(w.w, c);
-          op_value_v<T, V>((int)(w.x & 0xffu), a, c, r);
-          store16(wb + w.y + lane * 16, r);
+          op_value_v<T, W>((int)(w.x & 0xffu), a, c, r);
+          store_part<T, W>(mine + w.y, r);
           put(w.x >> 8, r);
         }
       }
-    } else {
-      // general path (shared subtrees, more rows than the table holds, variables beyond the
-      // rows): one row of 32 values per node, one value per lane
-      for (int64_t base = e0; base < e1; base += 32) {
-        const int64_t p = base + lane;
-        const bool valid = p < e1;
-        const int64_t q = valid ? p : e1 - 1;
-        const int64_t n = kMulti ? q / K : q;
-        const uint32_t kko = kMulti ? (uint32_t)(q - n * K) * (uint32_t)sizeof(T) : 0u;
-        auto fetch = [&](uint32_t w) {
-          return (w & kConstOperand) ? *reinterpret_cast<const T*>(wb + (w & ~kConstOperand) + kko)
-                                     : reinterpret_cast<const T*>(wb + w)[lane];
-        };
-        for (int j = 0; j < nleaf; ++j) {
-          const uint32_t w = leaf[-j], k = w & 0xfffu;
-          T x;
-          if (w & (1u << 12)) {
-            x = __ldg(X + n * n_x + (w >> 13));
-            reinterpret_cast<T*>(wb + ly.rows + k * row_bytes)[lane] = x;
-          } else {
-            x = *reinterpret_cast<const T*>(wb + ly.cval + (w >> 13) * (uint32_t)K * (uint32_t)sizeof(T) + kko);
-          }
-          if (valid) __stcs(out + (int64_t)k * rs + p * es, x);
-        }
-        for (int i = 0; i < nop; ++i) {
-          const uint4 w = prog[i];
-          const T r = op_value<T>((int)(w.x & 0xffu), fetch(w.z), fetch(w.w));
-          reinterpret_cast<T*>(wb + w.y)[lane] = r;
-          if (valid) __stcs(out + (int64_t)(w.x >> 8) * rs + p * es, r);
-        }
-      }
-    }
+    };
+    if (VV == V) passes(std::integral_constant<int, V>{});
+    else if (G > 1 && VV == G) passes(std::integral_constant<int, G>{});
+    else passes(std::integral_constant<int, 1>{});
     // rows after the last real node are filled with NaN by pad_fill_kernel
   }
 }

@@ -41,6 +41,31 @@ __device__ __forceinline__ void stream16(void* p, const double (&r)[2]) {
   __stcs(reinterpret_cast<double2*>(p), make_double2(r[0], r[1]));
 }
 
+// A lane's part of a row: VV values.
+template <typename T, int VV>
+__device__ __forceinline__ void load_part(const void* p, T (&r)[VV]) {
+  if constexpr (VV * sizeof(T) == 16) {
+    load16(p, r);
+  } else if constexpr (VV == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    r[0] = t.x; r[1] = t.y;
+  } else {
+    r[0] = *reinterpret_cast<const T*>(p);
+  }
+}
+template <typename T, int VV>
+__device__ __forceinline__ void store_part(void* p, const T (&r)[VV]) {
+  if constexpr (VV * sizeof(T) == 16) store16(p, r);
+  else if constexpr (VV == 2) *reinterpret_cast<float2*>(p) = make_float2(r[0], r[1]);
+  else *reinterpret_cast<T*>(p) = r[0];
+}
+template <typename T, int VV>
+__device__ __forceinline__ void stream_part(void* p, const T (&r)[VV]) {
+  if constexpr (VV * sizeof(T) == 16) stream16(p, r);
+  else if constexpr (VV == 2) __stcs(reinterpret_cast<float2*>(p), make_float2(r[0], r[1]));
+  else __stcs(reinterpret_cast<T*>(p), r[0]);
+}
+
 // How a unit takes the K constant sets of its tape: one set (K = 1), all of them as N K
 // consecutive values per node, or one set whose values lie K elements apart.
 enum SetMode : int { kSingle = 0, kFlat = 1, kStrided = 2 };

@@ -14,6 +14,8 @@
 #include <mutex>
 #include <type_traits>
 
+#include <cooperative_groups.h>
+
 #include "sr_eval.cuh"
 
 namespace sr {
@@ -192,45 +194,61 @@ __global__ void __launch_bounds__(32) pad_fill_kernel(const int32_t* __restrict_
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Work order: the tapes by falling meta[column], by one CTA (a histogram of the values, its
-// running sums, then a place for each tape).  The order decides only which warp takes which
-// tape, so tapes of one length come in any order.  What bounds it: two passes over meta by one
-// SM, so a thread reads kOrderLoads tapes at once and counts with plain
-// shared-memory atomics (16384 tapes: 13.5 us, all of one length 18; with the lanes of a warp
-// grouped by value first, 31); a library sort's five launches took the host longer than the
-// forward of a small batch.
-constexpr int kOrderLoads = 8;
+// Work order: the tapes by falling meta[column], by one cluster of CTAs (each counts the values of
+// its share of the tapes, all add up the counts through each other's shared memory, then each
+// places its share).  The order decides only which warp takes which tape, so tapes of one length
+// come in any order.  What bounds it: two passes over meta, so a thread reads kOrderLoads tapes at
+// once and counts with plain shared-memory atomics; with the lanes of a warp grouped by value
+// first one CTA took 31 us for 16384 tapes instead of 13.5.  A large batch is shared among
+// kOrderCtas CTAs (with the call, 1000000 tapes 637 to 97 us, 65536 61 to 27; 1000 24 with one CTA, 27
+// with eight); a
+// library sort's five launches took the host longer than the forward of a small batch.
+constexpr int kOrderLoads = 8, kOrderCtas = 8;
+constexpr int64_t kOrderOneCta = 8192;  // tapes that one CTA reads in one go
 
 __global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restrict__ meta, int64_t B, int column,
                                                           int add, int bins, int32_t* __restrict__ order) {
-  extern __shared__ int at[];  // per value: count, then the next place
+  namespace cg = cooperative_groups;
+  extern __shared__ int count[];  // per value: the count of this CTA's tapes
+  int* at = count + bins;         // the next place
   __shared__ int warp_sum_[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < bins; i += blockDim.x) at[i] = 0;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int ctas = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int64_t share = (B + ctas - 1) / ctas, from = share * rank, to = from + share < B ? from + share : B;
+  for (int i = tid; i < bins; i += blockDim.x) count[i] = 0;
   __syncthreads();
-  // f(b, key) for every tape, the lanes of a warp together; key 0 for the largest value, -1
-  // past the last tape
+  // f(b, key) for every tape of the share, the lanes of a warp together; key 0 for the largest
+  // value, -1 past the last tape
   auto each_tape = [&](auto f) {
-    for (int64_t b0 = 0; b0 < B; b0 += (int64_t)kOrderLoads * blockDim.x) {
+    for (int64_t b0 = from; b0 < to; b0 += (int64_t)kOrderLoads * blockDim.x) {
       int k[kOrderLoads];
 #pragma unroll
       for (int j = 0; j < kOrderLoads; ++j) {
         const int64_t b = b0 + j * (int)blockDim.x + tid;
-        k[j] = b < B ? bins - 1 - min(max(meta[b * 4 + column] + add, 0), bins - 1) : -1;
+        k[j] = b < to ? bins - 1 - min(max(meta[b * 4 + column] + add, 0), bins - 1) : -1;
       }
 #pragma unroll
       for (int j = 0; j < kOrderLoads; ++j)
-        if (b0 + j * (int)blockDim.x < B) f(b0 + j * (int)blockDim.x + tid, k[j]);
+        if (b0 + j * (int)blockDim.x < to) f(b0 + j * (int)blockDim.x + tid, k[j]);
     }
   };
   each_tape([&](int64_t, int k) {
-    if (k >= 0) atomicAdd(&at[k], 1);
+    if (k >= 0) atomicAdd(&count[k], 1);
   });
-  __syncthreads();
-  // exclusive running sums over the bins, a run of consecutive bins per thread
+  cluster.sync();
+  // exclusive running sums over the bins, a run of consecutive bins per thread; within a bin the
+  // shares in their order
   const int per = (bins + (int)blockDim.x - 1) / (int)blockDim.x, lo = min(bins, tid * per), hi = min(bins, lo + per);
   int sum = 0;
-  for (int i = lo; i < hi; ++i) sum += at[i];
+  for (int i = lo; i < hi; ++i) {
+    int before = 0;
+    for (int c = 0; c < ctas; ++c) {
+      if (c == rank) at[i] = before;
+      before += *cluster.map_shared_rank(count + i, c);
+    }
+    sum += before;
+  }
   int incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -242,11 +260,10 @@ __global__ void __launch_bounds__(1024) tape_order_kernel(const int32_t* __restr
   int before = incl - sum;
   for (int w = 0; w < warp; ++w) before += warp_sum_[w];
   for (int i = lo; i < hi; ++i) {
-    const int c = at[i];
-    at[i] = before;
-    before += c;
+    at[i] += before;
+    for (int c = 0; c < ctas; ++c) before += *cluster.map_shared_rank(count + i, c);
   }
-  __syncthreads();
+  cluster.sync();  // also: no CTA leaves while another reads its counts
   each_tape([&](int64_t b, int k) {
     if (k >= 0) order[atomicAdd(&at[k], 1)] = (int32_t)b;
   });
@@ -807,8 +824,19 @@ int sr_tape_order(const int32_t* meta, int64_t B, int64_t M, int32_t column, int
   if (B == 0) return SR_OK;
   if (!meta || !order) { set_error("null pointer argument"); return SR_ERR_INVALID_ARGUMENT; }
   const int bins = (int)M + 1;
-  tape_order_kernel<<<1, 1024, bins * sizeof(int), as_stream(stream)>>>(meta, B, column, column, bins, order);
-  return launch_check("tape_order_kernel");
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = B > kOrderOneCta ? kOrderCtas : 1;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(cluster.val.clusterDim.x);
+  config.blockDim = dim3(1024);
+  config.dynamicSmemBytes = 2 * bins * sizeof(int);
+  config.stream = as_stream(stream);
+  config.attrs = &cluster;
+  config.numAttrs = 1;
+  return cuda_check(cudaLaunchKernelEx(&config, tape_order_kernel, meta, B, (int)column, (int)column, bins, order),
+                    "tape_order_kernel");
 }
 
 int sr_any_nonzero(const int64_t* words, int64_t n, int32_t* out, void* stream) {

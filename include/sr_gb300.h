@@ -77,7 +77,8 @@ int sr_tape_compile(const int64_t *ops_dev, const int64_t *ch_dev, int64_t B, in
 
 /*
  * Work order for the kernels below: order_dev (B) int32 lists the tapes by falling
- * meta[column] (0: L_eff, 1: the root), tapes of one length in any order.  One launch.
+ * meta[column] (0: L_eff, 1: the root), tapes of one length in any order.  One launch (a
+ * cluster of eight CTAs for large batches).
  */
 int sr_tape_order(const int32_t *meta_dev, int64_t B, int64_t M, int32_t column, int32_t *order_dev, void *stream);
 

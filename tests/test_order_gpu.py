@@ -48,3 +48,8 @@ def test_compile_summary_is_the_maximum_over_tapes(B, M):
         ch[at] = -1
         c = tape.compile_tapes(torch.as_tensor(rows).cuda(), torch.as_tensor(ch).cuda(), 2)
         assert (c.max_len, c.max_root, c.max_consts) == want
+
+
+@pytest.mark.parametrize("B,M", [(8192, 64), (8193, 64), (65535, 1), (65536, 4095), (262145, 64), (1000003, 33)])
+def test_tape_order_over_the_shares_of_a_cluster(B, M):
+    test_tape_order_lists_every_tape_by_falling_length(B, M, 0)

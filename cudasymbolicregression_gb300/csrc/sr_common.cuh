@@ -29,16 +29,13 @@ int resident_ctas(const void* kern, int threads, size_t smem);
 int max_dyn_smem();  // dynamic shared memory that a block can have
 
 // Lets a kernel be launched with `bytes` of dynamic shared memory: a kernel that needs more than
-// it may take unasked is allowed all that a block can have beside its static arrays.  Never just
-// `bytes`: the limit belongs to the kernel, and a call that set it to its own size could lower it
-// under the launch of a larger call in another thread.
+// it may take unasked is allowed all that a block can have beside static arrays of up to 1 KB.
+// Never just `bytes`: the limit belongs to the kernel, and a call that set it to its own size
+// could lower it under the launch of a larger call in another thread.
 inline int allow_dynamic_smem(const void* kern, size_t bytes) {
   if (bytes <= 46 * 1024) return SR_OK;
-  cudaFuncAttributes a;
-  const int rc = cuda_check(cudaFuncGetAttributes(&a, kern), "kernel attributes");
-  if (rc) return rc;
-  return cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         max_dyn_smem() - (int)a.sharedSizeBytes), "shared memory attribute");
+  return cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dyn_smem() - 1024),
+                    "shared memory attribute");
 }
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }

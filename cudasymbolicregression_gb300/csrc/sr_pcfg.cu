@@ -194,6 +194,25 @@ __device__ __forceinline__ bool stage_grammar(const WideGrammar& W, int start, u
   return __syncthreads_and(ok);
 }
 
+// Whether every symbol id that a derivation can meet fits a byte; the same in every thread.
+__device__ __forceinline__ bool byte_symbols(const WideGrammar& W, int start) {
+  if (W.n_symbols > 256 || start > 255) return false;
+  const int rules = W.nt_ptr[W.n_symbols];
+  if (rules < 0) return false;
+  const int total = W.rhs_ptr[rules];
+  bool ok = total >= 0;
+  for (int s = threadIdx.x; s < W.n_symbols; s += blockDim.x) {
+    const int from = W.nt_ptr[s], to = W.nt_ptr[s + 1];
+    ok &= from >= 0 && from <= to && to <= rules;
+  }
+  for (int j = threadIdx.x; j < rules; j += blockDim.x) {
+    const int lo = W.rhs_ptr[j], hi = W.rhs_ptr[j + 1];
+    ok &= lo >= 0 && hi <= total;
+  }
+  for (int i = threadIdx.x; i < total; i += blockDim.x) ok &= (unsigned)W.rhs[i] < 256u;
+  return __syncthreads_and(ok);
+}
+
 // The CTA's warps derive the expressions [beg, beg + count).  Every lane works on one
 // expression; a turn of the loop emits at most one terminal and expands at most one
 // non-terminal of it, with the next symbol in a register and the next random number drawn
@@ -315,7 +334,9 @@ __device__ __forceinline__ void derive(const G& g, int start, int64_t beg, int64
 // (1051).  With the probabilities read one by one (indexes clamped to the symbol's last) the
 // first took 320 us; with two CTAs per SM, each with a longer queue, 425; with the streams of
 // 32 expressions seeded ahead by all lanes, 343.
-// Other grammars keep 16-bit symbols and their tables in global memory; `wide_threads`
+// Grammars with larger tables keep them in global memory, with symbols in a byte where all ids
+// fit (400 rules, 262144 expressions of up to 64 tokens: 308 us, with 16-bit symbols and half
+// the threads 401, with all 369).  Other ids keep 16 bits; `wide_threads`
 // threads of the CTA then work (all of them, or the half that shared memory sized for bytes
 // holds).
 __global__ void __launch_bounds__(kThreads) sample_infix_kernel(
@@ -334,11 +355,15 @@ __global__ void __launch_bounds__(kThreads) sample_infix_kernel(
   const WideGrammar W{nt_ptr, rhs_ptr, rhs, cum, n_symbols};
   SmallGrammar S;
   const bool small = stage_grammar(W, start, smem, S);
-  if (threadIdx.x == 0) queue = small ? kThreads : wide_threads;
+  const bool narrow = small || byte_symbols(W, start);
+  if (threadIdx.x == 0) queue = narrow ? kThreads : wide_threads;
   __syncthreads();
   if (small) {
     derive<uint8_t>(S, start, beg, count, &queue, max_len, max_tries, seed, smem + kTableBytes,
                     smem + kTableBytes + kThreads * odd_stride(kHardMax), out, errors);
+  } else if (narrow) {
+    derive<uint8_t>(W, start, beg, count, &queue, max_len, max_tries, seed, smem,
+                    smem + kThreads * odd_stride(kHardMax), out, errors);
   } else if ((int)threadIdx.x < wide_threads) {
     derive<int16_t>(W, start, beg, count, &queue, max_len, max_tries, seed, smem,
                     smem + wide_threads * odd_stride(kHardMax * (int)sizeof(int16_t)), out, errors);

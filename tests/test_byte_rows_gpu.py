@@ -184,3 +184,32 @@ def test_calls_of_several_threads_keep_their_shared_memory():
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("rules,symbols,top", [(209, 260, 255), (400, 500, 120), (3, 3000, 255), (209, 260, 256), (400, 600, 5000)])
+@pytest.mark.parametrize("B,length", [(1, 1), (65, 9), (3000, 64), (40000, 128)])
+def test_sampler_tables_larger_than_its_copy(rules, symbols, top, B, length):
+    """Grammars whose tables stay in global memory: more rules, or more symbols on their right-hand
+    sides, than the copy holds, with ids that fit a byte and ids that do not."""
+    from cudasymbolicregression_gb300 import _lib
+    rng = np.random.default_rng([rules, symbols, top])
+    per = symbols // rules
+    E = 1
+    rc, rp = [], [0]
+    for r in range(rules):
+        rc += [E if r % 5 == 0 and i % 2 == 0 and i < 3 else int(rng.integers(2, top + 1)) for i in range(max(1, per))]
+        rp.append(len(rc))
+    rc[-1] = top
+    n_symbols = min(256, top + 1)
+    nt = np.zeros(n_symbols + 1, np.int32)
+    nt[E + 1:] = rules
+    cum = ((np.arange(rules) + 1) / rules).astype(np.float32)
+    tables = [nt, cum, np.array(rp, np.int32), np.array(rc, np.int32)]
+    d = [torch.tensor(a).cuda() for a in tables]
+    out = torch.full((B, length), 77, dtype=torch.int64, device="cuda")
+    err = torch.full((B,), 77, dtype=torch.int64, device="cuda")
+    assert _lib.lib().sr_pcfg_sample_infix(*(_lib.ptr(a) for a in d), n_symbols, E, B, length, 5, 99, _lib.ptr(out),
+                                           _lib.ptr(err), _lib.stream_ptr(out.device)) == 0
+    want, want_err = oracle.pcfg_sample(tables, E, B, length, 5, 99)
+    np.testing.assert_array_equal(err.cpu().numpy(), want_err)
+    np.testing.assert_array_equal(out.cpu().numpy(), want)

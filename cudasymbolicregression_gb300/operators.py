@@ -133,6 +133,8 @@ _MESSAGES = {
     507: "Conversion failed: Malformed input (e.g., too many operands).",
     508: "Conversion failed: Resulting infix expression has multiple roots, which is not allowed.",
     509: "Conversion failed: Unexpected token encountered (e.g., an operator without operands).",
+    601: "A device kernel gave up waiting (its results are not complete).",
+    602: "A tape is longer than the tables the kernel was launched with.",
     1000: "An internal error occurred that does not fit into the above categories.",
 }
 

@@ -268,3 +268,12 @@ def test_optimize_argument_errors_in_reference_order():
         sr.optimize(X, Y, ops, ch[0], C)
     with pytest.raises(RuntimeError, match="expected scalar type Float but found Double"):
         sr.optimize(X, Y, ops, ch, C.double())
+
+
+def test_status_codes_of_the_library_have_a_message():
+    """The library's own status codes, which the reference does not have: a wait that ran out and a
+    tape longer than the launch's tables."""
+    from cudasymbolicregression_gb300 import _lib
+    from cudasymbolicregression_gb300.operators import error_message
+    assert error_message(_lib.MLP_TIMEOUT, "backward pass").startswith("Error during backward pass: A device kernel")
+    assert "longer than the tables" in error_message(_lib.TAPE_EXCEEDS_LAUNCH)

@@ -354,3 +354,47 @@ def test_warm_start_gains_on_the_readme_problem():
     print(f"mean closures plain {ep:.2f} warm {ew:.2f}; median MSE plain {mp:.5g} warm {mw:.5g}")
     assert ew < 0.95 * ep
     assert mw <= mp * 1.005 + 1e-9
+
+
+def test_adam_of_several_tensors_matches_oracle():
+    """sr_mlp_adam_all: every element goes to its own tensor, whose weight decay it takes, at
+    sizes around a block of 256, with an empty tensor between and up to 16 of them."""
+    from cudasymbolicregression_gb300 import _lib
+    L = _lib.lib()
+    rng = np.random.default_rng(21)
+    shapes = [(1, 1), (1, 255), (1, 257), (64, 96), (0, 5), (3, 256)] + [(2, 7 + i) for i in range(10)]
+    f = lambda s: torch.tensor(rng.standard_normal(s).astype(np.float32)).cuda()  # noqa: E731
+    w, g = [f(s) for s in shapes], [f(s) for s in shapes]
+    m, v = [[torch.zeros_like(t) for t in w] for _ in range(2)]
+    wb = [torch.zeros(s, dtype=torch.bfloat16, device="cuda") for s in shapes]
+    wbt = [torch.zeros(s[::-1], dtype=torch.bfloat16, device="cuda") for s in shapes]
+    decay = [0.01 * (i % 3) for i in range(len(shapes))]
+    ref = [[np32(t).astype(np.float64), np.zeros(s), np.zeros(s)] for t, s in zip(w, shapes)]
+    items = (_lib.MlpAdamTensor * 17)()
+    for i, s in enumerate(shapes):
+        copies = i % 4 != 1
+        items[i] = (w[i].data_ptr(), g[i].data_ptr(), m[i].data_ptr(), v[i].data_ptr(), *s,
+                    wb[i].data_ptr() if copies else None, wbt[i].data_ptr() if copies else None, decay[i])
+    for step in (1, 2, 3):
+        _lib.check(L.sr_mlp_adam_all(items, 16, 1e-2, 0.9, 0.999, 1e-8, step, None), "adam")
+        ref = [list(mo.adam(r[0], np32(g[i]).astype(np.float64), r[1], r[2], step, 1e-2, weight_decay=decay[i]))
+               for i, r in enumerate(ref)]
+    torch.cuda.synchronize()
+    for i in range(16):
+        np.testing.assert_allclose(np32(w[i]), ref[i][0], rtol=1e-5, atol=1e-6)
+        if i % 4 != 1:
+            np.testing.assert_array_equal(np32(wb[i]), mo.bf16(np32(w[i])))
+            np.testing.assert_array_equal(np32(wbt[i]), mo.bf16(np32(w[i])).T)
+    assert L.sr_mlp_adam_all(items, 17, 1e-2, 0.9, 0.999, 1e-8, 1, None) == -1
+
+
+@pytest.mark.parametrize("n,rows,ld", [(64, 128, 128), (256, 384, 512), (3, 5, 8)])
+def test_column_sums(n, rows, ld):
+    """sr_mlp_colsum: a warp's sums over the rows of each column, in float32."""
+    from cudasymbolicregression_gb300 import _lib
+    rng = np.random.default_rng([n, rows])
+    x = torch.tensor(rng.integers(-4, 5, (n, ld)).astype(np.float32)).to(torch.bfloat16).cuda()
+    out = torch.empty(n, device="cuda")
+    _lib.check(_lib.lib().sr_mlp_colsum(ctypes.c_void_p(x.data_ptr()), n, rows, ld, ctypes.c_void_p(out.data_ptr()), None),
+               "colsum")
+    np.testing.assert_array_equal(np32(out), np32(x)[:, :rows].sum(1))  # whole numbers: exact in any order

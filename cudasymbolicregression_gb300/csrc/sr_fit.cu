@@ -64,7 +64,6 @@ struct FitArgs {
   int Lmax, Kmax;
   int Imax;         // program entries: largest count of operator nodes
   int Amax;         // most operator-node adjoints live at once
-  int tight;        // see fit_layout
   int Rmax;         // rows of the per-warp table for operator values and adjoints (see stage_problem)
   int VR;           // rows of the per-warp table for variables (distinct variables of a tape)
   unsigned char* ws_hist;  // per CTA: the L-BFGS history block (hist_block_bytes), when not in shared memory
@@ -1351,7 +1350,8 @@ __device__ __forceinline__ bool variables_once(const FitArgs& A, const WarpSmem&
 // _alpha_zoom_corrected / _backtracking_line_search for one column.
 enum Phase : int { PH_INIT = 0, PH_BRACKET, PH_ZOOM_LO, PH_ZOOM, PH_BACKTRACK, PH_UPDATE, PH_DONE };
 
-template <int V, int U, int SPL>
+// kTight: see fit_layout (its own kernels: a flag in the way of the layout cost the fits 2%).
+template <int V, int U, int SPL, bool kTight>
 __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
   // L-BFGS constants in the iteration's arithmetic: eps as a float pair, the gradient
   // tolerance in float32 (the reference compares a float32 norm with it)
@@ -1359,7 +1359,7 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
   const float tolf = __double2float_rn(A.tol);
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, A.tight != 0);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, kTight);
   const WarpSmem S = carve(smem, l, warp);
   // the L-BFGS history of this CTA (used by warp 0)
   const History H = history_at<SPL>(
@@ -1746,12 +1746,12 @@ __global__ void __launch_bounds__(256, 2) fit_lbfgs_kernel(FitArgs A) {
 // loss_out[b, k] is the mean squared error from candidate k, as the fit's first
 // closure measures it (to the last bit but for the order of the lane sum).
 // Candidate k of problem b: C_sets + k c_sk + b c_sb, slot m at + m c_sm.
-template <int V, int U>
+template <int V, int U, bool kTight>
 __global__ void __launch_bounds__(256, 2) fit_screen_kernel(FitArgs A, const float* __restrict__ C_sets, int64_t c_sk,
                                                             int64_t K, float* __restrict__ loss_out) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, A.tight != 0);
+  const Layout l = fit_layout(A.Lmax, A.Imax, A.Rmax, A.Kmax, V, U, W, A.VR, kTight);
   const WarpSmem S = carve(smem, l, warp);
   for (int64_t b = blockIdx.x; b < A.B; b += gridDim.x) {
     const int L = A.meta[b * 4 + 1] + 1;
@@ -1971,25 +1971,39 @@ struct FitShape {
 
 
 template <int V, int U, int SPL>
-static void* fit_kernel_ptr() {
-  return reinterpret_cast<void*>(fit_lbfgs_kernel<V, U, SPL>);
+static void* fit_kernel_ptr(bool tight) {
+  if constexpr (U == 1) {  // a layout too large for its staging tables does not take two chunks either
+    if (tight) return reinterpret_cast<void*>(fit_lbfgs_kernel<V, U, SPL, true>);
+  }
+  return reinterpret_cast<void*>(fit_lbfgs_kernel<V, U, SPL, false>);
 }
 
-static void* pick_kernel(int V, int U, int SPL) {
+static void* pick_kernel(int V, int U, int SPL, bool tight) {
   switch (V * 100 + U * 10 + SPL) {
-    case 111: return fit_kernel_ptr<1, 1, 1>();
-    case 112: return fit_kernel_ptr<1, 1, 2>();
-    case 114: return fit_kernel_ptr<1, 1, 4>();
-    case 121: return fit_kernel_ptr<1, 2, 1>();
-    case 122: return fit_kernel_ptr<1, 2, 2>();
-    case 124: return fit_kernel_ptr<1, 2, 4>();
-    case 211: return fit_kernel_ptr<2, 1, 1>();
-    case 212: return fit_kernel_ptr<2, 1, 2>();
-    case 214: return fit_kernel_ptr<2, 1, 4>();
-    case 411: return fit_kernel_ptr<4, 1, 1>();
-    case 412: return fit_kernel_ptr<4, 1, 2>();
-    case 414: return fit_kernel_ptr<4, 1, 4>();
+    case 111: return fit_kernel_ptr<1, 1, 1>(tight);
+    case 112: return fit_kernel_ptr<1, 1, 2>(tight);
+    case 114: return fit_kernel_ptr<1, 1, 4>(tight);
+    case 121: return fit_kernel_ptr<1, 2, 1>(tight);
+    case 122: return fit_kernel_ptr<1, 2, 2>(tight);
+    case 124: return fit_kernel_ptr<1, 2, 4>(tight);
+    case 211: return fit_kernel_ptr<2, 1, 1>(tight);
+    case 212: return fit_kernel_ptr<2, 1, 2>(tight);
+    case 214: return fit_kernel_ptr<2, 1, 4>(tight);
+    case 411: return fit_kernel_ptr<4, 1, 1>(tight);
+    case 412: return fit_kernel_ptr<4, 1, 2>(tight);
+    case 414: return fit_kernel_ptr<4, 1, 4>(tight);
     default: return nullptr;
+  }
+}
+
+static void* screen_kernel(int V, bool tight) {
+  switch (V * 10 + (tight ? 1 : 0)) {
+    case 10: return reinterpret_cast<void*>(fit_screen_kernel<1, 1, false>);
+    case 11: return reinterpret_cast<void*>(fit_screen_kernel<1, 1, true>);
+    case 20: return reinterpret_cast<void*>(fit_screen_kernel<2, 1, false>);
+    case 21: return reinterpret_cast<void*>(fit_screen_kernel<2, 1, true>);
+    case 40: return reinterpret_cast<void*>(fit_screen_kernel<4, 1, false>);
+    default: return reinterpret_cast<void*>(fit_screen_kernel<4, 1, true>);
   }
 }
 
@@ -2039,7 +2053,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
   int bestPerSm = 0, onePerSm = 0;
   bool tight = false;
   auto resident = [&](int u, int w, size_t& bytes) -> int {  // CTAs per SM, 0 if they do not fit, < 0 for an error
-    void* k = pick_kernel(V, u, sh.SPL);
+    void* k = pick_kernel(V, u, sh.SPL, tight);
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess) return -1;
     bytes = fit_layout(Lmax, Imax, sh.Rmax, Kmax, V, u, w, sh.VR, tight).bytes;
     return bytes > (size_t)optin ? 0 : resident_ctas(k, w * 32, bytes);
@@ -2059,7 +2073,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
       sh.tight = tight;
       bestPerSm = onePerSm = one;
       sh.smem = bytes;
-      if (V == 1 && N > (int64_t)32 * w) {
+      if (V == 1 && !tight && N > (int64_t)32 * w) {
         const int two = resident(2, w, bytes);
         if (two > 0 && 2 * two >= one) {
           sh.U = 2;
@@ -2081,7 +2095,7 @@ static int fit_shape(int64_t B, int64_t N, int64_t n_x, int Lmax, int Kmax, cons
   sh.ring_off = 0;
   {
     const size_t off = fit_align16(sh.smem), with = off + hist_block_bytes(o.history_size, sh.SPL);
-    if (with <= (size_t)optin && resident_ctas(pick_kernel(V, sh.U, sh.SPL), W * 32, with) >= bestPerSm) {
+    if (with <= (size_t)optin && resident_ctas(pick_kernel(V, sh.U, sh.SPL, sh.tight), W * 32, with) >= bestPerSm) {
       sh.ring_off = off;
       sh.smem = with;
     }
@@ -2194,13 +2208,11 @@ int sr_fit_screen(const float* X, int64_t N, int64_t n_x, const float* Y, const 
   A.desc = desc; A.meta = meta; A.B = B; A.M = M;
   A.c_sb = c_sb; A.c_sm = c_sm;
   A.objective = o.objective;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR; A.tight = sh.tight;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
   A.status = status;
   // a forward pass alone gains less from two chunks at once than it loses with the CTAs that
   // the doubled rows displace (2048 problems of two starts, N = 512: 280 us against 237)
-  void* k = sh.V == 1 ? reinterpret_cast<void*>(fit_screen_kernel<1, 1>)
-                      : (sh.V == 2 ? reinterpret_cast<void*>(fit_screen_kernel<2, 1>)
-                                   : reinterpret_cast<void*>(fit_screen_kernel<4, 1>));
+  void* k = screen_kernel(sh.V, sh.tight);
   const size_t smem = fit_layout(Lmax, sh.Imax, sh.Rmax, max_consts, sh.V, 1, sh.warps, sh.VR, sh.tight).bytes;
   int dev = 0, optin = 0;
   if (cuda_check(cudaGetDevice(&dev), "cudaGetDevice") ||
@@ -2261,14 +2273,14 @@ int sr_fit_lbfgs(const float* X, int64_t N, int64_t n_x, const float* Y, const u
   A.order = order;
   A.max_iter = o.max_iter; A.hist = o.history_size; A.ls_kind = o.line_search; A.ls_max = o.line_search_max_iter;
   A.objective = o.objective; A.tol = o.tolerance_grad; A.eps = o.eps;
-  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR; A.tight = sh.tight;
+  A.Lmax = Lmax; A.Kmax = max_consts; A.Imax = sh.Imax; A.Amax = sh.Amax; A.Rmax = sh.Rmax; A.VR = sh.VR;
   A.counter = reinterpret_cast<int*>(ws);
   A.ws_hist = sh.ring_off ? nullptr : ws + 256;
   A.ring_off = (int)sh.ring_off;
   A.status = status;
   rc = cuda_check(cudaMemsetAsync(ws, 0, 256, st), "work counter reset");
   if (rc) return rc;
-  void* k = pick_kernel(sh.V, sh.U, sh.SPL);
+  void* k = pick_kernel(sh.V, sh.U, sh.SPL, sh.tight);
   void* args[] = {&A};
   rc = cuda_check(cudaLaunchKernel(k, dim3(sh.blocks), dim3(sh.warps * 32), args, sh.smem, st), "fit_lbfgs_kernel");
   return rc;

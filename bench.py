@@ -105,11 +105,9 @@ FIT_TRAFFIC_BYTES = {("ragged", 16384, 512): 4 * (10265344 + 1536),
 FIT_PROFILE = {"commit": "66b7445", "issue_active_pct": 54.8, "fp32_pipe_pct": 15.8, "xu_pipe_pct": 2.5,
                "alu_pipe_pct": 51.3, "lsu_pipe_pct": 13.9, "fp64_pipe_pct": 2.4, "warps_active_pct": 23.2,
                "capture": "ncu --set full, ragged B=4096, N=512"}
-# The adjoint call: its length-class grids (which read the cached value rows of the real
-# nodes beside the grad_out rows) and the concurrent padding check, captured with an earlier
-# kernel that staged the same rows in shared memory.
-EVAL_TRAFFIC_BYTES = {("eval_forward_kernel", 65536, 1024): 16 * (1611520 + 1012199000),
-                      ("eval_adjoint_kernel", 65536, 1024): 16 * (1364424192 + 13661696)}
+# DRAM bytes of the evaluation calls are not stated: the captures of their kernels
+# (profiles/eval_forward_B4096_N1024.txt, profiles/eval_backward_B4096_N1024.txt) hold none for the current ones.
+EVAL_TRAFFIC_BYTES = {}
 
 
 def peaks():
@@ -733,7 +731,11 @@ def run_eval(args, rank, world, local):
                    "sr_eval_backward_f32")
 
     ktimes = {}
-    for name, fn in (("eval_forward_kernel", fwd_k), ("eval_adjoint_kernel", bwd_k)):
+    # the adjoint of a batch this large goes to its staged kernel (launch_backward in csrc/sr_adjoint.cu)
+    sms = torch.cuda.get_device_properties(Xd.device).multi_processor_count
+    staged = B >= 192 * sms
+    adjoint = "eval_adjoint_staged_kernel" if staged else "eval_adjoint_kernel"
+    for name, fn in (("eval_forward_kernel", fwd_k), (adjoint, bwd_k)):
         for _ in range(3):
             fn()
         ts = []
@@ -788,7 +790,7 @@ def run_eval(args, rank, world, local):
         pk, pk_kind = peaks()
         hbm = float(pk["hbm_gbs"])
         dom = max(ktimes, key=ktimes.get)
-        dom_bytes = bwd_bytes if dom == "eval_adjoint_kernel" else fwd_bytes
+        dom_bytes = bwd_bytes if dom == adjoint else fwd_bytes
         ach = dom_bytes / ktimes[dom] / 1e9
         line = {"metric": EVAL_METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": t_step * 1000.0, "higher_is_better": True, "scaling": "weak",
@@ -799,12 +801,14 @@ def run_eval(args, rank, world, local):
                 "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                              "traffic": EVAL_TRAFFIC_BYTES.get((dom, B, N)), "kernel": dom, "peak_kind": pk_kind},
                 "kernels": {k: {"ms": v * 1000.0,
-                                "GB/s": (bwd_bytes if k == "eval_adjoint_kernel" else fwd_bytes) / v / 1e9}
+                                "GB/s": (bwd_bytes if k == adjoint else fwd_bytes) / v / 1e9}
                             for k, v in ktimes.items()},
                 "expressions_per_s": B * world / t_step,
                 # per step: tape compile, work order, padding fill, padding check, and one forward
-                # and one adjoint grid per length class the batch reaches (three at these lengths)
-                "gpu_launches": (4 + 2 * (1 + (tapes.max_len > 16) + (tapes.max_len > 32))) * args.steps,
+                # and one adjoint grid per length class the batch reaches (three at these lengths;
+                # the staged adjoint has a fourth above 48 nodes)
+                "gpu_launches": (4 + 2 * (1 + (tapes.max_len > 16) + (tapes.max_len > 32))
+                                 + (staged and tapes.max_len > 48)) * args.steps,
                 "clocks": clk.summary()}
         if e2e:
             line["e2e"] = e2e

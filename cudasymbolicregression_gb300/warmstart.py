@@ -321,6 +321,13 @@ def candidate_starts(X, Y, ops, C_plain, net: WarmStartMLP | None = None, extra:
     return torch.stack(cands)
 
 
+def _followed(t: torch.Tensor) -> bool:
+    """Whether autograd follows t, backwards or forwards (a tangent)."""
+    if t.requires_grad and torch.is_grad_enabled():
+        return True
+    return torch.autograd.forward_ad.unpack_dual(t).tangent is not None
+
+
 def screened_start(X, Y, ops, ch, C_sets: torch.Tensor) -> torch.Tensor:
     """Per problem, the candidate start (C_sets (K, B, M)) with the lowest initial loss,
     all candidates measured in one launch of the screening kernel; a non-finite loss
@@ -328,7 +335,7 @@ def screened_start(X, Y, ops, ch, C_sets: torch.Tensor) -> torch.Tensor:
     from .optimization import screen_starts
     loss = screen_starts(X, Y, ops, ch, C_sets)
     K, B, M = C_sets.shape
-    if C_sets.requires_grad and torch.is_grad_enabled():  # a start that autograd can follow
+    if _followed(C_sets):  # a start that autograd can follow
         loss = torch.where(torch.isfinite(loss), loss, torch.full_like(loss, float("inf")))
         return C_sets[torch.argmin(loss, dim=1), torch.arange(B, device=ops.device)]
     Cs = C_sets.contiguous()
@@ -353,7 +360,7 @@ def warm_start_constants(net: WarmStartMLP, X, Y, ops, C_plain, clip: float = 10
         raise RuntimeError(f"C_plain must be float32 and shaped like ops {tuple(ops.shape)}, got {C_plain.dtype} "
                            f"{tuple(C_plain.shape)}")
     pred = net.predict(ops, X, Y)
-    if C_plain.requires_grad and torch.is_grad_enabled():  # a start that autograd can follow
+    if _followed(C_plain):  # a start that autograd can follow
         sel, r, k = _first_slots(ops)
         C = C_plain.clone()
         C[sel] = pred.clamp(-clip, clip)[r, k]

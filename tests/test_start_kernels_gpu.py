@@ -34,3 +34,32 @@ def test_place_and_pick(B, M):
         out = torch.empty((B, M), device="cuda")
         _lib.check(L.sr_mlp_pick_start(_lib.ptr(loss), _lib.ptr(sets), K, B, M, _lib.ptr(out), st), "pick")
         assert torch.equal(out, sets[best, torch.arange(B, device="cuda")])
+
+
+def test_starts_carry_a_tangent():
+    """Forward-mode differentiation goes through the chosen start: the tangent of the chosen
+    candidate, zero where a prediction took the constant's place."""
+    import torch.autograd.forward_ad as fw
+
+    from cudasymbolicregression_gb300 import tapes, warmstart
+    rng = np.random.default_rng(3)
+    B, M, N = 40, 24, 60
+    tb = tapes.generate(B, M, seed=3, mean_length=10, n_vars=2, unary=(10, 11), binary=(40, 41, 42), p_const_leaf=0.5)
+    ops, ch = torch.as_tensor(tb.ops).cuda(), torch.as_tensor(tb.ch).cuda()
+    X = torch.as_tensor(rng.uniform(-1, 1, (N, 2)).astype(np.float32)).cuda()
+    Y = torch.as_tensor(rng.uniform(-1, 1, (B, N)).astype(np.float32)).cuda()
+    C = torch.as_tensor(rng.standard_normal((B, M)).astype(np.float32)).cuda()
+    net = warmstart.WarmStartMLP(seed=1)
+    plain = warmstart.warm_start_constants(net, X, Y, ops, C)
+    with fw.dual_level():
+        t = torch.as_tensor(rng.standard_normal((B, M)).astype(np.float32)).cuda()
+        out = fw.unpack_dual(warmstart.warm_start_constants(net, X, Y, ops, fw.make_dual(C, t)))
+        rank = torch.cumsum((ops == 1).int(), 1) - 1
+        assert torch.equal(out.primal, plain)
+        assert torch.equal(out.tangent, torch.where((ops == 1) & (rank < 8), torch.zeros_like(t), t))
+        sets, ts = torch.stack([C, plain]), torch.stack([t, -t])
+        out = fw.unpack_dual(warmstart.screened_start(X, Y, ops, ch, fw.make_dual(sets, ts)))
+        chosen = warmstart.screened_start(X, Y, ops, ch, sets)
+        assert torch.equal(out.primal, chosen)
+        first = (chosen == C).all(1, keepdim=True)
+        assert torch.equal(out.tangent, torch.where(first, t, -t))
